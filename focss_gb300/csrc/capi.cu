@@ -67,30 +67,29 @@ focss_status get_plan_split(Ctx* ctx, int N, int log2N1, const Plan** out) {
     p.log2N2 = lg - log2N1;
     p.N1 = 1 << p.log2N1;
     p.N2 = 1 << p.log2N2;
-    // Twiddle tables from FP64 as double-float pairs {re_hi, im_hi, re_lo, im_lo}
-    // (layout documented in internal.h).
-    std::vector<float4> h(2 * (size_t)p.N1 + 2 * (size_t)p.N2 + 512);
+    // Twiddle tables from FP64 (layout documented in internal.h).
+    std::vector<char> h(table_bytes(p.N1, p.N2));
+    const Tables t = tables_at(h.data(), p.N1);
     const double two_pi = 2.0 * 3.14159265358979323846;
-    auto df = [](double re, double im) {
-        const float rh = (float)re, ih = (float)im;
-        return make_float4(rh, ih, (float)(re - (double)rh), (float)(im - (double)ih));
-    };
-    // cos/sin of 2 pi e / L evaluated on an exactly reduced argument (e mod L).
-    auto w = [&](long long e, long long L) { return df(std::cos(two_pi * e / L), -std::sin(two_pi * e / L)); };
     // Threads per group of a length-L sub-FFT (must match PQ<L>::P in fft.cuh).
     auto groupP = [](int L) { return L <= 32 ? 4 : L <= 128 ? 8 : L <= 512 ? 16 : 32; };
-    auto fill_pq = [&](float4* dst, int L, int P) {
+    auto fill_pq = [&](float2* dst, int L, int P) {
         const int Q = L / P;
         for (int u = 0; u < Q; ++u)
-            for (int t = 0; t < P; ++t) dst[u * P + t] = w((long long)t * u % L, L);
+            for (int i = 0; i < P; ++i) {
+                const double th = -two_pi * (double)((i < P / 2 ? i : i - P) * (u < Q / 2 ? u : u - Q)) / L;
+                dst[u * P + i] = make_float2((float)std::tan(0.5 * th), (float)std::sin(th));
+            }
     };
-    fill_pq(h.data(), p.N1, col_group_p(p.N1));
-    fill_pq(h.data() + p.N1, p.N2, groupP(p.N2));
-    for (int j = 0; j < 512; ++j)
-        h[2 * p.N1 + 2 * p.N2 + j] = df(std::cos(two_pi * j / 512), std::sin(two_pi * j / 512));
-    cudaError_t e = cudaMalloc(&p.tw, sizeof(float4) * h.size());
+    fill_pq((float2*)t.col, p.N1, col_group_p(p.N1));
+    fill_pq((float2*)t.row, p.N2, groupP(p.N2));
+    for (int j = 0; j < 512; ++j) {
+        const float2 c = split_df(std::cos(two_pi * j / 512)), s = split_df(std::sin(two_pi * j / 512));
+        ((float4*)t.turn)[j] = make_float4(c.x, s.x, c.y, s.y);
+    }
+    cudaError_t e = cudaMalloc(&p.tw, h.size());
     if (e != cudaSuccess) return cuda_check(ctx, e, "twiddle alloc");
-    e = cudaMemcpy(p.tw, h.data(), sizeof(float4) * h.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(p.tw, h.data(), h.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(p.tw);
         return cuda_check(ctx, e, "twiddle upload");

@@ -53,23 +53,25 @@ __device__ __forceinline__ float2 phase_rotation(float phi) {
 // 1): a gain that repeats at every split step and grows the field error
 // quadratically along a link.  The increment form leaves one unbiased rounding
 // (the final additions).
-__device__ __forceinline__ float2 kerr_rotate(float2 v, float phi) {
-    float cm1, s;
-    if (fabsf(phi) <= 0.25f) {
-        // The increment multiplies v, so sin and cos - 1 need FP32 accuracy
-        // relative to themselves: Taylor to phi^5 and phi^6 (truncation below
-        // 5e-8 and 1.3e-8 relative at |phi| = 1/4).
-        const float p2 = phi * phi;
-        s = phi * fmaf(p2, fmaf(p2, 1.0f / 120.0f, -1.0f / 6.0f), 1.0f);
-        cm1 = p2 * fmaf(p2, fmaf(p2, -1.0f / 720.0f, 1.0f / 24.0f), -0.5f);
-    } else {
-        const float2 r = phase_rotation(phi);  // cos(phi) <= 0.97: cos - 1 is exact
-        cm1 = r.x - 1.0f;
-        s = r.y;
-    }
+__device__ __forceinline__ float2 kerr_increment(float2 v, float cm1, float s) {
     const float dx = fmaf(v.x, cm1, -v.y * s);
     const float dy = fmaf(v.y, cm1, v.x * s);
     return make_float2(v.x + dx, v.y + dy);
+}
+// |phi| <= kKerrSmall: the increment multiplies v, so sin and cos - 1 need
+// FP32 accuracy relative to themselves: Taylor to phi^5 and phi^6 (truncation
+// below 5e-8 and 1.3e-8 relative at |phi| = 1/4).
+constexpr float kKerrSmall = 0.25f;
+__device__ __forceinline__ float2 kerr_rotate_small(float2 v, float phi) {
+    const float p2 = phi * phi;
+    const float s = phi * fmaf(p2, fmaf(p2, 1.0f / 120.0f, -1.0f / 6.0f), 1.0f);
+    const float cm1 = p2 * fmaf(p2, fmaf(p2, -1.0f / 720.0f, 1.0f / 24.0f), -0.5f);
+    return kerr_increment(v, cm1, s);
+}
+__device__ __forceinline__ float2 kerr_rotate(float2 v, float phi) {
+    if (fabsf(phi) <= kKerrSmall) return kerr_rotate_small(v, phi);
+    const float2 r = phase_rotation(phi);  // cos(phi) <= 0.97: cos - 1 is exact
+    return kerr_increment(v, r.x - 1.0f, r.y);
 }
 
 // Block-wide reductions (blockDim.x multiple of 32, <= 1024).

@@ -81,37 +81,56 @@ cudaError_t launch_power(const float2* d, int modes, int samples, int batch, dou
     return cudaGetLastError();
 }
 
-// Transposed spectrum layout (k1*N2 + k2 holds bin k1 + N1*k2) <-> natural.
-// Tiled 32x32 transpose through shared memory; batch on grid.z.
-__global__ void transpose_kernel(const float2* __restrict__ src, float2* __restrict__ dst, int rows, int cols) {
+// Two-pass spectrum layout (row k1, column k2 holds bin k1' + N1 k2 mod N,
+// k1' = k1 or, from kc on, k1 - N1; see col_work) <-> natural order.  Tiled
+// 32x32 transpose through shared memory; batch on grid.z.  In the N2 x N1
+// matrix of natural order (row k / N1) the columns k1 >= kc sit one row up.
+__global__ void transpose_to_natural_kernel(const float2* __restrict__ src, float2* __restrict__ dst, int N1, int N2,
+                                            int kc) {
     __shared__ float2 tile[32][33];
-    const size_t off = (size_t)blockIdx.z * rows * cols;
-    const int x = blockIdx.x * 32 + threadIdx.x;
+    const size_t off = (size_t)blockIdx.z * N1 * N2;
+    const int x = blockIdx.x * 32 + threadIdx.x;  // k2
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int y = blockIdx.y * 32 + k;
-        if (x < cols && y < rows) tile[k][threadIdx.x] = src[off + (size_t)y * cols + x];
+        const int y = blockIdx.y * 32 + k;        // k1
+        if (x < N2 && y < N1) tile[k][threadIdx.x] = src[off + (size_t)y * N2 + x];
     }
     __syncthreads();
-    const int x2 = blockIdx.y * 32 + threadIdx.x;
+    const int k1 = blockIdx.y * 32 + threadIdx.x;
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int y2 = blockIdx.x * 32 + k;
-        if (x2 < rows && y2 < cols) dst[off + (size_t)y2 * rows + x2] = tile[threadIdx.x][k];
+        const int k2 = blockIdx.x * 32 + k;
+        if (k1 < N1 && k2 < N2) dst[off + (size_t)((k2 - (k1 >= kc)) & (N2 - 1)) * N1 + k1] = tile[threadIdx.x][k];
     }
 }
 
-cudaError_t launch_transpose_to_natural(const float2* src, float2* dst, int N1, int N2, int batch,
+__global__ void transpose_from_natural_kernel(const float2* __restrict__ src, float2* __restrict__ dst, int N1, int N2,
+                                              int kc) {
+    __shared__ float2 tile[32][33];
+    const size_t off = (size_t)blockIdx.z * N1 * N2;
+    const int k1 = blockIdx.x * 32 + threadIdx.x;
+    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+        const int k2 = blockIdx.y * 32 + k;
+        if (k1 < N1 && k2 < N2) tile[k][threadIdx.x] = src[off + (size_t)((k2 - (k1 >= kc)) & (N2 - 1)) * N1 + k1];
+    }
+    __syncthreads();
+    const int x = blockIdx.y * 32 + threadIdx.x;  // k2
+    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+        const int y = blockIdx.x * 32 + k;        // k1
+        if (x < N2 && y < N1) dst[off + (size_t)y * N2 + x] = tile[threadIdx.x][k];
+    }
+}
+
+cudaError_t launch_transpose_to_natural(const float2* src, float2* dst, int N1, int N2, int kc, int batch,
                                         cudaStream_t st) {
-    // src is N1 rows x N2 cols; natural index k1 + N1*k2 = dst row k2, col k1.
     dim3 grid((N2 + 31) / 32, (N1 + 31) / 32, batch);
-    transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(src, dst, N1, N2);
+    transpose_to_natural_kernel<<<grid, dim3(32, 8), 0, st>>>(src, dst, N1, N2, kc);
     count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_transpose_from_natural(const float2* src, float2* dst, int N1, int N2, int batch,
+cudaError_t launch_transpose_from_natural(const float2* src, float2* dst, int N1, int N2, int kc, int batch,
                                           cudaStream_t st) {
     dim3 grid((N1 + 31) / 32, (N2 + 31) / 32, batch);
-    transpose_kernel<<<grid, dim3(32, 8), 0, st>>>(src, dst, N2, N1);
+    transpose_from_natural_kernel<<<grid, dim3(32, 8), 0, st>>>(src, dst, N1, N2, kc);
     count_launch();
     return cudaGetLastError();
 }

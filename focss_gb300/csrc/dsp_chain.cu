@@ -17,7 +17,7 @@
 #include <string>
 #include <vector>
 
-#include "common.cuh"
+#include "fft.cuh"
 #include "internal.h"
 
 namespace fg {
@@ -185,20 +185,21 @@ __global__ void scale_taps_kernel(double* __restrict__ taps, int len, const doub
     }
 }
 
-// Decimation gather: out (M samples, transposed layout M1 x M2) takes bin
-// k_out of the N-point spectrum `in` (transposed layout N1 x N2), with the
-// reference's bin map (field.cpp:309-317).
+// Decimation gather: out (M samples, two-pass layout M1 x M2) takes bin
+// k_out of the N-point spectrum `in` (two-pass layout N1 x N2; rows from kc on
+// hold the bins k1 - N1 + N1 k2), with the reference's bin map (field.cpp:309-317).
 __global__ void decimate_gather_kernel(const float2* __restrict__ in, float2* __restrict__ out, int N, int N1,
-                                       int N2, int M, int M1, int M2, int rows) {
+                                       int N2, int kc_in, int M, int M1, int M2, int kc_out, int rows) {
     const int cutoff = M / 2, shift = N - M;
     const size_t total = (size_t)rows * M;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t r = i / M;
         const int p = (int)(i % M);
         const int k1 = p / M2, k2 = p % M2;
-        const int kout = k1 + M1 * k2;
+        const int kout = ((k1 < kc_out ? k1 : k1 - M1) + M1 * k2) & (M - 1);
         const int kin = kout < cutoff ? kout : kout + shift;
-        out[i] = in[r * N + (size_t)(kin % N1) * N2 + kin / N1];
+        const int r1 = kin % N1;
+        out[i] = in[r * N + (size_t)r1 * N2 + ((kin / N1 + (r1 >= kc_in)) & (N2 - 1))];
     }
 }
 
@@ -674,7 +675,7 @@ FOCSS_API focss_status focss_decimate(focss_ctx* c, const focss_field* in, int f
     st = fg::fft_forward_transposed(c, sp, in->samples, rows, 1.0f / (float)in->samples);
     if (st != FOCSS_OK) return st;
     FG_LAUNCH(fg::decimate_gather_kernel<<<fg::grid_for(out->n(), 256), 256, 0, c->stream>>>(
-        sp, out->d, pi->N, pi->N1, pi->N2, po->N, po->N1, po->N2, rows));
+        sp, out->d, pi->N, pi->N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1, po->N2, fg::col_kc(po->N1), rows));
     e = cudaGetLastError();
     if (e != cudaSuccess) return fg::cuda_check(c, e, "decimate gather");
     return fg::fft_inverse_transposed(c, out->d, out->samples, rows);

@@ -1,64 +1,35 @@
 // fft.cuh -- FFT building blocks for the SSFM kernels.
 //
-// Layout convention used throughout: a length-L sub-FFT (L = P*Q, Q a multiple
-// of P) is computed by a group of P threads; thread t holds the Q elements
-// x[t + P*j], j = 0..Q-1, in registers.  fft_pq() returns the transform in the
-// same layout (v[j] = X[t + P*j]), so a forward transform, a pointwise
-// operator and an inverse transform chain without any extra data movement.
-// One exchange through shared memory per transform:
+// A length-L sub-FFT (L = P*Q) is computed by a group of P threads of Q
+// elements each, with one exchange through shared memory per transform:
 //   1. Q-point DFT in registers over j          (radix-2 DIF, constant twiddles)
-//   2. twiddle W_L^{t*u}                        (table in shared memory)
-//   3. write (u, t), read (u = t + P*i, s)      (caller-chosen conflict-free layout)
-//   4. P-point DFT in registers over s.
+//   2. twiddle W_L^{t' u'}                      (table in shared memory)
+//   3. write (u, t), read row u of P elements   (caller-chosen conflict-free layout)
+//   4. P-point DFT in registers.
 // Sign convention: forward = exp(-2 pi i nk/L), unnormalized (FFTW_FORWARD).
+//
+// Centred indices.  Thread t stands for t' = t or, from P/2 on, t - P, and row
+// u of the exchange for u' = u or, from Q/2 on, u - Q: the twiddle angle
+// 2 pi t' u' / L is then at most pi/2, one lifting rotation (three FMAs, an
+// 8-byte table entry) without a quarter-turn placement.  The relabelling only
+// moves indices: thread t holds x[(t' + P j) mod L], j = 0..Q-1,
+// and the rows u' hold X[u' + Q s], which fft_pq puts back in order:
+//   Q = P:  register j holds X[(t' + P j) mod L] (the layout of the input),
+//   Q = 2P: register j holds X[t + P j].
+// The double-float twiddle product (16-byte entry, 8 FP32 instructions) that
+// this replaced cost ~10 of the row pass's 143 instructions per sample.
 //
 // Precision.  The split-step loop applies the same transforms thousands of
 // times, so a rounding error that depends only on a constant (a twiddle
 // factor) repeats identically every step and grows linearly with the step
 // count, while roundings that depend on the data decorrelate and grow like
-// sqrt(steps).  Every twiddle is therefore held as an unevaluated sum
-// hi + lo of two floats (about 48 significant bits) and applied with a
-// compensated product: the only roundings left are data-dependent.
+// sqrt(steps).  Every twiddle is therefore a lifting rotation that the inverse
+// transform undoes operation by operation (see lift_rot).
 #pragma once
 
 #include "common.cuh"
 
 namespace fg {
-
-// (hi, lo) with hi + lo = cos(pi*j/32) to ~2^-48, j = 0..16
-__host__ __device__ __forceinline__ constexpr float2 cos_pi32_df(int j) {
-    constexpr float2 t[17] = {
-        {1.0f, 0.0f},
-        {0.9951847195625305f, 7.109666189109021e-09f},
-        {0.9807852506637573f, 2.9739473106360492e-08f},
-        {0.9569403529167175f, -1.7184508038781132e-08f},
-        {0.9238795042037964f, 2.830748968563057e-08f},
-        {0.8819212913513184f, -2.7002963420841297e-08f},
-        {0.8314695954322815f, 1.687026340846387e-08f},
-        {0.7730104327201843f, 2.0642552556182636e-08f},
-        {0.7071067690849304f, 1.2101617485882343e-08f},
-        {0.6343932747840881f, 9.37955757507325e-09f},
-        {0.5555702447891235f, -1.1769521357507529e-08f},
-        {0.4713967442512512f, -7.425253745196869e-09f},
-        {0.3826834261417389f, 6.2233507236442165e-09f},
-        {0.290284663438797f, 1.3815665056426951e-08f},
-        {0.19509032368659973f, -1.670471427850373e-09f},
-        {0.0980171412229538f, -8.933931927579408e-10f},
-        {0.0f, 0.0f}};
-    return t[j];
-}
-
-// (cos, sin) of pi*idx/32 for idx in [0, 64) as double-float: {c_hi, c_lo, s_hi, s_lo}
-__host__ __device__ __forceinline__ constexpr float4 cs64_df(int idx) {
-    return idx <= 16   ? float4{cos_pi32_df(idx).x, cos_pi32_df(idx).y, cos_pi32_df(16 - idx).x,
-                              cos_pi32_df(16 - idx).y}
-           : idx <= 32 ? float4{-cos_pi32_df(32 - idx).x, -cos_pi32_df(32 - idx).y, cos_pi32_df(idx - 16).x,
-                                cos_pi32_df(idx - 16).y}
-           : idx <= 48 ? float4{-cos_pi32_df(idx - 32).x, -cos_pi32_df(idx - 32).y, -cos_pi32_df(48 - idx).x,
-                                -cos_pi32_df(48 - idx).y}
-                       : float4{cos_pi32_df(64 - idx).x, cos_pi32_df(64 - idx).y, -cos_pi32_df(idx - 48).x,
-                                -cos_pi32_df(idx - 48).y};
-}
 
 // a * (w_hi + w_lo) with w = {re_hi, im_hi, re_lo, im_lo}: compensated complex
 // product; the representation error of w drops out, data roundings remain.
@@ -67,26 +38,6 @@ __device__ __forceinline__ float2 cmul_df(float2 a, float4 w) {
     const float im = fmaf(a.x, w.y, fmaf(a.y, w.x, fmaf(a.x, w.w, a.y * w.z)));
     return make_float2(re, im);
 }
-// a * conj(w_hi + w_lo)
-__device__ __forceinline__ float2 cmulc_df(float2 a, float4 w) {
-    const float re = fmaf(a.x, w.x, fmaf(a.y, w.y, fmaf(a.x, w.z, a.y * w.w)));
-    const float im = fmaf(a.y, w.x, fmaf(-a.x, w.y, fmaf(a.y, w.z, -a.x * w.w)));
-    return make_float2(re, im);
-}
-
-// a * exp(-+ i*pi*idx/32): forward uses the minus sign.
-template <bool INV>
-__device__ __forceinline__ float2 twmul64(float2 a, int idx) {
-    idx &= 63;
-    if (idx == 0) return a;
-    if (idx == 32) return make_float2(-a.x, -a.y);
-    if (idx == 16) return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
-    if (idx == 48) return INV ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
-    const float4 w = cs64_df(idx);  // (c_hi, c_lo, s_hi, s_lo)
-    // forward multiplies by (c - i s), inverse by (c + i s)
-    return INV ? cmul_df(a, make_float4(w.x, w.z, w.y, w.w)) : cmul_df(a, make_float4(w.x, -w.z, w.y, -w.w));
-}
-
 __host__ __device__ __forceinline__ constexpr int bitrev(int i, int bits) {
     int r = 0;
     for (int b = 0; b < bits; ++b) r |= ((i >> b) & 1) << (bits - 1 - b);
@@ -94,33 +45,6 @@ __host__ __device__ __forceinline__ constexpr int bitrev(int i, int bits) {
 }
 
 __host__ __device__ __forceinline__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n >> 1); }
-
-// In-register DFT of size R (power of two <= 64), natural order in and out.
-template <int R, bool INV>
-__device__ __forceinline__ void dft(float2 (&v)[R]) {
-#pragma unroll
-    for (int half = R / 2; half >= 1; half >>= 1) {
-#pragma unroll
-        for (int base = 0; base < R; base += 2 * half) {
-#pragma unroll
-            for (int j = 0; j < half; ++j) {
-                const float2 a = v[base + j], b = v[base + j + half];
-                v[base + j] = cadd(a, b);
-                v[base + j + half] = twmul64<INV>(csub(a, b), j * (32 / half));
-            }
-        }
-    }
-    constexpr int bits = ilog2c(R);
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int r = bitrev(i, bits);
-        if (i < r) {
-            const float2 tmp = v[i];
-            v[i] = v[r];
-            v[r] = tmp;
-        }
-    }
-}
 
 // Thread-group shape for a sub-FFT of length L.
 template <int L>
@@ -147,11 +71,9 @@ struct ColLayout {
     __device__ __forceinline__ int operator()(int u, int s) const { return (u * P + s) * C + c; }
 };
 
-// XOR swizzle of a table index inside groups of 8 entries (16-byte entries:
-// 8 per 128-byte shared-memory wavefront), so strided reads spread over banks.
-__host__ __device__ __forceinline__ int swz8(int e) { return e ^ (((e >> 3) ^ (e >> 6)) & 7); }
-// The same for 8-byte entries (16 per wavefront).
-__host__ __device__ __forceinline__ int swz16(int e) { return e ^ ((e >> 4) & 15); }
+// Centred index of thread t of P.
+template <int P>
+__host__ __device__ __forceinline__ int centred(int t) { return t < P / 2 ? t : t - P; }
 
 // ---------------------------------------------------------------------------
 // Rotations by lifting (three shears, A. W. Paeth, "A fast algorithm for
@@ -177,16 +99,15 @@ __device__ __forceinline__ float2 lift_rot_inv(float2 v, float2 ts) {
     x = fmaf(ts.x, y, x);
     return make_float2(x, y);
 }
-// W_N^e = exp(-2 pi i e/N) = (-i)^q rot(theta), q = round(4e/N), |theta| <= pi/4,
-// for 0 <= e < N = 2^log2N: {tan(theta/2), sin(theta), q (int bits), 0}.  The
-// residual turn fraction is exact, so the pair is a deterministic function of
-// (e, N): a rotation applied in one launch is undone exactly in another.
-__device__ __forceinline__ float4 sixstep_factor(int e, int log2N) {
-    const int q = ((e << 2) + (1 << (log2N - 1))) >> log2N;
-    const float r = (float)(e - (q << (log2N - 2))) * __int_as_float((127 - log2N) << 23);
+// W_N^e = exp(-2 pi i e/N) as a lifting pair {tan(theta/2), sin(theta)} for
+// |e| <= ~N/4 (theta = -2 pi e/N, |theta| <= ~pi/2), N = 2^log2N.  e/N is exact,
+// so the pair is a deterministic function of (e, N): a rotation applied in one
+// launch is undone exactly in another.
+__device__ __forceinline__ float2 sixstep_factor(int e, int log2N) {
+    const float r = (float)e * __int_as_float((127 - log2N) << 23);
     float sp, cp;
     sincospif(r, &sp, &cp);  // sin, cos of pi*r;  theta = -2 pi r
-    return make_float4(-sp / cp, -2.0f * sp * cp, __int_as_float(q & 3), 0.0f);
+    return make_float2(-sp / cp, -2.0f * sp * cp);
 }
 
 // v * (-i)^q (exact).
@@ -195,40 +116,9 @@ __device__ __forceinline__ float2 quarter_turns(float2 v, int q) {
     return (q & 2) ? make_float2(-r.x, -r.y) : r;
 }
 
-// Group-wide sub-FFT (see file comment).  twPQ[u*P + t] = exp(-2 pi i t u / L)
-// as double-float {re_hi, im_hi, re_lo, im_lo}: the P threads of a group read
-// P consecutive entries (conflict-free).
-// BLOCK_SYNC selects __syncthreads (group spans warps) or __syncwarp.
-template <int P, int Q, bool INV, bool BLOCK_SYNC, class Lay>
-__device__ __forceinline__ void fft_pq(float2 (&v)[Q], float2* __restrict__ sm, const Lay lay, int t,
-                                       const float4* __restrict__ twPQ) {
-    static_assert(Q % P == 0, "Q must be a multiple of P");
-    constexpr int M = Q / P;
-    dft<Q, INV>(v);
-#pragma unroll
-    for (int u = 1; u < Q; ++u)
-        v[u] = INV ? cmulc_df(v[u], twPQ[u * P + t]) : cmul_df(v[u], twPQ[u * P + t]);
-#pragma unroll
-    for (int u = 0; u < Q; ++u) sm[lay(u, t)] = v[u];
-    if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
-#pragma unroll
-    for (int i = 0; i < M; ++i) {
-        float2 w[P];
-        const int u = t + P * i;
-#pragma unroll
-        for (int s = 0; s < P; ++s) w[s] = sm[lay(u, s)];
-        dft<P, INV>(w);
-#pragma unroll
-        for (int s = 0; s < P; ++s) v[i + M * s] = w[s];
-    }
-    if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
-}
-
 // ---------------------------------------------------------------------------
-// Mirrored sub-FFTs for the column pass: in-register DFT twiddles as lifting
-// rotations (quarter turns exact, residual |angle| <= pi/4 in three FMAs), and
-// an inverse that undoes the forward operation by operation in reverse order
-// (see lift_rot).  The inter-stage table twiddles stay double-float.
+// Mirrored sub-FFTs: twiddles as lifting rotations, and an inverse that undoes
+// the forward operation by operation in reverse order (see lift_rot).
 
 // {tan(theta/2), sin(theta)} for theta = -pi*r/32, r = 0..8 (forward sign).
 __host__ __device__ __forceinline__ constexpr float2 lift_pi32(int r) {
@@ -308,15 +198,18 @@ __device__ __forceinline__ void dft_lift_inv(float2 (&v)[R]) {
     }
 }
 
-// fft_pq with the mirrored pieces (same layouts; forward and L times inverse).
+// Forward sub-FFT on P threads (layouts in the file comment), and L times its
+// inverse.  twPQ[u*P + t] = lifting pair of W_L^{t' u'}: the P threads of a
+// group read P consecutive entries (conflict-free).
+// BLOCK_SYNC selects __syncthreads (group spans warps) or __syncwarp.
 template <int P, int Q, bool BLOCK_SYNC, class Lay>
 __device__ __forceinline__ void fft_pq_lift(float2 (&v)[Q], float2* __restrict__ sm, const Lay lay, int t,
-                                            const float4* __restrict__ twPQ) {
-    static_assert(Q % P == 0, "Q must be a multiple of P");
+                                            const float2* __restrict__ twPQ) {
+    static_assert(Q == P || Q == 2 * P, "one or two rows per thread");
     constexpr int M = Q / P;
     dft_lift<Q>(v);
 #pragma unroll
-    for (int u = 1; u < Q; ++u) v[u] = cmul_df(v[u], twPQ[u * P + t]);
+    for (int u = 1; u < Q; ++u) v[u] = lift_rot(v[u], twPQ[u * P + t]);
 #pragma unroll
     for (int u = 0; u < Q; ++u) sm[lay(u, t)] = v[u];
     if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
@@ -327,21 +220,22 @@ __device__ __forceinline__ void fft_pq_lift(float2 (&v)[Q], float2* __restrict__
 #pragma unroll
         for (int s = 0; s < P; ++s) w[s] = sm[lay(u, s)];
         dft_lift<P>(w);
+        // w[s] = X[u' + Q s]; rows from Q/2 on (i = 1 when Q = 2P) have u' = u - Q
 #pragma unroll
-        for (int s = 0; s < P; ++s) v[i + M * s] = w[s];
+        for (int s = 0; s < P; ++s) v[i + M * ((s - i) & (P - 1))] = w[s];
     }
     if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
 }
 template <int P, int Q, bool BLOCK_SYNC, class Lay>
 __device__ __forceinline__ void fft_pq_lift_inv(float2 (&v)[Q], float2* __restrict__ sm, const Lay lay, int t,
-                                                const float4* __restrict__ twPQ) {
-    static_assert(Q % P == 0, "Q must be a multiple of P");
+                                                const float2* __restrict__ twPQ) {
+    static_assert(Q == P || Q == 2 * P, "one or two rows per thread");
     constexpr int M = Q / P;
 #pragma unroll
     for (int i = 0; i < M; ++i) {
         float2 w[P];
 #pragma unroll
-        for (int s = 0; s < P; ++s) w[s] = v[i + M * s];
+        for (int s = 0; s < P; ++s) w[s] = v[i + M * ((s - i) & (P - 1))];
         dft_lift_inv<P>(w);
         const int u = t + P * i;
 #pragma unroll
@@ -352,26 +246,26 @@ __device__ __forceinline__ void fft_pq_lift_inv(float2 (&v)[Q], float2* __restri
     for (int u = 0; u < Q; ++u) v[u] = sm[lay(u, t)];
     if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
 #pragma unroll
-    for (int u = 1; u < Q; ++u) v[u] = cmulc_df(v[u], twPQ[u * P + t]);
+    for (int u = 1; u < Q; ++u) v[u] = lift_rot_inv(v[u], twPQ[u * P + t]);
     dft_lift_inv<Q>(v);
 }
 
 // ---------------------------------------------------------------------------
 // Column sub-FFT with half the registers: L = 2 Q^2 on P = 2Q threads of Q
-// elements (L = 32, 128, 512).  Thread t holds x[t + P j]; after an in-register
-// Q-point DFT over j, the twiddle W_L^{t u} and one exchange, lane pair
-// (u = t >> 1, h = t & 1) holds the even (h = 0) or odd (h = 1) half of the
-// P-point DFT over t for row u, transforms it in registers and finishes with
-// one radix-2 butterfly across the pair (__shfl_xor, the partner lane differs
-// by `pair_xor`).  Output: thread t holds X[k1], k1 = (t>>1) + Q k + Q^2 (t&1).
-// The inverse mirrors the forward operation by operation (lifting rotations).
+// elements (L = 32, 128, 512).  Thread t holds x[(t' + P j) mod L]; after an
+// in-register Q-point DFT over j, the twiddle W_L^{t' u'} and one exchange,
+// lane pair (u = t >> 1, h = t & 1) holds the even (h = 0) or odd (h = 1) half
+// of the P-point DFT over t for row u, transforms it in registers and finishes
+// with one radix-2 butterfly across the pair (__shfl_xor, the partner lane
+// differs by `pair_xor`).  Output: thread t holds X[(u' + Q k + Q^2 h) mod L],
+// k = 0..Q-1.  The inverse mirrors the forward operation by operation.
 template <int Q, bool BLOCK_SYNC, class Lay>
 __device__ __forceinline__ void fft_p2q_lift(float2 (&v)[Q], float2* __restrict__ sm, const Lay lay, int t,
-                                             const float4* __restrict__ twPQ, int pair_xor) {
+                                             const float2* __restrict__ twPQ, int pair_xor) {
     constexpr int P = 2 * Q;
     dft_lift<Q>(v);
 #pragma unroll
-    for (int u = 1; u < Q; ++u) v[u] = cmul_df(v[u], twPQ[u * P + t]);
+    for (int u = 1; u < Q; ++u) v[u] = lift_rot(v[u], twPQ[u * P + t]);
 #pragma unroll
     for (int u = 0; u < Q; ++u) sm[lay(u, t)] = v[u];
     if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
@@ -393,7 +287,7 @@ __device__ __forceinline__ void fft_p2q_lift(float2 (&v)[Q], float2* __restrict_
 }
 template <int Q, bool BLOCK_SYNC, class Lay>
 __device__ __forceinline__ void fft_p2q_lift_inv(float2 (&v)[Q], float2* __restrict__ sm, const Lay lay, int t,
-                                                 const float4* __restrict__ twPQ, int pair_xor) {
+                                                 const float2* __restrict__ twPQ, int pair_xor) {
     constexpr int P = 2 * Q;
     const int u = t >> 1, h = t & 1;
     const float sg = h ? -1.0f : 1.0f;
@@ -414,7 +308,7 @@ __device__ __forceinline__ void fft_p2q_lift_inv(float2 (&v)[Q], float2* __restr
     for (int w = 0; w < Q; ++w) v[w] = sm[lay(w, t)];
     if (BLOCK_SYNC) __syncthreads(); else __syncwarp();
 #pragma unroll
-    for (int w = 1; w < Q; ++w) v[w] = cmulc_df(v[w], twPQ[w * P + t]);
+    for (int w = 1; w < Q; ++w) v[w] = lift_rot_inv(v[w], twPQ[w * P + t]);
     dft_lift_inv<Q>(v);
 }
 
@@ -424,85 +318,51 @@ struct ColFFT {
     static constexpr bool PAIR = (L == 32 || L == 128 || L == 512);
     static constexpr int Q = PAIR ? (L == 32 ? 4 : L == 128 ? 8 : 16) : PQ<L>::Q;
     static constexpr int P = L / Q;
+    // Spectral rows k1 >= KC of the two-pass layout stand for the negative
+    // index k1 - L (see col_work); L/2 less the overhang of a thread's first
+    // element.
+    static constexpr int KC = L / 2 - (PAIR ? Q / 2 : P / 2);
+    static_assert(PAIR || P == Q, "column lengths 16, 64, 256, 1024 have P = Q");
 };
-// Threads per group of the column pass for length L (host side of ColFFT).
+// Threads per group of the column pass for length L, and KC (host side of ColFFT).
 __host__ __device__ __forceinline__ int col_group_p(int L) {
     return L == 32 ? 8 : L == 128 ? 16 : L == 512 ? 32 : (L <= 32 ? 4 : L <= 128 ? 8 : L <= 512 ? 16 : 32);
 }
+__host__ __device__ __forceinline__ int col_kc(int L) {
+    const int P = col_group_p(L), Q = L / P;
+    return L / 2 - (P == Q ? P / 2 : Q / 2);
+}
 
 // ---------------------------------------------------------------------------
-// exp(2 pi i x) for a 64-bit fixed-point turn fraction x = X / 2^64, returned
-// as a double-float rotation {re_hi, im_hi, re_lo, im_lo} accurate to ~1e-12.
-// x = j/512 + r with |r| <= 1/1024: T[j] = exp(2 pi i j/512) from a
-// double-float table, exp(i theta) (theta = 2 pi r, |theta| <= pi/512) from
-// its Taylor series, combined with error-free products and sums
-// (Dekker / Knuth two-product and two-sum).
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
-    s = a + b;
-    const float bv = s - a;
-    e = (a - (s - bv)) + (b - bv);
-}
-
-// Exact float of a 23-bit unsigned integer (exponent trick, no conversion unit).
-__device__ __forceinline__ float u23_to_float(unsigned u) { return __int_as_float(0x4B000000u | u) - 8388608.0f; }
-
-__device__ __forceinline__ float4 turns_rotation_df(unsigned long long X, const float4* __restrict__ T512) {
-    // Y = X + 2^54: j = Y >> 55 is the nearest multiple of 1/512 turn, and the
-    // remainder r = X - j 2^55 in [-2^54, 2^54) is (Y mod 2^55) - 2^54.
-    const unsigned long long Y = X + (1ull << 54);
+// v * exp(2 pi i x) for a 64-bit fixed-point turn fraction, given as
+// Y = 2^64 x + 2^54 (the 2^54 rounds the table index to nearest): w = v * T[j],
+// T[j] = exp(2 pi i j/512) (times the linear step's gain) as double-float
+// {re_hi, im_hi, re_lo, im_lo} in a compensated product, then
+// w + w * (cos(theta) - 1 + i sin(theta)) for the residual |theta| <= pi/512,
+// whose angle is carried as the exact split th + tl.
+__device__ __forceinline__ float2 turns_rotate(float2 v, unsigned long long Y, const float4* __restrict__ T512) {
     const unsigned yh = (unsigned)(Y >> 32);
-    const int j = (int)((yh >> 23) & 511u);
-    // r + 2^54 = A 2^32 + B 2^9 + (9 dropped bits, < 2e-16 rad), A, B < 2^23.
-    const unsigned A = yh & 0x7FFFFFu;
-    const unsigned B = (unsigned)(Y >> 9) & 0x7FFFFFu;
-    const float fA = u23_to_float(A) - 4194304.0f;  // exact, in [-2^22, 2^22)
-    const float fB = u23_to_float(B);
-    // theta = 2 pi r / 2^64 = fA * 2pi/2^32 + fB * 2pi/2^55, as th + tl
-    const float c32_hi = 1.462918119976564e-09f, c32_lo = -4.070940267922164e-17f;
-    const float c9 = 1.7439342975337076e-16f;
+    const int j = (int)(yh >> 23);
+    // r + 2^54 = A 2^32 + B 2^9 + (9 dropped bits, < 2e-16 rad), A, B < 2^23
+    const float fA = __int_as_float(0x4B000000u | (yh & 0x7FFFFFu)) - (8388608.0f + 4194304.0f);  // exact
+    const float fB = __int_as_float(0x4B000000u | ((unsigned)Y >> 9)) - 8388608.0f;
+    const float c32_hi = 1.462918119976564e-09f, c32_lo = -4.070940267922164e-17f;  // 2 pi / 2^32
+    const float c9 = 1.7439342975337076e-16f;                                       // 2 pi / 2^55
     const float th = fA * c32_hi;
-    const float tl = fmaf(fA, c32_hi, -th) + fmaf(fA, c32_lo, fB * c9);
+    const float tl = fmaf(fB, c9, fmaf(fA, c32_lo, fmaf(fA, c32_hi, -th)));
     const float th2 = th * th;
-    // sin(theta) = th + (tl - th^3/6),  cos(theta) - 1 = -th^2/2 - th*tl + th^4/24
-    const float s_hi = th;
-    const float s_lo = fmaf(-th2 * th, 1.0f / 6.0f, tl);
-    const float cm1 = fmaf(th2 * th2, 1.0f / 24.0f, fmaf(-0.5f, th2, -th * tl));
-    const float4 t = T512[j];  // {c_hi, s_hi, c_lo, s_lo}
-    // re = Tc (1 + cm1) - Ts s ;  im = Ts (1 + cm1) + Tc s
-    const float p = t.y * s_hi, pe = fmaf(t.y, s_hi, -p);
-    const float q = t.x * s_hi, qe = fmaf(t.x, s_hi, -q);
-    float re_hi, re_e, im_hi, im_e;
-    two_sum(t.x, -p, re_hi, re_e);
-    two_sum(t.y, q, im_hi, im_e);
-    const float re_lo = re_e + t.z + fmaf(t.x, cm1, -pe) - fmaf(t.y, s_lo, t.w * s_hi);
-    const float im_lo = im_e + t.w + fmaf(t.y, cm1, qe) + fmaf(t.x, s_lo, t.z * s_hi);
-    return make_float4(re_hi, im_hi, re_lo, im_lo);
-}
-
-// v * exp(2 pi i x), x = X / 2^64 as in turns_rotation_df, applied to the data
-// in two steps: w = v * T[j] (double-float table entry, compensated product),
-// then w + w * (cos(theta) - 1 + i sin(theta)) for the residual |theta| <=
-// pi/512, whose angle is carried as the exact split th + tl.  Every constant
-// stays at ~48 bits; the intermediate w adds one data rounding.
-__device__ __forceinline__ float2 turns_rotate(float2 v, unsigned long long X, const float4* __restrict__ T512) {
-    const unsigned long long Y = X + (1ull << 54);
-    const unsigned yh = (unsigned)(Y >> 32);
-    const int j = (int)((yh >> 23) & 511u);
-    const unsigned A = yh & 0x7FFFFFu;
-    const unsigned B = (unsigned)(Y >> 9) & 0x7FFFFFu;
-    const float fA = u23_to_float(A) - 4194304.0f;
-    const float fB = u23_to_float(B);
-    const float c32_hi = 1.462918119976564e-09f, c32_lo = -4.070940267922164e-17f;
-    const float c9 = 1.7439342975337076e-16f;
-    const float th = fA * c32_hi;
-    const float tl = fmaf(fA, c32_hi, -th) + fmaf(fA, c32_lo, fB * c9);
-    const float th2 = th * th;
-    const float sl = fmaf(-th2 * th, 1.0f / 6.0f, tl);                             // sin = th + sl
-    const float cm1 = fmaf(th2 * th2, 1.0f / 24.0f, fmaf(-0.5f, th2, -th * tl));  // cos - 1
+    const float sl = fmaf(th2 * th, -1.0f / 6.0f, tl);       // sin = th + sl (theta^5/120 < 8e-14)
+    const float cm1 = th2 * fmaf(th2, 1.0f / 24.0f, -0.5f);  // cos - 1 (th tl < 2e-12, its rounding 1e-12)
     const float2 w = cmul_df(v, T512[j]);
     const float re = w.x + fmaf(-w.y, th, fmaf(w.x, cm1, -(w.y * sl)));
     const float im = w.y + fmaf(w.x, th, fmaf(w.y, cm1, w.x * sl));
     return make_float2(re, im);
+}
+
+// A double-float table entry times an FP32 gain, renormalized.
+__device__ __forceinline__ float4 scale_df(float4 w, float g) {
+    const float re = g * w.x, im = g * w.y;
+    return make_float4(re, im, fmaf(g, w.z, fmaf(g, w.x, -re)), fmaf(g, w.w, fmaf(g, w.y, -im)));
 }
 
 }  // namespace fg

@@ -71,21 +71,34 @@ inline void ssfm_derive(SsfmParams& p) {
     p.inv_samples = 1.0 / (double)p.samples;  // exact: samples is a power of 2
 }
 
-// Twiddle tables, double-float {re_hi, im_hi, re_lo, im_lo}, packed in one
-// device buffer (offsets in entries):
-//   0            column sub-FFT table, entry u*P+t = W_N1^{t u}   (N1 entries)
-//   N1           row sub-FFT table,    entry u*P+t = W_N2^{t u}   (N2 entries)
-//   N1+N2        reserved (N1 entries; the column pass computes its six-step
-//                factors on the device, sixstep_factor in fft.cuh)
-//   2N1+N2       reserved (N2 entries)
-//   2N1+2N2      exp(+2 pi i j/512), j < 512                      (512 entries)
+// Twiddle tables of a plan, packed in one device buffer:
+//   col   column sub-FFT, entry u*P+t = lifting pair of W_N1^{t' u'}   (N1 float2)
+//   row   row sub-FFT, likewise for N2                                 (N2 float2)
+//   turn  exp(+2 pi i j/512), j < 512, double-float {re_hi, im_hi, re_lo, im_lo}
+// (centred indices t', u' and lifting pairs {tan(theta/2), sin(theta)} as in
+// fft.cuh; the column pass computes its six-step factors itself).
+struct Tables {
+    const float2* col = nullptr;
+    const float2* row = nullptr;
+    const float4* turn = nullptr;
+};
+constexpr size_t table_bytes(int N1, int N2) { return sizeof(float4) * 512 + sizeof(float2) * ((size_t)N1 + N2); }
+inline Tables tables_at(const void* buf, int N1) {
+    Tables t;
+    t.turn = (const float4*)buf;
+    t.col = (const float2*)(t.turn + 512);
+    t.row = t.col + N1;
+    return t;
+}
+
 struct PassArgs {
     float2* data;           // batch x N complex64
-    const float4* tw;
+    Tables tw;
     const float2* table;    // ROW_TABLE multiplier, transposed layout (k1*N2 + k2), length N
     SsfmState* state;       // null: plain transform driven by `op`
     SsfmParams prm;
     int N, N1, N2, log2N2;
+    int kc;                 // rows k1 >= kc hold the bins k1 - N1 + N1 k2 (set by the launch helpers)
     int batch;              // realizations (set by the launch helpers)
     int modes;              // modes per realization of an SSFM run (0 or 1: single mode)
     int op;
@@ -96,7 +109,7 @@ struct PassArgs {
 
 struct Plan {
     int N = 0, N1 = 0, N2 = 0, log2N1 = 0, log2N2 = 0;
-    float4* tw = nullptr;   // device tables (layout above)
+    void* tw = nullptr;     // device tables (tables_at)
     int staging = 0;        // FOCSS_STAGING_*: how the passes move their data
 };
 
@@ -220,7 +233,7 @@ focss_status fft_inverse(Ctx* ctx, float2* data, int N, int batch);   // natural
 // Forward then pointwise op then inverse, spectrum never leaves the two-pass layout.
 focss_status spectral_apply(Ctx* ctx, float2* data, int N, int batch, int row_op, const float2* table,
                             float scale, int bp_cut);
-// Transposed-layout spectrum (k1*N2 + k2 holds bin k1 + N1*k2), x scale.
+// Two-pass-layout spectrum (row k1, column k2 holds bin k1' + N1*k2 mod N, see col_work), x scale.
 focss_status fft_forward_transposed(Ctx* ctx, float2* data, int N, int batch, float scale);
 focss_status fft_inverse_transposed(Ctx* ctx, float2* data, int N, int batch);
 
@@ -230,9 +243,9 @@ cudaError_t launch_amplifier(float2* d, int modes, int samples, int batch, doubl
                              uint64_t seed, uint64_t counter, cudaStream_t st);
 cudaError_t launch_power(const float2* d, int modes, int samples, int batch, double* avg,
                          unsigned int* peak_bits, cudaStream_t st);
-cudaError_t launch_transpose_to_natural(const float2* src, float2* dst, int N1, int N2, int batch,
+cudaError_t launch_transpose_to_natural(const float2* src, float2* dst, int N1, int N2, int kc, int batch,
                                         cudaStream_t st);
-cudaError_t launch_transpose_from_natural(const float2* src, float2* dst, int N1, int N2, int batch,
+cudaError_t launch_transpose_from_natural(const float2* src, float2* dst, int N1, int N2, int kc, int batch,
                                           cudaStream_t st);
 
 }  // namespace fg

@@ -25,16 +25,14 @@ namespace {
 
 constexpr int kNoallocMaxLog2Samples = 17;   // N <= 2^17 samples per realization
 constexpr int kNoallocMaxBatch = 256;        // realizations per call
-// Largest table set: N = 2^17 -> N1 = 256, N2 = 512: 2*N1 + 2*N2 + 512 entries.
-constexpr int kNoallocTableEntries = 2 * 256 + 2 * 512 + 512;
-
+// Largest table set: N = 2^17 -> N1 = 256, N2 = 512.
 struct NoallocScratch {
-    float4 tw[kNoallocTableEntries];
+    alignas(16) unsigned char tw[table_bytes(256, 512)];
     SsfmState state[kNoallocMaxBatch];
     int counters[16];
 };
 
-// ~59 KB of device memory per device, for the lifetime of the process.
+// ~52 KB of device memory per device, for the lifetime of the process.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoallocScratch)];
 
 std::mutex g_noalloc_mutex;
@@ -57,30 +55,26 @@ cudaError_t noalloc_scratch(NoallocScratch** out) {
     return cudaSuccess;
 }
 
-__device__ __forceinline__ float4 df_rotation(double turns_times_2) {
-    double s, c;
-    sincospi(turns_times_2, &s, &c);
-    const float ch = (float)c, sh = (float)s;
-    return make_float4(ch, sh, (float)(c - (double)ch), (float)(s - (double)sh));
-}
-
 __host__ __device__ __forceinline__ int group_p(int L) { return L <= 32 ? 4 : L <= 128 ? 8 : L <= 512 ? 16 : 32; }
 
 // The plan tables of internal.h, computed on the device in FP64.
-__global__ void noalloc_tables_kernel(float4* __restrict__ tw, int N, int N1, int N2) {
-    const int total = 2 * N1 + 2 * N2 + 512;
+__global__ void noalloc_tables_kernel(float2* __restrict__ col, float4* __restrict__ turn, int N1, int N2) {
+    const int total = N1 + N2 + 512;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        double s, c;
         if (i < N1 + N2) {
             const int L = i < N1 ? N1 : N2;
             const int k = i < N1 ? i : i - N1;
-            const int P = i < N1 ? col_group_p(L) : group_p(L);
-            const long long e = (long long)(k % P) * (k / P) % L;
-            tw[i] = df_rotation(-2.0 * (double)e / L);
-        } else if (i < 2 * N1 + 2 * N2) {
-            tw[i] = make_float4(0.f, 0.f, 0.f, 0.f);  // reserved
+            const int P = i < N1 ? col_group_p(L) : group_p(L), Q = L / P;
+            const int t = k % P, u = k / P;
+            const double r = -(double)((t < P / 2 ? t : t - P) * (u < Q / 2 ? u : u - Q)) / L;  // turns
+            sincospi(r, &s, &c);  // half the angle
+            col[i] = make_float2((float)(s / c), (float)(2.0 * s * c));
         } else {
-            const int j = i - 2 * N1 - 2 * N2;
-            tw[i] = df_rotation(2.0 * (double)j / 512);
+            const int j = i - N1 - N2;
+            sincospi(2.0 * (double)j / 512, &s, &c);
+            const float2 cf = split_df(c), sf = split_df(s);
+            turn[j] = make_float4(cf.x, sf.x, cf.y, sf.y);
         }
     }
 }
@@ -123,7 +117,8 @@ extern "C" FOCSS_API focss_status focss_ssfm_run_noalloc(void* stream, void* dat
     e = cudaMemsetAsync(sc->state, 0, sizeof(SsfmState) * batch, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(sc->counters, 0, sizeof(int) * 16, s);
     if (e == cudaSuccess) {
-        noalloc_tables_kernel<<<8, 256, 0, s>>>(sc->tw, p.N, p.N1, p.N2);
+        const Tables t = tables_at(sc->tw, p.N1);
+        noalloc_tables_kernel<<<8, 256, 0, s>>>((float2*)t.col, (float4*)t.turn, p.N1, p.N2);
         count_launch();
         e = cudaGetLastError();
     }

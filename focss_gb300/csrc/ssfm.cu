@@ -11,15 +11,16 @@
 //   row pass     [forward length-N2 FFT] -> exp(-alpha*hl/2)/N *
 //                exp(i*beta2/2*hl*w_k^2) -> [inverse length-N2 FFT]
 //
-// The spectrum never leaves the transposed layout (row k1, column k2 holds
-// bin k = k1 + N1*k2), so no transposes are needed.  The merged half steps of
+// The spectrum never leaves the two-pass layout (row k1, column k2 holds bin
+// k1' + N1*k2 mod N with k1' = k1 or k1 - N1, see col_work), so no transposes
+// are needed.  The merged half steps of
 // the reference's Strang splitting (src/focss/solver/ssfm.cpp:62-118) appear
 // as one row pass with hl = (h_i + h_{i+1})/2.
 //
 // The dispersion phase is formed from an FP64 per-step scalar
-// a = beta2/2*hl*dw^2/(2*pi) (turns per k'^2) held as a 64-bit fixed-point
-// turn fraction; a*k'^2 mod 1 is then an exact wrapping 64-bit integer
-// product, so the FP32 sincospi argument is already range-reduced to [-1, 1).
+// a = beta2/2*hl*dw^2/(2*pi) (turns per k'^2) held as a 96-bit fixed-point
+// turn fraction; a*k'^2 mod 1 then follows in wrapping 64-bit integers
+// (PhaseRun), already range-reduced.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -199,13 +200,13 @@ cudaError_t launch_col(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
     const int C = narrow ? l.per_block_narrow : l.per_block;
     // s_fc (N1) + six-step table (Q x C, Q = N1/P) + exchange (N1 x C per mode)
     const int P = l.threads / l.per_block;
-    const size_t smem = sizeof(float4) * ((size_t)p.N1 + (size_t)(p.N1 / P) * C) +
-                        sizeof(float2) * (size_t)p.N1 * C * modes;
+    const size_t smem = sizeof(float2) * ((size_t)p.N1 + (size_t)(p.N1 / P) * C + (size_t)p.N1 * C * modes);
     a.N = p.N;
     a.N1 = p.N1;
     a.N2 = p.N2;
     a.log2N2 = p.log2N2;
-    a.tw = p.tw;
+    a.tw = tables_at(p.tw, p.N1);
+    a.kc = col_kc(p.N1);
     a.batch = batch;
     if (p.staging == FOCSS_STAGING_TMA) return launch_col_tma(p, a, batch, modes, smem + 128, s);
     cudaError_t e = cached_launch(narrow ? 4 : 0, p.log2N1, smem, &l);
@@ -224,14 +225,15 @@ cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
                         p.N1 % l.per_block_narrow == 0;
     const int kind = p.staging != FOCSS_STAGING_LOADS ? 2 : narrow ? 3 : 1;
     int R = narrow ? l.per_block_narrow : l.per_block;
-    const size_t smem = sizeof(float4) * ((size_t)p.N2 + 512) + sizeof(float2) * (size_t)R * Q * (P + 1);
+    const size_t smem = sizeof(float4) * 512 + sizeof(float2) * ((size_t)p.N2 + (size_t)R * Q * (P + 1));
     cudaError_t e = cached_launch(kind, p.log2N2, smem, &l);
     if (e != cudaSuccess) return e;
     a.N = p.N;
     a.N1 = p.N1;
     a.N2 = p.N2;
     a.log2N2 = p.log2N2;
-    a.tw = p.tw;
+    a.tw = tables_at(p.tw, p.N1);
+    a.kc = col_kc(p.N1);
     a.batch = batch;
     if (p.N1 % R != 0) return cudaErrorInvalidValue;
     return launch_pass(l, dim3(p.N1 / R, batch * (a.modes > 1 ? a.modes : 1)), l.threads, smem, s, a);
@@ -503,7 +505,7 @@ focss_status fft_forward(Ctx* ctx, float2* data, int N, int batch) {
     if (st != FOCSS_OK) return st;
     float2* tmp = (float2*)scratch_buffer(ctx, 0, sizeof(float2) * (size_t)N * batch);
     if (!tmp) return set_error(ctx, FOCSS_ERR_OOM, "fft scratch");
-    cudaError_t e = launch_transpose_to_natural(data, tmp, p->N1, p->N2, batch, ctx->stream);
+    cudaError_t e = launch_transpose_to_natural(data, tmp, p->N1, p->N2, col_kc(p->N1), batch, ctx->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(data, tmp, sizeof(float2) * (size_t)N * batch, cudaMemcpyDeviceToDevice, ctx->stream);
     return cuda_check(ctx, e, "fft transpose");
@@ -515,7 +517,7 @@ focss_status fft_inverse(Ctx* ctx, float2* data, int N, int batch) {
     if (st != FOCSS_OK) return st;
     float2* tmp = (float2*)scratch_buffer(ctx, 0, sizeof(float2) * (size_t)N * batch);
     if (!tmp) return set_error(ctx, FOCSS_ERR_OOM, "ifft scratch");
-    cudaError_t e = launch_transpose_from_natural(data, tmp, p->N1, p->N2, batch, ctx->stream);
+    cudaError_t e = launch_transpose_from_natural(data, tmp, p->N1, p->N2, col_kc(p->N1), batch, ctx->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(data, tmp, sizeof(float2) * (size_t)N * batch, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e != cudaSuccess) return cuda_check(ctx, e, "ifft transpose");

@@ -35,7 +35,8 @@ cudaError_t launch_block(const Plan& p, PassArgs a, int batch, int cap, cudaStre
     a.N1 = p.N1;
     a.N2 = p.N2;
     a.log2N2 = p.log2N2;
-    a.tw = p.tw;
+    a.tw = tables_at(p.tw, p.N1);
+    a.kc = col_kc(p.N1);
     a.batch = batch;
     switch (p.N) {
         case 1 << 12: return launch_block_t<64, 64>(a, batch, cap, s);

@@ -217,49 +217,60 @@ struct ColShape {
 // on columns [n2_0, n2_0 + C) of one mode of one realization; `data` points
 // at that mode's first sample and rows are `ld` samples apart (N2 in global
 // memory for the two-pass kernels; padded in the single-CTA kernel's shared
-// memory).  `sB` holds the six-step
-// factors W_N^{n2 a1 j} of these columns at sB[j * sB_stride + c].  Adds the
-// time-domain field's peak and sum of |A|^2 to pk / sm.
+// memory).  `sB` holds the column part of the six-step factors at
+// sB[j * sB_stride + c].  Adds the time-domain field's peak and sum of |A|^2
+// to pk / sm.
+//
+// Centred six-step factors.  Column n2 stands for n2' = n2 or, from N2/2 on,
+// n2 - N2, and spectral row k1 for k1' = k1 or, from KC (~N1/2) on, k1 - N1.
+// The factor W_N^{n2' k1'} then turns by at most ~pi/2, so it is a product of
+// two plain lifting rotations (a per-thread one and a per-column table over
+// j) where W_N^{n2 k1} needed a data-dependent quarter-turn placement (~8
+// instructions per element and direction).  W_N^{n2 k1} differs from it by
+// whole periods: time row n1 of a column n2' < 0 is index n1 + 1 of its
+// sub-FFT, and column k2 of a row k1' < 0 holds bin k1' + N1 k2 (see row_core),
+// i.e. only indices move.
 template <int N1, int C>
 __device__ __forceinline__ void col_work(const PassArgs& a, int op, const SsfmState* st, float2* data, int n2_0,
-                                         const float4* s_fc, const float4* sB, int sB_stride, float2* sx,
+                                         const float2* s_fc, const float2* sB, int sB_stride, float2* sx,
                                          float2* s_x0, int mo, int modes, int gt, int ld, float& pk, float& sm,
                                          const float2* src = nullptr, int src_ld = 0) {
     constexpr int P = ColFFT<N1>::P, Q = ColFFT<N1>::Q;
     constexpr bool PAIR = ColFFT<N1>::PAIR;
-    // Element j of a thread is time-domain row t + P j; in the spectral
-    // layout it is row a0 + a1 j (a0 = t, a1 = P for the PQ form; lane-pair
-    // form: a0 = (t>>1) + Q^2 (t&1), a1 = Q).  Six-step twiddle of column n2:
-    // W_N^{n2 (a0 + a1 j)} = W_N^{n2 a0} (per thread) x W_N^{n2 a1 j} (per
-    // column table over j), each a quarter turn times a lifting rotation whose
-    // inverse mirrors it exactly.
+    // Time domain: element j of a thread is index t' + P j of the sub-FFT.
+    // Spectral domain: row a0 + a1 j (PQ form: a0 = t', a1 = P; lane-pair form:
+    // a0 = u' + Q^2 h with u = t >> 1, h = t & 1, a1 = Q).  Only element 0 can
+    // be negative and wraps by N1.
     constexpr int a1 = PAIR ? Q : P;
     const int log2N = a.log2N2 + ilog2c(N1);
     const int c = gt % C, t = (gt / C) % P;
-    const int a0 = PAIR ? (t >> 1) + Q * Q * (t & 1) : t;
+    const int a0 = PAIR ? centred<Q>(t >> 1) + Q * Q * (t & 1) : centred<P>(t);
     const int n2 = n2_0 + c;
-    const float4 fa = sixstep_factor(n2 * a0, log2N);
-    const float2 tsA = make_float2(fa.x, fa.y);
-    const int qA = __float_as_int(fa.z);
+    const int neg = n2 >= (1 << a.log2N2) / 2;                 // n2' < 0
+    const int n2c = n2 - (neg << a.log2N2);
+    // thread part of the six-step factor (lane-pair form: rows of h = 1 are k1' = row - N1)
+    const float2 tsA = sixstep_factor(n2c * (PAIR ? a0 - N1 * (t & 1) : a0), log2N);
+    const int tbase = centred<P>(t) - neg;                     // time row of element 0
+    const int twrap = tbase < 0 ? tbase + N1 : tbase, awrap = a0 < 0 ? a0 + N1 : a0;
     float2* base = data + n2;
     // the columns come from `src` (a tile of C columns, rows src_ld apart,
     // staged in shared memory) when given, else from data
     const float2* lb = src ? src + c : base;
-    const size_t lld = src ? (size_t)src_ld : (size_t)ld;
+    const int lld = src ? src_ld : ld;
     float2 v[Q];
+    {
+        const int r0 = op == COL_FWD ? twrap : awrap, rb = op == COL_FWD ? tbase : a0, rs = op == COL_FWD ? P : a1;
+        v[0] = lb[(size_t)r0 * lld];
+        const float2* q = lb + (ptrdiff_t)rb * lld;
 #pragma unroll
-    for (int j = 0; j < Q; ++j) v[j] = lb[(size_t)(op == COL_FWD ? t + P * j : a0 + a1 * j) * lld];
+        for (int j = 1; j < Q; ++j) v[j] = q[(size_t)(rs * j) * lld];
+    }
     __syncthreads();
 
     const ColLayout<P, C> lay{c};
     if (op != COL_FWD) {
 #pragma unroll
-        for (int j = 0; j < Q; ++j) {
-            const float4 fb = sB[j * sB_stride + c];
-            v[j] = lift_rot_inv(lift_rot_inv(quarter_turns(v[j], -(qA + __float_as_int(fb.z)) & 3),
-                                             make_float2(fb.x, fb.y)),
-                                tsA);
-        }
+        for (int j = 0; j < Q; ++j) v[j] = lift_rot_inv(lift_rot_inv(v[j], sB[j * sB_stride + c]), tsA);
         if constexpr (PAIR)
             fft_p2q_lift_inv<Q, true>(v, sx, lay, t, s_fc, C);
         else
@@ -268,30 +279,48 @@ __device__ __forceinline__ void col_work(const PassArgs& a, int op, const SsfmSt
     if (op == COL_KERR) {
         // src/focss/solver/ssfm.cpp:160-164: A *= exp(i kappa gamma h |A|^2); the
         // peak is taken from |A|^2 before the rotation (which preserves it).
+        // A thread whose phases are all small takes kerr_rotate_small on its
+        // registers; the general rotation runs as a rolled loop over a copy in
+        // local memory, so that its long body is emitted once instead of Q
+        // times (the unrolled one stalled the kernel on instruction fetch).
         const float coef = st->kerr_coef;
+        const float* pw = reinterpret_cast<const float*>(s_x0);
+        const int stride = N1 * C;
+        float m = 0.0f;
         if (modes == 1) {
 #pragma unroll
-            for (int j = 0; j < Q; ++j) {
-                const float p = cnorm(v[j]);
-                v[j] = kerr_rotate(v[j], coef * p);
-                pk = fmaxf(pk, p);
-            }
+            for (int j = 0; j < Q; ++j) m = fmaxf(m, cnorm(v[j]));
         } else {
             // |A_0|^2 + |A_1|^2 through the (now free) exchange buffers
-            float* pw = reinterpret_cast<float*>(s_x0);
-            const int stride = N1 * C;
+            float* mine = reinterpret_cast<float*>(s_x0) + mo * stride;
 #pragma unroll
-            for (int j = 0; j < Q; ++j) pw[mo * stride + (t + P * j) * C + c] = cnorm(v[j]);
+            for (int j = 0; j < Q; ++j) mine[(t + P * j) * C + c] = cnorm(v[j]);
             __syncthreads();
+#pragma unroll
+            for (int j = 0; j < Q; ++j) m = fmaxf(m, pw[(t + P * j) * C + c] + pw[stride + (t + P * j) * C + c]);
+        }
+        pk = fmaxf(pk, m);
+        if (fabsf(coef) * m <= kKerrSmall) {
 #pragma unroll
             for (int j = 0; j < Q; ++j) {
                 const int i = (t + P * j) * C + c;
-                const float p = pw[i] + pw[stride + i];
-                v[j] = kerr_rotate(v[j], coef * p);
-                pk = fmaxf(pk, p);
+                const float p = modes == 1 ? cnorm(v[j]) : pw[i] + pw[stride + i];
+                v[j] = kerr_rotate_small(v[j], coef * p);
             }
-            __syncthreads();  // the forward transform reuses the buffers
+        } else {
+            float2 tmp[Q];
+#pragma unroll
+            for (int j = 0; j < Q; ++j) tmp[j] = v[j];
+#pragma unroll 1
+            for (int j = 0; j < Q; ++j) {
+                const int i = (t + P * j) * C + c;
+                const float p = modes == 1 ? cnorm(tmp[j]) : pw[i] + pw[stride + i];
+                tmp[j] = kerr_rotate(tmp[j], coef * p);
+            }
+#pragma unroll
+            for (int j = 0; j < Q; ++j) v[j] = tmp[j];
         }
+        if (modes > 1) __syncthreads();  // the forward transform reuses the buffers
     } else if (op == COL_FWD && st) {
         if (modes == 1) {
 #pragma unroll
@@ -324,13 +353,26 @@ __device__ __forceinline__ void col_work(const PassArgs& a, int op, const SsfmSt
         else
             fft_pq_lift<P, Q, true>(v, sx, lay, t, s_fc);
 #pragma unroll
-        for (int j = 0; j < Q; ++j) {
-            const float4 fb = sB[j * sB_stride + c];
-            v[j] = quarter_turns(lift_rot(lift_rot(v[j], tsA), make_float2(fb.x, fb.y)), qA + __float_as_int(fb.z));
-        }
+        for (int j = 0; j < Q; ++j) v[j] = lift_rot(lift_rot(v[j], tsA), sB[j * sB_stride + c]);
     }
+    {
+        const int r0 = op == COL_INV ? twrap : awrap, rb = op == COL_INV ? tbase : a0, rs = op == COL_INV ? P : a1;
+        base[(size_t)r0 * ld] = v[0];
+        float2* q = base + (ptrdiff_t)rb * ld;
 #pragma unroll
-    for (int j = 0; j < Q; ++j) base[(size_t)(op == COL_INV ? t + P * j : a0 + a1 * j) * ld] = v[j];
+        for (int j = 1; j < Q; ++j) q[(size_t)(rs * j) * ld] = v[j];
+    }
+}
+
+// Column part of the six-step factors, entry (j, column n2) of a table over
+// the elements j of a thread (col_work): W_N^{n2' e} with e = a1 j, in the PQ
+// form a1 j - N1 from j = Q/2 on (those rows are k1' = row - N1).
+template <int N1>
+__device__ __forceinline__ float2 sixstep_column(int j, int n2, int log2N2) {
+    constexpr int P = ColFFT<N1>::P, Q = ColFFT<N1>::Q;
+    const int n2c = n2 - ((n2 >= (1 << log2N2) / 2) << log2N2);
+    const int e = ColFFT<N1>::PAIR ? Q * j : P * j - (j >= Q / 2 ? N1 : 0);
+    return sixstep_factor(n2c * e, log2N2 + ilog2c(N1));
 }
 
 // The column-pass CTAs of realization b add their peak and energy to its
@@ -368,11 +410,10 @@ __device__ __forceinline__ void col_advance(const PassArgs& a, SsfmState* st, in
 template <int N1, int C>
 __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col_kernel(const PassArgs a) {
     constexpr int P = ColFFT<N1>::P, Q = ColFFT<N1>::Q;
-    constexpr int a1 = ColFFT<N1>::PAIR ? Q : P;
     extern __shared__ float4 smem4[];
-    float4* s_fc = smem4;                                  // column sub-FFT twiddles, (u,t) order
-    float4* s_B = s_fc + N1;                               // six-step factors W_N^{n2 a1 j}, [j][c]
-    float2* s_x0 = reinterpret_cast<float2*>(s_B + Q * C); // exchange buffers, N1*C per mode
+    float2* s_fc = reinterpret_cast<float2*>(smem4);       // column sub-FFT twiddles, (u,t) order
+    float2* s_B = s_fc + N1;                               // six-step factors (sixstep_column), [j][c]
+    float2* s_x0 = s_B + Q * C;                            // exchange buffers, N1*C per mode
     const int mo = threadIdx.x / (C * P);                  // mode of this thread group
     float2* sx = s_x0 + (size_t)mo * N1 * C;
     __shared__ float red[64];
@@ -380,9 +421,8 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
     // The six-step factors depend on nothing in memory: computed while the
     // previous pass finishes (programmatic dependent launch).
     pdl_trigger();
-    const int log2N = a.log2N2 + ilog2c(N1);
     for (int i = threadIdx.x; i < Q * C; i += blockDim.x)
-        s_B[i] = sixstep_factor((blockIdx.x * C + i % C) * a1 * (i / C), log2N);
+        s_B[i] = sixstep_column<N1>(i / C, blockIdx.x * C + i % C, a.log2N2);
     pdl_wait();
     const int b = blockIdx.y;
     SsfmState* st = a.state ? a.state + b : nullptr;
@@ -391,7 +431,7 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
         op = *(volatile int*)&st->action;
         if (op == COL_IDLE) return;
     }
-    for (int i = threadIdx.x; i < N1; i += blockDim.x) s_fc[i] = a.tw[i];
+    for (int i = threadIdx.x; i < N1; i += blockDim.x) s_fc[i] = a.tw.col[i];
     const int modes = a.modes > 1 ? a.modes : 1;
     float pk = 0.0f, sm = 0.0f;
     col_work<N1, C>(a, op, st, a.data + ((size_t)b * modes + mo) * a.N, blockIdx.x * C, s_fc, s_B, C, sx, s_x0, mo,
@@ -402,35 +442,54 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
 // ---------------------------------------------------------------- row pass
 // The work of the P threads of row k1 (`rl` the row's slot in the exchange
 // buffer, t the thread in the row) of one mode; `data` points at that mode's
-// first sample (global or shared memory), rows `ld` samples apart.  ROW_SSFM
-// applies exp(-alpha hl/2)/N (FP32 gain g) times the dispersion phase from the
-// 96-bit fraction dhi/dlo.
-// a k'^2 in turns as the 96-bit fixed-point product of the step's fraction
-// a (a96 = dhi 2^32 + the low 32 bits) and k'^2, carried exactly (mod 2^128)
-// along an arithmetic progression k' = k0 + delta i by second differences:
-// P_i = a k_i'^2, P_{i+1} = P_i + dP_i, dP_{i+1} = dP_i + 2 a delta^2.  next()
-// returns bits 32..95 of P_i, which equal dhi k'^2 + umulhi(dlo 2^32, k'^2)
-// mod 2^64.  |k0|, |delta| <= 2^19, so the integer factors fit in 64 bits.
+// first sample (global or shared memory), rows `ld` samples apart.  Column k2
+// of the row holds bin k = k1' + N1 k2 mod N, k1' = k1 or, from a.kc on,
+// k1 - N1 (col_work).  ROW_SSFM applies exp(-alpha hl/2)/N (in the table s_T)
+// times the dispersion phase from the 96-bit fraction dhi/dlo.
+
+// a k'^2 in turns for k' = k0 + delta j, j = 0, 1, ..., carried along the
+// arithmetic progression by second differences in 64-bit turn fractions, plus
+// 2^54 (turns_rotate's rounding).  The start value and the two differences
+// are formed from the step's 96-bit fraction a = hi 2^-64 + lo 2^-96 (lo < 2^32)
+// and truncated to 2^-64, which adds at most ~150 2^-64 = 2^-57 turns over 16
+// elements -- below the 2^-55 that turns_rotate reads.  (128-bit differences
+// gave the exact bits for 8 more instructions per element.)
+__device__ __forceinline__ unsigned long long turns_mul(unsigned long long hi, unsigned long long lo, long long m) {
+    // floor(a m 2^64) mod 2^64, |m| < 2^41: lo m / 2^32 from the halves of m
+    const unsigned long long ml = (unsigned)m;
+    return hi * (unsigned long long)m + (unsigned long long)((long long)lo * (m >> 32)) + ((lo * ml) >> 32);
+}
 struct PhaseRun {
-    unsigned __int128 P, dP, C2;
-    __device__ __forceinline__ PhaseRun(unsigned __int128 a, long long k0, long long delta) {
-        P = a * (unsigned __int128)(unsigned long long)(k0 * k0);
-        dP = a * (unsigned __int128)(__int128)(2 * delta * k0 + delta * delta);
-        C2 = a * (unsigned __int128)(unsigned long long)(2 * delta * delta);
+    unsigned long long P, dP, C2;
+    __device__ __forceinline__ PhaseRun(unsigned long long hi, unsigned long long lo, long long k0, long long delta) {
+        P = turns_mul(hi, lo, k0 * k0) + (1ull << 54);
+        dP = turns_mul(hi, lo, 2 * delta * k0 + delta * delta);
+        C2 = turns_mul(hi, lo, 2 * delta * delta);
     }
     __device__ __forceinline__ unsigned long long next() {
-        const unsigned long long X = (unsigned long long)(P >> 32);
+        const unsigned long long X = P;
         P += dP;
         dP += C2;
         return X;
     }
 };
 
-// The row work on the thread's elements v[j] = x[t + P j] of row k1, in
-// registers from load to store.
+// The row work on the thread's elements in registers: v[j] = sample
+// (t' + P j) mod N2 of row k1 in the n2 domain, on entry (but ROW_INV) and
+// exit (but ROW_FWD).  In the k2 domain (ROW_INV's entry, ROW_FWD's exit)
+// v[j] is column row_k2<N2>(t, j).
+template <int N2>
+__device__ __forceinline__ int row_k2_base(int t) {  // column of element 0 before wrapping
+    return PQ<N2>::Q == PQ<N2>::P ? centred<PQ<N2>::P>(t) : t;
+}
+template <int N2>
+__device__ __forceinline__ int row_k2(int t, int j) {
+    return (row_k2_base<N2>(t) + PQ<N2>::P * j) & (N2 - 1);
+}
+
 template <int N2>
 __device__ __forceinline__ void row_core(const PassArgs& a, int op, float2 (&v)[PQ<N2>::Q], int k1, int rl, int t,
-                                         const float4* s_tw, const float4* s_T, float2* sx, float g,
+                                         const float2* s_tw, const float4* s_T, float2* sx, float g,
                                          unsigned long long dhi, unsigned long long dlo) {
     constexpr int P = PQ<N2>::P, Q = PQ<N2>::Q;
     const RowLayout<P> lay{rl * Q * (P + 1)};
@@ -440,45 +499,32 @@ __device__ __forceinline__ void row_core(const PassArgs& a, int op, float2 (&v)[
     // with the (near-identity) Kerr step of the next column pass.
     if (op != ROW_INV) fft_pq_lift<P, Q, false>(v, sx, lay, t, s_tw);
     const int N = a.N, N1 = a.N1;
+    const int k1c = k1 < a.kc ? k1 : k1 - N1;
     if (op == ROW_SSFM) {
         // exp(-alpha hl/2)/N * exp(i beta2/2 hl w_k^2) (ssfm.cpp:142-158), w_k = k' dw,
-        // phase in turns = a k'^2 mod 1 formed exactly from the 96-bit fraction.
-        // The thread's own bins go through its column of the exchange buffer
-        // so that this long per-bin body is emitted once (a rolled loop), not
-        // Q times: the unrolled kernel overflowed the instruction cache.
-        //
-        // The thread's bins k = s0 + D j (s0 = k1 + N1 t, D = N1 P) fold to
-        // k' = s0 + D j for j < Q/2 and k' = N - s0 - D j above: two
-        // arithmetic progressions, along which a k'^2 is carried exactly by
-        // second differences (PhaseRun) instead of a 64 x 64-bit product per
-        // bin -- the same bits, so the same rotation.
-        float2* mine = sx + lay(0, t);
+        // phase in turns = a k'^2 mod 1 from the 96-bit fraction.  The
+        // thread's bins k = s0 + D j, s0 = k1' + N1 (column of element 0),
+        // D = N1 P = N/Q, |s0| < D, fold to k' = k below N/2 and k - N from
+        // there on: two arithmetic progressions that meet at j = Q/2, where
+        // k = N/2 + s0.
+        const long long s0 = (long long)k1c + (long long)N1 * row_k2_base<N2>(t), D = (long long)N1 * P;
+        PhaseRun lo(dhi, dlo, s0, D), up(dhi, dlo, s0 - (N >> 1), D);
 #pragma unroll
-        for (int j = 0; j < Q; ++j) mine[j * (P + 1)] = v[j];
-        const unsigned __int128 a96 = ((unsigned __int128)dhi << 32) | (unsigned __int128)(dlo >> 32);
-        const long long s0 = (long long)k1 + (long long)N1 * t, D = (long long)N1 * P;
+        for (int j = 0; j < Q / 2; ++j) v[j] = turns_rotate(v[j], lo.next(), s_T);
         {
-            PhaseRun run(a96, s0, D);
-#pragma unroll 1
-            for (int j = 0; j < Q / 2; ++j)
-                mine[j * (P + 1)] = turns_rotate(cscale(mine[j * (P + 1)], g), run.next(), s_T);
-        }
-        {
-            PhaseRun run(a96, (long long)(N >> 1) - s0, -D);
-#pragma unroll 1
-            for (int j = Q / 2; j < Q; ++j)
-                mine[j * (P + 1)] = turns_rotate(cscale(mine[j * (P + 1)], g), run.next(), s_T);
+            const unsigned long long X = up.next();
+            v[Q / 2] = turns_rotate(v[Q / 2], s0 < 0 ? lo.P : X, s_T);
         }
 #pragma unroll
-        for (int j = 0; j < Q; ++j) v[j] = mine[j * (P + 1)];
+        for (int j = Q / 2 + 1; j < Q; ++j) v[j] = turns_rotate(v[j], up.next(), s_T);
     } else if (op == ROW_TABLE) {
-        const float2* tb = a.table + (size_t)k1 * N2 + t;
+        const float2* tb = a.table + (size_t)k1 * N2;
 #pragma unroll
-        for (int j = 0; j < Q; ++j) v[j] = cscale(cmul(v[j], tb[P * j]), g);
+        for (int j = 0; j < Q; ++j) v[j] = cscale(cmul(v[j], tb[row_k2<N2>(t, j)]), g);
     } else if (op == ROW_BANDPASS) {
 #pragma unroll
         for (int j = 0; j < Q; ++j) {
-            const int k = k1 + N1 * (t + P * j);
+            const int k = (k1c + N1 * row_k2<N2>(t, j)) & (N - 1);
             v[j] = (k >= a.bp_cut && k <= N - a.bp_cut) ? make_float2(0.f, 0.f) : cscale(v[j], g);
         }
     } else if (op != ROW_INV) {  // ROW_SCALE, ROW_FWD
@@ -488,28 +534,62 @@ __device__ __forceinline__ void row_core(const PassArgs& a, int op, float2 (&v)[
     if (op != ROW_FWD) fft_pq_lift_inv<P, Q, false>(v, sx, lay, t, s_tw);
 }
 
+// Loads / stores the thread's elements of a row at `row` (either domain).
+template <int N2>
+__device__ __forceinline__ void row_load(float2 (&v)[PQ<N2>::Q], const float2* row, int first) {
+    v[0] = row[first & (N2 - 1)];
+#pragma unroll
+    for (int j = 1; j < PQ<N2>::Q; ++j) v[j] = row[first + PQ<N2>::P * j];
+}
+template <int N2>
+__device__ __forceinline__ void row_store(const float2 (&v)[PQ<N2>::Q], float2* row, int first) {
+    row[first & (N2 - 1)] = v[0];
+#pragma unroll
+    for (int j = 1; j < PQ<N2>::Q; ++j) row[first + PQ<N2>::P * j] = v[j];
+}
+
 template <int N2>
 __device__ __forceinline__ void row_work(const PassArgs& a, int op, float2* data, int k1, int rl, int t,
-                                         const float4* s_tw, const float4* s_T, float2* sx, float g,
+                                         const float2* s_tw, const float4* s_T, float2* sx, float g,
                                          unsigned long long dhi, unsigned long long dlo, int ld) {
     constexpr int P = PQ<N2>::P, Q = PQ<N2>::Q;
-    float2* base = data + (size_t)k1 * ld + t;
+    float2* row = data + (size_t)k1 * ld;
     float2 v[Q];
-#pragma unroll
-    for (int j = 0; j < Q; ++j) v[j] = base[P * j];
+    row_load<N2>(v, row, op == ROW_INV ? row_k2_base<N2>(t) : centred<P>(t));
     __syncthreads();
     row_core<N2>(a, op, v, k1, rl, t, s_tw, s_T, sx, g, dhi, dlo);
-#pragma unroll
-    for (int j = 0; j < Q; ++j) base[P * j] = v[j];
+    row_store<N2>(v, row, op == ROW_FWD ? row_k2_base<N2>(t) : centred<P>(t));
 }
+
+// Shared-memory tables of a row pass: the sub-FFT twiddles and, for the split
+// step, exp(2 pi i j/512) times the linear step's gain g.
+template <int N2>
+__device__ __forceinline__ void row_tables(const PassArgs& a, bool ssfm, float g, float2* s_tw, float4* s_T) {
+    for (int i = threadIdx.x; i < N2; i += blockDim.x) s_tw[i] = a.tw.row[i];
+    if (ssfm)
+        for (int i = threadIdx.x; i < 512; i += blockDim.x) s_T[i] = scale_df(a.tw.turn[i], g);
+}
+
+// Row-pass rows per block: must divide N1 (N1 >= max(16, N2/2) for every plan).
+template <int N2>
+struct RowShape {
+    static constexpr int P = PQ<N2>::P;
+    static constexpr int R0 = 256 / P;
+    static constexpr int RH = (N2 / 2 > 16 ? N2 / 2 : 16);
+    static constexpr int R = R0 < RH ? R0 : RH;
+    // 64-thread CTAs: when a launch has fewer row blocks than the GPU has SMs
+    // (a single field of 2^17 samples at a 128 x 1024 split has 16), four
+    // times as many SMs take part.
+    static constexpr int RN = 64 / P;
+};
 
 template <int N2, int R>
 __global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel(const PassArgs a) {
     constexpr int P = PQ<N2>::P;
     extern __shared__ float4 smem4[];
-    float4* s_tw = smem4;                                    // W_N2^e (double-float)
-    float4* s_T = s_tw + N2;                                 // exp(2 pi i j/512)
-    float2* sx = reinterpret_cast<float2*>(s_T + 512);       // R * Q * (P+1)
+    float4* s_T = smem4;                                     // g exp(2 pi i j/512)
+    float2* s_tw = reinterpret_cast<float2*>(s_T + 512);     // sub-FFT twiddles
+    float2* sx = s_tw + N2;                                  // R * Q * (P+1)
 
     pdl_trigger();
     pdl_wait();
@@ -520,12 +600,10 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel(const PassArgs a) 
     if (st) {
         if (!*(volatile const int*)&st->row_active) return;
         dhi = st->disp_hi;
-        dlo = st->disp_lo << 32;
+        dlo = st->disp_lo;
         g = st->lin_gain;
     }
-    for (int i = threadIdx.x; i < N2; i += blockDim.x) s_tw[i] = a.tw[a.N1 + i];
-    if (st)
-        for (int i = threadIdx.x; i < 512; i += blockDim.x) s_T[i] = a.tw[2 * a.N1 + 2 * N2 + i];
+    row_tables<N2>(a, st != nullptr, g, s_tw, s_T);
     const int rl = threadIdx.x / P, t = threadIdx.x % P;
     row_work<N2>(a, st ? (int)ROW_SSFM : a.op, a.data + (size_t)b * a.N, blockIdx.x * R + rl, rl, t, s_tw, s_T, sx,
                  g, dhi, dlo, N2);
@@ -563,9 +641,9 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel_bulk(const PassArg
     constexpr uint32_t kRowBytes = N2 * sizeof(float2);
     static_assert(kRowBytes % 16 == 0 && (Q * (P + 1) * sizeof(float2)) % 16 == 0, "bulk copies move 16-byte units");
     extern __shared__ float4 smem4[];
-    float4* s_tw = smem4;                                    // W_N2^e (double-float)
-    float4* s_T = s_tw + N2;                                 // exp(2 pi i j/512)
-    float2* sx = reinterpret_cast<float2*>(s_T + 512);       // R * Q * (P+1): landing zone and exchange
+    float4* s_T = smem4;                                     // g exp(2 pi i j/512)
+    float2* s_tw = reinterpret_cast<float2*>(s_T + 512);     // sub-FFT twiddles
+    float2* sx = s_tw + N2;                                  // R * Q * (P+1): landing zone and exchange
     __shared__ __align__(8) unsigned long long bar;
 
     pdl_trigger();
@@ -577,7 +655,7 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel_bulk(const PassArg
     if (st) {
         if (!*(volatile const int*)&st->row_active) return;  // before any copy is queued
         dhi = st->disp_hi;
-        dlo = st->disp_lo << 32;
+        dlo = st->disp_lo;
         g = st->lin_gain;
     }
     const int k1_0 = blockIdx.x * R;
@@ -594,9 +672,7 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel_bulk(const PassArg
                          "l"(rows + (size_t)r * N2), "r"(kRowBytes), "r"(ub)
                          : "memory");
     }
-    for (int i = threadIdx.x; i < N2; i += blockDim.x) s_tw[i] = a.tw[a.N1 + i];
-    if (st)
-        for (int i = threadIdx.x; i < 512; i += blockDim.x) s_T[i] = a.tw[2 * a.N1 + 2 * N2 + i];
+    row_tables<N2>(a, st != nullptr, g, s_tw, s_T);
     __syncthreads();  // barrier initialised, tables in place
     // every thread polls; the CTA leaves together if any of them gave up
     if (__syncthreads_or(!mbar_wait_bounded(ub, 0))) {
@@ -607,12 +683,11 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel_bulk(const PassArg
     const int rl = threadIdx.x / P, t = threadIdx.x % P;
     float2* row_s = sx + (size_t)rl * Q * (P + 1);
     float2 v[Q];
-#pragma unroll
-    for (int j = 0; j < Q; ++j) v[j] = row_s[t + P * j];
+    const int op = st ? (int)ROW_SSFM : a.op;
+    row_load<N2>(v, row_s, op == ROW_INV ? row_k2_base<N2>(t) : centred<P>(t));
     __syncwarp();  // the row's lanes (one warp holds whole rows) have read before the exchange writes
-    row_core<N2>(a, st ? (int)ROW_SSFM : a.op, v, k1_0 + rl, rl, t, s_tw, s_T, sx, g, dhi, dlo);
-#pragma unroll
-    for (int j = 0; j < Q; ++j) row_s[t + P * j] = v[j];
+    row_core<N2>(a, op, v, k1_0 + rl, rl, t, s_tw, s_T, sx, g, dhi, dlo);
+    row_store<N2>(v, row_s, op == ROW_FWD ? row_k2_base<N2>(t) : centred<P>(t));
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the writes, visible to the copy engine
     __syncwarp();
     if (t == 0) {
@@ -644,11 +719,10 @@ template <int N1, int C>
 __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB)
     col_kernel_tma(const __grid_constant__ CUtensorMap fmap, const PassArgs a) {
     constexpr int P = ColFFT<N1>::P, Q = ColFFT<N1>::Q;
-    constexpr int a1 = ColFFT<N1>::PAIR ? Q : P;
     constexpr int BOX = N1 < 256 ? N1 : 256;
     extern __shared__ float4 smem4[];
-    float4* s_fc = smem4;                                  // column sub-FFT twiddles, (u,t) order
-    float4* s_B = s_fc + N1;                               // six-step factors W_N^{n2 a1 j}, [j][c]
+    float2* s_fc = reinterpret_cast<float2*>(smem4);       // column sub-FFT twiddles, (u,t) order
+    float2* s_B = s_fc + N1;                               // six-step factors (sixstep_column), [j][c]
     // exchange buffers (the TMA landing tiles), N1*C per mode, from a
     // 128-byte boundary (the launch adds 128 bytes for it)
     const uint32_t xb = smem_addr(s_B + Q * C), xpad = (128u - (xb & 127u)) & 127u;
@@ -659,9 +733,8 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB)
     __shared__ __align__(8) unsigned long long bar;
 
     pdl_trigger();
-    const int log2N = a.log2N2 + ilog2c(N1);
     for (int i = threadIdx.x; i < Q * C; i += blockDim.x)
-        s_B[i] = sixstep_factor((blockIdx.x * C + i % C) * a1 * (i / C), log2N);
+        s_B[i] = sixstep_column<N1>(i / C, blockIdx.x * C + i % C, a.log2N2);
     pdl_wait();
     const int b = blockIdx.y;
     SsfmState* st = a.state ? a.state + b : nullptr;
@@ -683,7 +756,7 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB)
                 tma_load_2d(smem_addr(s_x0 + (size_t)m * N1 * C + (size_t)h * BOX * C), &fmap, blockIdx.x * C,
                             (b * modes + m) * N1 + h * BOX, ub);
     }
-    for (int i = threadIdx.x; i < N1; i += blockDim.x) s_fc[i] = a.tw[i];
+    for (int i = threadIdx.x; i < N1; i += blockDim.x) s_fc[i] = a.tw.col[i];
     __syncthreads();  // barrier initialised, tables in place
     if (__syncthreads_or(!mbar_wait_bounded(ub, 0))) {
         if (a.fault) atomicExch(a.fault, 1);
@@ -717,8 +790,8 @@ struct BlockShape {
     static constexpr size_t XCH = (size_t)G * N1 * C > (size_t)RPI * PQ<N2>::Q * (PQ<N2>::P + 1)
                                       ? (size_t)G * N1 * C
                                       : (size_t)RPI * PQ<N2>::Q * (PQ<N2>::P + 1);
-    static constexpr size_t SMEM = sizeof(float4) * ((size_t)N1 + (size_t)ColFFT<N1>::Q * N2 + N2 + 512) +
-                                   sizeof(float2) * ((size_t)N1 * LD + XCH);
+    static constexpr size_t SMEM = sizeof(float4) * 512 +
+                                   sizeof(float2) * ((size_t)N1 + (size_t)ColFFT<N1>::Q * N2 + N2 + (size_t)N1 * LD + XCH);
     static_assert(G >= 1 && N2 % (G * C) == 0 && N1 % RPI == 0, "single-CTA split");
 };
 
@@ -728,24 +801,21 @@ __global__ void __launch_bounds__(kBlockThreads, BlockShape<N1, N2>::SMEM <= 113
     using S = BlockShape<N1, N2>;
     constexpr int C = S::C, G = S::G, RPI = S::RPI;
     constexpr int Pc = ColFFT<N1>::P, Qc = ColFFT<N1>::Q, Pr = PQ<N2>::P;
-    constexpr int a1 = ColFFT<N1>::PAIR ? Qc : Pc;
     constexpr int N = N1 * N2, LD = S::LD;
     extern __shared__ float4 smem4[];
-    float4* s_fc = smem4;                                 // column sub-FFT twiddles
-    float4* s_B = s_fc + N1;                              // six-step factors, [j][n2]
-    float4* s_tw = s_B + Qc * N2;                         // row sub-FFT twiddles
-    float4* s_T = s_tw + N2;                              // exp(2 pi i j/512)
-    float2* s_f = reinterpret_cast<float2*>(s_T + 512);   // the field, N1 rows of LD
+    float4* s_T = smem4;                                  // g exp(2 pi i j/512) of the current step
+    float2* s_fc = reinterpret_cast<float2*>(s_T + 512);  // column sub-FFT twiddles
+    float2* s_B = s_fc + N1;                              // six-step factors, [j][n2]
+    float2* s_tw = s_B + Qc * N2;                         // row sub-FFT twiddles
+    float2* s_f = s_tw + N2;                              // the field, N1 rows of LD
     float2* s_x = s_f + (size_t)N1 * LD;                  // exchange buffers
     __shared__ float red[64];
 
     SsfmState* st = a.state + blockIdx.x;
-    const int log2N = a.log2N2 + ilog2c(N1);
-    for (int i = threadIdx.x; i < N1; i += kBlockThreads) s_fc[i] = a.tw[i];
-    for (int i = threadIdx.x; i < N2; i += kBlockThreads) s_tw[i] = a.tw[N1 + i];
-    for (int i = threadIdx.x; i < 512; i += kBlockThreads) s_T[i] = a.tw[2 * N1 + 2 * N2 + i];
+    for (int i = threadIdx.x; i < N1; i += kBlockThreads) s_fc[i] = a.tw.col[i];
+    for (int i = threadIdx.x; i < N2; i += kBlockThreads) s_tw[i] = a.tw.row[i];
     for (int i = threadIdx.x; i < Qc * N2; i += kBlockThreads)
-        s_B[i] = sixstep_factor((i % N2) * a1 * (i / N2), log2N);
+        s_B[i] = sixstep_column<N1>(i / N2, i % N2, a.log2N2);
     float4* g4 = reinterpret_cast<float4*>(a.data + (size_t)blockIdx.x * N);
     float4* f4 = reinterpret_cast<float4*>(s_f);
     for (int i = threadIdx.x; i < N / 2; i += kBlockThreads) f4[(i / (N2 / 2)) * (LD / 2) + i % (N2 / 2)] = g4[i];
@@ -769,7 +839,9 @@ __global__ void __launch_bounds__(kBlockThreads, BlockShape<N1, N2>::SMEM <= 113
         if (*(volatile const int*)&st->row_active) {
             const float g = *(volatile const float*)&st->lin_gain;
             const unsigned long long dhi = *(volatile const unsigned long long*)&st->disp_hi;
-            const unsigned long long dlo = *(volatile const unsigned long long*)&st->disp_lo << 32;
+            const unsigned long long dlo = *(volatile const unsigned long long*)&st->disp_lo;
+            // the step's rotation table; row_work synchronizes before its first use
+            for (int i = threadIdx.x; i < 512; i += kBlockThreads) s_T[i] = scale_df(a.tw.turn[i], g);
             for (int rb = 0; rb < N1 / RPI; ++rb) {
                 row_work<N2>(a, ROW_SSFM, s_f, rb * RPI + rl, rl, t, s_tw, s_T, s_x, g, dhi, dlo, LD);
                 __syncthreads();
@@ -790,19 +862,6 @@ struct Launch {
     int threads = 0, per_block = 0;
     size_t smem = 0;
     bool attr_set = false;
-};
-
-// Row-pass rows per block: must divide N1 (N1 >= max(16, N2/2) for every plan).
-template <int N2>
-struct RowShape {
-    static constexpr int P = PQ<N2>::P;
-    static constexpr int R0 = 256 / P;
-    static constexpr int RH = (N2 / 2 > 16 ? N2 / 2 : 16);
-    static constexpr int R = R0 < RH ? R0 : RH;
-    // 64-thread CTAs: when a launch has fewer row blocks than the GPU has SMs
-    // (a single field of 2^17 samples at a 128 x 1024 split has 16), four
-    // times as many SMs take part.
-    static constexpr int RN = 64 / P;
 };
 
 Launch col_launch_for(int log2N1);

@@ -508,7 +508,7 @@ FOCSS_API focss_status focss_cnn_adam_step(focss_cnn* model, double lr, double b
  * `data` is the caller's device buffer of batch*samples complex64
  * (interleaved float pairs), propagated in place on `stream` (a
  * cudaStream_t; NULL = legacy default stream).  The library allocates
- * nothing: step state and twiddle tables live in one fixed 59 KB
+ * nothing: step state and twiddle tables live in one fixed 52 KB
  * __device__ array per device, held until the process exits.
  * Limits: samples a power of two in [2^8, 2^17], batch <= 256; larger shapes
  * return FOCSS_ERR_UNSUPPORTED before any GPU work.  Single-mode fields only.
