@@ -335,28 +335,24 @@ __host__ __device__ __forceinline__ int col_kc(int L) {
 
 // ---------------------------------------------------------------------------
 // v * exp(2 pi i x) for a 64-bit fixed-point turn fraction, given as
-// Y = 2^64 x + 2^54 (the 2^54 rounds the table index to nearest): w = v * T[j],
-// T[j] = exp(2 pi i j/512) (times the linear step's gain) as double-float
-// {re_hi, im_hi, re_lo, im_lo} in a compensated product, then
-// w + w * (cos(theta) - 1 + i sin(theta)) for the residual |theta| <= pi/512,
-// whose angle is carried as the exact split th + tl.
+// Y = 2^64 x + 2^54 (the 2^54 rounds the table index to nearest).  T[j] =
+// exp(2 pi i j/512) (times the linear step's gain) is a double-float table
+// {re_hi, im_hi, re_lo, im_lo}; the residual rotation theta = 2 pi r, |theta| <=
+// pi/512, goes into the low words, T (cos theta - 1 + i sin theta) + T_lo, which
+// are at most 6e-3 and so carry it to ~2e-10 in FP32; one compensated product
+// then rotates the data.
 __device__ __forceinline__ float2 turns_rotate(float2 v, unsigned long long Y, const float4* __restrict__ T512) {
     const unsigned yh = (unsigned)(Y >> 32);
-    const int j = (int)(yh >> 23);
-    // r + 2^54 = A 2^32 + B 2^9 + (9 dropped bits, < 2e-16 rad), A, B < 2^23
-    const float fA = __int_as_float(0x4B000000u | (yh & 0x7FFFFFu)) - (8388608.0f + 4194304.0f);  // exact
-    const float fB = __int_as_float(0x4B000000u | ((unsigned)Y >> 9)) - 8388608.0f;
-    const float c32_hi = 1.462918119976564e-09f, c32_lo = -4.070940267922164e-17f;  // 2 pi / 2^32
-    const float c9 = 1.7439342975337076e-16f;                                       // 2 pi / 2^55
-    const float th = fA * c32_hi;
-    const float tl = fmaf(fB, c9, fmaf(fA, c32_lo, fmaf(fA, c32_hi, -th)));
+    const float4 t = T512[yh >> 23];
+    // 32 bits of the residual below the table index, in units of 2^-41 turn
+    const int r = (int)((unsigned)(Y >> 23) ^ 0x80000000u);
+    const float th = (float)r * 2.857261873568671e-12f;  // 2 pi / 2^41
     const float th2 = th * th;
-    const float sl = fmaf(th2 * th, -1.0f / 6.0f, tl);       // sin = th + sl (theta^5/120 < 8e-14)
-    const float cm1 = th2 * fmaf(th2, 1.0f / 24.0f, -0.5f);  // cos - 1 (th tl < 2e-12, its rounding 1e-12)
-    const float2 w = cmul_df(v, T512[j]);
-    const float re = w.x + fmaf(-w.y, th, fmaf(w.x, cm1, -(w.y * sl)));
-    const float im = w.y + fmaf(w.x, th, fmaf(w.y, cm1, w.x * sl));
-    return make_float2(re, im);
+    const float s = fmaf(th * th2, -1.0f / 6.0f, th);
+    const float cm1 = th2 * fmaf(th2, 1.0f / 24.0f, -0.5f);
+    const float lr = fmaf(t.x, cm1, fmaf(-t.y, s, t.z));
+    const float li = fmaf(t.y, cm1, fmaf(t.x, s, t.w));
+    return cmul_df(v, make_float4(t.x, t.y, lr, li));
 }
 
 // A double-float table entry times an FP32 gain, renormalized.
