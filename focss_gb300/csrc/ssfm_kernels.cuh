@@ -571,20 +571,27 @@ __device__ __forceinline__ void row_tables(const PassArgs& a, bool ssfm, float g
 }
 
 // Row-pass rows per block: must divide N1 (N1 >= max(16, N2/2) for every plan).
+// 128-thread CTAs, four per SM, start and finish more staggered than two of
+// 256 and overlap one's loads with the others' work (row pass of 16 x 2^17
+// 16.4 -> 15.5 us, 64 x 2^15 16.0 -> 14.2 us); at N2 = 1024 the tables a CTA
+// loads (16 KB) cost more than that gains (126 x 2^19: 300 us with 256 threads,
+// 341 us with 128).
 template <int N2>
 struct RowShape {
     static constexpr int P = PQ<N2>::P;
-    static constexpr int R0 = 256 / P;
+    static constexpr int R0 = (N2 >= 1024 ? 256 : 128) / P;
     static constexpr int RH = (N2 / 2 > 16 ? N2 / 2 : 16);
     static constexpr int R = R0 < RH ? R0 : RH;
     // 64-thread CTAs: when a launch has fewer row blocks than the GPU has SMs
     // (a single field of 2^17 samples at a 128 x 1024 split has 16), four
     // times as many SMs take part.
     static constexpr int RN = 64 / P;
+    // CTAs of r rows per SM the register budget (128 at 512 threads) is sized for
+    static constexpr int min_blocks(int r) { return r == RN ? 2 : (512 / (r * P) > 2 ? 512 / (r * P) : 2); }
 };
 
 template <int N2, int R>
-__global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel(const PassArgs a) {
+__global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row_kernel(const PassArgs a) {
     constexpr int P = PQ<N2>::P;
     extern __shared__ float4 smem4[];
     float4* s_T = smem4;                                     // g exp(2 pi i j/512)
