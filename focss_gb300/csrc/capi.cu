@@ -261,6 +261,7 @@ FOCSS_API focss_status focss_ctx_destroy(focss_ctx* c) {
     for (cudaEvent_t e : c->prof_events) cudaEventDestroy(e);
     for (auto& kv : c->tables) cudaFree(kv.second);
     fg::free_loop_graphs(c);
+    fg::free_term_cache(c->terms);
     cudaFree(c->d_state);
     cudaFree(c->d_counters);
     cudaFree(c->d_red);

@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "tcgen05.cuh"
 #include "tma_map.h"
 
 namespace fg {
@@ -60,7 +61,7 @@ __device__ __forceinline__ uint32_t pack2(bf16 lo, bf16 hi) {
 namespace tc {
 constexpr int M = 128, ROWS = M + 2 * HALF;
 constexpr uint32_t SBO = 128;
-constexpr long long kWaitCap = 1ll << 22;  // mbarrier polls before giving up
+using namespace tcg;
 
 constexpr int STAGES = 4;                  // activation tiles in flight per CTA
 constexpr int FWD_THREADS = 320;           // producer, MMA, two groups of four epilogue warps
@@ -80,13 +81,7 @@ struct Shape {
     static constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;           // two: a power of two >= 32
 };
 
-// Shared-memory matrix descriptor: start address, LBO and SBO in 16-byte
-// units, the descriptor version 1 at bit 46, base offset 0, no swizzling.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
-           (1ull << 46);
-}
-// The same for a K-major operand in the 128-byte swizzled layout (TMA
+// smem_desc for a K-major operand in the 128-byte swizzled layout (TMA
 // CU_TENSOR_MAP_SWIZZLE_128B): rows of 128 bytes, 8-row groups SBO = 1024 B
 // apart, swizzling mode 2 at bit 61; LBO is not used (encoded 1).  `addr`
 // must be 1024-byte aligned (base offset 0).
@@ -101,82 +96,13 @@ __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-// Waits for the phase of parity `parity` of `bar`, at most kWaitCap polls.
-// Gives up early when *abort is set, and sets it when the polls run out.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity, volatile int* abort) {
-    const uint32_t a = smem_addr(bar);
-    for (long long it = 0; it < kWaitCap; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (abort && *abort) return false;
-    }
-    if (abort) *abort = 1;
-    return false;
-}
-// D (tensor memory) = A B (+ D when `accumulate`), kind::f16, one CTA.
-__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate));
-}
-// Arrives on `bar` once every tcgen05 operation this thread issued so far completes.
-__device__ __forceinline__ void mma_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_addr(bar))
-                 : "memory");
-}
 constexpr int FWD_EPI = FWD_THREADS - 64;  // epilogue threads
-
-// TMA tensor copy of one box at (x, y, z) of a 3-D tensor map into shared
-// memory, completing on `bar` (x * element size must be a multiple of 16 bytes).
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z,
-                                            unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];\n" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
-        : "memory");
-}
 
 // 16-byte asynchronous copy global -> shared; `bytes` = 0 writes zeros.
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// tcgen05.ld of 16 columns without the wait; wait_ld then waits for every
-// load in flight and ties these registers to the wait, so that no use of
-// them can be scheduled before it.
-__device__ __forceinline__ void ld_x16_async(uint32_t taddr, uint32_t (&u)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
-          "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void wait_ld(uint32_t (&u)[16]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
-                 : "+r"(u[0]), "+r"(u[1]), "+r"(u[2]), "+r"(u[3]), "+r"(u[4]), "+r"(u[5]), "+r"(u[6]), "+r"(u[7]),
-                   "+r"(u[8]), "+r"(u[9]), "+r"(u[10]), "+r"(u[11]), "+r"(u[12]), "+r"(u[13]), "+r"(u[14]), "+r"(u[15])
-                 :
-                 : "memory");
-}
 __device__ __forceinline__ void ld_x16(uint32_t taddr, float (&r)[16]) {
     uint32_t u[16];
     asm volatile(
@@ -310,7 +236,7 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
                     for (int kk = 0; kk < KW; ++kk)
 #pragma unroll
                         for (int kc = 0; kc < CIN / 16; ++kc)
-                            tc::mma_bf16(d, adesc + (uint64_t)((kk * 128 + kc * 32) >> 4),
+                            tc::mma_f16(d, adesc + (uint64_t)((kk * 128 + kc * 32) >> 4),
                                          bdesc + (uint64_t)(((kk * KG + kc * 2) * S::LBO_B) >> 4), tc::idesc(COUT),
                                          (kk | kc) != 0);
                 } else {
@@ -319,7 +245,7 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
                     for (int kk = 0; kk < KW; ++kk)
 #pragma unroll
                         for (int kc = 0; kc < CIN / 16; ++kc)  // 16 input channels = 2 K core matrices per MMA
-                            tc::mma_bf16(d, adesc + (uint64_t)((kk * 16 + kc * 2 * S::LBO_A) >> 4),
+                            tc::mma_f16(d, adesc + (uint64_t)((kk * 16 + kc * 2 * S::LBO_A) >> 4),
                                          bdesc + (uint64_t)(((kk * KG + kc * 2) * S::LBO_B) >> 4), tc::idesc(COUT),
                                          (kk | kc) != 0);
                 }
@@ -523,7 +449,7 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(const __grid_constan
                 for (int ks = 0; ks < tcw::P / 16; ++ks) {  // 16 positions = 2 K core matrices per MMA
                     const uint64_t gd = tc::smem_desc(gb + ks * 2 * tcw::LBO, tcw::LBO, tcw::P * 16);
                     const uint64_t id = tc::smem_desc(ib + kk * 16 + ks * 2 * tcw::LBO, tcw::LBO, tcw::PR * 16);
-                    tc::mma_bf16(tmem + (uint32_t)(S::NC * j), S::G_IS_A ? gd : id, S::G_IS_A ? id : gd, S::IDESC,
+                    tc::mma_f16(tmem + (uint32_t)(S::NC * j), S::G_IS_A ? gd : id, S::G_IS_A ? id : gd, S::IDESC,
                                  (t | ks) != 0);
                 }
             }

@@ -114,6 +114,7 @@ struct Plan {
 };
 
 struct LoopGraph;  // span_loop.cu
+struct TermCache;  // triplet.cu
 
 struct Ctx {
     int device = 0;
@@ -141,6 +142,7 @@ struct Ctx {
     // split-step FFT split (log2 N1) per length picked by the autotuner or
     // pinned by the caller; lengths absent here use the balanced split
     std::map<int, int> ssfm_split;
+    TermCache* terms = nullptr;      // device tables of recent triplet term lists
     int staging = 0;                 // FOCSS_STAGING_* for new plans (focss_set_pass_staging)
     // instantiated span-loop graphs keyed by shape and parameters, and the
     // streams/events their capture uses (span_loop.cu)
@@ -218,6 +220,7 @@ bool amplifier_coeffs(int op, double gain, double noise_factor, double f0, doubl
                       double* sigma);
 
 // ---- triplet.cu
+void free_term_cache(TermCache* t);
 // Triplet sum over `modes` consecutive rows of each realization of `in`
 // (realizations in_bstride apart) into out (batch x modes x samples); with rx
 // the equalizer (rx - y) * inv_lw.

@@ -8,30 +8,33 @@
 // so box-shaped term sets (|m|, |n| <= R) are accepted as well as the
 // reference's diamond |m| + |n| <= R.
 //
-// Kernel: one CTA per tile of TK = T*NT consecutive outputs.  Terms are
-// grouped by m on the host into dense n-runs (zero-padded to multiples of T).
-// Per m the CTA hoists Q_m[j] = sum_p A_p[j] conj(A_p[j+m]) for the tile into
-// shared memory; each thread then owns T consecutive outputs and slides a
-// register window over Q_m along n, so one shared-memory load feeds T complex
-// multiply-adds (FP32 CUDA cores; the sum has no GEMM structure).  Shared
-// arrays use a padded index j + j/T so the per-thread stride T+1 is odd and
-// reads are conflict-free.
+// Terms are grouped by m on the host into dense n-runs, and outputs into tiles
+// of TK = 1024.  Per m a tile forms Q_m[j] = sum_p A_p[j] conj(A_p[j+m]) once;
+// S_m[k] = sum_n C_mn Q_m[k+n] is then a correlation with a fixed tap vector,
+// i.e. a product of the Hankel matrix Q_m[8 i + x] (k = 8 i + r) with a
+// Toeplitz matrix T_m[x][r] = C_m,nlo+x-r, and y += A[k+m] S_m[k].
+//
+// triplet_tc_kernel runs that product on the tensor cores in split FP16;
+// triplet_tile_fp32 is the same sum in FP32 on the CUDA cores, for tiles and
+// term lists outside the split's range (see use_tensor and the tile check).
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <cmath>
-#include <cstdio>
-#include <map>
-#include <mutex>
+#include <cstring>
+#include <list>
 #include <string>
 #include <vector>
 
 #include "common.cuh"
 #include "internal.h"
+#include "tcgen05.cuh"
 
 namespace fg {
 namespace {
 
-constexpr int TT = 8;     // outputs per thread and n-steps per window refill
-constexpr int NT = 128;   // threads per CTA
+constexpr int TT = 8;     // outputs per thread
+constexpr int NT = 128;   // threads of the FP32 sum
 constexpr int TK = TT * NT;
 
 __device__ __forceinline__ int padi(int j) { return j + (j >> 3); }
@@ -50,14 +53,51 @@ struct TripletArgs {
     const float2* coef;     // dense C_mn runs
     int halo_q;             // max |n| + TT over groups (Q range beyond the tile)
     int halo_a;             // halo_q + max |m| (A range beyond the tile)
+    // tensor cores
+    const int4* grp;        // {m, nlo, K steps of 16, byte offset into bmat} of each group
+    const unsigned char* bmat;  // Toeplitz matrices (toeplitz_kernel)
+    int a_lo, alen;         // the tile reads samples k0 + a_lo + [0, alen)
+    int qcap;               // elements of a Q array, a multiple of 8
+    int bslot;              // bytes of a Toeplitz buffer
+    float coef_unscale;     // 1 / (power-of-two scale of the matrices)
+    float2* part;           // splits > 1: partial sums, splits x batch x modes x N
+    int splits;
 };
 
+// Output o = sample k of a row: zero outside [radius, N - radius), and the equalizer.
+__device__ __forceinline__ void finish_output(const TripletArgs& a, size_t o, int k, float2 acc) {
+    float2 y = (k >= a.radius && k < a.samples - a.radius) ? acc : make_float2(0.f, 0.f);
+    if (a.rx) y = cmul(csub(a.rx[o], y), a.inv_lw);
+    a.out[o] = y;
+}
+__device__ __forceinline__ void write_output(const TripletArgs& a, int b, int modes, int p, int k, float2 acc) {
+    if (k >= a.samples) return;
+    const size_t o = ((size_t)b * modes + p) * a.samples + k;
+    if (a.splits > 1)
+        a.part[(size_t)blockIdx.z * gridDim.y * modes * a.samples + o] = acc;
+    else
+        finish_output(a, o, k, acc);
+}
+// Joins the partial sums of the splits in order.
+__global__ void triplet_join_kernel(const TripletArgs a, size_t n) {
+    for (size_t o = blockIdx.x * (size_t)blockDim.x + threadIdx.x; o < n; o += (size_t)gridDim.x * blockDim.x) {
+        float2 y = a.part[o];
+        for (int z = 1; z < a.splits; ++z) y = cadd(y, a.part[z * n + o]);
+        finish_output(a, o, (int)(o % a.samples), y);
+    }
+}
+
+// One tile in FP32, by NT threads: each owns TT consecutive outputs and slides
+// a register window over Q_m along n, so one shared-memory load feeds TT
+// complex multiply-adds.  Shared arrays use a padded index j + j/8 so the
+// per-thread stride is odd and reads are conflict-free.  Sums groups
+// [g0, g1).  Out of line: the tensor-core kernel calls it for single tiles.
+__device__ __forceinline__ void tile_sync() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
 template <int MODES>
-__global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
-    extern __shared__ float2 sh[];
+__device__ __noinline__ void triplet_tile_fp32(const TripletArgs& a, float2* sh, int k0, int g0, int g1) {
     const int N = a.samples;
     const int b = blockIdx.y;
-    const int k0 = blockIdx.x * TK;
+    tile_sync();  // the buffers are free (second tile of a CTA)
     const int alen = TK + 2 * a.halo_a;
     const int qlen = TK + 2 * a.halo_q;
     float2* As = sh;                           // MODES x padi(alen)
@@ -79,11 +119,11 @@ __global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
         for (int r = 0; r < TT; ++r) acc[p][r] = make_float2(0.f, 0.f);
 
     const int kl = threadIdx.x * TT;  // first local output of this thread
-    for (int g = 0; g < a.groups; ++g) {
+    for (int g = g0; g < g1; ++g) {
         const int m = a.g_m[g];
         const int nlo = a.g_nlo[g];
         const int off = a.g_off[g], len = a.g_off[g + 1] - off;
-        __syncthreads();  // previous Q consumed (and A tile ready on g = 0)
+        tile_sync();  // previous Q consumed (and A tile ready on the first)
         // Q tile: index i <-> j = k0 - halo_q + i
         for (int i = threadIdx.x; i < qlen; i += NT) {
             const int ia = i + (a.halo_a - a.halo_q);  // A index of j
@@ -93,7 +133,7 @@ __global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
                 q = cadd(q, cmulc(As[p * astride + padi(ia)], As[p * astride + padi(ia + m)]));
             Qs[padi(i)] = q;
         }
-        __syncthreads();
+        tile_sync();
         float2 s[TT];
 #pragma unroll
         for (int r = 0; r < TT; ++r) s[r] = make_float2(0.f, 0.f);
@@ -126,144 +166,531 @@ __global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
                 acc[p][r] = cadd(acc[p][r], cmul(As[p * astride + padi(kl + r + m + a.halo_a)], s[r]));
     }
 
-    const float2* rx = a.rx ? a.rx + (size_t)b * MODES * N : nullptr;
-    float2* out = a.out + (size_t)b * MODES * N;
 #pragma unroll
     for (int p = 0; p < MODES; ++p)
 #pragma unroll
-        for (int r = 0; r < TT; ++r) {
-            const int k = k0 + kl + r;
-            if (k >= N) continue;
-            const bool valid = k >= a.radius && k < N - a.radius;
-            float2 y = valid ? acc[p][r] : make_float2(0.f, 0.f);
-            if (rx) y = cmul(csub(rx[(size_t)p * N + k], y), a.inv_lw);
-            out[(size_t)p * N + k] = y;
+        for (int r = 0; r < TT; ++r) write_output(a, b, MODES, p, k0 + kl + r, acc[p][r]);
+}
+
+template <int MODES>
+__global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
+    extern __shared__ float2 sh[];
+    triplet_tile_fp32<MODES>(a, sh, blockIdx.x * TK, 0, a.groups);
+}
+
+// ---------------------------------------------------------------- tensor cores
+// S_m on tcgen05: for k = 16 i + r, A[i][x] = Q[16 i + x] (M = 128 rows, one of
+// Re Q / Im Q) and B the Toeplitz matrix B[x][r] = C_m,nlo+x-r (re and im
+// columns); Re Q B and Im Q B accumulate apart and join as a complex product
+// in the epilogue, so one B serves both.  Rows of the 32-byte-swizzled K-major
+// layout are 32 bytes = 16 FP16 values apart, exactly the Hankel row pitch, so
+// the (swizzled) array Q itself is the operand and a step of 16 taps is an
+// address offset.
+//
+// Precision.  Q and C are scaled by powers of two to at most 1 and split into
+// FP16 pairs hi + lo 2^-11 (22 bits, absolute error below 2^-36), and the
+// products hi hi, hi lo, lo hi accumulate in FP32, the last two in columns of
+// their own that join with the factor 2^-11 at the end; lo lo (2^-22 of a
+// product at most) is left out.  The sum over m is compensated (Kahan).  The
+// scale of Q is the tile's largest power; tiles whose power spans more than
+// 2^12 between its largest sample and the mean of its weakest 32-sample run,
+// or with non-finite values, take the FP32 sum.  Relative error against 64
+// bits at R = 75 on 2^20 symbols: 1.9e-7 .. 2.3e-7 (the FP32 sum 2.7e-7 ..
+// 4.2e-7 on the same inputs).
+//
+// One CTA per 2048 outputs and SM: warps 8-13 form and split Q_m (a thread of
+// them starts the bulk copy of the group's B matrix), warps 14 and 15 issue 4
+// MMAs per 16 taps, warps 0-7 read the accumulators back and add A[k+m] S_m.
+// What bounds it: shared-memory bandwidth.  An MMA reads 4 KB of A and 1 or 2
+// KB of B, ~44 cycles whatever its N, hence 16 outputs per row of A; forming
+// Q costs another ~660 cycles of it per group and the epilogue ~130, together
+// ~1900 of the ~2300 cycles a group of R = 75 takes.
+// R = 75 (11 389 terms) on 2^20 symbols: 0.69 ms = 141 TFLOP/s of the sum's 8
+// flops per term, where the FP32 kernel took 2.30 ms (42 TFLOP/s, 53 % of the
+// FP32 FMA peak); on the way 0.86 ms with 8 outputs per row of A, 0.82 ms
+// with one thread issuing from divergent code, 0.75 ms with one issuing warp.
+constexpr int TC_ROW = 16;                // outputs per row of A
+constexpr int TC_K = NT * TC_ROW;         // outputs per CTA
+constexpr int TC_THREADS = 512;
+constexpr int kSt = 4;                    // groups in flight: Q buffers and accumulators
+constexpr int kEpiWarps = 8, kProdWarps = 6;
+constexpr int kPairs = 2 * 32 * kProdWarps, kBatch = 3;
+constexpr int kMaxKSteps = 14;            // taps per group: 16 * kMaxKSteps - 15
+constexpr int kMaxTcGroups = 512;
+constexpr uint32_t kDCols = 128;          // FP32 columns: (Re Q | Im Q) x (hi hi | mixed) x C re/im x 16 r
+constexpr uint32_t kStepBytes = 2048;     // B bytes per 16 taps: 2 x 64 rows x 16 bytes
+// kind::f16, FP32 accumulator (bits 4-5 = 1), FP16 operands, both K-major
+__host__ __device__ constexpr uint32_t tri_idesc(int n) {
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(NT >> 4) << 24);
+}
+__device__ __forceinline__ int padt(int j) { return j + (j >> 4); }
+// Byte offset `o` in the 32-byte-swizzled layout: 16-byte chunks swapped in
+// every other 128 bytes (address bit 4 ^= bit 7).
+__device__ __forceinline__ uint32_t swz32(uint32_t o) { return o ^ ((o >> 3) & 0x10u); }
+
+template <int MODES>
+__global__ void __launch_bounds__(TC_THREADS, 1) triplet_tc_kernel(const TripletArgs a) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) unsigned long long full[kSt], done[kSt], bfull[kSt], drain[2];
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int abort_flag;
+    __shared__ unsigned s_max, s_min;
+    __shared__ int s_bad;
+    // kSt buffers of {re hi, im hi, re lo, im lo}, each 2 qcap bytes, on a
+    // 1024-byte boundary (the swizzle follows absolute address bits)
+    unsigned char* Qs = sm + ((1024u - (tcg::smem_addr(sm) & 1023u)) & 1023u);
+    unsigned char* Bs = Qs + (size_t)kSt * 8 * a.qcap;                     // kSt buffers of B
+    int4* s_grp = reinterpret_cast<int4*>(Bs + (size_t)kSt * a.bslot);
+    float2* As = reinterpret_cast<float2*>(s_grp + a.groups);              // MODES x padt(alen)
+    const int astride = padt(a.alen) + 1;
+    const int N = a.samples, b = blockIdx.y, k0 = blockIdx.x * TC_K;
+    const int g0 = (int)((long long)a.groups * blockIdx.z / a.splits);
+    const int g1 = (int)((long long)a.groups * (blockIdx.z + 1) / a.splits), ng = g1 - g0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        s_max = 0u;
+        s_min = 0x7F7FFFFFu;
+        s_bad = 0;
+        for (int i = 0; i < kSt; ++i) {
+            tcg::mbar_init(&full[i], kProdWarps + kEpiWarps);
+            tcg::mbar_init(&done[i], 1);
+            tcg::mbar_init(&bfull[i], 1);
         }
+        tcg::mbar_init(&drain[0], 1);
+        tcg::mbar_init(&drain[1], 1);
+        tcg::fence_mbar_init();
+    }
+    __syncthreads();
+    // A tile (zero outside [0, N)), its largest sample power and the smallest
+    // non-zero power of a run of 32
+    {
+        const float2* in = a.in + (size_t)b * a.in_bstride;
+        float mx = 0.f, mn = 3.4e38f;
+        bool bad = false;
+        for (int i0 = warp * 32; i0 < a.alen; i0 += TC_THREADS) {
+            const int i = i0 + lane, s = k0 + a.a_lo + i;
+            float pw = 0.f;
+#pragma unroll
+            for (int p = 0; p < MODES; ++p) {
+                const float2 v = (i < a.alen && s >= 0 && s < N) ? in[(size_t)p * N + s] : make_float2(0.f, 0.f);
+                if (i < a.alen) As[p * astride + padt(i)] = v;
+                pw += cnorm(v);
+            }
+            const float sum = warp_sum(pw);
+            bad = bad || !(sum <= 1e30f);
+            if (sum > 0.f) mn = fminf(mn, sum);
+            mx = fmaxf(mx, pw);
+        }
+        mx = warp_max(mx);
+        if (lane == 0) {
+            atomicMax(&s_max, __float_as_uint(mx));
+            atomicMin(&s_min, __float_as_uint(mn));
+            if (bad) s_bad = 1;
+        }
+        for (int g = threadIdx.x; g < a.groups; g += TC_THREADS) s_grp[g] = a.grp[g];
+    }
+    __syncthreads();
+    const float pmax = __uint_as_float(s_max), pmin = __uint_as_float(s_min);
+    if (s_bad || (pmax > 0.f && (!(pmax > 1e-30f) || pmax > 128.f * pmin))) {  // 2^12 over the run's mean
+        if (threadIdx.x < NT)
+            for (int k = k0; k < k0 + TC_K && k < N; k += TK)
+                triplet_tile_fp32<MODES>(a, reinterpret_cast<float2*>(sm), k, g0, g1);
+        return;
+    }
+    // |Q| <= pmax < 2^e: scale by 2^-e
+    const int e = pmax > 0.f ? (int)((__float_as_uint(pmax) >> 23) & 255u) - 126 : 0;
+    const float qscale = __uint_as_float((unsigned)(127 - e) << 23);
+    if (warp == 14) tcg::tmem_alloc(&tmem_base, kSt * kDCols);
+    tcg::fence_before_sync();
+    __syncthreads();
+    tcg::fence_after_sync();
+    const uint32_t tmem = tmem_base;
+
+    // epilogue threads: row 32 (warp & 3) + lane, outputs 8 (warp >> 2) .. + 7 of it
+    const int kl = (32 * (warp & 3) + lane) * TC_ROW + TT * (warp >> 2);
+    float2 acc[MODES][TT], low[MODES][TT];  // sum and its compensation
+#pragma unroll
+    for (int p = 0; p < MODES; ++p)
+#pragma unroll
+        for (int r = 0; r < TT; ++r) acc[p][r] = low[p][r] = make_float2(0.f, 0.f);
+    int loads = 0;                          // loader: groups whose copy was queued
+    if (warp < 8) {
+        const uint32_t t0 = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(TT * (warp >> 2));
+        if (lane == 0)
+            for (int i = 0; i < kSt; ++i) tcg::mbar_arrive(&full[i]);  // every accumulator is free
+        for (int i = 0; i < ng; ++i) {
+            const int st = i % kSt, m = s_grp[g0 + i].x;
+            if (!tcg::mbar_wait(&done[st], (i / kSt) & 1, &abort_flag)) break;
+            tcg::fence_after_sync();
+            const uint32_t t = t0 + (uint32_t)st * kDCols;
+            float2 sv[TT];  // S_m of the thread's outputs
+            {
+                // Re S = Re Q Re C - Im Q Im C
+                uint32_t h0[8], l0[8], h1[8], l1[8];
+                tcg::ld_x8_async(t, h0);
+                tcg::ld_x8_async(t + 32, l0);
+                tcg::ld_x8_async(t + 80, h1);
+                tcg::ld_x8_async(t + 112, l1);
+                tcg::wait_ld8(h0, l0, h1, l1);
+#pragma unroll
+                for (int r = 0; r < TT; ++r)
+                    sv[r].x = fmaf(__uint_as_float(l0[r]) - __uint_as_float(l1[r]), 0x1p-11f,
+                                   __uint_as_float(h0[r]) - __uint_as_float(h1[r]));
+            }
+            {
+                // Im S = Re Q Im C + Im Q Re C
+                uint32_t h0[8], l0[8], h1[8], l1[8];
+                tcg::ld_x8_async(t + 16, h0);
+                tcg::ld_x8_async(t + 48, l0);
+                tcg::ld_x8_async(t + 64, h1);
+                tcg::ld_x8_async(t + 96, l1);
+                tcg::wait_ld8(h0, l0, h1, l1);
+#pragma unroll
+                for (int r = 0; r < TT; ++r)
+                    sv[r].y = fmaf(__uint_as_float(l0[r]) + __uint_as_float(l1[r]), 0x1p-11f,
+                                   __uint_as_float(h0[r]) + __uint_as_float(h1[r]));
+            }
+            tcg::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tcg::mbar_arrive(&full[st]);
+            const int ia = kl + m - a.a_lo;
+#pragma unroll
+            for (int r = 0; r < TT; ++r) {
+#pragma unroll
+                for (int p = 0; p < MODES; ++p) {
+                    const float2 x = cmul(As[p * astride + padt(ia + r)], sv[r]);
+                    const float2 sum = cadd(acc[p][r], x);
+                    low[p][r] = cadd(low[p][r], csub(x, csub(sum, acc[p][r])));
+                    acc[p][r] = sum;
+                }
+            }
+        }
+    } else if (warp < 14) {
+        const int pt = threadIdx.x - 256;
+        for (int i = 0; i < ng; ++i) {
+            const int st = i % kSt;
+            const int4 G = s_grp[g0 + i];
+            if (i >= kSt && !tcg::mbar_wait(&done[st], (i / kSt - 1) & 1, &abort_flag)) break;
+            if (threadIdx.x == 256) {
+                const uint32_t bytes = kStepBytes * G.z;
+                tcg::mbar_expect_tx(&bfull[st], bytes);
+                tcg::bulk_load(tcg::smem_addr(Bs) + (uint32_t)st * a.bslot, a.bmat + G.w, bytes, &bfull[st]);
+                loads = i + 1;
+            }
+            unsigned char* q = Qs + (size_t)st * 8 * a.qcap;
+            const int len = 16 * G.z + TC_K - 16, m = G.x;
+            // pairs el, el + 1; kBatch pairs of a thread in flight at a time
+            // (a pair alone waits out the latency of its loads and conversions)
+            for (int e0 = 2 * pt; e0 < len; e0 += kBatch * kPairs) {
+                float2 q0[kBatch], q1[kBatch];
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) q0[u] = q1[u] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int p = 0; p < MODES; ++p) {
+                    const float2* A = As + p * astride;
+                    float2 x0[kBatch], x1[kBatch], y0[kBatch], y1[kBatch];
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        const int ia = G.y - a.a_lo + min(e0 + u * kPairs, len - 2);
+                        x0[u] = A[padt(ia)];
+                        x1[u] = A[padt(ia + 1)];
+                        y0[u] = A[padt(ia + m)];
+                        y1[u] = A[padt(ia + 1 + m)];
+                    }
+#pragma unroll
+                    for (int u = 0; u < kBatch; ++u) {
+                        q0[u].x = fmaf(x0[u].x, y0[u].x, fmaf(x0[u].y, y0[u].y, q0[u].x));
+                        q0[u].y = fmaf(x0[u].y, y0[u].x, fmaf(-x0[u].x, y0[u].y, q0[u].y));
+                        q1[u].x = fmaf(x1[u].x, y1[u].x, fmaf(x1[u].y, y1[u].y, q1[u].x));
+                        q1[u].y = fmaf(x1[u].y, y1[u].x, fmaf(-x1[u].x, y1[u].y, q1[u].y));
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    const int el = e0 + u * kPairs;
+                    const float2 re = make_float2(q0[u].x * qscale, q1[u].x * qscale);
+                    const float2 im = make_float2(q0[u].y * qscale, q1[u].y * qscale);
+                    const __half2 rh = __floats2half2_rn(re.x, re.y), ih = __floats2half2_rn(im.x, im.y);
+                    const float2 rf = __half22float2(rh), jf = __half22float2(ih);
+                    const __half2 rl = __floats2half2_rn((re.x - rf.x) * 2048.f, (re.y - rf.y) * 2048.f);
+                    const __half2 il = __floats2half2_rn((im.x - jf.x) * 2048.f, (im.y - jf.y) * 2048.f);
+                    if (el < len) {
+                        unsigned char* w = q + swz32(2u * el);
+                        *reinterpret_cast<__half2*>(w) = rh;
+                        *reinterpret_cast<__half2*>(w + 2 * a.qcap) = ih;
+                        *reinterpret_cast<__half2*>(w + 4 * a.qcap) = rl;
+                        *reinterpret_cast<__half2*>(w + 6 * a.qcap) = il;
+                    }
+                }
+            }
+            // warp 8 also vouches for the group's B copy, so that the issuing
+            // warp has one barrier per group to look at
+            if (warp == 8 && !tcg::mbar_wait(&bfull[st], (i / kSt) & 1, &abort_flag)) break;
+            tcg::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) tcg::mbar_arrive(&full[st]);
+        }
+    } else {
+        // Two issuing warps take turns: a single one gets an MMA out every ~70
+        // cycles, where its operands need 48 of shared-memory bandwidth.  A
+        // look at a barrier takes ~250 cycles even when its phase is over, so
+        // the warp's next barrier is looked at between this group's MMAs.
+        int i = warp - 14;
+        bool ready = i < ng && tcg::mbar_wait_warp(&full[i], 0, &abort_flag);
+        for (; i < ng && ready; i += 2) {
+            const int st = i % kSt;
+            const int ks = __shfl_sync(0xffffffffu, s_grp[g0 + i].z, 0);
+            tcg::fence_after_sync();
+            const uint32_t d = tmem + (uint32_t)st * kDCols;
+            // A: the four Q arrays; B: 1024 bytes (64 rows) per 8 taps,
+            // rows 0-31 the hi words, 32-63 the lo words
+            const uint32_t qa = tcg::smem_addr(Qs) + (uint32_t)st * 8u * a.qcap, qn = 2u * a.qcap;
+            uint64_t arh = tcg::smem_desc_sw32(qa), aih = tcg::smem_desc_sw32(qa + qn);
+            uint64_t arl = tcg::smem_desc_sw32(qa + 2 * qn), ail = tcg::smem_desc_sw32(qa + 3 * qn);
+            uint64_t bd = tcg::smem_desc(tcg::smem_addr(Bs) + (uint32_t)st * a.bslot, 1024, 128);
+            for (int k = 0; k < ks; ++k) {
+                tcg::mma_f16_warp(d, arh, bd, tri_idesc(64), k != 0);
+                tcg::mma_f16_warp(d + 64, aih, bd, tri_idesc(64), k != 0);
+                tcg::mma_f16_warp(d + 32, arl, bd, tri_idesc(32), true);
+                tcg::mma_f16_warp(d + 96, ail, bd, tri_idesc(32), true);
+                arh += 2;  // 16 taps: 32 bytes along Q, 2048 along B
+                aih += 2;
+                arl += 2;
+                ail += 2;
+                bd += 128;
+                if (k == (ks - 1) / 2 && i + 2 < ng)
+                    ready = tcg::mbar_wait_warp(&full[(i + 2) % kSt], ((i + 2) / kSt) & 1, &abort_flag);
+            }
+            tcg::mma_commit_warp(&done[st]);
+        }
+    }
+    __syncthreads();
+    const bool ok = !abort_flag;
+    if (!ok) {
+        // a wait ran out: the queued copies and MMAs land before the CTA
+        // leaves (bounded again), and the tile is marked invalid
+        if (threadIdx.x == 256)
+            for (int i = loads > kSt ? loads - kSt : 0; i < loads; ++i)
+                tcg::mbar_wait(&bfull[i % kSt], (i / kSt) & 1, nullptr);
+        if (warp >= 14) {
+            tcg::mma_commit_warp(&drain[warp - 14]);
+            tcg::mbar_wait_warp(&drain[warp - 14], 0, nullptr);
+        }
+        __syncthreads();
+    }
+    if (warp < 8) {
+        const float un = ok ? a.coef_unscale : __int_as_float(0x7fc00000);
+        const float uq = __uint_as_float((unsigned)(127 + e) << 23);
+#pragma unroll
+        for (int p = 0; p < MODES; ++p)
+#pragma unroll
+            for (int r = 0; r < TT; ++r) write_output(a, b, MODES, p, k0 + kl + r, cscale(cscale(cadd(acc[p][r], low[p][r]), uq), un));
+    }
+    tcg::fence_before_sync();
+    __syncthreads();
+    tcg::fence_after_sync();
+    if (warp == 14) tcg::tmem_free(tmem, kSt * kDCols);
 }
 
 struct Terms {
-    std::vector<int> gm, gnlo, goff;
+    std::vector<int> gm, gnlo, goff, len;  // len: taps of a run before its padding
     std::vector<float2> coef;
     int halo_q = 0, halo_a = 0;
+    // tensor cores (empty grp: outside its range)
+    std::vector<int4> grp;
+    size_t bmat_bytes = 0;
+    int a_lo = 0, a_hi = 0, ksteps = 0;
+    float unscale = 1.f;
 };
 
-bool build_terms(int n_terms, const int32_t* m, const int32_t* n, const double* c, Terms& t) {
-    std::map<int, std::map<int, std::pair<double, double>>> by_m;
-    for (int i = 0; i < n_terms; ++i) {
-        auto& slot = by_m[m[i]][n[i]];
-        slot.first += c[2 * i];
-        slot.second += c[2 * i + 1];
+// Toeplitz matrices of the groups in B's shared-memory layout, FP16: each
+// 8-tap chunk holds 64 rows of 16 bytes, rows r / 16 + r = the real /
+// imaginary output r, rows 32.. the same in the lo words.  One CTA per group.
+__global__ void toeplitz_kernel(const float2* __restrict__ coef, const int* __restrict__ off, const int4* __restrict__ grp,
+                                const int* __restrict__ len, float scale, __half* __restrict__ bmat) {
+    const int g = blockIdx.x, ks = grp[g].z, taps = len[g];
+    const float2* c = coef + off[g];
+    __half* b = bmat + grp[g].w / 2;
+    for (int i = threadIdx.x; i < ks * 1024; i += blockDim.x) {
+        const int x = (i >> 9) * 8 + (i & 7), row = (i >> 3) & 63, r = row & 15;
+        const int d = x - r;
+        float v = 0.f;
+        if (d >= 0 && d < taps) v = ((row >> 4) & 1 ? c[d].y : c[d].x) * scale;
+        const __half hi = __float2half_rn(v);
+        b[i] = row < 32 ? hi : __float2half_rn((v - __half2float(hi)) * 2048.f);
     }
+}
+
+// Groups of the tensor-core sum.  Left empty when a run has
+// more than 16 kMaxKSteps - 15 taps, there are more than kMaxTcGroups groups
+// or the coefficients' magnitude leaves [2^-100, 2^100].
+void plan_tensor(Terms& t) {
+    float cmax = 0.f;
+    for (const float2& c : t.coef) {
+        if (!std::isfinite(c.x) || !std::isfinite(c.y)) return;
+        cmax = std::max({cmax, std::fabs(c.x), std::fabs(c.y)});
+    }
+    if (!(cmax > 0x1p-100f && cmax < 0x1p100f) || (int)t.gm.size() > kMaxTcGroups) return;
+    for (int l : t.len)
+        if (l + 15 > 16 * kMaxKSteps) return;
+    int ex = 0;
+    std::frexp(cmax, &ex);
+    t.unscale = std::ldexp(1.f, ex);
+    t.a_lo = 0;
+    t.a_hi = TC_K;
+    for (size_t g = 0; g < t.gm.size(); ++g) {
+        const int ks = (t.len[g] + 15 + 15) / 16, m = t.gm[g], nlo = t.gnlo[g];
+        t.grp.push_back(make_int4(m, nlo, ks, (int)t.bmat_bytes));
+        t.bmat_bytes += kStepBytes * (size_t)ks;
+        t.ksteps = std::max(t.ksteps, ks);
+        t.a_lo = std::min({t.a_lo, m, nlo, nlo + m});
+        t.a_hi = std::max({t.a_hi, TC_K + m, nlo + 16 * ks + TC_K - 16, nlo + m + 16 * ks + TC_K - 16});
+    }
+}
+
+// Terms sorted by (m, n) through an index array (duplicates add in list order).
+void build_terms(int n_terms, const int32_t* m, const int32_t* n, const double* c, Terms& t) {
+    std::vector<int> at(n_terms);
+    for (int i = 0; i < n_terms; ++i) at[i] = i;
+    auto before = [&](int i, int j) { return m[i] != m[j] ? m[i] < m[j] : n[i] < n[j]; };
+    if (!std::is_sorted(at.begin(), at.end(), before)) std::stable_sort(at.begin(), at.end(), before);
     int max_n = 0, max_m = 0;
     t.goff.push_back(0);
-    for (auto& kv : by_m) {
-        const int mm = kv.first;
-        const int nlo = kv.second.begin()->first, nhi = kv.second.rbegin()->first;
-        int len = nhi - nlo + 1;
-        len = (len + TT - 1) / TT * TT;
+    for (int i = 0; i < n_terms;) {
+        int e = i;
+        const int mm = m[at[i]], nlo = n[at[i]];
+        while (e < n_terms && m[at[e]] == mm) ++e;
+        const int run = n[at[e - 1]] - nlo + 1, len = (run + TT - 1) / TT * TT;
         t.gm.push_back(mm);
         t.gnlo.push_back(nlo);
+        t.len.push_back(run);
         const size_t base = t.coef.size();
         t.coef.resize(base + len, make_float2(0.f, 0.f));
-        for (auto& e : kv.second) t.coef[base + (e.first - nlo)] = make_float2((float)e.second.first, (float)e.second.second);
+        while (i < e) {
+            const int nn = n[at[i]];
+            double re = 0, im = 0;
+            for (; i < e && n[at[i]] == nn; ++i) {
+                re += c[2 * at[i]];
+                im += c[2 * at[i] + 1];
+            }
+            t.coef[base + (nn - nlo)] = make_float2((float)re, (float)im);
+        }
         t.goff.push_back((int)t.coef.size());
         max_m = std::max(max_m, std::abs(mm));
         max_n = std::max({max_n, std::abs(nlo), std::abs(nlo + len - 1)});
     }
     t.halo_q = max_n + TT;
     t.halo_a = t.halo_q + max_m;
-    return true;
+    plan_tensor(t);
 }
+}  // namespace
 
-// Device term tables of recent term lists, per context: an equalizer applied
-// again with the same coefficients skips the host grouping and the upload.
-// The device buffer lives in ctx->tables (freed with the context); its
-// layout is {gm[ng], gnlo[ng], goff[ng+1], pad to 16 B, coef runs}.
-struct TermPlan {
-    int ng = 0, halo_q = 0, halo_a = 0;
-    size_t coef_offset = 0;
+// Device term tables of recent term lists, per context, most recent first: an
+// equalizer applied again with the same coefficients skips the host grouping
+// and the upload.  A list is recognised by its contents (compared with a host
+// copy: ~20 us for the 11 361 terms of R = 75, where hashing them took 0.6 ms
+// of every call).
+struct TermEntry {
+    std::vector<int32_t> m, n;
+    std::vector<double> coef;
+    void* dev = nullptr;
+    int ng = 0, halo_q = 0, halo_a = 0, a_lo = 0, alen = 0, ksteps = 0;
+    float unscale = 1.f;
+    size_t coef_offset = 0, grp_offset = 0, len_offset = 0, bmat_offset = 0;
 };
-std::mutex g_term_mutex;
-std::map<std::pair<const Ctx*, std::string>, TermPlan> g_term_plans;
-constexpr int kMaxTermPlans = 16;
-
-uint64_t fnv1a(const void* p, size_t n, uint64_t h) {
-    const unsigned char* b = (const unsigned char*)p;
-    for (size_t i = 0; i < n; ++i) {
-        h ^= b[i];
-        h *= 1099511628211ull;
-    }
-    return h;
+struct TermCache {
+    std::list<TermEntry> entries;
+};
+void free_term_cache(TermCache* t) {
+    if (!t) return;
+    for (TermEntry& e : t->entries) cudaFree(e.dev);
+    delete t;
 }
 
-std::string term_key(int n_terms, const int32_t* m, const int32_t* n, const double* c) {
-    uint64_t h1 = 1469598103934665603ull, h2 = 0x9E3779B97F4A7C15ull;
-    h1 = fnv1a(&n_terms, sizeof n_terms, h1);
-    h1 = fnv1a(m, sizeof(int32_t) * n_terms, h1);
-    h1 = fnv1a(n, sizeof(int32_t) * n_terms, h1);
-    h1 = fnv1a(c, sizeof(double) * 2 * n_terms, h1);
-    h2 = fnv1a(c, sizeof(double) * 2 * n_terms, h2);
-    h2 = fnv1a(n, sizeof(int32_t) * n_terms, h2);
-    h2 = fnv1a(m, sizeof(int32_t) * n_terms, h2);
-    char buf[64];
-    std::snprintf(buf, sizeof buf, "triplet:%016llx%016llx:%d", (unsigned long long)h1, (unsigned long long)h2,
-                  n_terms);
-    return buf;
+namespace {
+constexpr size_t kMaxTermPlans = 16;
+
+bool same_terms(const TermEntry& e, int n_terms, const int32_t* m, const int32_t* n, const double* c) {
+    const size_t k = (size_t)n_terms;
+    return e.m.size() == k && !std::memcmp(e.m.data(), m, sizeof(int32_t) * k) &&
+           !std::memcmp(e.n.data(), n, sizeof(int32_t) * k) && !std::memcmp(e.coef.data(), c, sizeof(double) * 2 * k);
 }
 
 // The cached device tables of a term list (built and uploaded on a miss).
 focss_status term_plan(Ctx* c, int n_terms, const int32_t* m, const int32_t* n, const double* coef,
-                       const char** dev, TermPlan* plan) {
-    const std::string key = term_key(n_terms, m, n, coef);
-    std::lock_guard<std::mutex> lock(g_term_mutex);
-    auto it = g_term_plans.find({c, key});
-    auto tt = c->tables.find(key);
-    if (it != g_term_plans.end() && tt != c->tables.end()) {
-        *dev = (const char*)tt->second;
-        *plan = it->second;
-        return FOCSS_OK;
-    }
-    int cached = 0;
-    for (auto& kv : c->tables) cached += kv.first.compare(0, 8, "triplet:") == 0;
-    if (cached >= kMaxTermPlans) {  // drop them all (in-flight kernels finish first)
-        cudaStreamSynchronize(c->stream);
-        for (auto kv = c->tables.begin(); kv != c->tables.end();) {
-            if (kv->first.compare(0, 8, "triplet:") == 0) {
-                cudaFree(kv->second);
-                g_term_plans.erase({c, kv->first});
-                kv = c->tables.erase(kv);
-            } else {
-                ++kv;
-            }
+                       const TermEntry** out) {
+    if (!c->terms) c->terms = new TermCache();
+    std::list<TermEntry>& es = c->terms->entries;
+    for (auto it = es.begin(); it != es.end(); ++it)
+        if (same_terms(*it, n_terms, m, n, coef)) {
+            es.splice(es.begin(), es, it);
+            *out = &es.front();
+            return FOCSS_OK;
         }
-    }
+    for (int i = 0; i < n_terms; ++i)
+        if (std::abs(m[i]) > 4096 || std::abs(n[i]) > 4096)
+            return set_error(c, FOCSS_ERR_INVALID_ARG, "triplet: |m|, |n| must be <= 4096");
     Terms t;
     build_terms(n_terms, m, n, coef, t);
-    TermPlan p;
+    TermEntry p;
     p.ng = (int)t.gm.size();
     p.halo_q = t.halo_q;
     p.halo_a = t.halo_a;
-    const size_t bytes_i = sizeof(int) * (3 * (size_t)p.ng + 1);
-    p.coef_offset = (bytes_i + 15) / 16 * 16;
-    std::vector<char> host(p.coef_offset + sizeof(float2) * t.coef.size(), 0);
+    p.a_lo = t.a_lo;
+    p.alen = t.a_hi - t.a_lo;
+    p.ksteps = t.ksteps;
+    p.unscale = t.unscale;
+    auto up16 = [](size_t v) { return (v + 15) / 16 * 16; };
+    p.coef_offset = up16(sizeof(int) * (3 * (size_t)p.ng + 1));
+    p.grp_offset = up16(p.coef_offset + sizeof(float2) * t.coef.size());
+    p.len_offset = up16(p.grp_offset + sizeof(int4) * t.grp.size());
+    p.bmat_offset = up16(p.len_offset + sizeof(int) * p.ng);
+    std::vector<char> host(p.bmat_offset, 0);
     int* hi = (int*)host.data();
     std::copy(t.gm.begin(), t.gm.end(), hi);
     std::copy(t.gnlo.begin(), t.gnlo.end(), hi + p.ng);
     std::copy(t.goff.begin(), t.goff.end(), hi + 2 * p.ng);
     std::copy(t.coef.begin(), t.coef.end(), (float2*)(host.data() + p.coef_offset));
-    void* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, host.size());
+    std::copy(t.grp.begin(), t.grp.end(), (int4*)(host.data() + p.grp_offset));
+    std::copy(t.len.begin(), t.len.end(), (int*)(host.data() + p.len_offset));
+    p.m.assign(m, m + n_terms);
+    p.n.assign(n, n + n_terms);
+    p.coef.assign(coef, coef + 2 * (size_t)n_terms);
+    if (es.size() >= kMaxTermPlans) {  // drop the oldest (in-flight kernels finish first)
+        cudaStreamSynchronize(c->stream);
+        cudaFree(es.back().dev);
+        es.pop_back();
+    }
+    cudaError_t e = cudaMalloc(&p.dev, p.bmat_offset + t.bmat_bytes);
     if (e != cudaSuccess) return cuda_check(c, e, "triplet tables");
-    e = cudaMemcpy(d, host.data(), host.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(p.dev, host.data(), host.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !t.grp.empty()) {
+        char* d = (char*)p.dev;
+        toeplitz_kernel<<<p.ng, 256, 0, c->stream>>>((const float2*)(d + p.coef_offset), (const int*)d + 2 * (size_t)p.ng,
+                                                     (const int4*)(d + p.grp_offset), (const int*)(d + p.len_offset),
+                                                     1.f / p.unscale, (__half*)(d + p.bmat_offset));
+        count_launch();
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) {
-        cudaFree(d);
+        cudaFree(p.dev);
         return cuda_check(c, e, "triplet upload");
     }
-    c->tables[key] = d;
-    g_term_plans[{c, key}] = p;
-    *dev = (const char*)d;
-    *plan = p;
+    es.push_front(std::move(p));
+    *out = &es.front();
     return FOCSS_OK;
+}
+
+template <int MODES>
+cudaError_t launch_triplet(const TripletArgs& a, size_t smem, bool tensor, dim3 grid, cudaStream_t s) {
+    auto kern = tensor ? triplet_tc_kernel<MODES> : triplet_kernel<MODES>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, tensor ? TC_THREADS : NT, smem, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -277,17 +704,11 @@ focss_status run_triplet_rows(Ctx* c, const float2* in, size_t in_bstride, int m
     if (modes < 1 || modes > 2)
         return set_error(c, FOCSS_ERR_UNSUPPORTED, "triplet: 1 or 2 modes");
     if (n_terms <= 0 || !m || !n || !coef) return set_error(c, FOCSS_ERR_INVALID_ARG, "triplet: empty term list");
-    for (int i = 0; i < n_terms; ++i)
-        if (std::abs(m[i]) > 4096 || std::abs(n[i]) > 4096)
-            return set_error(c, FOCSS_ERR_INVALID_ARG, "triplet: |m|, |n| must be <= 4096");
-    const char* d = nullptr;
-    TermPlan t;
-    focss_status st = term_plan(c, n_terms, m, n, coef, &d, &t);
+    const TermEntry* t = nullptr;
+    focss_status st = term_plan(c, n_terms, m, n, coef, &t);
     if (st != FOCSS_OK) return st;
-    const size_t ng = (size_t)t.ng;
-    const float2* dcoef = (const float2*)(d + t.coef_offset);
-    cudaStream_t s = c->stream;
-    cudaError_t e = cudaSuccess;
+    const size_t ng = (size_t)t->ng;
+    const char* d = (const char*)t->dev;
     TripletArgs a{};
     a.in = in;
     a.in_bstride = in_bstride;
@@ -301,22 +722,48 @@ focss_status run_triplet_rows(Ctx* c, const float2* in, size_t in_bstride, int m
     a.g_m = (const int*)d;
     a.g_nlo = (const int*)d + ng;
     a.g_off = (const int*)d + 2 * ng;
-    a.coef = dcoef;
-    a.halo_q = t.halo_q;
-    a.halo_a = t.halo_a;
-    const int alen = TK + 2 * t.halo_a, qlen = TK + 2 * t.halo_q;
-    const size_t smem = sizeof(float2) * ((size_t)modes * (alen + alen / 8 + 2) + qlen + qlen / 8 + 2);
+    a.coef = (const float2*)(d + t->coef_offset);
+    a.halo_q = t->halo_q;
+    a.halo_a = t->halo_a;
+    const int alen = TK + 2 * t->halo_a, qlen = TK + 2 * t->halo_q;
+    size_t smem = sizeof(float2) * ((size_t)modes * (alen + alen / 8 + 2) + qlen + qlen / 8 + 2);
     if (smem > 200 * 1024) return set_error(c, FOCSS_ERR_UNSUPPORTED, "triplet: term offsets too large for a tile");
-    dim3 grid((samples + TK - 1) / TK, batch);
-    if (modes == 1) {
-        cudaFuncSetAttribute(triplet_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        triplet_kernel<1><<<grid, NT, smem, s>>>(a);
-    } else {
-        cudaFuncSetAttribute(triplet_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        triplet_kernel<2><<<grid, NT, smem, s>>>(a);
+    bool tensor = t->ksteps > 0;
+    a.splits = 1;
+    if (tensor) {
+        a.grp = (const int4*)(d + t->grp_offset);
+        a.bmat = (const unsigned char*)(d + t->bmat_offset);
+        a.bslot = (int)kStepBytes * t->ksteps;
+        a.a_lo = t->a_lo;
+        a.alen = t->alen;
+        a.qcap = (16 * t->ksteps + TC_K - 16 + 127) / 128 * 128;
+        a.coef_unscale = t->unscale;
+        const size_t need = 1024 + (size_t)kSt * (8 * (size_t)a.qcap + a.bslot) + sizeof(int4) * ng +
+                            sizeof(float2) * (size_t)modes * (a.alen + a.alen / 16 + 2);
+        tensor = need <= 220 * 1024;
+        if (tensor) smem = std::max(smem, need);  // a tile may take the FP32 sum
     }
-    count_launch();
-    e = cudaGetLastError();
+    const int tile = tensor ? TC_K : TK;
+    dim3 grid((samples + tile - 1) / tile, batch);
+    const size_t total = (size_t)batch * modes * samples;
+    if (tensor) {
+        // fewer tiles than half the SMs: the groups split over CTAs, whose
+        // partial sums a second kernel joins (at least 4 groups each)
+        const long long tiles = (long long)grid.x * batch;
+        a.splits = (int)std::max(1ll, std::min<long long>({sm_count() / std::max(1ll, tiles), (long long)ng / 4, 32}));
+        if (a.splits > 1) {
+            a.part = (float2*)scratch_buffer(c, 7, sizeof(float2) * total * a.splits);
+            if (!a.part) return set_error(c, FOCSS_ERR_OOM, "triplet scratch");
+            grid.z = a.splits;
+        }
+    }
+    const cudaError_t e = modes == 1 ? launch_triplet<1>(a, smem, tensor, grid, c->stream)
+                                     : launch_triplet<2>(a, smem, tensor, grid, c->stream);
+    if (e == cudaSuccess && a.splits > 1) {
+        triplet_join_kernel<<<(unsigned)std::min<size_t>((total + 255) / 256, (size_t)sm_count() * 8), 256, 0, c->stream>>>(a, total);
+        count_launch();
+        return cuda_check(c, cudaGetLastError(), "triplet join");
+    }
     return cuda_check(c, e, "triplet");
 }
 
