@@ -504,31 +504,42 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(const __grid_constan
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(S::TMEM_COLS));
 }
 
-// bias gradient: gb[co] += sum_p g[p][co].  Each lane sums one channel pair
-// over a slot of positions, so a warp reads whole 128-byte rows; warps and
-// then CTAs combine in shared memory and one atomic per channel per CTA.
+// bias gradient: gb[co] += sum_p g[p][co].  A lane reads 16 bytes (8 channels)
+// of kBiasRows positions before it adds any of them, so that a warp keeps 2 KB
+// in flight; warps and then CTAs combine in shared memory and one atomic per
+// channel per CTA.  12 x 2^15 positions of 64 channels (50 MB): 13.7 us
+// (41 us with one 4-byte load in flight per lane).
+constexpr int kBiasRows = 4;
 template <int C>
 __global__ void __launch_bounds__(256) bias_grad_kernel(const bf16* __restrict__ g, size_t positions,
                                                         float* __restrict__ gb) {
-    constexpr int HC = C / 2, PW = 32 / HC;  // channel pairs; positions per warp step
+    constexpr int L = C / 8, PW = 32 / L;  // lanes per position; positions per warp step
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int cp = lane % HC, po = lane / HC;
-    float a0 = 0.f, a1 = 0.f;
+    const int cg = lane % L, po = lane / L;
+    float a[8] = {};
     const size_t step = (size_t)gridDim.x * nw * PW;
-    for (size_t p = ((size_t)blockIdx.x * nw + warp) * PW + po; p < positions; p += step) {
-        const __nv_bfloat162 v = reinterpret_cast<const __nv_bfloat162*>(g + p * C)[cp];
-        a0 += __low2float(v);
-        a1 += __high2float(v);
+    for (size_t p = ((size_t)blockIdx.x * nw + warp) * PW + po; p < positions; p += kBiasRows * step) {
+        uint4 v[kBiasRows];
+#pragma unroll
+        for (int u = 0; u < kBiasRows; ++u)
+            v[u] = p + u * step < positions ? reinterpret_cast<const uint4*>(g + (p + u * step) * C)[cg] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < kBiasRows; ++u) {
+            const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                a[2 * e] += __uint_as_float(w[e] << 16);  // BF16 is the upper half of FP32
+                a[2 * e + 1] += __uint_as_float(w[e] & 0xFFFF0000u);
+            }
+        }
     }
-    for (int o = HC; o < 32; o <<= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        for (int o = L; o < 32; o <<= 1) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
     __shared__ float sh[8][C];
-    if (po == 0) {
-        sh[warp][2 * cp] = a0;
-        sh[warp][2 * cp + 1] = a1;
-    }
+    if (po == 0)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sh[warp][8 * cg + e] = a[e];
     __syncthreads();
     if (threadIdx.x < C) {
         float t = 0.f;
