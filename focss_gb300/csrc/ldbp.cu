@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fir_tc.cuh"
 #include "internal.h"
 
 namespace fg {
@@ -128,6 +129,270 @@ __global__ void __launch_bounds__(FIR_THREADS) fir_kernel(const float2* __restri
 #pragma unroll
     for (int i = 0; i < FIR_OUT; ++i)
         if (n0 + o0 + i < N) yb[i] = acc[i];
+}
+
+// ---------------------------------------------------------------- chains of layers
+// A chain of up to kMaxChain layers, each y = FIR(x, h_l) gain_l and, with xi,
+// x' = y exp(i xi_l |y|^2), in one launch.  A CTA takes `owned` samples of one
+// realization through all of them: layer l's product (fir_tc.cuh) gives 2048
+// outputs, of which the T - 1 at the end are no longer valid inputs' sums, so
+// owned = 2048 - (layers - 1)(T - 1), and between layers the samples stay in
+// shared memory (split FP16) and registers (FP32).
+//
+// The input of every layer is scaled by the tile's largest sample (precision:
+// fir_tc.cuh).  Tiles whose input spans more
+// than 2^12 in power (largest sample over the mean of the weakest 32-sample
+// run) or holds non-finite samples run the layers in FP32.  20 x 4 steps of
+// 63 taps: relative error of the symbols FIGURE_ERR.
+//
+// What bounds it: per tile and layer ~1040 cycles of shared-memory bandwidth
+// for the products and ~1200 issue cycles for the epilogue (nonlinear phase,
+// splits), with two CTAs per SM (tensor memory) to overlap them.  FIGURE_TIME
+constexpr int kMaxChain = 8;
+struct ChainArgs {
+    const float2* x;            // batch x N
+    float2* y;                  // batch x N, or batch x N/2 (decimate: even samples only)
+    float2* keep;               // with keep: y of layer l (before the phase) at keep + l keep_stride
+    size_t keep_stride;
+    const unsigned char* bmat;  // Toeplitz matrices of the layers, ks * 2048 bytes each
+    const float* unscale;       // their scales
+    const float2* h;            // taps, T per layer (tiles in FP32)
+    const float* xi;            // gains of the nonlinear phase, or null
+    float gain[kMaxChain];
+    int layers, T, N, owned, decimate;
+};
+
+__device__ __forceinline__ int wrap_index(int s, int N) {
+    if (s < 0 || s >= N) {
+        s %= N;
+        if (s < 0) s += N;
+    }
+    return s;
+}
+
+// The CTA's owned samples of a layer's output `v(i)`, i = 0 .. owned-1, to dst.
+template <class V>
+__device__ __forceinline__ void chain_store(const ChainArgs& a, float2* dst, int b, int n0, bool last, V v) {
+    for (int i = threadIdx.x; i < a.owned; i += firtc::THREADS) {
+        const int n = n0 + i;
+        if (n >= a.N) break;
+        if (last && a.decimate) {
+            if (!(n & 1)) dst[(size_t)b * (a.N / 2) + n / 2] = v(i);
+        } else {
+            dst[(size_t)b * a.N + n] = v(i);
+        }
+    }
+}
+
+// The layers of one tile in FP32 on plain shared-memory buffers.
+__device__ __noinline__ void chain_tile_fp32(const ChainArgs& a, float2* buf, int b, int n0) {
+    const int c = (a.T - 1) / 2, span = firtc::TILE + a.T - 1;
+    float2 *cur = buf, *nxt = buf + span;
+    int valid = a.owned + a.layers * (a.T - 1);
+    __syncthreads();
+    for (int i = threadIdx.x; i < valid; i += firtc::THREADS)
+        cur[i] = a.x[(size_t)b * a.N + wrap_index(n0 - a.layers * c + i, a.N)];
+    for (int l = 0; l < a.layers; ++l) {
+        const float2* h = a.h + (size_t)l * a.T;
+        const bool last = l + 1 == a.layers;
+        const int first = (a.layers - 1 - l) * c;
+        valid -= a.T - 1;
+        __syncthreads();
+        for (int i = threadIdx.x; i < valid; i += firtc::THREADS) {
+            float2 s = make_float2(0.f, 0.f);
+            for (int t = 0; t < a.T; ++t) {
+                const float2 hv = h[t], xv = cur[i + t];
+                s.x = fmaf(hv.x, xv.x, fmaf(-hv.y, xv.y, s.x));
+                s.y = fmaf(hv.x, xv.y, fmaf(hv.y, xv.x, s.y));
+            }
+            s = cscale(s, a.gain[l]);
+            const int n = n0 + i - first;
+            if (a.keep && i >= first && i < first + a.owned && n < a.N)
+                a.keep[l * a.keep_stride + (size_t)b * a.N + n] = s;
+            nxt[i] = a.xi ? cmul(s, phase_rotation(a.xi[l] * cnorm(s))) : s;
+        }
+        __syncthreads();
+        float2* t = cur;
+        cur = nxt;
+        nxt = t;
+        if (last) chain_store(a, a.y, b, n0, true, [&](int i) { return cur[i]; });
+    }
+}
+
+__global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const ChainArgs a) {
+    using namespace firtc;
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) unsigned long long done, bfull[2];
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int abort_flag;
+    __shared__ unsigned s_max[kMaxChain], s_min;
+    __shared__ int s_bad;
+    const int ks = ksteps(a.T), cap = qcap(ks), c = (a.T - 1) / 2;
+    const uint32_t pitch = 2u * cap, bbytes = STEP_BYTES * ks;
+    unsigned char* xs = sm + ((1024u - (tcg::smem_addr(sm) & 1023u)) & 1023u);  // {re hi, im hi, re lo, im lo}
+    unsigned char* bs = xs + 4 * (size_t)pitch;                                 // Toeplitz matrices, two for a chain
+    float2* stage = reinterpret_cast<float2*>(bs + (a.layers > 1 ? 2 : 1) * (size_t)bbytes);  // TILE outputs, padded
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.y, n0 = blockIdx.x * a.owned;
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < kMaxChain; ++i) s_max[i] = 0u;
+        s_min = 0x7F7FFFFFu;
+        s_bad = 0;
+        tcg::mbar_init(&done, 1);
+        tcg::mbar_init(&bfull[0], 1);
+        tcg::mbar_init(&bfull[1], 1);
+        tcg::fence_mbar_init();
+        for (int l = 0; l < 2 && l < a.layers; ++l) {
+            tcg::mbar_expect_tx(&bfull[l], bbytes);
+            tcg::bulk_load(tcg::smem_addr(bs) + l * bbytes, a.bmat + (size_t)l * bbytes, bbytes, &bfull[l]);
+        }
+    }
+    if (warp == 0) tcg::tmem_alloc(&tmem_base, D_COLS);
+    __syncthreads();
+    // input: element e of the tile is sample n0 - layers c + e; 8 per thread at a time
+    constexpr int LOADS = (TILE + 16 * 17 + 8 * THREADS - 1) / (8 * THREADS);
+    float2 v[LOADS][8];
+    {
+        const float2* xb = a.x + (size_t)b * a.N;
+        const int base = n0 - a.layers * c, len = TILE + a.T - 1;
+        float mx = 0.f, mn = 3.4e38f;
+        bool bad = false;
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int e = 8 * (threadIdx.x + THREADS * u) + j;
+                v[u][j] = e < len ? xb[wrap_index(base + e, a.N)] : make_float2(0.f, 0.f);
+            }
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u) {
+            float sum = 0.f;  // 8 samples; four neighbouring lanes hold a run of 32
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float p = cnorm(v[u][j]);
+                sum += p;
+                mx = fmaxf(mx, p);
+            }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            bad = bad || !(sum <= 1e30f);
+            if (sum > 0.f) mn = fminf(mn, sum);
+        }
+        mx = warp_max(mx);
+        mn = -warp_max(-mn);
+        bad = __any_sync(0xffffffffu, bad);
+        if (lane == 0) {
+            atomicMax(&s_max[0], __float_as_uint(mx));
+            atomicMin(&s_min, __float_as_uint(mn));
+            if (bad) s_bad = 1;
+        }
+    }
+    tcg::fence_before_sync();
+    __syncthreads();
+    tcg::fence_after_sync();
+    const uint32_t tmem = tmem_base;
+    const float pmax = __uint_as_float(s_max[0]);
+    bool ok = true;
+    if (s_bad || (pmax > 0.f && (!(pmax > 1e-30f) || pmax > 128.f * __uint_as_float(s_min)))) {  // 2^12 over a run's mean
+        ok = tcg::mbar_wait(&bfull[0], 0, &abort_flag);  // the copies land before the buffers are reused
+        if (a.layers > 1) ok = tcg::mbar_wait(&bfull[1], 0, &abort_flag) && ok;
+        chain_tile_fp32(a, reinterpret_cast<float2*>(sm), b, n0);
+        __syncthreads();
+        if (warp == 0) tcg::tmem_free(tmem, D_COLS);
+        return;
+    }
+    {
+        const float sc = pow2(-split_exponent(s_max[0]));
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u) {
+            const int e = 8 * (threadIdx.x + THREADS * u);
+            if (e < cap) split_store8(xs, pitch, e, v[u], sc);
+        }
+    }
+    const int o0 = ROW * (32 * (warp & 3) + lane) + OUT * (warp >> 2);  // first output of the thread
+    for (int l = 0; l < a.layers; ++l) {
+        const bool last = l + 1 == a.layers;
+        tcg::fence_async_smem();
+        tcg::fence_before_sync();
+        __syncthreads();  // the split input is in place, the accumulator read
+        if (warp == 0) {
+            tcg::fence_after_sync();
+            ok = tcg::mbar_wait_warp(&bfull[l & 1], (l >> 1) & 1, &abort_flag);
+            if (ok) issue(tmem, tcg::smem_addr(xs), pitch, tcg::smem_addr(bs) + (l & 1) * bbytes, ks, &done);
+        }
+        ok = ok && tcg::mbar_wait(&done, l & 1, &abort_flag);
+        if (__syncthreads_or(!ok)) {
+            ok = false;
+            break;
+        }
+        tcg::fence_after_sync();
+        if (threadIdx.x == 0 && l + 2 < a.layers) {
+            tcg::mbar_expect_tx(&bfull[l & 1], bbytes);
+            tcg::bulk_load(tcg::smem_addr(bs) + (l & 1) * bbytes, a.bmat + (size_t)(l + 2) * bbytes, bbytes, &bfull[l & 1]);
+        }
+        float2 y[OUT];
+        read_outputs(tmem, warp, pow2(split_exponent(s_max[l])) * a.unscale[l], y);
+        const int first = (a.layers - 1 - l) * c;  // first owned output
+        if (a.gain[l] != 1.0f) {
+#pragma unroll
+            for (int r = 0; r < OUT; ++r) y[r] = cscale(y[r], a.gain[l]);
+        }
+        if (a.keep) {
+#pragma unroll
+            for (int r = 0; r < OUT; ++r) stage[pad(o0 + r)] = y[r];
+            __syncthreads();
+            chain_store(a, a.keep + l * a.keep_stride, b, n0, false, [&](int i) { return stage[pad(first + i)]; });
+        }
+        if (a.xi) {
+            const float k = a.xi[l];
+#pragma unroll
+            for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation(k * cnorm(y[r])));
+        }
+        if (last) {
+            if (a.keep) __syncthreads();
+#pragma unroll
+            for (int r = 0; r < OUT; ++r) stage[pad(o0 + r)] = y[r];
+            __syncthreads();
+            chain_store(a, a.y, b, n0, true, [&](int i) { return stage[pad(i)]; });
+            break;
+        }
+        // the outputs are the next layer's inputs at the same places; the
+        // elements behind them (no longer valid) become zero
+        float mx = 0.f;
+#pragma unroll
+        for (int r = 0; r < OUT; ++r) mx = fmaxf(mx, cnorm(y[r]));
+        mx = warp_max(mx);
+        if (lane == 0) atomicMax(&s_max[l + 1], __float_as_uint(mx));
+        if (l == 0)
+            for (int e = TILE / 8 + threadIdx.x; e < cap / 8; e += THREADS) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    *reinterpret_cast<uint4*>(xs + q * pitch + swz32(16u * e)) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        __syncthreads();
+        split_store8(xs, pitch, o0, y, pow2(-split_exponent(s_max[l + 1])));
+    }
+    if (!ok) {
+        // a wait ran out: the copies and MMAs in flight land (bounded) before
+        // the CTA leaves, and its outputs are marked invalid
+        if (warp == 0) {
+            tcg::mma_commit_warp(&done);
+            for (int p = 0; p < 2; ++p) tcg::mbar_wait_warp(&done, p, nullptr);
+            for (int p = 0; p < 2; ++p) {
+                tcg::mbar_wait_warp(&bfull[0], p, nullptr);
+                if (a.layers > 1) tcg::mbar_wait_warp(&bfull[1], p, nullptr);
+            }
+        }
+        __syncthreads();
+        const float nan = __int_as_float(0x7fc00000);
+        chain_store(a, a.y, b, n0, true, [&](int) { return make_float2(nan, nan); });
+    }
+    tcg::fence_before_sync();
+    __syncthreads();
+    tcg::fence_after_sync();
+    if (warp == 0) tcg::tmem_free(tmem, D_COLS);
 }
 
 // g_h[t] += sum_n g_y[n] conj(x[(n + t - c) mod N]) over all realizations.
@@ -279,6 +544,9 @@ struct LdbpModel {
     float2* work = nullptr;  // 2 work buffers of batch*samples
     float2* sym = nullptr;   // batch*samples/2
     double* loss = nullptr;
+    unsigned char* bmat = nullptr;  // Toeplitz matrices of the layers, then of the matched filter
+    float* unscale = nullptr;       // their scales
+    bool stale = true;              // parameters changed since they were built
     size_t field_n() const { return (size_t)batch * samples; }
     float2* h(int k) const { return (float2*)params + (size_t)k * taps; }
     float* xi(int k) const { return params + (size_t)spans * steps * taps * 2 + k; }
@@ -302,6 +570,80 @@ using fg::count_launch;
 
 static focss_status ldbp_err(focss_ctx* c, cudaError_t e, const char* what) { return fg::cuda_check(c, e, what); }
 
+// Toeplitz matrices of the current parameters.
+static size_t layer_bytes(const LdbpModel& M) { return (size_t)fg::firtc::STEP_BYTES * fg::firtc::ksteps(M.taps); }
+static cudaError_t ldbp_matrices(LdbpModel& M) {
+    if (!M.stale) return cudaSuccess;
+    const int L = M.spans * M.steps;
+    fg::firtc::toeplitz_kernel<<<L, 256, 0, M.ctx->stream>>>(M.h(0), M.taps, 0, (__half*)M.bmat, M.unscale);
+    fg::firtc::toeplitz_kernel<<<1, 256, 0, M.ctx->stream>>>(M.hmf(), M.mf_taps, 0, (__half*)(M.bmat + L * layer_bytes(M)),
+                                                            M.unscale + L);
+    count_launch(2);
+    M.stale = false;
+    return cudaGetLastError();
+}
+
+static cudaError_t launch_chain(const LdbpModel& M, fg::ChainArgs& a) {
+    using namespace fg::firtc;
+    a.N = M.samples;
+    a.owned = TILE - (a.layers - 1) * (a.T - 1);
+    const int ks = ksteps(a.T);
+    const size_t smem = 1024 + 8 * (size_t)qcap(ks) + (a.layers > 1 ? 2 : 1) * (size_t)STEP_BYTES * ks +
+                        sizeof(float2) * (TILE + TILE / 16);
+    // a tile in FP32 takes two plain buffers instead
+    const size_t need = std::max(smem, sizeof(float2) * 2 * (size_t)(TILE + a.T - 1));
+    cudaError_t e = cudaFuncSetAttribute(fg::ldbp_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    if (e != cudaSuccess) return e;
+    fg::ldbp_chain_kernel<<<dim3((M.samples + a.owned - 1) / a.owned, M.batch), THREADS, need, M.ctx->stream>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// All learned steps from `in` (left in M.work), in chains; keep: every
+// layer's FIR output (times the span's gain) in M.acts.  Then the matched
+// filter's symbols (even samples) into `symbols`.
+static cudaError_t ldbp_chains(LdbpModel& M, const float2* in, bool keep, float2* symbols) {
+    const size_t n = M.field_n();
+    const int L = M.spans * M.steps;
+    cudaError_t e = ldbp_matrices(M);
+    float2* bufs[2] = {M.work, M.work + n};
+    // layers per launch: the halo a chain computes twice stays below an eighth
+    const int F = std::max(1, std::min(fg::kMaxChain, 1 + 256 / std::max(1, M.taps - 1)));
+    const float2* src = in;
+    int w = 0;
+    for (int k = 0; k < L && e == cudaSuccess; k += F) {
+        fg::ChainArgs a{};
+        a.layers = std::min(F, L - k);
+        a.T = M.taps;
+        a.x = src;
+        a.y = bufs[w];
+        a.keep = keep ? M.acts + (size_t)k * n : nullptr;
+        a.keep_stride = n;
+        a.bmat = M.bmat + k * layer_bytes(M);
+        a.unscale = M.unscale + k;
+        a.h = M.h(k);
+        a.xi = M.xi(k);
+        for (int l = 0; l < a.layers; ++l) a.gain[l] = (k + l) % M.steps == 0 ? M.span_scale : 1.0f;
+        e = launch_chain(M, a);
+        src = bufs[w];
+        w ^= 1;
+    }
+    if (e == cudaSuccess) {
+        fg::ChainArgs a{};
+        a.layers = 1;
+        a.T = M.mf_taps;
+        a.x = src;
+        a.y = symbols;
+        a.decimate = 1;
+        a.bmat = M.bmat + L * layer_bytes(M);
+        a.unscale = M.unscale + L;
+        a.h = M.hmf();
+        a.gain[0] = 1.0f;
+        e = launch_chain(M, a);
+    }
+    return e;
+}
+
 static cudaError_t fir(const LdbpModel& M, const float2* x, const float2* h, int T, int conj_rev, float2* y,
                        float gain = 1.0f, const float* xi = nullptr) {
     dim3 g((M.samples + fg::FIR_TILE - 1) / fg::FIR_TILE, M.batch);
@@ -310,30 +652,8 @@ static cudaError_t fir(const LdbpModel& M, const float2* x, const float2* h, int
     return cudaGetLastError();
 }
 
-// Inference forward pass: one launch per learned step (FIR, the span's
-// drop_power factor applied to the filter output, nonlinear phase), reading
-// the input field directly, then the matched filter into work[1].
-static cudaError_t ldbp_infer(LdbpModel& M, const float2* in) {
-    const size_t n = M.field_n();
-    float2* bufs[2] = {M.work, M.work + n};
-    const int layers = M.spans * M.steps;
-    int w = (layers - 1) & 1;  // the last step lands in work[0]
-    const float2* src = in;
-    cudaError_t e = cudaSuccess;
-    for (int sp = 0; sp < M.spans && e == cudaSuccess; ++sp)
-        for (int st = 0; st < M.steps && e == cudaSuccess; ++st) {
-            const int k = sp * M.steps + st;
-            e = fir(M, src, M.h(k), M.taps, 0, bufs[w], st == 0 ? M.span_scale : 1.0f, M.xi(k));
-            src = bufs[w];
-            w ^= 1;
-        }
-    if (e == cudaSuccess) e = fir(M, src, M.hmf(), M.mf_taps, 0, M.work + n);
-    return e;
-}
-
 // Forward pass; keeps every layer input in M.acts when `keep`.
 static cudaError_t ldbp_forward(LdbpModel& M, const float2* in, bool keep) {
-    if (!keep && M.steps > 0) return ldbp_infer(M, in);
     cudaStream_t s = M.ctx->stream;
     const size_t n = M.field_n();
     float2* cur = M.work;
@@ -397,11 +717,17 @@ FOCSS_API focss_status focss_ldbp_create(focss_ctx* c, int spans, int steps_per_
     if (e == cudaSuccess) e = cudaMalloc(&m->work, sizeof(float2) * n * 3);
     m->sym = m->work + 2 * n;
     if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(double) * 2);
+    const size_t nl = (size_t)spans * steps_per_span;
+    if (e == cudaSuccess)
+        e = cudaMalloc(&m->bmat, nl * layer_bytes(*m) + (size_t)fg::firtc::STEP_BYTES * fg::firtc::ksteps(mf_taps));
+    if (e == cudaSuccess) e = cudaMalloc(&m->unscale, sizeof(float) * (nl + 1));
     if (e != cudaSuccess) {
         cudaFree(m->params);
         cudaFree(m->acts);
         cudaFree(m->work);
         cudaFree(m->loss);
+        cudaFree(m->bmat);
+        cudaFree(m->unscale);
         delete m;
         return ldbp_err(c, e, "ldbp alloc");
     }
@@ -416,6 +742,8 @@ FOCSS_API focss_status focss_ldbp_destroy(focss_ldbp* m) {
     cudaFree(m->acts);
     cudaFree(m->work);
     cudaFree(m->loss);
+    cudaFree(m->bmat);
+    cudaFree(m->unscale);
     delete m;
     return FOCSS_OK;
 }
@@ -428,6 +756,7 @@ FOCSS_API focss_status focss_ldbp_set_params(focss_ldbp* m, const float* host, i
     if (e == cudaSuccess) e = cudaMemsetAsync(m->m1, 0, sizeof(float) * 2 * n, m->ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->ctx->stream);
     m->adam_t = 0;
+    m->stale = true;
     return ldbp_err(m->ctx, e, "ldbp set params");
 }
 
@@ -446,15 +775,7 @@ FOCSS_API focss_status focss_ldbp_forward(focss_ldbp* m, const focss_field* in, 
     if (in->modes != 1 || in->samples != m->samples || in->batch != m->batch || symbols->modes != 1 ||
         symbols->samples != m->samples / 2 || symbols->batch != m->batch)
         return fg::set_error(m->ctx, FOCSS_ERR_INVALID_ARG, "ldbp_forward: shapes");
-    cudaError_t e = ldbp_forward(*m, in->d, false);
-    const size_t ns = (size_t)m->batch * (m->samples / 2);
-    if (e == cudaSuccess) {
-        fg::mse_decimate_kernel<<<gridn(ns), 256, 0, m->ctx->stream>>>(m->work + m->field_n(), nullptr, m->samples, ns,
-                                                                       1.f, symbols->d, nullptr, nullptr);
-        count_launch();
-        e = cudaGetLastError();
-    }
-    return ldbp_err(m->ctx, e, "ldbp forward");
+    return ldbp_err(m->ctx, ldbp_chains(*m, in->d, false, symbols->d), "ldbp forward");
 }
 
 // One forward + backward over the batch: gradients into the model (overwritten),
@@ -522,6 +843,7 @@ FOCSS_API focss_status focss_ldbp_adam_step(focss_ldbp* m, double lr, double lr_
                                             double eps) {
     if (!m) return FOCSS_ERR_INVALID_ARG;
     m->adam_t += 1;
+    m->stale = true;
     const float c1 = (float)(1.0 / (1.0 - std::pow(beta1, m->adam_t)));
     const float c2 = (float)(1.0 / (1.0 - std::pow(beta2, m->adam_t)));
     // complex gradients g = dL/dconj(z) -> real gradient 2 g; xi gradients are already real:
