@@ -45,14 +45,15 @@ __device__ __forceinline__ float cnorm(float2 a) { return fmaf(a.x, a.x, a.y * a
 // nonlinear phase is bounded by construction): Taylor polynomials to degree
 // 8/9 (truncation < 3e-13), about one FP32 rounding; larger phases take the
 // reduced path below.
+constexpr float kPhaseSmall = 0.25f;
+__device__ __forceinline__ float2 phase_rotation_small(float phi) {
+    const float p2 = phi * phi;
+    const float s = phi * fmaf(p2, fmaf(p2, fmaf(p2, -1.0f / 5040.0f, 1.0f / 120.0f), -1.0f / 6.0f), 1.0f);
+    const float c = fmaf(p2, fmaf(p2, fmaf(p2, fmaf(p2, 1.0f / 40320.0f, -1.0f / 720.0f), 1.0f / 24.0f), -0.5f), 1.0f);
+    return make_float2(c, s);
+}
 __device__ __forceinline__ float2 phase_rotation(float phi) {
-    if (fabsf(phi) <= 0.25f) {
-        const float p2 = phi * phi;
-        const float s = phi * fmaf(p2, fmaf(p2, fmaf(p2, -1.0f / 5040.0f, 1.0f / 120.0f), -1.0f / 6.0f), 1.0f);
-        const float c = fmaf(p2, fmaf(p2, fmaf(p2, fmaf(p2, 1.0f / 40320.0f, -1.0f / 720.0f), 1.0f / 24.0f), -0.5f),
-                             1.0f);
-        return make_float2(c, s);
-    }
+    if (fabsf(phi) <= kPhaseSmall) return phase_rotation_small(phi);
     // Larger phases: Cody-Waite reduction by q quarter turns (pi/2 as a
     // two-float constant), Taylor series on |r| <= pi/4 (truncation below
     // 3e-9), exact quarter-turn placement.  Straight-line code with no local

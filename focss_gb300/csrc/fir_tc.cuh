@@ -34,13 +34,14 @@ __host__ __device__ constexpr int ksteps(int taps) { return (taps + ROW - 1 + 15
 // FP16 elements of one array of the split input: the taps' reach behind the
 // last row, rounded up to the swizzle's period
 __host__ __device__ constexpr int qcap(int ks) { return (16 * ks + TILE - ROW + 127) / 128 * 128; }
+constexpr int CAP_MAX = qcap(ksteps(255));  // for the longest filter
 // kind::f16, FP32 accumulator, FP16 operands, both K-major
 __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 __device__ __forceinline__ uint32_t swz32(uint32_t o) { return o ^ ((o >> 3) & 0x10u); }
 // staging index: 8 consecutive float2 per lane, lanes 16 apart, conflict-free
-__device__ __forceinline__ int pad(int o) { return o + (o >> 4); }
+__host__ __device__ constexpr int pad(int o) { return o + (o >> 4); }
 
 // Toeplitz matrices of `gridDim.x` filters of T taps, B[x][r] = h[x - r]: per
 // 8 taps 128 rows of 16 bytes, 32 rows (r / 16 + r = real / imaginary part of

@@ -251,26 +251,33 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
     }
     if (warp == 0) tcg::tmem_alloc(&tmem_base, D_COLS);
     __syncthreads();
-    // input: element e of the tile is sample n0 - layers c + e; 8 per thread at a time
-    constexpr int LOADS = (TILE + 16 * 17 + 8 * THREADS - 1) / (8 * THREADS);
+    // input: element e of the tile is sample n0 - layers c + e, coalesced into
+    // the staging buffer, then 8 consecutive per thread
+    constexpr int LOADS = 2;  // 8 x 256 x 2 >= CAP_MAX
     float2 v[LOADS][8];
     {
         const float2* xb = a.x + (size_t)b * a.N;
         const int base = n0 - a.layers * c, len = TILE + a.T - 1;
+        constexpr int K = CAP_MAX / THREADS;
+        static_assert(CAP_MAX % THREADS == 0 && CAP_MAX >= TILE + FIR_MAX_TAPS - 1 && CAP_MAX <= 8 * LOADS * THREADS, "tile");
+        float2 t[K];
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const int e = threadIdx.x + THREADS * u;
+            t[u] = e < len ? xb[wrap_index(base + e, a.N)] : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < K; ++u) stage[pad(threadIdx.x + THREADS * u)] = t[u];
+        __syncthreads();
         float mx = 0.f, mn = 3.4e38f;
         bool bad = false;
 #pragma unroll
-        for (int u = 0; u < LOADS; ++u)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int e = 8 * (threadIdx.x + THREADS * u) + j;
-                v[u][j] = e < len ? xb[wrap_index(base + e, a.N)] : make_float2(0.f, 0.f);
-            }
-#pragma unroll
         for (int u = 0; u < LOADS; ++u) {
+            const int e0 = 8 * (threadIdx.x + THREADS * u);
             float sum = 0.f;  // 8 samples; four neighbouring lanes hold a run of 32
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
+                v[u][j] = e0 < CAP_MAX ? stage[pad(e0 + j)] : make_float2(0.f, 0.f);
                 const float p = cnorm(v[u][j]);
                 sum += p;
                 mx = fmaxf(mx, p);
@@ -333,22 +340,34 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
             tcg::bulk_load(tcg::smem_addr(bs) + (l & 1) * bbytes, a.bmat + (size_t)(l + 2) * bbytes, bbytes, &bfull[l & 1]);
         }
         float2 y[OUT];
-        read_outputs(tmem, warp, pow2(split_exponent(s_max[l])) * a.unscale[l], y);
+        read_outputs(tmem, warp, pow2(split_exponent(s_max[l])) * a.unscale[l] * a.gain[l], y);
         const int first = (a.layers - 1 - l) * c;  // first owned output
-        if (a.gain[l] != 1.0f) {
-#pragma unroll
-            for (int r = 0; r < OUT; ++r) y[r] = cscale(y[r], a.gain[l]);
-        }
         if (a.keep) {
 #pragma unroll
             for (int r = 0; r < OUT; ++r) stage[pad(o0 + r)] = y[r];
             __syncthreads();
             chain_store(a, a.keep + l * a.keep_stride, b, n0, false, [&](int i) { return stage[pad(first + i)]; });
         }
+        // the phase keeps |y|, whose largest value scales the next layer's input
+        float pw[OUT], mx = 0.f;
+#pragma unroll
+        for (int r = 0; r < OUT; ++r) {
+            pw[r] = cnorm(y[r]);
+            mx = fmaxf(mx, pw[r]);
+        }
+        if (!last) {
+            const float wm = warp_max(mx);
+            if (lane == 0) atomicMax(&s_max[l + 1], __float_as_uint(wm));
+        }
         if (a.xi) {
             const float k = a.xi[l];
+            if (fabsf(k) * mx <= kPhaseSmall) {
 #pragma unroll
-            for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation(k * cnorm(y[r])));
+                for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation_small(k * pw[r]));
+            } else {
+#pragma unroll
+                for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation(k * pw[r]));
+            }
         }
         if (last) {
             if (a.keep) __syncthreads();
@@ -360,11 +379,6 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         }
         // the outputs are the next layer's inputs at the same places; the
         // elements behind them (no longer valid) become zero
-        float mx = 0.f;
-#pragma unroll
-        for (int r = 0; r < OUT; ++r) mx = fmaxf(mx, cnorm(y[r]));
-        mx = warp_max(mx);
-        if (lane == 0) atomicMax(&s_max[l + 1], __float_as_uint(mx));
         if (l == 0)
             for (int e = TILE / 8 + threadIdx.x; e < cap / 8; e += THREADS) {
 #pragma unroll
@@ -589,7 +603,7 @@ static cudaError_t launch_chain(const LdbpModel& M, fg::ChainArgs& a) {
     a.owned = TILE - (a.layers - 1) * (a.T - 1);
     const int ks = ksteps(a.T);
     const size_t smem = 1024 + 8 * (size_t)qcap(ks) + (a.layers > 1 ? 2 : 1) * (size_t)STEP_BYTES * ks +
-                        sizeof(float2) * (TILE + TILE / 16);
+                        sizeof(float2) * pad(CAP_MAX);
     // a tile in FP32 takes two plain buffers instead
     const size_t need = std::max(smem, sizeof(float2) * 2 * (size_t)(TILE + a.T - 1));
     cudaError_t e = cudaFuncSetAttribute(fg::ldbp_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
