@@ -43,13 +43,13 @@ __device__ __forceinline__ uint32_t swz32(uint32_t o) { return o ^ ((o >> 3) & 0
 // staging index: 8 consecutive float2 per lane, lanes 16 apart, conflict-free
 __host__ __device__ constexpr int pad(int o) { return o + (o >> 4); }
 
-// Toeplitz matrices of `gridDim.x` filters of T taps, B[x][r] = h[x - r]: per
+// Toeplitz matrices of n filters of T taps and (block n) one of T2 taps, B[x][r] = h[x - r]: per
 // 8 taps 128 rows of 16 bytes, 32 rows (r / 16 + r = real / imaginary part of
 // output r) each of h_mid, h_hi, h_lo 2^11, h_mid 2^11.  h is scaled to at most
 // 1 by a power of two, whose inverse goes to unscale.  conj_rev: the adjoint
 // filter conj(h[T-1-t]).
-__global__ void toeplitz_kernel(const float2* __restrict__ h, int T, int conj_rev, __half* __restrict__ bmat,
-                                float* __restrict__ unscale) {
+__global__ void toeplitz_kernel(const float2* __restrict__ h, int T, int n, const float2* __restrict__ h2, int T2,
+                                int conj_rev, __half* __restrict__ bmat, float* __restrict__ unscale) {
     __shared__ unsigned s_max;
     __shared__ float s_sum;
     if (threadIdx.x == 0) {
@@ -57,7 +57,12 @@ __global__ void toeplitz_kernel(const float2* __restrict__ h, int T, int conj_re
         s_sum = 0.f;
     }
     __syncthreads();
+    bmat += (size_t)blockIdx.x * ksteps(T) * (STEP_BYTES / 2);
     h += (size_t)blockIdx.x * T;
+    if ((int)blockIdx.x == n) {
+        h = h2;
+        T = T2;
+    }
     float mx = 0.f, re = 0.f, im = 0.f;
     for (int t = threadIdx.x; t < T; t += blockDim.x) {
         mx = fmaxf(mx, fmaxf(fabsf(h[t].x), fabsf(h[t].y)));
@@ -81,7 +86,6 @@ __global__ void toeplitz_kernel(const float2* __restrict__ h, int T, int conj_re
     const int a = 11 - (bits < 1 ? 1 : bits > 10 ? 10 : bits);
     const float grid = __uint_as_float((unsigned)(127 + a) << 23), inv_grid = __uint_as_float((unsigned)(127 - a) << 23);
     const int ks = ksteps(T);
-    __half* b = bmat + (size_t)blockIdx.x * ks * (STEP_BYTES / 2);
     for (int i = threadIdx.x; i < ks * (int)(STEP_BYTES / 2); i += blockDim.x) {
         const int x = (i >> 10) * 8 + (i & 7), row = (i >> 3) & 127, word = row >> 5;
         const int d = x - (row & 15);
@@ -93,7 +97,7 @@ __global__ void toeplitz_kernel(const float2* __restrict__ h, int T, int conj_re
         const float hi = rintf(v * grid) * inv_grid, rest = v - hi;   // exact
         const __half mid = __float2half_rn(rest * 2048.f);
         const float low = rest - __half2float(mid) * 0x1p-11f;        // exact
-        b[i] = word == 0 ? __float2half_rn(rest) : word == 1 ? __float2half_rn(hi) : word == 2 ? __float2half_rn(low * 2048.f) : mid;
+        bmat[i] = word == 0 ? __float2half_rn(rest) : word == 1 ? __float2half_rn(hi) : word == 2 ? __float2half_rn(low * 2048.f) : mid;
     }
 }
 

@@ -22,40 +22,51 @@
 
 namespace fg {
 
-constexpr int FIR_THREADS = 128;                    // fir_kernel
 constexpr int FIR_GRAD_THREADS = 256;               // fir_grad_taps_kernel: 8 warps x 8 taps
-constexpr int FIR_OUT = 4;                          // consecutive outputs per thread
-constexpr int FIR_TILE = FIR_THREADS * FIR_OUT;     // outputs per CTA of fir_kernel
 constexpr int FIR_GRAD_TILE = 2048;                 // samples per CTA of fir_grad_taps_kernel
 constexpr int FIR_MAX_TAPS = 255;
 constexpr int FIR_TAPS_PAD = (FIR_MAX_TAPS + 7) / 8 * 8;
 // Shared-memory sample windows keep one padding slot after every R samples,
-// R the run a thread reads from a multiple of R: runs of 4 (forward) start
-// 40 bytes apart across a half-warp and runs of 8 (tap gradient) 72 bytes
-// apart, both on distinct bank pairs.
+// R the run a thread reads from a multiple of R: runs of 8 start 72 bytes
+// apart across a half-warp, on distinct bank pairs.
 template <int R>
 __device__ __forceinline__ int fir_pad(int i) { return i + i / R; }
-constexpr int FIR_XS = (FIR_TILE + FIR_TAPS_PAD + 8) * (FIR_OUT + 1) / FIR_OUT;
 constexpr int FIR_GRAD_XS = (FIR_GRAD_TILE + FIR_TAPS_PAD + 8) * 9 / 8;
+
+__device__ __forceinline__ int wrap_index(int s, int N) {
+    if (s < 0 || s >= N) {
+        s %= N;
+        if (s < 0) s += N;
+    }
+    return s;
+}
 
 // Loads samples [n0 - c, n0 - c + span) of one realization (circular) into
 // the padded window: all of a thread's loads are issued before the first
 // store (a load-store loop would wait for one load latency per iteration).
+// With xi, the samples' nonlinear phase exp(i xi |x|^2) is applied.
 template <int THREADS, int TILE, int R>
 __device__ __forceinline__ void fir_load_window(float2* xs, const float2* __restrict__ xb, int n0, int c, int span,
-                                                int N) {
+                                                int N, const float* xi) {
     constexpr int K = (TILE + FIR_TAPS_PAD + THREADS - 1) / THREADS;
     float2 v[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         const int i = threadIdx.x + k * THREADS;
-        if (i < span) {
-            int s = n0 - c + i;
-            if (s < 0 || s >= N) {
-                s %= N;
-                if (s < 0) s += N;
-            }
-            v[k] = xb[s];
+        v[k] = i < span ? xb[wrap_index(n0 - c + i, N)] : make_float2(0.f, 0.f);
+    }
+    if (xi) {
+        const float g = *xi;
+        float mx = 0.f;
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            mx = fmaxf(mx, cnorm(v[k]));
+        if (fabsf(g) * mx <= kPhaseSmall) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) v[k] = cmul(v[k], phase_rotation_small(g * cnorm(v[k])));
+        } else {
+#pragma unroll
+            for (int k = 0; k < K; ++k) v[k] = cmul(v[k], phase_rotation(g * cnorm(v[k])));
         }
     }
 #pragma unroll
@@ -63,72 +74,6 @@ __device__ __forceinline__ void fir_load_window(float2* xs, const float2* __rest
         const int i = threadIdx.x + k * THREADS;
         if (i < span) xs[fir_pad<R>(i)] = v[k];
     }
-}
-
-// y = FIR(x, h) for every realization; conj_rev: use h'[t] = conj(h[T-1-t])
-// (the adjoint filter, for the input gradient).  Register-blocked: a thread
-// computes 4 consecutive outputs from an 11-sample register window per 8 taps
-// (taps zero-padded to a multiple of 8), so a product costs 19/32 of a
-// shared-memory load instead of two; each output still sums its taps in
-// ascending order with the same fused multiply-adds.
-//
-// Inference epilogue (both optional): the output is multiplied by `gain`
-// (the span's drop_power factor, moved past the linear filter) and then
-// rotated by exp(i xi |.|^2) (the step's nonlinear phase, as nl_kernel), so
-// one launch does a whole learned step.
-__global__ void __launch_bounds__(FIR_THREADS) fir_kernel(const float2* __restrict__ x, const float2* __restrict__ h,
-                                                          int T, int conj_rev, float2* __restrict__ y, int N,
-                                                          float gain, const float* __restrict__ xi) {
-    __shared__ float2 xs[FIR_XS];
-    __shared__ float2 hs[FIR_TAPS_PAD];
-    const int b = blockIdx.y;
-    const int n0 = blockIdx.x * FIR_TILE;
-    const int c = (T - 1) / 2;
-    const int Tp = (T + 7) & ~7;
-    for (int t = threadIdx.x; t < Tp; t += blockDim.x) {
-        float2 v = make_float2(0.f, 0.f);
-        if (t < T) {
-            v = conj_rev ? h[T - 1 - t] : h[t];
-            if (conj_rev) v.y = -v.y;
-        }
-        hs[t] = v;
-    }
-    fir_load_window<FIR_THREADS, FIR_TILE, FIR_OUT>(xs, x + (size_t)b * N, n0, c, FIR_TILE + Tp, N);
-    __syncthreads();
-    const int o0 = threadIdx.x * FIR_OUT;
-    float2 acc[FIR_OUT];
-#pragma unroll
-    for (int i = 0; i < FIR_OUT; ++i) acc[i] = make_float2(0.f, 0.f);
-    for (int tb = 0; tb < Tp; tb += 8) {
-        constexpr int WN = FIR_OUT + 7;  // window of 8 taps x FIR_OUT outputs
-        float2 w[WN], hv[8];
-        const int base = ((o0 + tb) / FIR_OUT) * (FIR_OUT + 1);
-#pragma unroll
-        for (int j = 0; j < WN; ++j) w[j] = xs[base + j + j / FIR_OUT];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) hv[u] = hs[tb + u];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-#pragma unroll
-            for (int i = 0; i < FIR_OUT; ++i) {
-                const float2 xv = w[i + u];
-                acc[i].x = fmaf(hv[u].x, xv.x, fmaf(-hv[u].y, xv.y, acc[i].x));
-                acc[i].y = fmaf(hv[u].x, xv.y, fmaf(hv[u].y, xv.x, acc[i].y));
-            }
-    }
-    if (gain != 1.0f) {
-#pragma unroll
-        for (int i = 0; i < FIR_OUT; ++i) acc[i] = cscale(acc[i], gain);
-    }
-    if (xi) {
-        const float k = *xi;
-#pragma unroll
-        for (int i = 0; i < FIR_OUT; ++i) acc[i] = cmul(acc[i], phase_rotation(k * cnorm(acc[i])));
-    }
-    float2* yb = y + (size_t)b * N + n0 + o0;
-#pragma unroll
-    for (int i = 0; i < FIR_OUT; ++i)
-        if (n0 + o0 + i < N) yb[i] = acc[i];
 }
 
 // ---------------------------------------------------------------- chains of layers
@@ -143,31 +88,41 @@ __global__ void __launch_bounds__(FIR_THREADS) fir_kernel(const float2* __restri
 // fir_tc.cuh).  Tiles whose input spans more
 // than 2^12 in power (largest sample over the mean of the weakest 32-sample
 // run) or holds non-finite samples run the layers in FP32.  20 x 4 steps of
-// 63 taps: relative error of the symbols FIGURE_ERR.
+// 63 taps: relative error of the symbols 1.1e-6 (1.4e-6 with plain FP32 filters).
 //
 // What bounds it: per tile and layer ~1040 cycles of shared-memory bandwidth
 // for the products and ~1200 issue cycles for the epilogue (nonlinear phase,
-// splits), with two CTAs per SM (tensor memory) to overlap them.  FIGURE_TIME
+// splits), with two CTAs per SM (tensor memory) to overlap them.  20 x 4 steps of 63 taps on
+// 16 x 65536 samples: 1368 -> 582 us against one FP32 launch per layer.
 constexpr int kMaxChain = 8;
 struct ChainArgs {
-    const float2* x;            // batch x N
+    const float2* x;            // batch x N: samples, or (backward) the gradient
     float2* y;                  // batch x N, or batch x N/2 (decimate: even samples only)
-    float2* keep;               // with keep: y of layer l (before the phase) at keep + l keep_stride
-    size_t keep_stride;
-    const unsigned char* bmat;  // Toeplitz matrices of the layers, ks * 2048 bytes each
+    int dir;                    // layer l's data is at l dir strides: 1, or -1 backward
+    float2* keep;               // forward, optional: y of a layer (before the phase); backward: the gradient there
+    const float2* act;          // backward: the kept y of the layers
+    size_t stride;              // of keep and act
+    const unsigned char* bmat;  // Toeplitz matrices of the layers, ks * STEP_BYTES each
     const float* unscale;       // their scales
     const float2* h;            // taps, T per layer (tiles in FP32)
     const float* xi;            // gains of the nonlinear phase, or null
+    float* gxi;                 // backward: their gradients (added to)
     float gain[kMaxChain];
     int layers, T, N, owned, decimate;
 };
 
-__device__ __forceinline__ int wrap_index(int s, int N) {
-    if (s < 0 || s >= N) {
-        s %= N;
-        if (s < 0) s += N;
-    }
-    return s;
+// Gradient through y e^{i phi}, phi = xi |y|^2, from g = dL/dconj of the output:
+//   g_y = g e^{-i phi} (1 - i xi p) + conj(g) i xi y^2 e^{i phi},
+//   dL/dxi += 2 Re(conj(g) i p y e^{i phi})
+__device__ __forceinline__ float2 phase_grad(float2 g, float2 y, float k, float& gxi) {
+    const float p = cnorm(y);
+    const float2 e = phase_rotation(k * p);
+    const float2 z = cmul(y, e);
+    const float2 a = cmul(cmul(g, make_float2(e.x, -e.y)), make_float2(1.f, -k * p));
+    const float2 gc = make_float2(g.x, -g.y);
+    const float2 b = cmul(cmul(gc, cmul(y, y)), e);
+    gxi = -2.f * p * cmul(gc, z).y;
+    return make_float2(a.x - k * b.y, a.y + k * b.x);
 }
 
 // The CTA's owned samples of a layer's output `v(i)`, i = 0 .. owned-1, to dst.
@@ -185,90 +140,127 @@ __device__ __forceinline__ void chain_store(const ChainArgs& a, float2* dst, int
 }
 
 // The layers of one tile in FP32 on plain shared-memory buffers.
+template <bool BWD>
 __device__ __noinline__ void chain_tile_fp32(const ChainArgs& a, float2* buf, int b, int n0) {
     const int c = (a.T - 1) / 2, span = firtc::TILE + a.T - 1;
     float2 *cur = buf, *nxt = buf + span;
     int valid = a.owned + a.layers * (a.T - 1);
+    const size_t row = (size_t)b * a.N;
     __syncthreads();
-    for (int i = threadIdx.x; i < valid; i += firtc::THREADS)
-        cur[i] = a.x[(size_t)b * a.N + wrap_index(n0 - a.layers * c + i, a.N)];
+    for (int i = threadIdx.x; i < valid; i += firtc::THREADS) cur[i] = a.x[row + wrap_index(n0 - a.layers * c + i, a.N)];
     for (int l = 0; l < a.layers; ++l) {
-        const float2* h = a.h + (size_t)l * a.T;
-        const bool last = l + 1 == a.layers;
+        const ptrdiff_t at = (ptrdiff_t)a.dir * l;
+        const float2* h = a.h + at * a.T;
+        __syncthreads();
+        if (BWD && a.xi) {
+            const int first = (a.layers - l) * c;
+            float acc = 0.f;
+            for (int i = threadIdx.x; i < valid; i += firtc::THREADS) {
+                const int n = n0 + i - first;
+                float d;
+                cur[i] = phase_grad(cur[i], a.act[at * (ptrdiff_t)a.stride + row + wrap_index(n, a.N)], a.xi[at], d);
+                if (i >= first && i < first + a.owned && n < a.N) {
+                    a.keep[at * (ptrdiff_t)a.stride + row + n] = cur[i];
+                    acc += d;
+                }
+            }
+            acc = warp_sum(acc);
+            if ((threadIdx.x & 31) == 0) atomicAdd(a.gxi + at, acc);
+            __syncthreads();
+        }
         const int first = (a.layers - 1 - l) * c;
         valid -= a.T - 1;
-        __syncthreads();
         for (int i = threadIdx.x; i < valid; i += firtc::THREADS) {
             float2 s = make_float2(0.f, 0.f);
             for (int t = 0; t < a.T; ++t) {
-                const float2 hv = h[t], xv = cur[i + t];
+                const float2 hv = BWD ? make_float2(h[a.T - 1 - t].x, -h[a.T - 1 - t].y) : h[t], xv = cur[i + t];
                 s.x = fmaf(hv.x, xv.x, fmaf(-hv.y, xv.y, s.x));
                 s.y = fmaf(hv.x, xv.y, fmaf(hv.y, xv.x, s.y));
             }
             s = cscale(s, a.gain[l]);
-            const int n = n0 + i - first;
-            if (a.keep && i >= first && i < first + a.owned && n < a.N)
-                a.keep[l * a.keep_stride + (size_t)b * a.N + n] = s;
-            nxt[i] = a.xi ? cmul(s, phase_rotation(a.xi[l] * cnorm(s))) : s;
+            if (!BWD) {
+                const int n = n0 + i - first;
+                if (a.keep && i >= first && i < first + a.owned && n < a.N) a.keep[at * (ptrdiff_t)a.stride + row + n] = s;
+                if (a.xi) s = cmul(s, phase_rotation(a.xi[at] * cnorm(s)));
+            }
+            nxt[i] = s;
         }
         __syncthreads();
         float2* t = cur;
         cur = nxt;
         nxt = t;
-        if (last) chain_store(a, a.y, b, n0, true, [&](int i) { return cur[i]; });
     }
+    chain_store(a, a.y, b, n0, true, [&](int i) { return cur[i]; });
 }
 
+// BWD: the same chain run backwards on gradients -- per layer the gradient
+// through the phase (kept for the tap gradients, and summed for the gain's),
+// then the adjoint filter times the gain.  `dir` is then -1 and the matrices
+// are the adjoint filters'.
+template <bool BWD>
 __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const ChainArgs a) {
     using namespace firtc;
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) unsigned long long done, bfull[2];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
-    __shared__ unsigned s_max[kMaxChain], s_min;
+    __shared__ unsigned s_in, s_max[kMaxChain], s_min;  // largest |.|^2: input, filter inputs
+    __shared__ float s_gxi[kMaxChain];
     __shared__ int s_bad;
     const int ks = ksteps(a.T), cap = qcap(ks), c = (a.T - 1) / 2;
     const uint32_t pitch = 2u * cap, bbytes = STEP_BYTES * ks;
     unsigned char* xs = sm + ((1024u - (tcg::smem_addr(sm) & 1023u)) & 1023u);  // {re hi, im hi, re lo, im lo}
     unsigned char* bs = xs + 4 * (size_t)pitch;                                 // Toeplitz matrices, two for a chain
-    float2* stage = reinterpret_cast<float2*>(bs + (a.layers > 1 ? 2 : 1) * (size_t)bbytes);  // TILE outputs, padded
+    float2* stage = reinterpret_cast<float2*>(bs + (a.layers > 1 ? 2 : 1) * (size_t)bbytes);  // CAP_MAX samples, padded
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.y, n0 = blockIdx.x * a.owned;
+    const size_t row = (size_t)b * a.N;
+    auto load_matrix = [&](int l) {
+        tcg::mbar_expect_tx(&bfull[l & 1], bbytes);
+        tcg::bulk_load(tcg::smem_addr(bs) + (l & 1) * bbytes, a.bmat + (ptrdiff_t)a.dir * l * (ptrdiff_t)bbytes, bbytes,
+                       &bfull[l & 1]);
+    };
 
+    pdl_trigger();
     if (threadIdx.x == 0) {
         abort_flag = 0;
-        for (int i = 0; i < kMaxChain; ++i) s_max[i] = 0u;
+        for (int i = 0; i < kMaxChain; ++i) {
+            s_max[i] = 0u;
+            s_gxi[i] = 0.f;
+        }
+        s_in = 0u;
         s_min = 0x7F7FFFFFu;
         s_bad = 0;
         tcg::mbar_init(&done, 1);
         tcg::mbar_init(&bfull[0], 1);
         tcg::mbar_init(&bfull[1], 1);
         tcg::fence_mbar_init();
-        for (int l = 0; l < 2 && l < a.layers; ++l) {
-            tcg::mbar_expect_tx(&bfull[l], bbytes);
-            tcg::bulk_load(tcg::smem_addr(bs) + l * bbytes, a.bmat + (size_t)l * bbytes, bbytes, &bfull[l]);
-        }
     }
     if (warp == 0) tcg::tmem_alloc(&tmem_base, D_COLS);
+    pdl_wait();  // nothing in global memory is touched before the launches it depends on are done
     __syncthreads();
+    if (threadIdx.x == 0)
+        for (int l = 0; l < 2 && l < a.layers; ++l) load_matrix(l);
     // input: element e of the tile is sample n0 - layers c + e, coalesced into
     // the staging buffer, then 8 consecutive per thread
     constexpr int LOADS = 2;  // 8 x 256 x 2 >= CAP_MAX
-    float2 v[LOADS][8];
-    {
-        const float2* xb = a.x + (size_t)b * a.N;
-        const int base = n0 - a.layers * c, len = TILE + a.T - 1;
-        constexpr int K = CAP_MAX / THREADS;
-        static_assert(CAP_MAX % THREADS == 0 && CAP_MAX >= TILE + FIR_MAX_TAPS - 1 && CAP_MAX <= 8 * LOADS * THREADS, "tile");
+    constexpr int K = CAP_MAX / THREADS;
+    static_assert(CAP_MAX % THREADS == 0 && CAP_MAX >= TILE + FIR_MAX_TAPS - 1 && CAP_MAX <= 8 * LOADS * THREADS, "tile");
+    const int base = n0 - a.layers * c, len = TILE + a.T - 1;
+    auto stage_in = [&](const float2* src, int first) {
         float2 t[K];
 #pragma unroll
         for (int u = 0; u < K; ++u) {
             const int e = threadIdx.x + THREADS * u;
-            t[u] = e < len ? xb[wrap_index(base + e, a.N)] : make_float2(0.f, 0.f);
+            t[u] = e < len ? src[wrap_index(first + e, a.N)] : make_float2(0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < K; ++u) stage[pad(threadIdx.x + THREADS * u)] = t[u];
-        __syncthreads();
+    };
+    float2 v[LOADS][8];
+    stage_in(a.x + row, base);
+    __syncthreads();
+    {
         float mx = 0.f, mn = 3.4e38f;
         bool bad = false;
 #pragma unroll
@@ -291,7 +283,8 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         mn = -warp_max(-mn);
         bad = __any_sync(0xffffffffu, bad);
         if (lane == 0) {
-            atomicMax(&s_max[0], __float_as_uint(mx));
+            atomicMax(&s_in, __float_as_uint(mx));
+            if (!BWD || !a.xi) atomicMax(&s_max[0], __float_as_uint(mx));
             atomicMin(&s_min, __float_as_uint(mn));
             if (bad) s_bad = 1;
         }
@@ -300,15 +293,59 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
     __syncthreads();
     tcg::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const float pmax = __uint_as_float(s_max[0]);
+    const float pmax = __uint_as_float(s_in);
     bool ok = true;
-    if (s_bad || (pmax > 0.f && (!(pmax > 1e-30f) || pmax > 128.f * __uint_as_float(s_min)))) {  // 2^12 over a run's mean
+    if (s_bad || (pmax > 0.f && (!(pmax > 1e-36f) || pmax > 128.f * __uint_as_float(s_min)))) {  // 2^12 over a run's mean
         ok = tcg::mbar_wait(&bfull[0], 0, &abort_flag);  // the copies land before the buffers are reused
         if (a.layers > 1) ok = tcg::mbar_wait(&bfull[1], 0, &abort_flag) && ok;
-        chain_tile_fp32(a, reinterpret_cast<float2*>(sm), b, n0);
+        chain_tile_fp32<BWD>(a, reinterpret_cast<float2*>(sm), b, n0);
         __syncthreads();
         if (warp == 0) tcg::tmem_free(tmem, D_COLS);
         return;
+    }
+    const int o0 = ROW * (32 * (warp & 3) + lane) + OUT * (warp >> 2);  // first output of the thread
+    // Backward, before a layer's filter: the gradient through the phase of the
+    // thread's 8 samples at tile elements e0 .. (layer l, its y in the staging
+    // buffer), with the gain's gradient over the owned samples.
+    auto grad8 = [&](float2 (&g)[8], int e0, int l, float& mx) {
+        const float k = a.xi[(ptrdiff_t)a.dir * l];
+        const int first = (a.layers - l) * c, left = min(a.owned, a.N - n0);
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float d;
+            g[j] = phase_grad(g[j], stage[pad(e0 + j)], k, d);
+            const int i = e0 + j - first;
+            if (i >= 0 && i < left) acc += d;
+            mx = fmaxf(mx, cnorm(g[j]));
+        }
+        return acc;
+    };
+    if (BWD && a.xi) {
+        stage_in(a.act + row, base);
+        __syncthreads();
+        float acc = 0.f, mx = 0.f;
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u) {
+            const int e0 = 8 * (threadIdx.x + THREADS * u);
+            if (e0 < CAP_MAX) acc += grad8(v[u], e0, 0, mx);
+        }
+        mx = warp_max(mx);
+        acc = warp_sum(acc);
+        if (lane == 0) {
+            atomicMax(&s_max[0], __float_as_uint(mx));
+            atomicAdd(&s_gxi[0], acc);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u) {
+            const int e0 = 8 * (threadIdx.x + THREADS * u);
+            if (e0 < CAP_MAX)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) stage[pad(e0 + j)] = v[u][j];
+        }
+        __syncthreads();
+        chain_store(a, a.keep, b, n0, false, [&](int i) { return stage[pad(a.layers * c + i)]; });
     }
     {
         const float sc = pow2(-split_exponent(s_max[0]));
@@ -318,7 +355,6 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
             if (e < cap) split_store8(xs, pitch, e, v[u], sc);
         }
     }
-    const int o0 = ROW * (32 * (warp & 3) + lane) + OUT * (warp >> 2);  // first output of the thread
     for (int l = 0; l < a.layers; ++l) {
         const bool last = l + 1 == a.layers;
         tcg::fence_async_smem();
@@ -329,53 +365,76 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
             ok = tcg::mbar_wait_warp(&bfull[l & 1], (l >> 1) & 1, &abort_flag);
             if (ok) issue(tmem, tcg::smem_addr(xs), pitch, tcg::smem_addr(bs) + (l & 1) * bbytes, ks, &done);
         }
+        // backward: the next layer's y, in flight while the product runs
+        float2 ny[BWD ? TILE / THREADS : 1];
+        if (BWD && !last) {
+            const float2* src = a.act + (ptrdiff_t)a.dir * (l + 1) * (ptrdiff_t)a.stride + row;
+#pragma unroll
+            for (int u = 0; u < TILE / THREADS; ++u)
+                ny[u] = src[wrap_index(base + (l + 1) * c + threadIdx.x + THREADS * u, a.N)];
+        }
         ok = ok && tcg::mbar_wait(&done, l & 1, &abort_flag);
         if (__syncthreads_or(!ok)) {
             ok = false;
             break;
         }
         tcg::fence_after_sync();
-        if (threadIdx.x == 0 && l + 2 < a.layers) {
-            tcg::mbar_expect_tx(&bfull[l & 1], bbytes);
-            tcg::bulk_load(tcg::smem_addr(bs) + (l & 1) * bbytes, a.bmat + (size_t)(l + 2) * bbytes, bbytes, &bfull[l & 1]);
-        }
+        if (threadIdx.x == 0 && l + 2 < a.layers) load_matrix(l + 2);
         float2 y[OUT];
-        read_outputs(tmem, warp, pow2(split_exponent(s_max[l])) * a.unscale[l] * a.gain[l], y);
+        read_outputs(tmem, warp, pow2(split_exponent(s_max[l])) * a.unscale[(ptrdiff_t)a.dir * l] * a.gain[l], y);
         const int first = (a.layers - 1 - l) * c;  // first owned output
-        if (a.keep) {
+        float mx = 0.f;
+        if (BWD) {
+            if (!last) {
 #pragma unroll
-            for (int r = 0; r < OUT; ++r) stage[pad(o0 + r)] = y[r];
-            __syncthreads();
-            chain_store(a, a.keep + l * a.keep_stride, b, n0, false, [&](int i) { return stage[pad(first + i)]; });
-        }
-        // the phase keeps |y|, whose largest value scales the next layer's input
-        float pw[OUT], mx = 0.f;
+                for (int u = 0; u < TILE / THREADS; ++u) stage[pad(threadIdx.x + THREADS * u)] = ny[u];
+                __syncthreads();
+                const float acc = warp_sum(grad8(y, o0, l + 1, mx));
+                if (lane == 0) atomicAdd(&s_gxi[l + 1], acc);
+                __syncthreads();
+            }
+        } else {
+            if (a.keep) {
 #pragma unroll
-        for (int r = 0; r < OUT; ++r) {
-            pw[r] = cnorm(y[r]);
-            mx = fmaxf(mx, pw[r]);
-        }
-        if (!last) {
-            const float wm = warp_max(mx);
-            if (lane == 0) atomicMax(&s_max[l + 1], __float_as_uint(wm));
-        }
-        if (a.xi) {
-            const float k = a.xi[l];
-            if (fabsf(k) * mx <= kPhaseSmall) {
+                for (int r = 0; r < OUT; ++r) stage[pad(o0 + r)] = y[r];
+                __syncthreads();
+                chain_store(a, a.keep + (ptrdiff_t)a.dir * l * (ptrdiff_t)a.stride, b, n0, false,
+                            [&](int i) { return stage[pad(first + i)]; });
+            }
+            // the phase keeps |y|, whose largest value scales the next layer's input
+            float pw[OUT];
 #pragma unroll
-                for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation_small(k * pw[r]));
-            } else {
+            for (int r = 0; r < OUT; ++r) {
+                pw[r] = cnorm(y[r]);
+                mx = fmaxf(mx, pw[r]);
+            }
+            if (a.xi) {
+                const float k = a.xi[(ptrdiff_t)a.dir * l];
+                if (fabsf(k) * mx <= kPhaseSmall) {
 #pragma unroll
-                for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation(k * pw[r]));
+                    for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation_small(k * pw[r]));
+                } else {
+#pragma unroll
+                    for (int r = 0; r < OUT; ++r) y[r] = cmul(y[r], phase_rotation(k * pw[r]));
+                }
             }
         }
-        if (last) {
-            if (a.keep) __syncthreads();
+        if (!last) {
+            mx = warp_max(mx);
+            if (lane == 0) atomicMax(&s_max[l + 1], __float_as_uint(mx));
+        }
+        if (last || BWD) {
+            // staged: the result, or backward the gradient behind the next phase
+            if (a.keep && !BWD) __syncthreads();
 #pragma unroll
             for (int r = 0; r < OUT; ++r) stage[pad(o0 + r)] = y[r];
             __syncthreads();
-            chain_store(a, a.y, b, n0, true, [&](int i) { return stage[pad(i)]; });
-            break;
+            if (last) {
+                chain_store(a, a.y, b, n0, true, [&](int i) { return stage[pad(i)]; });
+                break;
+            }
+            chain_store(a, a.keep + (ptrdiff_t)a.dir * (l + 1) * (ptrdiff_t)a.stride, b, n0, false,
+                        [&](int i) { return stage[pad(first + i)]; });
         }
         // the outputs are the next layer's inputs at the same places; the
         // elements behind them (no longer valid) become zero
@@ -402,28 +461,47 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         __syncthreads();
         const float nan = __int_as_float(0x7fc00000);
         chain_store(a, a.y, b, n0, true, [&](int) { return make_float2(nan, nan); });
+        if (threadIdx.x < a.layers) s_gxi[threadIdx.x] = nan;
     }
+    if (BWD && a.xi && threadIdx.x < a.layers) atomicAdd(a.gxi + (ptrdiff_t)a.dir * (int)threadIdx.x, s_gxi[threadIdx.x]);
     tcg::fence_before_sync();
     __syncthreads();
     tcg::fence_after_sync();
     if (warp == 0) tcg::tmem_free(tmem, D_COLS);
 }
 
-// g_h[t] += sum_n g_y[n] conj(x[(n + t - c) mod N]) over all realizations.
+// Tap gradients of the layers first .. first + gridDim.z - 1 in one launch:
+//   g_h[t] += scale sum_n g_y[n] conj(x[(n + t - c) mod N]) over all realizations,
+// x = the input for layer 0, else the phase of layer k - 1 applied to its kept
+// y again, scale = span_scale in the first layer of a span.
 // Warp w takes taps 8w .. 8w + 7 (+ 64 per round for longer filters), lane l
 // the 8 consecutive samples 8l .. 8l + 7 of each 256-sample chunk of the
 // 2048-sample tile: per (chunk, 8 taps) a 15-sample register window and 8 gradient
 // samples give 64 products; lanes meet in a warp sum, CTAs in atomics.
-__global__ void __launch_bounds__(FIR_GRAD_THREADS) fir_grad_taps_kernel(const float2* __restrict__ x,
-                                                                         const float2* __restrict__ gy, int T,
-                                                                         float2* __restrict__ gh, int N) {
+struct TapGrad {
+    const float2* x0;    // batch x N: the input of layer 0
+    const float2* act;   // kept y of all layers, `stride` apart
+    const float2* gy;    // gradients of y, from layer `first` on, `stride` apart
+    size_t stride;
+    const float* xi;     // gains of all layers
+    float2* gh;          // T per layer, from layer `first` on
+    float span_scale;
+    int first, steps, T, N;
+};
+__global__ void __launch_bounds__(FIR_GRAD_THREADS) fir_grad_taps_kernel(const TapGrad p) {
     __shared__ float2 xs[FIR_GRAD_XS];
     __shared__ float2 gs[FIR_GRAD_TILE * 9 / 8];
-    const int b = blockIdx.y;
+    const int b = blockIdx.y, N = p.N, T = p.T;
     const int n0 = blockIdx.x * FIR_GRAD_TILE;
     const int c = (T - 1) / 2;
     const int Tp = (T + 7) & ~7;
-    fir_load_window<FIR_GRAD_THREADS, FIR_GRAD_TILE, 8>(xs, x + (size_t)b * N, n0, c, FIR_GRAD_TILE + Tp, N);
+    const int k = p.first + blockIdx.z;
+    const float2* x = k ? p.act + (size_t)(k - 1) * p.stride : p.x0;
+    const float2* gy = p.gy + (size_t)blockIdx.z * p.stride;
+    float2* gh = p.gh + (size_t)blockIdx.z * T;
+    const float scale = k % p.steps == 0 ? p.span_scale : 1.0f;
+    fir_load_window<FIR_GRAD_THREADS, FIR_GRAD_TILE, 8>(xs, x + (size_t)b * N, n0, c, FIR_GRAD_TILE + Tp, N,
+                                                        k ? p.xi + (k - 1) : nullptr);
     {
         constexpr int K = FIR_GRAD_TILE / FIR_GRAD_THREADS;
         float2 v[K];
@@ -456,7 +534,7 @@ __global__ void __launch_bounds__(FIR_GRAD_THREADS) fir_grad_taps_kernel(const f
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const float sx = warp_sum(acc[j].x), sy = warp_sum(acc[j].y);
+            const float sx = warp_sum(acc[j].x) * scale, sy = warp_sum(acc[j].y) * scale;
             if (lane == 0 && t0 + j < T) {
                 atomicAdd(&gh[t0 + j].x, sx);
                 atomicAdd(&gh[t0 + j].y, sy);
@@ -465,62 +543,18 @@ __global__ void __launch_bounds__(FIR_GRAD_THREADS) fir_grad_taps_kernel(const f
     }
 }
 
-// y = x exp(i xi |x|^2)
-__global__ void nl_kernel(const float2* __restrict__ x, const float* __restrict__ xi, float2* __restrict__ y,
-                          size_t n) {
-    const float k = *xi;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        y[i] = cmul(x[i], phase_rotation(k * cnorm(x[i])));
-}
-
-// Backward of y = x e^{i phi}, phi = xi |x|^2:
-//   g_x = g_y e^{-i phi} (1 - i xi p) + conj(g_y) i xi x^2 e^{i phi}
-//   dL/dxi = 2 Re(conj(g_y) i p y)
-__global__ void nl_grad_kernel(const float2* __restrict__ x, const float* __restrict__ xi,
-                               const float2* __restrict__ gy, float2* __restrict__ gx, float* __restrict__ gxi,
-                               size_t n) {
-    const float k = *xi;
-    float acc = 0.f;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float2 xv = x[i], g = gy[i];
-        const float p = cnorm(xv);
-        const float2 e = phase_rotation(k * p);                  // e^{i phi}
-        const float2 y = cmul(xv, e);
-        const float2 t1 = cmul(g, make_float2(e.x, -e.y));       // g e^{-i phi}
-        const float2 a = cmul(t1, make_float2(1.f, -k * p));     // (1 - i xi p)
-        const float2 x2 = cmul(xv, xv);
-        const float2 b = cmul(cmul(make_float2(g.x, -g.y), x2), e);  // conj(g) x^2 e^{i phi}
-        gx[i] = make_float2(a.x - k * b.y, a.y + k * b.x);       // + i xi b
-        // 2 Re(conj(g) * i p y) = -2 p Im(conj(g) y)
-        const float2 gy_ = cmul(make_float2(g.x, -g.y), y);
-        acc += -2.f * p * gy_.y;
-    }
-    __shared__ float red[64];
-    float dummy = 0.f;
-    float s = acc;
-    block_max_sum(dummy, s, red);
-    if (threadIdx.x == 0) atomicAdd(gxi, s);
-}
-
-// symbols = y[0::2]; loss = mean |symbols - t|^2, g_y = 0 at odd samples.
-__global__ void mse_decimate_kernel(const float2* __restrict__ y, const float2* __restrict__ tx, int N,
-                                    size_t n_sym_total, float inv_count, float2* __restrict__ sym,
-                                    float2* __restrict__ gy, double* __restrict__ loss) {
+// loss = mean |sym - t|^2 and the gradient at 2 samples/symbol (0 at odd samples).
+__global__ void mse_kernel(const float2* __restrict__ sym, const float2* __restrict__ tx, size_t n_sym_total,
+                           float inv_count, float4* __restrict__ gy, double* __restrict__ loss) {
     double acc = 0.0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n_sym_total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t b = i / (N / 2), k = i % (N / 2);
-        const float2 v = y[b * N + 2 * k];
-        if (sym) sym[i] = v;
-        if (gy) {
-            const float2 d = csub(v, tx[i]);
-            gy[b * N + 2 * k] = cscale(d, inv_count);
-            gy[b * N + 2 * k + 1] = make_float2(0.f, 0.f);
-            acc += (double)cnorm(d);
-        }
+        const float2 d = csub(sym[i], tx[i]);
+        gy[i] = make_float4(d.x * inv_count, d.y * inv_count, 0.f, 0.f);
+        acc += (double)cnorm(d);
     }
     __shared__ double sd[32];
     acc = block_sum_d(acc, sd);
-    if (threadIdx.x == 0 && loss) atomicAdd(loss, acc * inv_count);
+    if (threadIdx.x == 0) atomicAdd(loss, acc * inv_count);
 }
 
 // Adam on n real parameters (complex parameters as interleaved pairs; the
@@ -554,13 +588,13 @@ struct LdbpModel {
     float* m1 = nullptr;
     float* m2 = nullptr;
     int adam_t = 0;
-    float2* acts = nullptr;  // (2*spans*steps + 1) activations of batch*samples
+    float2* acts = nullptr;  // per layer y, then per layer the gradient there, of batch*samples
     float2* work = nullptr;  // 2 work buffers of batch*samples
     float2* sym = nullptr;   // batch*samples/2
     double* loss = nullptr;
-    unsigned char* bmat = nullptr;  // Toeplitz matrices of the layers, then of the matched filter
+    unsigned char* bmat = nullptr;  // Toeplitz matrices of the layers, of the matched filter; the adjoints'
     float* unscale = nullptr;       // their scales
-    bool stale = true;              // parameters changed since they were built
+    bool stale[2] = {true, true};   // parameters changed since they were built: filters, adjoint filters
     size_t field_n() const { return (size_t)batch * samples; }
     float2* h(int k) const { return (float2*)params + (size_t)k * taps; }
     float* xi(int k) const { return params + (size_t)spans * steps * taps * 2 + k; }
@@ -584,31 +618,46 @@ using fg::count_launch;
 
 static focss_status ldbp_err(focss_ctx* c, cudaError_t e, const char* what) { return fg::cuda_check(c, e, what); }
 
-// Toeplitz matrices of the current parameters.
+// Toeplitz matrices of the current parameters' filters, or of their adjoints.
 static size_t layer_bytes(const LdbpModel& M) { return (size_t)fg::firtc::STEP_BYTES * fg::firtc::ksteps(M.taps); }
-static cudaError_t ldbp_matrices(LdbpModel& M) {
-    if (!M.stale) return cudaSuccess;
+static size_t matrices_bytes(const LdbpModel& M) {
+    return (size_t)M.spans * M.steps * layer_bytes(M) + (size_t)fg::firtc::STEP_BYTES * fg::firtc::ksteps(M.mf_taps);
+}
+static unsigned char* matrix(const LdbpModel& M, int k, int adjoint) {
+    return M.bmat + adjoint * matrices_bytes(M) + k * layer_bytes(M);
+}
+static float* unscale(const LdbpModel& M, int k, int adjoint) { return M.unscale + adjoint * (M.spans * M.steps + 1) + k; }
+static cudaError_t ldbp_matrices(LdbpModel& M, int adjoint) {
+    if (!M.stale[adjoint]) return cudaSuccess;
     const int L = M.spans * M.steps;
-    fg::firtc::toeplitz_kernel<<<L, 256, 0, M.ctx->stream>>>(M.h(0), M.taps, 0, (__half*)M.bmat, M.unscale);
-    fg::firtc::toeplitz_kernel<<<1, 256, 0, M.ctx->stream>>>(M.hmf(), M.mf_taps, 0, (__half*)(M.bmat + L * layer_bytes(M)),
-                                                            M.unscale + L);
-    count_launch(2);
-    M.stale = false;
-    return cudaGetLastError();
+    fg::firtc::toeplitz_kernel<<<L + 1, 256, 0, M.ctx->stream>>>(M.h(0), M.taps, L, M.hmf(), M.mf_taps, adjoint,
+                                                                (__half*)matrix(M, 0, adjoint), unscale(M, 0, adjoint));
+    count_launch();
+    const cudaError_t e = cudaGetLastError();
+    M.stale[adjoint] = e != cudaSuccess;
+    return e;
 }
 
+// layers per launch: the halo a chain computes twice stays below an eighth
+static int chain_length(const LdbpModel& M) {
+    return std::max(1, std::min(fg::kMaxChain, 1 + 256 / std::max(1, M.taps - 1)));
+}
+
+template <bool BWD>
 static cudaError_t launch_chain(const LdbpModel& M, fg::ChainArgs& a) {
     using namespace fg::firtc;
     a.N = M.samples;
+    a.dir = BWD ? -1 : 1;
+    a.stride = M.field_n();
     a.owned = TILE - (a.layers - 1) * (a.T - 1);
     const int ks = ksteps(a.T);
     const size_t smem = 1024 + 8 * (size_t)qcap(ks) + (a.layers > 1 ? 2 : 1) * (size_t)STEP_BYTES * ks +
                         sizeof(float2) * pad(CAP_MAX);
     // a tile in FP32 takes two plain buffers instead
     const size_t need = std::max(smem, sizeof(float2) * 2 * (size_t)(TILE + a.T - 1));
-    cudaError_t e = cudaFuncSetAttribute(fg::ldbp_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    cudaError_t e = cudaFuncSetAttribute(fg::ldbp_chain_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
     if (e != cudaSuccess) return e;
-    fg::ldbp_chain_kernel<<<dim3((M.samples + a.owned - 1) / a.owned, M.batch), THREADS, need, M.ctx->stream>>>(a);
+    fg::ldbp_chain_kernel<BWD><<<dim3((M.samples + a.owned - 1) / a.owned, M.batch), THREADS, need, M.ctx->stream>>>(a);
     count_launch();
     return cudaGetLastError();
 }
@@ -619,10 +668,9 @@ static cudaError_t launch_chain(const LdbpModel& M, fg::ChainArgs& a) {
 static cudaError_t ldbp_chains(LdbpModel& M, const float2* in, bool keep, float2* symbols) {
     const size_t n = M.field_n();
     const int L = M.spans * M.steps;
-    cudaError_t e = ldbp_matrices(M);
+    cudaError_t e = ldbp_matrices(M, 0);
     float2* bufs[2] = {M.work, M.work + n};
-    // layers per launch: the halo a chain computes twice stays below an eighth
-    const int F = std::max(1, std::min(fg::kMaxChain, 1 + 256 / std::max(1, M.taps - 1)));
+    const int F = chain_length(M);
     const float2* src = in;
     int w = 0;
     for (int k = 0; k < L && e == cudaSuccess; k += F) {
@@ -632,13 +680,12 @@ static cudaError_t ldbp_chains(LdbpModel& M, const float2* in, bool keep, float2
         a.x = src;
         a.y = bufs[w];
         a.keep = keep ? M.acts + (size_t)k * n : nullptr;
-        a.keep_stride = n;
-        a.bmat = M.bmat + k * layer_bytes(M);
-        a.unscale = M.unscale + k;
+        a.bmat = matrix(M, k, 0);
+        a.unscale = unscale(M, k, 0);
         a.h = M.h(k);
         a.xi = M.xi(k);
         for (int l = 0; l < a.layers; ++l) a.gain[l] = (k + l) % M.steps == 0 ? M.span_scale : 1.0f;
-        e = launch_chain(M, a);
+        e = launch_chain<false>(M, a);
         src = bufs[w];
         w ^= 1;
     }
@@ -649,54 +696,66 @@ static cudaError_t ldbp_chains(LdbpModel& M, const float2* in, bool keep, float2
         a.x = src;
         a.y = symbols;
         a.decimate = 1;
-        a.bmat = M.bmat + L * layer_bytes(M);
-        a.unscale = M.unscale + L;
+        a.bmat = matrix(M, L, 0);
+        a.unscale = unscale(M, L, 0);
         a.h = M.hmf();
         a.gain[0] = 1.0f;
-        e = launch_chain(M, a);
+        e = launch_chain<false>(M, a);
     }
     return e;
 }
 
-static cudaError_t fir(const LdbpModel& M, const float2* x, const float2* h, int T, int conj_rev, float2* y,
-                       float gain = 1.0f, const float* xi = nullptr) {
-    dim3 g((M.samples + fg::FIR_TILE - 1) / fg::FIR_TILE, M.batch);
-    fg::fir_kernel<<<g, fg::FIR_THREADS, 0, M.ctx->stream>>>(x, h, T, conj_rev, y, M.samples, gain, xi);
-    count_launch();
-    return cudaGetLastError();
-}
-
-// Forward pass; keeps every layer input in M.acts when `keep`.
-static cudaError_t ldbp_forward(LdbpModel& M, const float2* in, bool keep) {
-    cudaStream_t s = M.ctx->stream;
+// Gradients of everything from gy, the gradient of the matched filter's output
+// (in M.work): the adjoint chains, then the tap gradients from what they and
+// the forward pass kept.
+static cudaError_t ldbp_backward(LdbpModel& M, const float2* in) {
     const size_t n = M.field_n();
-    float2* cur = M.work;
-    float2* nxt = M.work + n;
-    cudaError_t e = cudaMemcpyAsync(cur, in, sizeof(float2) * n, cudaMemcpyDeviceToDevice, s);
-    int a = 0;
-    for (int sp = 0; sp < M.spans && e == cudaSuccess; ++sp) {
-        e = fg::launch_scale(cur, n, make_float2(M.span_scale, 0.f), s);
-        for (int st = 0; st < M.steps && e == cudaSuccess; ++st) {
-            const int k = sp * M.steps + st;
-            if (keep) e = cudaMemcpyAsync(M.acts + (size_t)(a++) * n, cur, sizeof(float2) * n, cudaMemcpyDeviceToDevice, s);
-            if (e == cudaSuccess) e = fir(M, cur, M.h(k), M.taps, 0, nxt);
-            std::swap(cur, nxt);
-            if (keep && e == cudaSuccess)
-                e = cudaMemcpyAsync(M.acts + (size_t)(a++) * n, cur, sizeof(float2) * n, cudaMemcpyDeviceToDevice, s);
-            if (e == cudaSuccess) {
-                fg::nl_kernel<<<gridn(n), 256, 0, s>>>(cur, M.xi(k), nxt, n);
-                count_launch();
-                e = cudaGetLastError();
-            }
-            std::swap(cur, nxt);
-        }
+    const int L = M.spans * M.steps;
+    cudaStream_t s = M.ctx->stream;
+    const dim3 tiles((M.samples + fg::FIR_GRAD_TILE - 1) / fg::FIR_GRAD_TILE, M.batch);
+    float2* bufs[2] = {M.work, M.work + n};
+    fg::TapGrad t{in, M.acts, M.work, n, M.xi(0), M.ghmf(), 1.0f, L, M.steps, M.mf_taps, M.samples};
+    cudaError_t e = ldbp_matrices(M, 1);
+    if (e != cudaSuccess) return e;
+    fg::fir_grad_taps_kernel<<<tiles, fg::FIR_GRAD_THREADS, 0, s>>>(t);
+    count_launch();
+    e = cudaGetLastError();
+    fg::ChainArgs m{};
+    m.layers = 1;
+    m.T = M.mf_taps;
+    m.x = bufs[0];
+    m.y = bufs[1];
+    m.bmat = matrix(M, L, 1);
+    m.unscale = unscale(M, L, 1);
+    m.h = M.hmf();
+    m.gain[0] = 1.0f;
+    if (e == cudaSuccess) e = launch_chain<true>(M, m);
+    const int F = chain_length(M);
+    int w = 1;
+    for (int k = L - 1; k >= 0 && e == cudaSuccess; k -= F) {
+        fg::ChainArgs a{};
+        a.layers = std::min(F, k + 1);
+        a.T = M.taps;
+        a.x = bufs[w];
+        a.y = bufs[w ^ 1];
+        a.keep = M.acts + (size_t)(L + k) * n;
+        a.act = M.acts + (size_t)k * n;
+        a.bmat = matrix(M, k, 1);
+        a.unscale = unscale(M, k, 1);
+        a.h = M.h(k);
+        a.xi = M.xi(k);
+        a.gxi = M.gxi(k);
+        for (int l = 0; l < a.layers; ++l) a.gain[l] = (k - l) % M.steps == 0 ? M.span_scale : 1.0f;
+        e = launch_chain<true>(M, a);
+        w ^= 1;
     }
-    if (keep && e == cudaSuccess)
-        e = cudaMemcpyAsync(M.acts + (size_t)(a++) * n, cur, sizeof(float2) * n, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = fir(M, cur, M.hmf(), M.mf_taps, 0, nxt);
-    // result (2 sps, before decimation) is left in work[1] when the layer count is even
-    if (nxt != M.work + n && e == cudaSuccess)
-        e = cudaMemcpyAsync(M.work + n, nxt, sizeof(float2) * n, cudaMemcpyDeviceToDevice, s);
+    // gridDim.z is at most 65535
+    for (int k = 0; k < L && e == cudaSuccess; k += 32768) {
+        fg::TapGrad a{in, M.acts, M.acts + (size_t)(L + k) * n, n, M.xi(0), M.gh(k), M.span_scale, k, M.steps, M.taps, M.samples};
+        fg::fir_grad_taps_kernel<<<dim3(tiles.x, tiles.y, std::min(L - k, 32768)), fg::FIR_GRAD_THREADS, 0, s>>>(a);
+        count_launch();
+        e = cudaGetLastError();
+    }
     return e;
 }
 
@@ -721,7 +780,7 @@ FOCSS_API focss_status focss_ldbp_create(focss_ctx* c, int spans, int steps_per_
     m->span_scale = (float)span_scale;
     m->n_params = spans * steps_per_span * 2 * taps + m->xi_count() + 2 * mf_taps;
     const size_t n = m->field_n();
-    const size_t n_acts = (size_t)2 * spans * steps_per_span + 1;
+    const size_t n_acts = (size_t)2 * spans * steps_per_span;
     cudaError_t e = cudaMalloc(&m->params, sizeof(float) * 4 * (size_t)m->n_params);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->params, 0, sizeof(float) * 4 * (size_t)m->n_params, c->stream);
     m->grads = m->params + m->n_params;
@@ -733,8 +792,8 @@ FOCSS_API focss_status focss_ldbp_create(focss_ctx* c, int spans, int steps_per_
     if (e == cudaSuccess) e = cudaMalloc(&m->loss, sizeof(double) * 2);
     const size_t nl = (size_t)spans * steps_per_span;
     if (e == cudaSuccess)
-        e = cudaMalloc(&m->bmat, nl * layer_bytes(*m) + (size_t)fg::firtc::STEP_BYTES * fg::firtc::ksteps(mf_taps));
-    if (e == cudaSuccess) e = cudaMalloc(&m->unscale, sizeof(float) * (nl + 1));
+        e = cudaMalloc(&m->bmat, 2 * matrices_bytes(*m));
+    if (e == cudaSuccess) e = cudaMalloc(&m->unscale, sizeof(float) * 2 * (nl + 1));
     if (e != cudaSuccess) {
         cudaFree(m->params);
         cudaFree(m->acts);
@@ -770,7 +829,7 @@ FOCSS_API focss_status focss_ldbp_set_params(focss_ldbp* m, const float* host, i
     if (e == cudaSuccess) e = cudaMemsetAsync(m->m1, 0, sizeof(float) * 2 * n, m->ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->ctx->stream);
     m->adam_t = 0;
-    m->stale = true;
+    m->stale[0] = m->stale[1] = true;
     return ldbp_err(m->ctx, e, "ldbp set params");
 }
 
@@ -801,51 +860,16 @@ FOCSS_API focss_status focss_ldbp_loss_grad(focss_ldbp* m, const focss_field* in
         tx->samples != m->samples / 2 || tx->batch != m->batch)
         return fg::set_error(m->ctx, FOCSS_ERR_INVALID_ARG, "ldbp_loss_grad: shapes");
     cudaStream_t s = m->ctx->stream;
-    const size_t n = m->field_n();
     const size_t ns = (size_t)m->batch * (m->samples / 2);
-    cudaError_t e = ldbp_forward(*m, in->d, true);
+    cudaError_t e = ldbp_chains(*m, in->d, true, m->sym);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->grads, 0, sizeof(float) * m->n_params, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->loss, 0, sizeof(double), s);
-    float2* g = m->work;           // gradient w.r.t. the current layer output
-    float2* g2 = m->work + n;      // (work[1] holds y; reused after the loss)
-    float2* ybuf = m->work + n;
     if (e == cudaSuccess) {
-        // y lives in work[1]; write the output gradient into work[0]
-        fg::mse_decimate_kernel<<<gridn(ns), 256, 0, s>>>(ybuf, tx->d, m->samples, ns, 1.f / (float)ns, m->sym, g,
-                                                          m->loss);
+        fg::mse_kernel<<<gridn(ns), 256, 0, s>>>(m->sym, tx->d, ns, 1.f / (float)ns, (float4*)m->work, m->loss);
         count_launch();
         e = cudaGetLastError();
     }
-    const int L = m->spans * m->steps;
-    int a = 2 * L;  // index of the matched filter's input activation
-    dim3 gg((m->samples + fg::FIR_GRAD_TILE - 1) / fg::FIR_GRAD_TILE, m->batch);
-    // matched filter
-    if (e == cudaSuccess) {
-        fg::fir_grad_taps_kernel<<<gg, fg::FIR_GRAD_THREADS, 0, s>>>(m->acts + (size_t)a * n, g, m->mf_taps, m->ghmf(), m->samples);
-        count_launch();
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = fir(*m, g, m->hmf(), m->mf_taps, 1, g2);
-    std::swap(g, g2);
-    for (int sp = m->spans - 1; sp >= 0 && e == cudaSuccess; --sp) {
-        for (int st = m->steps - 1; st >= 0 && e == cudaSuccess; --st) {
-            const int k = sp * m->steps + st;
-            --a;  // NL input
-            fg::nl_grad_kernel<<<gridn(n), 256, 0, s>>>(m->acts + (size_t)a * n, m->xi(k), g, g2, m->gxi(k), n);
-            count_launch();
-            e = cudaGetLastError();
-            std::swap(g, g2);
-            --a;  // FIR input
-            if (e == cudaSuccess) {
-                fg::fir_grad_taps_kernel<<<gg, fg::FIR_GRAD_THREADS, 0, s>>>(m->acts + (size_t)a * n, g, m->taps, m->gh(k), m->samples);
-                count_launch();
-                e = cudaGetLastError();
-            }
-            if (e == cudaSuccess) e = fir(*m, g, m->h(k), m->taps, 1, g2);
-            std::swap(g, g2);
-        }
-        if (e == cudaSuccess) e = fg::launch_scale(g, n, make_float2(m->span_scale, 0.f), s);
-    }
+    if (e == cudaSuccess) e = ldbp_backward(*m, in->d);
     double h_loss = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -857,7 +881,7 @@ FOCSS_API focss_status focss_ldbp_adam_step(focss_ldbp* m, double lr, double lr_
                                             double eps) {
     if (!m) return FOCSS_ERR_INVALID_ARG;
     m->adam_t += 1;
-    m->stale = true;
+    m->stale[0] = m->stale[1] = true;
     const float c1 = (float)(1.0 / (1.0 - std::pow(beta1, m->adam_t)));
     const float c2 = (float)(1.0 / (1.0 - std::pow(beta2, m->adam_t)));
     // complex gradients g = dL/dconj(z) -> real gradient 2 g; xi gradients are already real:
