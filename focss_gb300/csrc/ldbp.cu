@@ -22,16 +22,7 @@
 
 namespace fg {
 
-constexpr int FIR_GRAD_THREADS = 256;               // fir_grad_taps_kernel: 8 warps x 8 taps
-constexpr int FIR_GRAD_TILE = 2048;                 // samples per CTA of fir_grad_taps_kernel
 constexpr int FIR_MAX_TAPS = 255;
-constexpr int FIR_TAPS_PAD = (FIR_MAX_TAPS + 7) / 8 * 8;
-// Shared-memory sample windows keep one padding slot after every R samples,
-// R the run a thread reads from a multiple of R: runs of 8 start 72 bytes
-// apart across a half-warp, on distinct bank pairs.
-template <int R>
-__device__ __forceinline__ int fir_pad(int i) { return i + i / R; }
-constexpr int FIR_GRAD_XS = (FIR_GRAD_TILE + FIR_TAPS_PAD + 8) * 9 / 8;
 
 __device__ __forceinline__ int wrap_index(int s, int N) {
     if (s < 0 || s >= N) {
@@ -39,41 +30,6 @@ __device__ __forceinline__ int wrap_index(int s, int N) {
         if (s < 0) s += N;
     }
     return s;
-}
-
-// Loads samples [n0 - c, n0 - c + span) of one realization (circular) into
-// the padded window: all of a thread's loads are issued before the first
-// store (a load-store loop would wait for one load latency per iteration).
-// With xi, the samples' nonlinear phase exp(i xi |x|^2) is applied.
-template <int THREADS, int TILE, int R>
-__device__ __forceinline__ void fir_load_window(float2* xs, const float2* __restrict__ xb, int n0, int c, int span,
-                                                int N, const float* xi) {
-    constexpr int K = (TILE + FIR_TAPS_PAD + THREADS - 1) / THREADS;
-    float2 v[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int i = threadIdx.x + k * THREADS;
-        v[k] = i < span ? xb[wrap_index(n0 - c + i, N)] : make_float2(0.f, 0.f);
-    }
-    if (xi) {
-        const float g = *xi;
-        float mx = 0.f;
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            mx = fmaxf(mx, cnorm(v[k]));
-        if (fabsf(g) * mx <= kPhaseSmall) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) v[k] = cmul(v[k], phase_rotation_small(g * cnorm(v[k])));
-        } else {
-#pragma unroll
-            for (int k = 0; k < K; ++k) v[k] = cmul(v[k], phase_rotation(g * cnorm(v[k])));
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int i = threadIdx.x + k * THREADS;
-        if (i < span) xs[fir_pad<R>(i)] = v[k];
-    }
 }
 
 // ---------------------------------------------------------------- chains of layers
@@ -114,15 +70,12 @@ struct ChainArgs {
 // Gradient through y e^{i phi}, phi = xi |y|^2, from g = dL/dconj of the output:
 //   g_y = g e^{-i phi} (1 - i xi p) + conj(g) i xi y^2 e^{i phi},
 //   dL/dxi += 2 Re(conj(g) i p y e^{i phi})
-__device__ __forceinline__ float2 phase_grad(float2 g, float2 y, float k, float& gxi) {
-    const float p = cnorm(y);
-    const float2 e = phase_rotation(k * p);
-    const float2 z = cmul(y, e);
-    const float2 a = cmul(cmul(g, make_float2(e.x, -e.y)), make_float2(1.f, -k * p));
-    const float2 gc = make_float2(g.x, -g.y);
-    const float2 b = cmul(cmul(gc, cmul(y, y)), e);
-    gxi = -2.f * p * cmul(gc, z).y;
-    return make_float2(a.x - k * b.y, a.y + k * b.x);
+// `e` = e^{i phi}, p = |y|^2.
+__device__ __forceinline__ float2 phase_grad(float2 g, float2 y, float p, float2 e, float k, float& gxi) {
+    const float2 q = cmul(make_float2(g.x, -g.y), cmul(y, e)), b = cmul(q, y), ge = cmulc(g, e);
+    const float kp = k * p;
+    gxi = -2.f * p * q.y;
+    return make_float2(fmaf(-k, b.y, fmaf(kp, ge.y, ge.x)), fmaf(k, b.x, fmaf(-kp, ge.x, ge.y)));
 }
 
 // The CTA's owned samples of a layer's output `v(i)`, i = 0 .. owned-1, to dst.
@@ -157,8 +110,10 @@ __device__ __noinline__ void chain_tile_fp32(const ChainArgs& a, float2* buf, in
             float acc = 0.f;
             for (int i = threadIdx.x; i < valid; i += firtc::THREADS) {
                 const int n = n0 + i - first;
+                const float2 y = a.act[at * (ptrdiff_t)a.stride + row + wrap_index(n, a.N)];
+                const float p = cnorm(y), k = a.xi[at];
                 float d;
-                cur[i] = phase_grad(cur[i], a.act[at * (ptrdiff_t)a.stride + row + wrap_index(n, a.N)], a.xi[at], d);
+                cur[i] = phase_grad(cur[i], y, p, phase_rotation(k * p), k, d);
                 if (i >= first && i < first + a.owned && n < a.N) {
                     a.keep[at * (ptrdiff_t)a.stride + row + n] = cur[i];
                     acc += d;
@@ -310,13 +265,25 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
     auto grad8 = [&](float2 (&g)[8], int e0, int l, float& mx) {
         const float k = a.xi[(ptrdiff_t)a.dir * l];
         const int first = (a.layers - l) * c, left = min(a.owned, a.N - n0);
-        float acc = 0.f;
+        float2 y[8];
+        float p[8], d[8], pm = 0.f, acc = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            float d;
-            g[j] = phase_grad(g[j], stage[pad(e0 + j)], k, d);
+            y[j] = stage[pad(e0 + j)];
+            p[j] = cnorm(y[j]);
+            pm = fmaxf(pm, p[j]);
+        }
+        if (fabsf(k) * pm <= kPhaseSmall) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) g[j] = phase_grad(g[j], y[j], p[j], phase_rotation_small(k * p[j]), k, d[j]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) g[j] = phase_grad(g[j], y[j], p[j], phase_rotation(k * p[j]), k, d[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
             const int i = e0 + j - first;
-            if (i >= 0 && i < left) acc += d;
+            if (i >= 0 && i < left) acc += d[j];
             mx = fmaxf(mx, cnorm(g[j]));
         }
         return acc;
@@ -470,14 +437,34 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
     if (warp == 0) tcg::tmem_free(tmem, D_COLS);
 }
 
-// Tap gradients of the layers first .. first + gridDim.z - 1 in one launch:
+// ---------------------------------------------------------------- tap gradients
+// Of the layers first .. first + gridDim.z - 1 in one launch:
 //   g_h[t] += scale sum_n g_y[n] conj(x[(n + t - c) mod N]) over all realizations,
 // x = the input for layer 0, else the phase of layer k - 1 applied to its kept
 // y again, scale = span_scale in the first layer of a span.
-// Warp w takes taps 8w .. 8w + 7 (+ 64 per round for longer filters), lane l
-// the 8 consecutive samples 8l .. 8l + 7 of each 256-sample chunk of the
-// 2048-sample tile: per (chunk, 8 taps) a 15-sample register window and 8 gradient
-// samples give 64 products; lanes meet in a warp sum, CTAs in atomics.
+//
+// On the tensor cores: with the window w[i] = x[n0 - c + i] and n = n0 + 32 b + r,
+//   D[m][r] = sum_b w[32 b + m] g_y[32 b + r],  g_h[t] = sum_r D[t + r][r],
+// a product over the 64 blocks b of a 2048-sample tile whose operands are the
+// plain arrays w and g_y: element (k = b, m) of an MN-major operand with 64-byte
+// rows lies 32 k + m elements from the start, so the Hankel matrix is w itself
+// with its 32-element groups along M 64 bytes apart.  M = 128 takes filters of
+// up to 97 taps; longer ones take further CTAs (blockIdx.y) 128 samples on.
+// Both are split in two FP16 words, the leading ones multiples of 2^-11 (their
+// products add up exactly while a sum stays below 4, and truncate by at most
+// 2^-19 of the largest product there could be beyond); the columns are
+//   (Re w: E0 E1 | Im w: E0 E1) x g re/im x 32,
+// E0 = w_hi g_hi and E1 = 2^11 (w_hi g_lo + w_lo g_hi).  Per tile the result is
+// rescaled and added to FP32 registers, once per CTA along the diagonals.
+// Tiles whose power spans more than 2^10 (largest sample over the weakest
+// run of 32's largest) or holds non-finite samples sum in FP32.
+//
+// What bounds it: issue (~1150 instructions per warp and tile: loads, phase,
+// splits, the way back), with the tensor core working on the tile before and
+// two CTAs per SM (tensor memory).  With the backward chains' shorter phase
+// gradient, loss and gradients of 20 x 4 steps of 63 taps on 16 x 65536 samples
+// took 3167 us with FP32 sums of 8 taps x 8 samples per thread (of which these
+// 1540), 2122 us so.
 struct TapGrad {
     const float2* x0;    // batch x N: the input of layer 0
     const float2* act;   // kept y of all layers, `stride` apart
@@ -487,59 +474,260 @@ struct TapGrad {
     float2* gh;          // T per layer, from layer `first` on
     float span_scale;
     int first, steps, T, N;
+    int tiles, chunk;    // tiles in all (tiles per realization x batch), and per CTA
 };
-__global__ void __launch_bounds__(FIR_GRAD_THREADS) fir_grad_taps_kernel(const TapGrad p) {
-    __shared__ float2 xs[FIR_GRAD_XS];
-    __shared__ float2 gs[FIR_GRAD_TILE * 9 / 8];
-    const int b = blockIdx.y, N = p.N, T = p.T;
-    const int n0 = blockIdx.x * FIR_GRAD_TILE;
-    const int c = (T - 1) / 2;
-    const int Tp = (T + 7) & ~7;
+namespace tapgrad {
+constexpr int TILE = 2048, W = 32, M = 128, THREADS = 256;
+constexpr int WIN = TILE - W + M;                    // window elements: 63 x 32 + 128
+constexpr int XK = (WIN + THREADS - 1) / THREADS, GK = TILE / THREADS;
+constexpr uint32_t XP = 4608, GP = 4096;             // bytes between the words of w, of g_y (multiples of 512)
+constexpr int RP = W + 1;                            // pitch of the matrix summed along its diagonals
+constexpr uint32_t BUF = 4 * XP + 4 * GP;            // one tile's words; two tiles
+constexpr size_t SMEM = 2 * (size_t)BUF + 1024;
+constexpr uint32_t D_COLS = 256;
+static_assert(2 * WIN <= XP && 2 * TILE <= GP && XP % 512 == 0 && GP % 512 == 0, "words");
+static_assert(BUF % 512 == 0 && sizeof(float2) * M * RP <= BUF && sizeof(float2) * (2 * TILE + M) <= BUF, "reuse");
+// kind::f16, FP32 accumulator, FP16 operands, both MN-major
+__host__ __device__ constexpr uint32_t idesc(int n) {
+    return (1u << 4) | (1u << 15) | (1u << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// One scaled sample as {re hi, im hi, re lo, im lo} at element e, words `pitch` apart.
+__device__ __forceinline__ void store(unsigned char* p, uint32_t pitch, int e, float2 v, float sc) {
+    const float re = v.x * sc, im = v.y * sc;
+    const float rf = (re + 6144.f) - 6144.f, jf = (im + 6144.f) - 6144.f;  // multiples of 2^-11
+    const uint32_t o = 2u * (uint32_t)e;
+    p += o ^ ((o >> 3) & 0x30u);
+    *reinterpret_cast<__half*>(p) = __float2half_rn(rf);
+    *reinterpret_cast<__half*>(p + pitch) = __float2half_rn(jf);
+    *reinterpret_cast<__half*>(p + 2 * pitch) = __float2half_rn((re - rf) * 2048.f);
+    *reinterpret_cast<__half*>(p + 3 * pitch) = __float2half_rn((im - jf) * 2048.f);
+}
+// One tile in FP32 on plain buffers: the taps of this CTA's 128 window offsets.
+__device__ __noinline__ void tile_fp32(float2* buf, const float2* x, const float2* gy, const float* xi, float2* gh,
+                                       float scale, int n0, int off, int T, int N) {
+    float2 *w = buf, *g = buf + TILE + M;
+    const int c = (T - 1) / 2, lane = threadIdx.x & 31;
+    __syncthreads();
+    for (int i = threadIdx.x; i < TILE + M; i += THREADS) {
+        const float2 v = x[wrap_index(n0 - c + off + i, N)];
+        w[i] = xi ? cmul(v, phase_rotation(*xi * cnorm(v))) : v;
+    }
+    for (int i = threadIdx.x; i < TILE; i += THREADS) g[i] = n0 + i < N ? gy[n0 + i] : make_float2(0.f, 0.f);
+    __syncthreads();
+    for (int t = threadIdx.x >> 5; t < M && off + t < T; t += THREADS / 32) {
+        float2 acc = make_float2(0.f, 0.f);
+        for (int i = lane; i < TILE; i += 32) acc = cadd(acc, cmulc(g[i], w[i + t]));
+        acc.x = warp_sum(acc.x) * scale;
+        acc.y = warp_sum(acc.y) * scale;
+        if (lane == 0) {
+            atomicAdd(&gh[off + t].x, acc.x);
+            atomicAdd(&gh[off + t].y, acc.y);
+        }
+    }
+    __syncthreads();
+}
+}  // namespace tapgrad
+
+__global__ void __launch_bounds__(tapgrad::THREADS, 2) tap_grad_kernel(const TapGrad p) {
+    using namespace tapgrad;
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ __align__(8) unsigned long long done;
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int abort_flag;
+    __shared__ unsigned s_max[2][2], s_min[2][2];  // of w, g_y; by the tile's parity
+    unsigned char* xs = sm + ((1024u - (tcg::smem_addr(sm) & 1023u)) & 1023u);
+    const int N = p.N, T = p.T, off = M * blockIdx.y, c = (T - 1) / 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = p.first + blockIdx.z;
     const float2* x = k ? p.act + (size_t)(k - 1) * p.stride : p.x0;
+    const float* xi = k ? p.xi + (k - 1) : nullptr;
     const float2* gy = p.gy + (size_t)blockIdx.z * p.stride;
     float2* gh = p.gh + (size_t)blockIdx.z * T;
     const float scale = k % p.steps == 0 ? p.span_scale : 1.0f;
-    fir_load_window<FIR_GRAD_THREADS, FIR_GRAD_TILE, 8>(xs, x + (size_t)b * N, n0, c, FIR_GRAD_TILE + Tp, N,
-                                                        k ? p.xi + (k - 1) : nullptr);
-    {
-        constexpr int K = FIR_GRAD_TILE / FIR_GRAD_THREADS;
-        float2 v[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int i = threadIdx.x + k * FIR_GRAD_THREADS;
-            v[k] = (n0 + i < N) ? gy[(size_t)b * N + n0 + i] : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int k = 0; k < K; ++k) gs[fir_pad<8>(threadIdx.x + k * FIR_GRAD_THREADS)] = v[k];
+    const int per_row = (N + TILE - 1) / TILE;
+    const int q0 = blockIdx.x * p.chunk, q1 = min(q0 + p.chunk, p.tiles);
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < 2; ++i)
+            for (int j = 0; j < 2; ++j) {
+                s_max[i][j] = 0u;
+                s_min[i][j] = 0xFFFFFFFFu;
+            }
+        tcg::mbar_init(&done, 1);
+        tcg::fence_mbar_init();
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int t0 = warp * 8; t0 < Tp; t0 += 64) {
-        float2 acc[8];
+    if (warp == 0) tcg::tmem_alloc(&tmem_base, D_COLS);
+    float2 xr[XK], gr[GK];
+    auto load = [&](int q) {
+        const int b = q / per_row, n0 = (q - b * per_row) * TILE, w0 = n0 - c + off;
+        const float2* xb = x + (size_t)b * N;
+        const float2* gb = gy + (size_t)b * N;
+        if (w0 >= 0 && w0 + WIN <= N && n0 + TILE <= N) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = make_float2(0.f, 0.f);
-        for (int q = 0; q < FIR_GRAD_TILE; q += 256) {
-            const int nl = q + 8 * lane;  // first local sample of this lane
-            float2 g[8], w[16];
-            const int gb = (nl >> 3) * 9, xb = ((nl + t0) >> 3) * 9;
+            for (int u = 0; u < XK; ++u) {
+                const int e = threadIdx.x + THREADS * u;
+                xr[u] = e < WIN ? xb[w0 + e] : make_float2(0.f, 0.f);
+            }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) g[i] = gs[gb + i];
+            for (int u = 0; u < GK; ++u) gr[u] = gb[n0 + threadIdx.x + THREADS * u];
+        } else {
 #pragma unroll
-            for (int k = 0; k < 15; ++k) w[k] = xs[xb + k + (k >> 3)];
+            for (int u = 0; u < XK; ++u) {
+                const int e = threadIdx.x + THREADS * u;
+                xr[u] = e < WIN ? xb[wrap_index(w0 + e, N)] : make_float2(0.f, 0.f);
+            }
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[j] = cadd(acc[j], cmulc(g[i], w[i + j]));
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float sx = warp_sum(acc[j].x) * scale, sy = warp_sum(acc[j].y) * scale;
-            if (lane == 0 && t0 + j < T) {
-                atomicAdd(&gh[t0 + j].x, sx);
-                atomicAdd(&gh[t0 + j].y, sy);
+            for (int u = 0; u < GK; ++u) {
+                const int n = n0 + threadIdx.x + THREADS * u;
+                gr[u] = n < N ? gb[n] : make_float2(0.f, 0.f);
             }
         }
+    };
+    load(q0);
+    tcg::fence_before_sync();
+    __syncthreads();
+    tcg::fence_after_sync();
+    const uint32_t tmem = tmem_base;
+    float2 acc[W / 2];
+#pragma unroll
+    for (int r = 0; r < W / 2; ++r) acc[r] = make_float2(0.f, 0.f);
+    bool ok = true, pending = false;  // pending: the last tile's product
+    uint32_t parity = 0;
+    float back = 1.f;                 // its scale
+    // a tile is split while the tensor core is on the one before
+    for (int q = q0; q <= q1; ++q) {
+        const int z = (q - q0) & 1;
+        unsigned char* buf = xs + z * BUF;
+        float sc[2], scale_back = 1.f;
+        bool wide = false;
+        if (q < q1) {
+            if (xi) {
+                const float g = *xi;
+                float mx = 0.f;
+#pragma unroll
+                for (int u = 0; u < XK; ++u) mx = fmaxf(mx, cnorm(xr[u]));
+                if (fabsf(g) * mx <= kPhaseSmall) {
+#pragma unroll
+                    for (int u = 0; u < XK; ++u) xr[u] = cmul(xr[u], phase_rotation_small(g * cnorm(xr[u])));
+                } else {
+#pragma unroll
+                    for (int u = 0; u < XK; ++u) xr[u] = cmul(xr[u], phase_rotation(g * cnorm(xr[u])));
+                }
+            }
+            // a warp's 32 samples are one run; non-negative floats order as integers, NaN above infinity
+            unsigned mx[2] = {0u, 0u}, mn[2] = {0xFFFFFFFFu, 0xFFFFFFFFu};
+#pragma unroll
+            for (int u = 0; u < XK; ++u) {
+                const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(cnorm(xr[u])) & 0x7FFFFFFFu);
+                mx[0] = max(mx[0], m);
+                if (m) mn[0] = min(mn[0], m);
+            }
+#pragma unroll
+            for (int u = 0; u < GK; ++u) {
+                const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(cnorm(gr[u])) & 0x7FFFFFFFu);
+                mx[1] = max(mx[1], m);
+                if (m) mn[1] = min(mn[1], m);
+            }
+            if (lane < 2) {
+                atomicMax(&s_max[z][lane], lane ? mx[1] : mx[0]);
+                atomicMin(&s_min[z][lane], lane ? mn[1] : mn[0]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const unsigned m = s_max[z][i];
+                const float pmax = __uint_as_float(m), pmin = __uint_as_float(s_min[z][i]);
+                wide = wide || !(pmax <= 1e30f) || (m && (!(pmax > 1e-36f) || pmax > 1024.f * pmin));
+                const int e = firtc::split_exponent(m);
+                sc[i] = firtc::pow2(-e);
+                scale_back *= firtc::pow2(e);
+            }
+            if (wide) {
+                const int b = q / per_row;
+                tile_fp32(reinterpret_cast<float2*>(buf), x + (size_t)b * N, gy + (size_t)b * N, xi, gh, scale,
+                          (q - b * per_row) * TILE, off, T, N);
+            } else {
+#pragma unroll
+                for (int u = 0; u < XK; ++u) {
+                    const int e = threadIdx.x + THREADS * u;
+                    if (e < WIN) store(buf, XP, e, xr[u], sc[0]);
+                }
+#pragma unroll
+                for (int u = 0; u < GK; ++u) store(buf + 4 * XP, GP, threadIdx.x + THREADS * u, gr[u], sc[1]);
+            }
+            if (q + 1 < q1) load(q + 1);
+        }
+        if (pending) {
+            ok = tcg::mbar_wait(&done, parity, &abort_flag);
+            parity ^= 1;
+            tcg::fence_after_sync();
+            const uint32_t t = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 16 * (uint32_t)(warp >> 2);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {  // (w re/im, g re/im)
+                const uint32_t col = t + 128 * (i >> 1) + 32 * (i & 1);
+                uint32_t e0[16], e1[16];
+                tcg::ld_x16_async(col, e0);
+                tcg::ld_x16_async(col + 64, e1);
+                tcg::wait_ld(e0);
+                tcg::wait_ld(e1);
+                const float f = i == 2 ? -back : back;
+#pragma unroll
+                for (int r = 0; r < W / 2; ++r) {
+                    const float v = fmaf(__uint_as_float(e1[r]), 0x1p-11f, __uint_as_float(e0[r]));
+                    if (i == 0 || i == 3)
+                        acc[r].x = fmaf(v, f, acc[r].x);
+                    else
+                        acc[r].y = fmaf(v, f, acc[r].y);
+                }
+            }
+        }
+        tcg::fence_async_smem();
+        tcg::fence_before_sync();
+        if (__syncthreads_or(!ok)) {
+            ok = false;
+            break;
+        }
+        pending = q < q1 && !wide;
+        back = scale_back;
+        if (threadIdx.x < 2) {  // for the tile after the next; read before the barrier above
+            s_max[z][threadIdx.x] = 0u;
+            s_min[z][threadIdx.x] = 0xFFFFFFFFu;
+        }
+        if (pending && warp == 0) {
+            tcg::fence_after_sync();
+            uint64_t a = tcg::smem_desc_sw64_mn(tcg::smem_addr(buf), 2 * W);
+            uint64_t g = tcg::smem_desc_sw64_mn(tcg::smem_addr(buf + 4 * XP), GP);
+            for (int s = 0; s < TILE / W / 16; ++s) {
+                tcg::mma_f16_warp(tmem, a, g, idesc(128), s != 0);
+                tcg::mma_f16_warp(tmem + 128, a + XP / 16, g, idesc(128), s != 0);
+                tcg::mma_f16_warp(tmem + 64, a + 2 * (XP / 16), g, idesc(64), true);
+                tcg::mma_f16_warp(tmem + 192, a + 3 * (XP / 16), g, idesc(64), true);
+                a += 1024 / 16;  // 16 blocks of 64 bytes
+                g += 1024 / 16;
+            }
+            tcg::mma_commit_warp(&done);
+        }
+    }
+    if (!ok && warp == 0) {  // a wait ran out: the MMAs in flight end (bounded) before the CTA leaves
+        tcg::mma_commit_warp(&done);
+        for (int i = 0; i < 2; ++i) tcg::mbar_wait_warp(&done, i, nullptr);
+    }
+    tcg::fence_before_sync();
+    __syncthreads();
+    tcg::fence_after_sync();
+    if (warp == 0) tcg::tmem_free(tmem, D_COLS);
+    float2* mat = reinterpret_cast<float2*>(xs);
+#pragma unroll
+    for (int r = 0; r < W / 2; ++r) mat[(32 * (warp & 3) + lane) * RP + (W / 2) * (warp >> 2) + r] = acc[r];
+    __syncthreads();
+    const int d = (int)threadIdx.x - (W - 1), t = off + d;  // m = d + r
+    if (d < M && t >= 0 && t < T) {
+        float2 s = make_float2(0.f, 0.f);
+        for (int r = max(0, -d); r < min(W, M - d); ++r) s = cadd(s, mat[(d + r) * RP + r]);
+        if (!ok) s.x = s.y = __int_as_float(0x7fc00000);
+        atomicAdd(&gh[t].x, s.x * scale);
+        atomicAdd(&gh[t].y, s.y * scale);
     }
 }
 
@@ -705,21 +893,34 @@ static cudaError_t ldbp_chains(LdbpModel& M, const float2* in, bool keep, float2
     return e;
 }
 
+static cudaError_t launch_tap_grad(const LdbpModel& M, fg::TapGrad& p, int layers) {
+    using namespace fg::tapgrad;
+    const size_t tiles = (size_t)((M.samples + TILE - 1) / TILE) * M.batch;
+    if (tiles > 0x7FFFFFFFu) return cudaErrorInvalidValue;
+    const unsigned blocks = (p.T + W - 1 + fg::tapgrad::M - 1) / fg::tapgrad::M;  // window offsets 0 .. T + 30
+    p.tiles = (int)tiles;
+    // tiles per CTA: the sum along the diagonals once per 16 tiles, fewer where
+    // that leaves an SM without its two CTAs
+    const size_t slots = 2 * (size_t)fg::sm_count();
+    p.chunk = (int)std::min<size_t>(16, (tiles * layers * blocks + slots - 1) / slots);
+    cudaError_t e = cudaFuncSetAttribute(fg::tap_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    if (e != cudaSuccess) return e;
+    fg::tap_grad_kernel<<<dim3((p.tiles + p.chunk - 1) / p.chunk, blocks, layers), THREADS, SMEM, M.ctx->stream>>>(p);
+    count_launch();
+    return cudaGetLastError();
+}
+
 // Gradients of everything from gy, the gradient of the matched filter's output
 // (in M.work): the adjoint chains, then the tap gradients from what they and
 // the forward pass kept.
 static cudaError_t ldbp_backward(LdbpModel& M, const float2* in) {
     const size_t n = M.field_n();
     const int L = M.spans * M.steps;
-    cudaStream_t s = M.ctx->stream;
-    const dim3 tiles((M.samples + fg::FIR_GRAD_TILE - 1) / fg::FIR_GRAD_TILE, M.batch);
     float2* bufs[2] = {M.work, M.work + n};
-    fg::TapGrad t{in, M.acts, M.work, n, M.xi(0), M.ghmf(), 1.0f, L, M.steps, M.mf_taps, M.samples};
+    fg::TapGrad t{in, M.acts, M.work, n, M.xi(0), M.ghmf(), 1.0f, L, M.steps, M.mf_taps, M.samples, 0, 0};
     cudaError_t e = ldbp_matrices(M, 1);
     if (e != cudaSuccess) return e;
-    fg::fir_grad_taps_kernel<<<tiles, fg::FIR_GRAD_THREADS, 0, s>>>(t);
-    count_launch();
-    e = cudaGetLastError();
+    e = launch_tap_grad(M, t, 1);
     fg::ChainArgs m{};
     m.layers = 1;
     m.T = M.mf_taps;
@@ -751,10 +952,8 @@ static cudaError_t ldbp_backward(LdbpModel& M, const float2* in) {
     }
     // gridDim.z is at most 65535
     for (int k = 0; k < L && e == cudaSuccess; k += 32768) {
-        fg::TapGrad a{in, M.acts, M.acts + (size_t)(L + k) * n, n, M.xi(0), M.gh(k), M.span_scale, k, M.steps, M.taps, M.samples};
-        fg::fir_grad_taps_kernel<<<dim3(tiles.x, tiles.y, std::min(L - k, 32768)), fg::FIR_GRAD_THREADS, 0, s>>>(a);
-        count_launch();
-        e = cudaGetLastError();
+        fg::TapGrad a{in, M.acts, M.acts + (size_t)(L + k) * n, n, M.xi(0), M.gh(k), M.span_scale, k, M.steps, M.taps, M.samples, 0, 0};
+        e = launch_tap_grad(M, a, std::min(L - k, 32768));
     }
     return e;
 }

@@ -84,6 +84,14 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 __device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61);
 }
+// An MN-major operand in the 64-byte swizzled layout: rows of 32 elements (64
+// bytes), one per k, 8-row groups 512 bytes apart, 32-element groups along M or
+// N `lbo` bytes apart; mode 4 (16-byte chunks XORed with address bits 7 and 8,
+// again of the absolute address).
+__device__ __forceinline__ uint64_t smem_desc_sw64_mn(uint32_t addr, uint32_t lbo) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) |
+           (1ull << 46) | (4ull << 61);
+}
 // D (tensor memory) = A B (+ D when `accumulate`), kind::f16, one CTA.
 __device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
     asm volatile(
