@@ -122,6 +122,39 @@ focss_status ensure_red(Ctx* ctx, size_t doubles) {
     return FOCSS_OK;
 }
 
+void* result_buffer(Ctx* ctx, size_t bytes) {
+    if (bytes <= ctx->result_cap) return ctx->h_result;
+    cudaStreamSynchronize(ctx->stream);
+    if (ctx->h_result) cudaFreeHost(ctx->h_result);
+    ctx->h_result = nullptr;
+    ctx->result_cap = 0;
+    bytes = std::max<size_t>(bytes, 4096);
+    if (cudaMallocHost(&ctx->h_result, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->h_result = nullptr;
+        return nullptr;
+    }
+    ctx->result_cap = bytes;
+    return ctx->h_result;
+}
+
+unsigned* tickets(Ctx* ctx, size_t n) {
+    if (n <= ctx->ticket_cap) return ctx->d_ticket;
+    cudaFree(ctx->d_ticket);
+    ctx->d_ticket = nullptr;
+    ctx->ticket_cap = 0;
+    n = std::max<size_t>(n, 64);
+    if (cudaMalloc(&ctx->d_ticket, sizeof(unsigned) * n) != cudaSuccess ||
+        cudaMemsetAsync(ctx->d_ticket, 0, sizeof(unsigned) * n, ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(ctx->d_ticket);
+        ctx->d_ticket = nullptr;
+        return nullptr;
+    }
+    ctx->ticket_cap = n;
+    return ctx->d_ticket;
+}
+
 int sm_count() {
     static int cached[64] = {};
     int dev = 0;
@@ -265,7 +298,9 @@ FOCSS_API focss_status focss_ctx_destroy(focss_ctx* c) {
     cudaFree(c->d_state);
     cudaFree(c->d_counters);
     cudaFree(c->d_red);
+    cudaFree(c->d_ticket);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
+    if (c->h_result) cudaFreeHost(c->h_result);
     if (c->stream) cudaStreamDestroy(c->stream);
     // fields still alive keep their blocks; the pool goes when they are freed
     if (c->pool) cudaMemPoolDestroy(c->pool);

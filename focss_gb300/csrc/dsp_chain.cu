@@ -10,6 +10,8 @@
 // layout, and applied by the row pass (ROW_TABLE) between the column passes.
 // Decisions and metric sums run in FP64 (O(N), off the split-step hot loop)
 // so that symbol decisions reproduce the reference's FP64 comparisons.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -232,39 +234,91 @@ __global__ void wdm_mux_kernel(const float2* __restrict__ ch, int n_ch, int mode
     }
 }
 
+// Sum of |A|^2 in FP64 over the samples first, first + step, ... of a realization.
+__device__ __forceinline__ double power_partial(const float2* __restrict__ d, size_t per, size_t first, size_t step) {
+    double a = 0.0, b = 0.0;
+    for (size_t i = first; i < per; i += step) {
+        const float2 z = d[i];
+        a = fma((double)z.x, (double)z.x, a);
+        b = fma((double)z.y, (double)z.y, b);
+    }
+    return a + b;
+}
+
 // Per-realization FP64 power sum over all modes and samples (for decision scales).
 __global__ void power_sum_kernel(const float2* __restrict__ d, size_t per, double* __restrict__ out) {
     const int b = blockIdx.y;
-    const float2* base = d + (size_t)b * per;
-    double acc = 0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < per; i += (size_t)gridDim.x * blockDim.x) {
-        const double x = base[i].x, y = base[i].y;
-        acc += x * x + y * y;
-    }
+    double acc = power_partial(d + (size_t)b * per, per, blockIdx.x * (size_t)blockDim.x + threadIdx.x,
+                               (size_t)gridDim.x * blockDim.x);
     __shared__ double sd[32];
     acc = block_sum_d(acc, sd);
     if (threadIdx.x == 0) atomicAdd(out + b, acc);
 }
 
+// Short realizations: the decision kernels below run as one cluster of
+// kCluster CTAs per realization and form its power sum themselves (partial
+// sums through distributed shared memory), so a call is one launch instead of
+// a memset, a power sum and the decision.  The sum, and the square root and
+// division after it, are a serial FP64 chain of a few microseconds, done by one
+// thread per CTA (formed by every thread, they took longer than the samples).
+// Four calls on 4000 samples (decision, codes, errors, Q): 139 -> 94 us with
+// launches and synchronization.  Above kClusterSamples a cluster's share of
+// the FP64 sums takes longer than a second launch over more CTAs.
+constexpr int kCluster = 8, kClusterThreads = 512;
+constexpr size_t kClusterSamples = 16384;
+
+// sum over the realization, valid in thread 0.  CL: by its cluster, whose CTAs
+// end with cluster_done (the partial sums are read remotely), else from psum.
+template <bool CL>
+__device__ __forceinline__ double realization_power(const float2* __restrict__ d, size_t per, const double* psum) {
+    if constexpr (CL) {
+        namespace cg = cooperative_groups;
+        __shared__ double sd[32], part;
+        const cg::cluster_group cluster = cg::this_cluster();
+        const double v = block_sum_d(power_partial(d, per, blockIdx.x * (size_t)blockDim.x + threadIdx.x,
+                                                   (size_t)gridDim.x * blockDim.x), sd);
+        if (threadIdx.x == 0) part = v;
+        cluster.sync();
+        double total = 0.0;
+        if (threadIdx.x == 0)
+            for (int r = 0; r < kCluster; ++r) total += *cluster.map_shared_rank(&part, r);
+        return total;
+    } else {
+        return *psum;
+    }
+}
+template <bool CL>
+__device__ __forceinline__ void cluster_done() {
+    if constexpr (CL) cooperative_groups::this_cluster().sync();
+}
+
 // hard_decision_16qam (modulation.cpp:112-120): power = avg/modes,
 // out = sqrt(power) * gray[demod(in / sqrt(power))].
 // Grid (samples, realization): the realization's scale is formed once per thread.
-__global__ void hard_decision_kernel(const float2* __restrict__ in, float2* __restrict__ out, int modes, int samples,
-                                     size_t per, const double* __restrict__ psum) {
+template <bool CL>
+__global__ void hard_decision_kernel(const float2* in, float2* out, int modes, int samples, size_t per,
+                                     const double* __restrict__ psum) {
     const double s10 = 1.0 / sqrt(10.0);
     const int b = blockIdx.y;
-    const double power = psum[b] / samples / modes;
-    const double sp = sqrt(power);
     in += (size_t)b * per;
     out += (size_t)b * per;
     // the 16 outputs, formed once per CTA (a per-sample lookup with divergent
     // codes would serialize in the constant cache)
     __shared__ float2 s_out[16];
+    __shared__ double s_sp;
+    __shared__ float s_inv;
+    const double total = realization_power<CL>(in, per, psum + b);
+    if (threadIdx.x == 0) {
+        s_sp = sqrt(total / samples / modes);
+        s_inv = (float)(1.0 / s_sp);
+    }
+    __syncthreads();
+    const double sp = s_sp;
     if (threadIdx.x < 16)
         s_out[threadIdx.x] = make_float2((float)(sp * (c_gray_re[threadIdx.x] * s10)),
                                          (float)(sp * (c_gray_im[threadIdx.x] * s10)));
     __syncthreads();
-    const float inv = (float)(1.0 / sp);
+    const float inv = s_inv;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < per; i += (size_t)gridDim.x * blockDim.x) {
         const float2 z = in[i];
         bool near;
@@ -272,6 +326,7 @@ __global__ void hard_decision_kernel(const float2* __restrict__ in, float2* __re
         if (near) c = demod16_div(z.x, z.y, sp);
         out[i] = s_out[c];
     }
+    cluster_done<CL>();
 }
 
 // The FP64 forms of one soft decision (modulation.cpp:122-146) and one
@@ -407,12 +462,17 @@ __global__ void certainty_decision_kernel(const float2* __restrict__ in, float2*
 }
 
 // hd_sequence_16qam (modulation.cpp:148-156): scale = sqrt(modes / average_power).
+template <bool CL>
 __global__ void hd_codes_kernel(const float2* __restrict__ in, int32_t* __restrict__ codes, int modes, int samples,
                                 size_t per, const double* __restrict__ psum) {
     const int b = blockIdx.y;
-    const double sc = sqrt(modes / (psum[b] / samples));
     in += (size_t)b * per;
     codes += (size_t)b * per;
+    __shared__ double s_sc;
+    const double total = realization_power<CL>(in, per, psum + b);
+    if (threadIdx.x == 0) s_sc = sqrt(modes / (total / samples));
+    __syncthreads();
+    const double sc = s_sc;
     const float sc32 = (float)sc;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < per; i += (size_t)gridDim.x * blockDim.x) {
         const float2 z = in[i];
@@ -421,16 +481,23 @@ __global__ void hd_codes_kernel(const float2* __restrict__ in, int32_t* __restri
         if (near) c = demod16_mul(z.x, z.y, sc);
         codes[i] = (int32_t)c;
     }
+    cluster_done<CL>();
 }
 
 // Decision errors over samples [cut, samples - cut) (modulation.cpp:158-223);
 // both sequences scaled by sqrt(modes / average_power(tx)).
+// counts is zeroed by the caller, or (CL) written.
+template <bool CL>
 __global__ void error_count_kernel(const float2* __restrict__ tx, const float2* __restrict__ rx, int modes,
                                    int samples, int cut, const double* __restrict__ psum_tx,
                                    unsigned long long* __restrict__ counts) {
     const int b = blockIdx.y;
     const size_t per = (size_t)modes * samples;
-    const double sc = sqrt(modes / (psum_tx[b] / samples));
+    __shared__ double s_sc;
+    const double power = realization_power<CL>(tx + (size_t)b * per, per, psum_tx + b);
+    if (threadIdx.x == 0) s_sc = sqrt(modes / (power / samples));
+    __syncthreads();
+    const double sc = s_sc;
     const float sc32 = (float)sc;
     const int span = samples - 2 * cut;
     unsigned long long be = 0, se = 0;
@@ -455,79 +522,182 @@ __global__ void error_count_kernel(const float2* __restrict__ tx, const float2* 
         be += __shfl_xor_sync(0xffffffffu, be, o);
         se += __shfl_xor_sync(0xffffffffu, se, o);
     }
-    if ((threadIdx.x & 31) == 0) {
+    if constexpr (CL) {
+        namespace cg = cooperative_groups;
+        __shared__ unsigned long long s_n[2];
+        const cg::cluster_group cluster = cg::this_cluster();
+        if (threadIdx.x < 2) s_n[threadIdx.x] = 0ull;
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&s_n[0], be);
+            atomicAdd(&s_n[1], se);
+        }
+        cluster.sync();
+        if (blockIdx.x == 0 && threadIdx.x < 2) {
+            unsigned long long n = 0ull;
+            for (int r = 0; r < kCluster; ++r) n += *cluster.map_shared_rank(&s_n[threadIdx.x], r);
+            counts[2 * b + threadIdx.x] = n;
+        }
+        cluster_done<CL>();
+    } else if ((threadIdx.x & 31) == 0) {
         atomicAdd(counts + 2 * b, be);
         atomicAdd(counts + 2 * b + 1, se);
     }
 }
 
-// FP64 pair sums over samples [lo, hi) of every mode:
-// out[8b + 0] = sum |t|^2, 1 = sum |r|^2, 2 = sum |t - r|^2, 3/4 = sum conj(r) t (re/im),
-// 5/6 = sum conj(t) r (re/im).
-__global__ void pair_sums_kernel(const float2* __restrict__ t, const float2* __restrict__ r, int modes, int samples,
-                                 int lo, int hi, double* __restrict__ out) {
-    const int b = blockIdx.y;
-    const size_t per = (size_t)modes * samples;
-    const int span = hi - lo;
-    double a[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (span > 0) {
-        const size_t total = (size_t)modes * span;
-        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-            const int m = (int)(i / span);
-            const int s = lo + (int)(i % span);
-            const size_t k = (size_t)b * per + (size_t)m * samples + s;
-            const double tr = t[k].x, ti = t[k].y, rr = r[k].x, ri = r[k].y;
-            const double dr = tr - rr, di = ti - ri;
-            a[0] += tr * tr + ti * ti;
-            a[1] += rr * rr + ri * ri;
-            a[2] += dr * dr + di * di;
-            a[3] += rr * tr + ri * ti;  // conj(r) t
-            a[4] += rr * ti - ri * tr;
-            a[5] += tr * rr + ti * ri;  // conj(t) r
-            a[6] += tr * ri - ti * rr;
-        }
-    }
-    __shared__ double sd[32];
-    for (int q = 0; q < 7; ++q) {
-        const double v = block_sum_d(a[q], sd);
-        if (threadIdx.x == 0) atomicAdd(out + 8 * b + q, v);
-        __syncthreads();
-    }
-}
+// FP64 pair sums over samples [lo, hi) of every mode, and what becomes of them:
+//   PAIR_Q2      out[2b] = sum |t|^2, [1] = sum |t - r|^2
+//   PAIR_SCALAR  out[3b] = sum |t|^2, [1], [2] = sum conj(t) r (re, im)
+//   PAIR_PHASE   out[b] = the phase-shift equalizer's angle, from sum conj(t) r
+// CTAs leave their partial sums in `part` and the realization's last one adds
+// them up (ticket, which it sets back to zero), so one launch does a call and
+// the result can go straight to host memory.  FP64 (~2 operations per cycle and
+// SM) bounds the sums: only the ones asked for are formed, 4 conversions and 4
+// or 6 fused multiply-adds per sample instead of 18 operations.  Estimating and
+// applying the angle of 12 x 32768 samples: 125 -> 85 us, of which the sums
+// and the angle took 65.
+enum { PAIR_Q2 = 0, PAIR_SCALAR = 1, PAIR_PHASE = 2 };
+__host__ __device__ constexpr int pair_sums_of(int what) { return what == PAIR_SCALAR ? 3 : 2; }
+constexpr int kPairBlocks = 64;  // CTAs per realization, at most
 
-// PhaseShiftEqualizer::estimate argmax over i = 0..steps-1 (first maximum
-// wins): q2 is monotone in Re(e^{i angle} sum conj(t) r).
-__global__ void pse_argmax_kernel(const double* __restrict__ sums, int steps, double* __restrict__ angle) {
-    const int b = blockIdx.x;
-    const double cr = sums[8 * b + 5], ci = sums[8 * b + 6];
+// PhaseShiftEqualizer::estimate argmax over i = 0..steps-1 of
+// Re(e^{i 2 pi i / steps} (cr + i ci)) (q2 is monotone in it), the first maximum
+// wins.  Around the peak at -arg(cr + i ci) neighbours fall off by at least
+// ~(2 pi / steps)^2 / 2 of it, far above rounding up to 65536 steps, so the
+// five steps around it decide; otherwise (or without a usable argument) all
+// steps are tried.  Called by a whole CTA, result in thread 0.
+__device__ int phase_argmax(double cr, double ci, int steps) {
     const double two_pi = 2 * 3.14159265358979323846264338;
+    const double mag = fmax(fabs(cr), fabs(ci));
+    const bool near = steps >= 8 && steps <= 65536 && mag > 1e-290 && mag < 1e290 && !isnan(cr) && !isnan(ci);
+    int first = 0, count = steps;
+    if (near) {
+        first = __double2int_rn(-atan2(ci, cr) / two_pi * steps) - 2;
+        count = 5;
+    }
     double best = -1e308;
     int bi = 0;
-    for (int i = threadIdx.x; i < steps; i += blockDim.x) {
+    for (int k = threadIdx.x; k < count; k += blockDim.x) {
+        int i = first + k;
+        if (i < 0) i += steps;
+        if (i >= steps) i -= steps;
         const double ang = two_pi * (double)i / steps;
         const double v = cr * cos(ang) - ci * sin(ang);
-        if (v > best) {
+        if (v > best || (v == best && i < bi)) {
             best = v;
             bi = i;
         }
     }
-    __shared__ double sv[1024];
-    __shared__ int si[1024];
-    sv[threadIdx.x] = best;
-    si[threadIdx.x] = bi;
+    __shared__ double sv[32];
+    __shared__ int si[32];
+    for (int round = 0; round < 2; ++round) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, best, o);
+            const int i = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (v > best || (v == best && i < bi)) {
+                best = v;
+                bi = i;
+            }
+        }
+        if (round) break;
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (lane == 0) {
+            sv[warp] = best;
+            si[warp] = bi;
+        }
+        __syncthreads();
+        if (warp) break;
+        best = lane < (int)blockDim.x / 32 ? sv[lane] : -1e308;
+        bi = lane < (int)blockDim.x / 32 ? si[lane] : 0x7FFFFFFF;
+    }
+    return bi;
+}
+
+template <int WHAT>
+__global__ void __launch_bounds__(256) pair_sums_kernel(const float2* __restrict__ t, const float2* __restrict__ r, int modes,
+                                                       int samples, int lo, int hi, double* part, unsigned* ticket,
+                                                       int steps, double* out) {
+    constexpr int K = pair_sums_of(WHAT);
+    const int b = blockIdx.y;
+    const size_t per = (size_t)modes * samples;
+    const int span = hi - lo;
+    double a[3] = {0, 0, 0};
+    if (span > 0) {
+        t += (size_t)b * per;
+        r += (size_t)b * per;
+        const unsigned step = gridDim.x * blockDim.x;
+        for (int m = 0; m < modes; ++m)
+            for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)span; i += step) {
+                const size_t k = (size_t)m * samples + lo + i;
+                const float2 tf = t[k], rf = r[k];
+                const double tr = tf.x, ti = tf.y, rr = rf.x, ri = rf.y;
+                if (WHAT != PAIR_PHASE) {
+                    a[0] = fma(tr, tr, a[0]);
+                    a[0] = fma(ti, ti, a[0]);
+                }
+                if (WHAT == PAIR_Q2) {
+                    const double dr = tr - rr, di = ti - ri;
+                    a[1] = fma(dr, dr, a[1]);
+                    a[1] = fma(di, di, a[1]);
+                } else {  // conj(t) r
+                    constexpr int o = WHAT == PAIR_SCALAR ? 1 : 0;
+                    a[o] = fma(tr, rr, a[o]);
+                    a[o] = fma(ti, ri, a[o]);
+                    a[o + 1] = fma(tr, ri, a[o + 1]);
+                    a[o + 1] = fma(-ti, rr, a[o + 1]);
+                }
+            }
+    }
+    __shared__ double s_w[K][8], s_sum[K];
+    __shared__ bool s_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        const double v = warp_sum_d(a[q]);
+        if (lane == 0) s_w[q][warp] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < K) {
+        double v = 0;
+        for (int w = 0; w < 8; ++w) v += s_w[threadIdx.x][w];
+        part[((size_t)b * gridDim.x + blockIdx.x) * K + threadIdx.x] = v;
+        __threadfence();
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double bv = sv[0];
-        int bidx = si[0];
-        for (int k = 1; k < (int)blockDim.x; ++k)
-            if (sv[k] > bv || (sv[k] == bv && si[k] < bidx)) {
-                bv = sv[k];
-                bidx = si[k];
-            }
-        angle[b] = two_pi * (double)bidx / steps;
+        s_last = atomicAdd(ticket + b, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    if (threadIdx.x == 0) ticket[b] = 0u;
+    if (warp < K) {
+        double v = 0;
+        for (int x = lane; x < (int)gridDim.x; x += 32) v += __ldcg(part + ((size_t)b * gridDim.x + x) * K + warp);
+        v = warp_sum_d(v);
+        if (lane == 0) s_sum[warp] = v;
+    }
+    __syncthreads();
+    if (WHAT == PAIR_PHASE) {
+        const int i = phase_argmax(s_sum[0], s_sum[1], steps);
+        if (threadIdx.x == 0) out[b] = 2 * 3.14159265358979323846264338 * (double)i / steps;
+    } else if (threadIdx.x < K) {
+        out[(size_t)b * K + threadIdx.x] = s_sum[threadIdx.x];
     }
 }
 
+// Multiplies each realization by its factor, passed by value for small batches
+// (no copy to wait for).
+constexpr int kScalesByValue = 64;
+struct Scales {
+    float2 s[kScalesByValue];
+};
+__global__ void scale_some_kernel(float2* __restrict__ d, size_t per, const __grid_constant__ Scales s) {
+    const float2 f = s.s[blockIdx.y];
+    d += (size_t)blockIdx.y * per;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < per; i += (size_t)gridDim.x * blockDim.x)
+        d[i] = cmul(d[i], f);
+}
 __global__ void scale_each_kernel(float2* __restrict__ d, size_t per, size_t n, const float2* __restrict__ s) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         d[i] = cmul(d[i], s[i / per]);
@@ -594,19 +764,43 @@ focss_status apply_filter(Ctx* c, float2* d, int samples, int rows, const float2
     return spectral_apply(c, d, samples, rows, ROW_TABLE, H, (float)g, 0);
 }
 
-focss_status sums_for(Ctx* c, const Field* t, const Field* r, int lo, int hi, std::vector<double>& host) {
-    focss_status st = ensure_red(c, 8 * (size_t)t->batch);
+// Pair sums (or the angle) of every realization into host[pair_sums_of(what)
+// (or 1) per realization]; the kernel writes them to pinned memory itself.
+template <int WHAT>
+focss_status pair_sums(Ctx* c, const Field* t, const Field* r, int lo, int hi, int steps, const double** host) {
+    const int B = t->batch;
+    // 2 samples per thread before the CTAs of a realization meet, up to 64 CTAs
+    const int gx = std::max(1, std::min(kPairBlocks, (int)(((size_t)t->modes * std::max(hi - lo, 1) + 511) / 512)));
+    constexpr int K = pair_sums_of(WHAT);
+    const size_t results = sizeof(double) * B * K;
+    double* out = (double*)result_buffer(c, results);
+    unsigned* ticket = tickets(c, B);
+    if (!out || !ticket) return set_error(c, FOCSS_ERR_OOM, "pair sums scratch");
+    focss_status st = ensure_red(c, (size_t)K * gx * B);
     if (st != FOCSS_OK) return st;
-    cudaStream_t s = c->stream;
-    cudaError_t e = cudaMemsetAsync(c->d_red, 0, sizeof(double) * 8 * t->batch, s);
-    const int gx = std::max(1, std::min(64, (int)(((size_t)t->modes * std::max(hi - lo, 1) + 1023) / 1024)));
-    if (e == cudaSuccess) FG_LAUNCH(pair_sums_kernel<<<dim3(gx, t->batch), 256, 0, s>>>(t->d, r->d, t->modes, t->samples, lo, hi, c->d_red));
-    if (e == cudaSuccess) e = cudaGetLastError();
-    host.assign(8 * (size_t)t->batch, 0.0);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(host.data(), c->d_red, sizeof(double) * 8 * t->batch, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    FG_LAUNCH(pair_sums_kernel<WHAT><<<dim3(gx, B), 256, 0, c->stream>>>(t->d, r->d, t->modes, t->samples, lo, hi, c->d_red, ticket, steps, out));
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    *host = out;
     return cuda_check(c, e, "pair sums");
+}
+
+// Launch of a decision kernel's cluster form (kCluster CTAs per realization).
+template <class... P, class... A>
+cudaError_t launch_cluster(void (*k)(P...), int batch, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kCluster, batch);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kCluster;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    count_launch();
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 
 focss_status power_sums(Ctx* c, const Field* f, double* dst_device) {
@@ -803,11 +997,14 @@ FOCSS_API focss_status focss_wdm_mux(focss_ctx* c, const focss_field* ch, double
 FOCSS_API focss_status focss_hard_decision(focss_ctx* c, const focss_field* in, focss_field* out) {
     if (!c || !in || !out) return FOCSS_ERR_INVALID_ARG;
     focss_status st = fg::check_same(c, in, out);
+    const size_t per = (size_t)in->modes * in->samples;
+    if (st == FOCSS_OK && per <= fg::kClusterSamples)
+        return fg::cuda_check(c, fg::launch_cluster(fg::hard_decision_kernel<true>, in->batch, c->stream, in->d, out->d, in->modes,
+                                                    in->samples, per, nullptr), "hard_decision");
     if (st == FOCSS_OK) st = fg::ensure_red(c, (size_t)in->batch);
     if (st == FOCSS_OK) st = fg::power_sums(c, in, c->d_red);
     if (st != FOCSS_OK) return st;
-    const size_t per = (size_t)in->modes * in->samples;
-    FG_LAUNCH(fg::hard_decision_kernel<<<fg::grid_per_realization(per, in->batch), 256, 0, c->stream>>>(in->d, out->d, in->modes, in->samples, per, c->d_red));
+    FG_LAUNCH(fg::hard_decision_kernel<false><<<fg::grid_per_realization(per, in->batch), 256, 0, c->stream>>>(in->d, out->d, in->modes, in->samples, per, c->d_red));
     return fg::cuda_check(c, cudaGetLastError(), "hard_decision");
 }
 
@@ -870,15 +1067,23 @@ FOCSS_API focss_status focss_certainty_decision(focss_ctx* c, const focss_field*
 
 FOCSS_API focss_status focss_hd_codes(focss_ctx* c, const focss_field* in, int32_t* codes) {
     if (!c || !in || !codes) return FOCSS_ERR_INVALID_ARG;
+    const size_t per = (size_t)in->modes * in->samples, bytes = sizeof(int32_t) * in->n();
+    if (per <= fg::kClusterSamples && bytes <= fg::kResultCap) {  // written to pinned host memory by the kernel
+        int32_t* d = (int32_t*)fg::result_buffer(c, bytes);
+        if (!d) return fg::set_error(c, FOCSS_ERR_OOM, "hd_codes scratch");
+        cudaError_t e = fg::launch_cluster(fg::hd_codes_kernel<true>, in->batch, c->stream, in->d, d, in->modes, in->samples, per, nullptr);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        if (e == cudaSuccess) std::memcpy(codes, d, bytes);
+        return fg::cuda_check(c, e, "hd_codes");
+    }
     focss_status st = fg::ensure_red(c, (size_t)in->batch);
     if (st == FOCSS_OK) st = fg::power_sums(c, in, c->d_red);
     if (st != FOCSS_OK) return st;
-    int32_t* d = (int32_t*)fg::scratch_buffer(c, 1, sizeof(int32_t) * in->n());
+    int32_t* d = (int32_t*)fg::scratch_buffer(c, 1, bytes);
     if (!d) return fg::set_error(c, FOCSS_ERR_OOM, "hd_codes scratch");
-    const size_t per = (size_t)in->modes * in->samples;
-    FG_LAUNCH(fg::hd_codes_kernel<<<fg::grid_per_realization(per, in->batch), 256, 0, c->stream>>>(in->d, d, in->modes, in->samples, per, c->d_red));
+    FG_LAUNCH(fg::hd_codes_kernel<false><<<fg::grid_per_realization(per, in->batch), 256, 0, c->stream>>>(in->d, d, in->modes, in->samples, per, c->d_red));
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(codes, d, sizeof(int32_t) * in->n(), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(codes, d, bytes, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     return fg::cuda_check(c, e, "hd_codes");
 }
@@ -890,17 +1095,24 @@ FOCSS_API focss_status focss_error_counts(focss_ctx* c, const focss_field* tx, c
     if (st != FOCSS_OK) return st;
     cut = fg::clamp_cut(cut);
     const int B = tx->batch;
-    st = fg::ensure_red(c, 3 * (size_t)B);
-    if (st == FOCSS_OK) st = fg::power_sums(c, tx, c->d_red);
-    if (st != FOCSS_OK) return st;
-    unsigned long long* cnt = (unsigned long long*)(c->d_red + B);
+    const size_t per = (size_t)tx->modes * tx->samples, bytes = sizeof(unsigned long long) * 2 * B;
     cudaStream_t s = c->stream;
-    cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * 2 * B, s);
-    const int gx = std::max(1, std::min(64, (int)(((size_t)tx->modes * tx->samples + 1023) / 1024)));
-    if (e == cudaSuccess) FG_LAUNCH(fg::error_count_kernel<<<dim3(gx, B), 256, 0, s>>>(tx->d, rx->d, tx->modes, tx->samples, cut, c->d_red, cnt));
-    if (e == cudaSuccess) e = cudaGetLastError();
-    std::vector<unsigned long long> h(2 * (size_t)B);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), cnt, sizeof(unsigned long long) * 2 * B, cudaMemcpyDeviceToHost, s);
+    unsigned long long* h = (unsigned long long*)fg::result_buffer(c, bytes);
+    if (!h) return fg::set_error(c, FOCSS_ERR_OOM, "error_counts scratch");
+    cudaError_t e;
+    if (per <= fg::kClusterSamples) {
+        e = fg::launch_cluster(fg::error_count_kernel<true>, B, s, tx->d, rx->d, tx->modes, tx->samples, cut, nullptr, h);
+    } else {
+        st = fg::ensure_red(c, 3 * (size_t)B);
+        if (st == FOCSS_OK) st = fg::power_sums(c, tx, c->d_red);
+        if (st != FOCSS_OK) return st;
+        unsigned long long* cnt = (unsigned long long*)(c->d_red + B);
+        e = cudaMemsetAsync(cnt, 0, bytes, s);
+        const int gx = std::max(1, std::min(64, (int)((per + 1023) / 1024)));
+        if (e == cudaSuccess) FG_LAUNCH(fg::error_count_kernel<false><<<dim3(gx, B), 256, 0, s>>>(tx->d, rx->d, tx->modes, tx->samples, cut, c->d_red, cnt));
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h, cnt, bytes, cudaMemcpyDeviceToHost, s);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fg::cuda_check(c, e, "error_counts");
     for (int b = 0; b < B; ++b) {
@@ -940,10 +1152,10 @@ FOCSS_API focss_status focss_q2_factor(focss_ctx* c, const focss_field* tx, cons
     focss_status st = fg::check_same(c, tx, rx);
     if (st != FOCSS_OK) return st;
     cut = fg::clamp_cut(cut);
-    std::vector<double> h;
-    st = fg::sums_for(c, tx, rx, cut, tx->samples - cut, h);
+    const double* h = nullptr;
+    st = fg::pair_sums<fg::PAIR_Q2>(c, tx, rx, cut, tx->samples - cut, 0, &h);
     if (st != FOCSS_OK) return st;
-    for (int b = 0; b < tx->batch; ++b) q2[b] = -10 * std::log10(h[8 * b + 2] / h[8 * b + 0]);
+    for (int b = 0; b < tx->batch; ++b) q2[b] = -10 * std::log10(h[2 * b + 1] / h[2 * b]);
     return FOCSS_OK;
 }
 
@@ -952,18 +1164,11 @@ FOCSS_API focss_status focss_pse_estimate(focss_ctx* c, const focss_field* desir
     if (!c || !desired || !actual || !angle || angle_steps <= 0) return FOCSS_ERR_INVALID_ARG;
     focss_status st = fg::check_same(c, desired, actual);
     if (st != FOCSS_OK) return st;
-    const int B = desired->batch;
-    st = fg::ensure_red(c, 9 * (size_t)B);
+    const double* h = nullptr;
+    st = fg::pair_sums<fg::PAIR_PHASE>(c, desired, actual, 0, desired->samples, angle_steps, &h);
     if (st != FOCSS_OK) return st;
-    cudaStream_t s = c->stream;
-    cudaError_t e = cudaMemsetAsync(c->d_red, 0, sizeof(double) * 8 * B, s);
-    const int gx = std::max(1, std::min(64, (int)(((size_t)desired->modes * desired->samples + 1023) / 1024)));
-    if (e == cudaSuccess) FG_LAUNCH(fg::pair_sums_kernel<<<dim3(gx, B), 256, 0, s>>>(desired->d, actual->d, desired->modes, desired->samples, 0, desired->samples, c->d_red));
-    if (e == cudaSuccess) FG_LAUNCH(fg::pse_argmax_kernel<<<B, 256, 0, s>>>(c->d_red, angle_steps, c->d_red + 8 * B));
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(angle, c->d_red + 8 * B, sizeof(double) * B, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    return fg::cuda_check(c, e, "pse_estimate");
+    std::copy(h, h + desired->batch, angle);
+    return FOCSS_OK;
 }
 
 FOCSS_API focss_status focss_scalar_estimate(focss_ctx* c, const focss_field* desired, const focss_field* actual,
@@ -971,22 +1176,28 @@ FOCSS_API focss_status focss_scalar_estimate(focss_ctx* c, const focss_field* de
     if (!c || !desired || !actual || !scalar) return FOCSS_ERR_INVALID_ARG;
     focss_status st = fg::check_same(c, desired, actual);
     if (st != FOCSS_OK) return st;
-    std::vector<double> h;
+    const double* h = nullptr;
     // t = actual, r = desired: sum |actual|^2 and sum conj(actual) desired.
-    st = fg::sums_for(c, actual, desired, 0, actual->samples, h);
+    st = fg::pair_sums<fg::PAIR_SCALAR>(c, actual, desired, 0, actual->samples, 0, &h);
     if (st != FOCSS_OK) return st;
     for (int b = 0; b < actual->batch; ++b) {
-        scalar[2 * b] = h[8 * b + 5] / h[8 * b + 0];
-        scalar[2 * b + 1] = h[8 * b + 6] / h[8 * b + 0];
+        scalar[2 * b] = h[3 * b + 1] / h[3 * b];
+        scalar[2 * b + 1] = h[3 * b + 2] / h[3 * b];
     }
     return FOCSS_OK;
 }
 
 static focss_status scale_each(focss_ctx* c, focss_field* f, const std::vector<float2>& s) {
+    const size_t per = (size_t)f->modes * f->samples;
+    if (f->batch <= fg::kScalesByValue) {
+        fg::Scales v{};
+        std::copy(s.begin(), s.end(), v.s);
+        FG_LAUNCH(fg::scale_some_kernel<<<fg::grid_per_realization(per, f->batch), 256, 0, c->stream>>>(f->d, per, v));
+        return fg::cuda_check(c, cudaGetLastError(), "scale_each");
+    }
     float2* d = (float2*)fg::scratch_buffer(c, 6, sizeof(float2) * f->batch);
     if (!d) return fg::set_error(c, FOCSS_ERR_OOM, "scale scratch");
     cudaError_t e = cudaMemcpyAsync(d, s.data(), sizeof(float2) * f->batch, cudaMemcpyHostToDevice, c->stream);
-    const size_t per = (size_t)f->modes * f->samples;
     if (e == cudaSuccess) FG_LAUNCH(fg::scale_each_kernel<<<fg::grid_for(f->n(), 256), 256, 0, c->stream>>>(f->d, per, f->n(), d));
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);

@@ -130,6 +130,10 @@ struct Ctx {
     int* h_pinned = nullptr;         // pinned polling buffer
     double* d_red = nullptr;         // reduction scratch
     size_t red_cap = 0;
+    void* h_result = nullptr;        // pinned, written by kernels (result_buffer)
+    size_t result_cap = 0;
+    unsigned* d_ticket = nullptr;    // zeroed counters (tickets)
+    size_t ticket_cap = 0;
     std::vector<void*> scratch;      // generic device scratch buffers
     std::vector<size_t> scratch_cap;
     // device-resident derived tables keyed by their parameters (RRC spectra, ...)
@@ -181,6 +185,12 @@ int default_split(int N);
 bool split_supported(int N, int log2N1);
 focss_status ensure_state(Ctx* ctx, int batch);
 focss_status ensure_red(Ctx* ctx, size_t doubles);
+// Pinned host memory that kernels write small results to (read after a stream
+// synchronize, before the next call that uses it), and per-realization
+// counters that are zero between kernels; null when out of memory.
+constexpr size_t kResultCap = 256 << 10;  // codes beyond this go through device memory
+void* result_buffer(Ctx* ctx, size_t bytes);
+unsigned* tickets(Ctx* ctx, size_t n);
 void* scratch_buffer(Ctx* ctx, int slot, size_t bytes);
 
 // ---- ssfm.cu
