@@ -626,7 +626,7 @@ FOCSS_API focss_status focss_cd_compensation(focss_ctx* c, focss_field* f, const
     d.length *= spans;
     if (spans == 0) return FOCSS_OK;
     focss_ssfm_opts o{FOCSS_UNIFORM, 1, 0.0, 0.0};
-    return focss_ssfm_run(c, f, &d, &o, FOCSS_BACKWARD, nullptr);
+    return fg::linear_run(c, f, d, o, FOCSS_BACKWARD);
 }
 
 FOCSS_API focss_status focss_profile_enable(focss_ctx* c, int enable) {

@@ -205,15 +205,35 @@ __global__ void decimate_gather_kernel(const float2* __restrict__ in, float2* __
     }
 }
 
+// Spectrum of a zero-stuffed sequence times a filter: inserting osf - 1 zeros
+// repeats the n-point spectrum `in` (layout N1i x N2i) osf times, so pulse
+// shaping needs no transform of the N-point sequence: out (layout N1 x N2)
+// takes bin k mod n times H times g.  Shaping 5 x 2^19 samples from 2^15 symbols
+// each: 72 -> 62 us.
+__global__ void repeat_filter_kernel(const float2* __restrict__ in, const float2* __restrict__ H, float2* __restrict__ out,
+                                     float g, int n, int N1i, int N2i, int kc_in, int N, int N1, int N2, int kc_out,
+                                     int rows) {
+    const size_t total = (size_t)rows * N;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = i / N;
+        const int p = (int)(i % N);
+        const int k1 = p / N2, k2 = p % N2;
+        const int k = ((k1 < kc_out ? k1 : k1 - N1) + N1 * k2) & (n - 1);
+        const int r1 = k % N1i;
+        const float2 v = in[r * n + (size_t)r1 * N2i + ((k / N1i + (r1 >= kc_in)) & (N2i - 1))];
+        out[i] = cscale(cmul(v, H[p]), g);
+    }
+}
+
 // A *= exp(2 pi i x n), x = X / 2^64 turns per sample (two's complement),
 // X n formed exactly modulo 2^64 (modulation.cpp:255-264).
-__global__ void freq_shift_kernel(float2* __restrict__ d, int samples, size_t n, unsigned long long X) {
+__global__ void freq_shift_kernel(const float2* d, float2* out, int samples, size_t n, unsigned long long X) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const unsigned long long s = (unsigned long long)(i % (size_t)samples);
         const float x = (float)(long long)(X * s) * 1.0842021724855044e-19f;
         float sn, cs;
         sincospif(x, &sn, &cs);
-        d[i] = cmul(d[i], make_float2(cs, sn));
+        out[i] = cmul(d[i], make_float2(cs, sn));
     }
 }
 
@@ -759,9 +779,9 @@ focss_status rrc_table(Ctx* c, int samples, int n_symbols, int osf, double roll_
 
 // In place: data <- IFFT(FFT(data)/N * H/N) * extra for H in transposed layout
 // (Field::filter_inplace, field.cpp:358-372).
-focss_status apply_filter(Ctx* c, float2* d, int samples, int rows, const float2* H, double extra) {
+focss_status apply_filter(Ctx* c, float2* d, int samples, int rows, const float2* H, double extra, const float2* src = nullptr) {
     const double g = extra / ((double)samples * (double)samples);
-    return spectral_apply(c, d, samples, rows, ROW_TABLE, H, (float)g, 0);
+    return spectral_apply(c, d, samples, rows, ROW_TABLE, H, (float)g, 0, src);
 }
 
 // Pair sums (or the angle) of every realization into host[pair_sums_of(what)
@@ -864,13 +884,11 @@ FOCSS_API focss_status focss_decimate(focss_ctx* c, const focss_field* in, int f
     const int rows = in->batch * in->modes;
     float2* sp = (float2*)fg::scratch_buffer(c, 2, sizeof(float2) * in->n());
     if (!sp) return fg::set_error(c, FOCSS_ERR_OOM, "decimate scratch");
-    cudaError_t e = cudaMemcpyAsync(sp, in->d, sizeof(float2) * in->n(), cudaMemcpyDeviceToDevice, c->stream);
-    if (e != cudaSuccess) return fg::cuda_check(c, e, "decimate copy");
-    st = fg::fft_forward_transposed(c, sp, in->samples, rows, 1.0f / (float)in->samples);
+    st = fg::fft_forward_transposed(c, sp, in->samples, rows, 1.0f / (float)in->samples, in->d);
     if (st != FOCSS_OK) return st;
     FG_LAUNCH(fg::decimate_gather_kernel<<<fg::grid_for(out->n(), 256), 256, 0, c->stream>>>(
         sp, out->d, pi->N, pi->N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1, po->N2, fg::col_kc(po->N1), rows));
-    e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fg::cuda_check(c, e, "decimate gather");
     return fg::fft_inverse_transposed(c, out->d, out->samples, rows);
 }
@@ -921,9 +939,30 @@ FOCSS_API focss_status focss_rrc_shaping(focss_ctx* c, const focss_field* symbol
                                          double gain, focss_field* out) {
     // modulation.cpp:86-90: upsample(osf).filter_inplace(rrc(n, osf, roll_off)) * (sqrt(gain) * osf)
     if (!c || !symbols || !out || osf <= 0) return FOCSS_ERR_INVALID_ARG;
-    focss_status st = focss_upsample(c, symbols, osf, out);
-    if (st != FOCSS_OK) return st;
+    focss_status st;
     const float2* H = nullptr;
+    const int n = symbols->samples;
+    if (fg::fft_size_supported(n) && out->modes == symbols->modes && out->batch == symbols->batch &&
+        (long long)out->samples == (long long)n * osf && fg::fft_size_supported(out->samples)) {
+        const fg::Plan *pi = nullptr, *po = nullptr;
+        st = fg::get_plan(c, n, &pi);
+        if (st == FOCSS_OK) st = fg::get_plan(c, out->samples, &po);
+        if (st == FOCSS_OK) st = fg::rrc_table(c, out->samples, n, osf, roll_off, &H);
+        if (st != FOCSS_OK) return st;
+        const int rows = symbols->batch * symbols->modes;
+        float2* sp = (float2*)fg::scratch_buffer(c, 2, sizeof(float2) * symbols->n());
+        if (!sp) return fg::set_error(c, FOCSS_ERR_OOM, "rrc_shaping scratch");
+        const double N = out->samples;
+        st = fg::fft_forward_transposed(c, sp, n, rows, 1.0f, symbols->d);
+        if (st != FOCSS_OK) return st;
+        FG_LAUNCH(fg::repeat_filter_kernel<<<fg::grid_for(out->n(), 256), 256, 0, c->stream>>>(
+            sp, H, out->d, (float)(std::sqrt(gain) * osf / (N * N)), pi->N, pi->N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1,
+            po->N2, fg::col_kc(po->N1), rows));
+        st = fg::cuda_check(c, cudaGetLastError(), "rrc_shaping spectrum");
+        return st == FOCSS_OK ? fg::fft_inverse_transposed(c, out->d, out->samples, rows) : st;
+    }
+    st = focss_upsample(c, symbols, osf, out);
+    if (st != FOCSS_OK) return st;
     st = fg::rrc_table(c, out->samples, symbols->samples, osf, roll_off, &H);
     if (st != FOCSS_OK) return st;
     return fg::apply_filter(c, out->d, out->samples, out->batch * out->modes, H, std::sqrt(gain) * osf);
@@ -937,11 +976,9 @@ FOCSS_API focss_status focss_rrc_sampling(focss_ctx* c, const focss_field* signa
         return fg::set_error(c, FOCSS_ERR_INVALID_ARG, "rrc_sampling: output shape");
     float2* tmp = (float2*)fg::scratch_buffer(c, 2, sizeof(float2) * signal->n());
     if (!tmp) return fg::set_error(c, FOCSS_ERR_OOM, "rrc_sampling scratch");
-    cudaError_t e = cudaMemcpyAsync(tmp, signal->d, sizeof(float2) * signal->n(), cudaMemcpyDeviceToDevice, c->stream);
-    if (e != cudaSuccess) return fg::cuda_check(c, e, "rrc_sampling copy");
     const float2* H = nullptr;
     focss_status st = fg::rrc_table(c, signal->samples, signal->samples / osf, osf, roll_off, &H);
-    if (st == FOCSS_OK) st = fg::apply_filter(c, tmp, signal->samples, signal->batch * signal->modes, H, 1.0);
+    if (st == FOCSS_OK) st = fg::apply_filter(c, tmp, signal->samples, signal->batch * signal->modes, H, 1.0, signal->d);
     if (st != FOCSS_OK) return st;
     FG_LAUNCH(fg::downsample_kernel<<<fg::grid_for(out->n(), 256), 256, 0, c->stream>>>(tmp, out->d, out->n(), osf, (float)std::sqrt(gain)));
     return fg::cuda_check(c, cudaGetLastError(), "rrc_sampling");
@@ -951,16 +988,19 @@ FOCSS_API focss_status focss_frequency_shift(focss_ctx* c, focss_field* f, doubl
     if (!c || !f) return FOCSS_ERR_INVALID_ARG;
     // modulation.cpp:255-264: A(mode, s) *= i_exp(2 pi f dt s)
     const unsigned long long X = fg::turns_fix64_host(frequency * f->dt);
-    FG_LAUNCH(fg::freq_shift_kernel<<<fg::grid_for(f->n(), 256), 256, 0, c->stream>>>(f->d, f->samples, f->n(), X));
+    FG_LAUNCH(fg::freq_shift_kernel<<<fg::grid_for(f->n(), 256), 256, 0, c->stream>>>(f->d, f->d, f->samples, f->n(), X));
     return fg::cuda_check(c, cudaGetLastError(), "frequency_shift");
 }
 
-FOCSS_API focss_status focss_bandpass(focss_ctx* c, focss_field* f, double frequency) {
-    if (!c || !f) return FOCSS_ERR_INVALID_ARG;
-    // modulation.cpp:266-277: cut = int(f * duration) + 1; zero bins [cut, N - cut].
+// modulation.cpp:266-277: cut = int(f * duration) + 1; zero bins [cut, N - cut].
+static focss_status bandpass(focss_ctx* c, focss_field* f, double frequency, const float2* src) {
     const int cut = (int)(frequency * (f->samples * f->dt)) + 1;
     return fg::spectral_apply(c, f->d, f->samples, f->batch * f->modes, fg::ROW_BANDPASS, nullptr,
-                              1.0f / (float)f->samples, cut);
+                              1.0f / (float)f->samples, cut, src);
+}
+FOCSS_API focss_status focss_bandpass(focss_ctx* c, focss_field* f, double frequency) {
+    if (!c || !f) return FOCSS_ERR_INVALID_ARG;
+    return bandpass(c, f, frequency, f->d);
 }
 
 FOCSS_API focss_status focss_wdm_select(focss_ctx* c, const focss_field* in, int channel_index,
@@ -968,13 +1008,18 @@ FOCSS_API focss_status focss_wdm_select(focss_ctx* c, const focss_field* in, int
     if (!c || !in || !out) return FOCSS_ERR_INVALID_ARG;
     focss_status st = fg::check_same(c, in, out);
     if (st != FOCSS_OK) return st;
-    if (out != in) {
-        cudaError_t e = cudaMemcpyAsync(out->d, in->d, sizeof(float2) * in->n(), cudaMemcpyDeviceToDevice, c->stream);
-        if (e != cudaSuccess) return fg::cuda_check(c, e, "wdm_select copy");
+    // shift, then band-pass (modulation.cpp:255-277) without a copy first: the
+    // shift, or where it is none the column pass, reads the input itself (centre
+    // channel of 12 x 2^19 samples: 125 -> 92 us)
+    const unsigned long long X = fg::turns_fix64_host(-channel_bandwidth * channel_index * out->dt);
+    const float2* src = in->d;
+    if (X) {
+        FG_LAUNCH(fg::freq_shift_kernel<<<fg::grid_for(in->n(), 256), 256, 0, c->stream>>>(in->d, out->d, in->samples, in->n(), X));
+        st = fg::cuda_check(c, cudaGetLastError(), "wdm_select shift");
+        if (st != FOCSS_OK) return st;
+        src = out->d;
     }
-    st = focss_frequency_shift(c, out, -channel_bandwidth * channel_index);
-    if (st != FOCSS_OK) return st;
-    return focss_bandpass(c, out, 0.5 * channel_bandwidth);
+    return bandpass(c, out, 0.5 * channel_bandwidth, src);
 }
 
 FOCSS_API focss_status focss_wdm_mux(focss_ctx* c, const focss_field* ch, double channel_bandwidth,

@@ -104,6 +104,8 @@ struct PassArgs {
     int op;
     float scale;
     int bp_cut;
+    long long src_off;      // stateless forward column pass: samples from data to its input (0: in place)
+    unsigned long long disp_hi, disp_lo;  // stateless ROW_SSFM: dispersion phase as in SsfmState, gain in scale
     int* fault;             // set to 1 by a kernel whose bounded wait ran out (may be null)
 };
 
@@ -209,6 +211,8 @@ focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ss
                       int* steps_out, const StepGrid* grid = nullptr, int* recorded_out = nullptr);
 // Argument checks of ssfm_run and the pass arguments of one run (state and
 // finished-realization counter supplied by the caller).
+// Dispersion only (alpha = gamma = 0) over fib.length, o a single UNIFORM step.
+focss_status linear_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ssfm_opts& o, double dir);
 focss_status ssfm_validate(Ctx* ctx, const Field* f, const focss_fiber& fib, const focss_ssfm_opts& o);
 PassArgs ssfm_args(const Field* f, const focss_fiber& fib, const focss_ssfm_opts& o, double dir, SsfmState* state,
                    int* n_done);
@@ -245,9 +249,10 @@ focss_status fft_forward(Ctx* ctx, float2* data, int N, int batch);   // natural
 focss_status fft_inverse(Ctx* ctx, float2* data, int N, int batch);   // natural order, unnormalized
 // Forward then pointwise op then inverse, spectrum never leaves the two-pass layout.
 focss_status spectral_apply(Ctx* ctx, float2* data, int N, int batch, int row_op, const float2* table,
-                            float scale, int bp_cut);
+                            float scale, int bp_cut, const float2* src = nullptr);
 // Two-pass-layout spectrum (row k1, column k2 holds bin k1' + N1*k2 mod N, see col_work), x scale.
-focss_status fft_forward_transposed(Ctx* ctx, float2* data, int N, int batch, float scale);
+// src: the input, left as it is (null: data, in place)
+focss_status fft_forward_transposed(Ctx* ctx, float2* data, int N, int batch, float scale, const float2* src = nullptr);
 focss_status fft_inverse_transposed(Ctx* ctx, float2* data, int N, int batch);
 
 // ---- dsp.cu

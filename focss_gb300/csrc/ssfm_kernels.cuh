@@ -57,13 +57,13 @@ __device__ __forceinline__ double log_step(const SsfmParams& p, int K, int i) {
 }
 
 // a (turns, any sign) -> 96-bit two's-complement turn fraction hi*2^-64 + lo*2^-96.
-__device__ __forceinline__ void turns_fix96(double a, unsigned long long& hi, unsigned long long& lo) {
+__host__ __device__ __forceinline__ void turns_fix96(double a, unsigned long long& hi, unsigned long long& lo) {
     const double ab = fabs(a);
     const double fr = ab - floor(ab);             // exact
     const double s64 = fr * 0x1p64;               // exact, < 2^64
     const double h = floor(s64);
-    hi = __double2ull_rz(h);
-    lo = __double2ull_rz((s64 - h) * 0x1p32);     // < 2^32
+    hi = (unsigned long long)h;
+    lo = (unsigned long long)((s64 - h) * 0x1p32);  // < 2^32
     if (a < 0) {
         if (lo == 0) {
             hi = 0ull - hi;
@@ -255,7 +255,7 @@ __device__ __forceinline__ void col_work(const PassArgs& a, int op, const SsfmSt
     float2* base = data + n2;
     // the columns come from `src` (a tile of C columns, rows src_ld apart,
     // staged in shared memory) when given, else from data
-    const float2* lb = src ? src + c : base;
+    const float2* lb = src ? src + c : base + a.src_off;
     const int lld = src ? src_ld : ld;
     float2 v[Q];
     {
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row
     pdl_wait();
     const int b = blockIdx.y;  // realization * modes + mode
     const SsfmState* st = a.state ? a.state + b / (a.modes > 1 ? a.modes : 1) : nullptr;
-    unsigned long long dhi = 0ull, dlo = 0ull;
+    unsigned long long dhi = a.disp_hi, dlo = a.disp_lo;
     float g = a.scale;
     if (st) {
         if (!*(volatile const int*)&st->row_active) return;
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row
         dlo = st->disp_lo;
         g = st->lin_gain;
     }
-    row_tables<N2>(a, st != nullptr, g, s_tw, s_T);
+    row_tables<N2>(a, st || a.op == ROW_SSFM, g, s_tw, s_T);
     const int rl = threadIdx.x / P, t = threadIdx.x % P;
     row_work<N2>(a, st ? (int)ROW_SSFM : a.op, a.data + (size_t)b * a.N, blockIdx.x * R + rl, rl, t, s_tw, s_T, sx,
                  g, dhi, dlo, N2);
