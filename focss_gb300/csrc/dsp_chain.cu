@@ -573,9 +573,8 @@ __global__ void error_count_kernel(const float2* __restrict__ tx, const float2* 
 // them up (ticket, which it sets back to zero), so one launch does a call and
 // the result can go straight to host memory.  FP64 (~2 operations per cycle and
 // SM) bounds the sums: only the ones asked for are formed, 4 conversions and 4
-// or 6 fused multiply-adds per sample instead of 18 operations.  Estimating and
-// applying the angle of 12 x 32768 samples: 125 -> 85 us, of which the sums
-// and the angle took 65.
+// or 6 fused multiply-adds per sample instead of 18 operations.  12 x 32768
+// samples: sums 34 us and angle 31 us, 16 us in one launch.
 enum { PAIR_Q2 = 0, PAIR_SCALAR = 1, PAIR_PHASE = 2 };
 __host__ __device__ constexpr int pair_sums_of(int what) { return what == PAIR_SCALAR ? 3 : 2; }
 constexpr int kPairBlocks = 64;  // CTAs per realization, at most
@@ -584,51 +583,41 @@ constexpr int kPairBlocks = 64;  // CTAs per realization, at most
 // Re(e^{i 2 pi i / steps} (cr + i ci)) (q2 is monotone in it), the first maximum
 // wins.  Around the peak at -arg(cr + i ci) neighbours fall off by at least
 // ~(2 pi / steps)^2 / 2 of it, far above rounding up to 65536 steps, so the
-// five steps around it decide; otherwise (or without a usable argument) all
-// steps are tried.  Called by a whole CTA, result in thread 0.
+// five steps around it decide (an FP32 argument is off by less than 0.01 step);
+// otherwise, or without a usable argument, all steps are tried.  Called by one
+// warp: the FP64 pipe serves ~2 lanes per cycle, so idle warps' copies of the
+// same arithmetic would cost as much again each.
 __device__ int phase_argmax(double cr, double ci, int steps) {
     const double two_pi = 2 * 3.14159265358979323846264338;
     const double mag = fmax(fabs(cr), fabs(ci));
-    const bool near = steps >= 8 && steps <= 65536 && mag > 1e-290 && mag < 1e290 && !isnan(cr) && !isnan(ci);
+    const int lane = threadIdx.x & 31;
     int first = 0, count = steps;
-    if (near) {
-        first = __double2int_rn(-atan2(ci, cr) / two_pi * steps) - 2;
+    if (steps >= 8 && steps <= 65536 && mag > 1e-290 && mag < 1e290 && !isnan(cr) && !isnan(ci)) {
+        first = __float2int_rn(-atan2f((float)(ci / mag), (float)(cr / mag)) * 0.15915494f * (float)steps) - 2;
         count = 5;
     }
     double best = -1e308;
     int bi = 0;
-    for (int k = threadIdx.x; k < count; k += blockDim.x) {
+    for (int k = lane; k < count; k += 32) {
         int i = first + k;
         if (i < 0) i += steps;
         if (i >= steps) i -= steps;
         const double ang = two_pi * (double)i / steps;
-        const double v = cr * cos(ang) - ci * sin(ang);
+        double sn, cs;
+        sincos(ang, &sn, &cs);
+        const double v = cr * cs - ci * sn;
         if (v > best || (v == best && i < bi)) {
             best = v;
             bi = i;
         }
     }
-    __shared__ double sv[32];
-    __shared__ int si[32];
-    for (int round = 0; round < 2; ++round) {
-        for (int o = 16; o > 0; o >>= 1) {
-            const double v = __shfl_xor_sync(0xffffffffu, best, o);
-            const int i = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (v > best || (v == best && i < bi)) {
-                best = v;
-                bi = i;
-            }
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, best, o);
+        const int i = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (v > best || (v == best && i < bi)) {
+            best = v;
+            bi = i;
         }
-        if (round) break;
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        if (lane == 0) {
-            sv[warp] = best;
-            si[warp] = bi;
-        }
-        __syncthreads();
-        if (warp) break;
-        best = lane < (int)blockDim.x / 32 ? sv[lane] : -1e308;
-        bi = lane < (int)blockDim.x / 32 ? si[lane] : 0x7FFFFFFF;
     }
     return bi;
 }
@@ -699,8 +688,9 @@ __global__ void __launch_bounds__(256) pair_sums_kernel(const float2* __restrict
     }
     __syncthreads();
     if (WHAT == PAIR_PHASE) {
+        if (warp) return;
         const int i = phase_argmax(s_sum[0], s_sum[1], steps);
-        if (threadIdx.x == 0) out[b] = 2 * 3.14159265358979323846264338 * (double)i / steps;
+        if (lane == 0) out[b] = 2 * 3.14159265358979323846264338 * (double)i / steps;
     } else if (threadIdx.x < K) {
         out[(size_t)b * K + threadIdx.x] = s_sum[threadIdx.x];
     }
@@ -789,8 +779,10 @@ focss_status apply_filter(Ctx* c, float2* d, int samples, int rows, const float2
 template <int WHAT>
 focss_status pair_sums(Ctx* c, const Field* t, const Field* r, int lo, int hi, int steps, const double** host) {
     const int B = t->batch;
-    // 2 samples per thread before the CTAs of a realization meet, up to 64 CTAs
-    const int gx = std::max(1, std::min(kPairBlocks, (int)(((size_t)t->modes * std::max(hi - lo, 1) + 511) / 512)));
+    // at least 2 samples per thread before the CTAs of a realization meet, and
+    // about two CTAs per SM (their FP64 sums over the CTA add up otherwise)
+    const int fill = std::max(1, std::min(kPairBlocks, 2 * sm_count() / B));
+    const int gx = std::max(1, std::min(fill, (int)(((size_t)t->modes * std::max(hi - lo, 1) + 511) / 512)));
     constexpr int K = pair_sums_of(WHAT);
     const size_t results = sizeof(double) * B * K;
     double* out = (double*)result_buffer(c, results);
