@@ -91,12 +91,15 @@ inline Tables tables_at(const void* buf, int N1) {
     return t;
 }
 
+// Kernel arguments: what every pass reads first is kept together (constant-bank
+// lines are cold at a launch), the step parameters last.
 struct PassArgs {
     float2* data;           // batch x N complex64
-    Tables tw;
-    const float2* table;    // ROW_TABLE multiplier, transposed layout (k1*N2 + k2), length N
+    // realizations of several fields in one SSFM launch (both or none): each
+    // one's samples (modes x N) and parameters, in place of data and prm
+    float2* const* datas;
     SsfmState* state;       // null: plain transform driven by `op`
-    SsfmParams prm;
+    Tables tw;
     int N, N1, N2, log2N2;
     int kc;                 // rows k1 >= kc hold the bins k1 - N1 + N1 k2 (set by the launch helpers)
     int batch;              // realizations (set by the launch helpers)
@@ -106,6 +109,9 @@ struct PassArgs {
     int bp_cut;
     long long src_off;      // stateless forward column pass: samples from data to its input (0: in place)
     unsigned long long disp_hi, disp_lo;  // stateless ROW_SSFM: dispersion phase as in SsfmState, gain in scale
+    const float2* table;    // ROW_TABLE multiplier, transposed layout (k1*N2 + k2), length N
+    const SsfmParams* prms;
+    SsfmParams prm;
     int* fault;             // set to 1 by a kernel whose bounded wait ran out (may be null)
 };
 

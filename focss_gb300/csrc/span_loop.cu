@@ -7,9 +7,11 @@
 // a UNIFORM grid, a data-dependent number for ADAPTIVE / LOGARITHMIC) and
 // another optional amplifier.  Here the whole chain, for every field of the
 // call, is captured once into one graph:
-//   * each field is one branch (fields of different lengths and batches run
+//   * fields of different lengths and batches are branches (they run
 //     concurrently and fill the GPU together);
-//   * UNIFORM spans are plain pass sequences;
+//   * UNIFORM spans are plain pass sequences, those of all fields of one length
+//     in one branch (record_group): a pass pair of 25 short fields is two
+//     launches instead of 50, and launches are what such a call is bound by;
 //   * ADAPTIVE / LOGARITHMIC spans are a conditional WHILE node whose body is
 //     kChunk pass pairs plus a one-thread check kernel; the check ends the loop
 //     once the SSFM state machines of all realizations report the span done
@@ -31,13 +33,26 @@
 
 namespace fg {
 
+// A field's amplifier operations in a group (amp_group_kernel).
+struct AmpField {
+    float2* d;
+    size_t n;
+    int samples;
+    float2 scale[2];  // before, after
+    float sigma[2];
+};
+
 struct LoopGraph {
     cudaGraphExec_t exec = nullptr;
     SsfmState* d_state = nullptr;         // every field's realizations
     int* d_ctr = nullptr;                 // kCtr counters per field
     int* d_steps = nullptr;               // steps per realization, summed over spans
     unsigned long long* d_amp = nullptr;  // {seed, counter0} per field
+    float2** d_data = nullptr;            // every realization's samples (grouped fields)
+    SsfmParams* d_prm = nullptr;          // and parameters
+    AmpField* d_ampf = nullptr;           // grouped fields' amplifiers
     std::vector<int> offset, batch;       // first realization and batch of each field
+    std::vector<int> slot;                // place of each field in d_ctr, d_amp and d_ampf
     int total = 0;
     long long static_kernels = 0;         // kernel nodes outside loop bodies
     std::vector<int> body_kernels;        // kernels per loop-body iteration, per field
@@ -78,6 +93,27 @@ __global__ void amp_graph_kernel(float2* __restrict__ d, int samples, size_t n, 
         d[i] = amplifier_sample(d[i], i, samples, scale, sigma, key, (uint32_t)counter, (uint32_t)(counter >> 32));
 }
 
+// The amplifiers of a group of fields (blockIdx.y), before or after a span.
+__global__ void amp_group_kernel(const AmpField* __restrict__ fields, const unsigned long long* __restrict__ sc, int after,
+                                 int span) {
+    const AmpField f = fields[blockIdx.y];
+    const unsigned long long seed = sc[2 * blockIdx.y], counter = sc[2 * blockIdx.y + 1] + (unsigned long long)span;
+    const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
+    const float2 scale = f.scale[after];
+    const float sigma = f.sigma[after];
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < f.n; i += (size_t)gridDim.x * blockDim.x)
+        f.d[i] = amplifier_sample(f.d[i], i, f.samples, scale, sigma, key, (uint32_t)counter, (uint32_t)(counter >> 32));
+}
+
+// span_end_kernel for a group of UNIFORM fields: a realization's counters are
+// found by its n_done.
+__global__ void span_end_group_kernel(const SsfmState* __restrict__ st, const SsfmParams* __restrict__ prm, int n, int* steps) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x) {
+        if (st[b].action != COL_IDLE) atomicOr(prm[b].n_done + 3, 1);
+        steps[b] += st[b].n_steps;
+    }
+}
+
 int amp_grid(size_t n) {
     size_t g = (n + 255) / 256;
     if (g > (size_t)sm_count() * 32) g = (size_t)sm_count() * 32;
@@ -110,6 +146,9 @@ void destroy_graph(LoopGraph* g) {
     cudaFree(g->d_ctr);
     cudaFree(g->d_steps);
     cudaFree(g->d_amp);
+    cudaFree(g->d_data);
+    cudaFree(g->d_prm);
+    cudaFree(g->d_ampf);
     delete g;
 }
 
@@ -136,7 +175,7 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
                           cudaStream_t body_stream) {
     const int B = f->batch;
     SsfmState* state = g->d_state + g->offset[i];
-    int* ctr = g->d_ctr + kCtr * i;
+    int* ctr = g->d_ctr + kCtr * g->slot[i];
     int* steps = g->d_steps + g->offset[i];
     const size_t n = f->n();
     double sc_b = 1, sg_b = 0, sc_a = 1, sg_a = 0;
@@ -148,7 +187,7 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
     for (int span = 0; span < spans && e == cudaSuccess; ++span) {
         if (amp.before != FOCSS_AMP_NONE) {
             amp_graph_kernel<<<amp_grid(n), 256, 0, s>>>(f->d, f->samples, n, split_df(sc_b), (float)sg_b,
-                                                         g->d_amp + 2 * i, span);
+                                                         g->d_amp + 2 * g->slot[i], span);
             e = cudaGetLastError();
             g->static_kernels += 1;
         }
@@ -162,9 +201,9 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
         } else if (o.grid == FOCSS_UNIFORM) {
             for (int k = 0; k < o.total_steps + 2 && e == cudaSuccess; ++k) {
                 e = launch_col(p, a, B, s);
-                if (e == cudaSuccess) e = launch_row(p, a, B, s);
+                if (e == cudaSuccess && k <= o.total_steps) e = launch_row(p, a, B, s);
             }
-            g->static_kernels += 2ll * (o.total_steps + 2);
+            g->static_kernels += 2ll * (o.total_steps + 2) - 1;
         } else {
             // Conditional WHILE node appended to the branch's capture.
             cudaStreamCaptureStatus cs;
@@ -213,10 +252,63 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
         g->static_kernels += 1;
         if (e == cudaSuccess && amp.after != FOCSS_AMP_NONE) {
             amp_graph_kernel<<<amp_grid(n), 256, 0, s>>>(f->d, f->samples, n, split_df(sc_a), (float)sg_a,
-                                                         g->d_amp + 2 * i, span);
+                                                         g->d_amp + 2 * g->slot[i], span);
             e = cudaGetLastError();
             g->static_kernels += 1;
         }
+    }
+    return e;
+}
+
+// Records a group (UNIFORM fields of one length, by descending step count) as
+// one branch: each pass runs all of its realizations that are not done with
+// the span.  Back-propagation of 25 fields of 5 realizations (five lengths from 2^13
+// to 2^17, 15 spans of 1 to 16 steps): 13.7 -> 10.2 ms.
+cudaError_t record_group(LoopGraph* g, const std::vector<int>& group, Field* const* fs, const Plan& p,
+                         const focss_ssfm_opts* opts, const focss_amp& amp, int spans, cudaStream_t s) {
+    const int first = group[0], off = g->offset[first], slot = g->slot[first], nf = (int)group.size();
+    int B = 0;
+    size_t largest = 0;
+    for (int i : group) {
+        B += g->batch[i];
+        largest = std::max(largest, fs[i]->n());
+    }
+    PassArgs a{};
+    a.modes = fs[first]->modes;
+    a.state = g->d_state + off;
+    a.datas = g->d_data + off;
+    a.prms = g->d_prm + off;
+    int* ctr = g->d_ctr + kCtr * slot;
+    // realizations of the fields with more than `steps` steps
+    auto active = [&](int steps) {
+        int n = 0;
+        for (int i : group)
+            if (opts[i].total_steps > steps) n += g->batch[i];
+        return n;
+    };
+    auto amplify = [&](int after, int span) {
+        amp_group_kernel<<<dim3(amp_grid(largest), nf), 256, 0, s>>>(g->d_ampf + slot, g->d_amp + 2 * slot, after, span);
+        g->static_kernels += 1;
+        return cudaGetLastError();
+    };
+    cudaError_t e = cudaMemsetAsync(g->d_steps + off, 0, sizeof(int) * B, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctr, 0, sizeof(int) * kCtr * nf, s);
+    for (int span = 0; span < spans && e == cudaSuccess; ++span) {
+        if (amp.before != FOCSS_AMP_NONE) e = amplify(0, span);
+        if (e == cudaSuccess) e = cudaMemsetAsync(g->d_state + off, 0, sizeof(SsfmState) * B, s);
+        // K steps take K + 2 column passes with a row pass between any two
+        const int passes = opts[first].total_steps + 2;
+        for (int k = 0; k < passes && e == cudaSuccess; ++k) {
+            e = launch_col(p, a, active(k - 2), s);
+            const int rows = active(k - 1);
+            if (e == cudaSuccess && rows) e = launch_row(p, a, rows, s);
+            g->static_kernels += rows ? 2 : 1;
+        }
+        if (e != cudaSuccess) break;
+        span_end_group_kernel<<<(B + 255) / 256, 256, 0, s>>>(a.state, a.prms, B, g->d_steps + off);
+        e = cudaGetLastError();
+        g->static_kernels += 1;
+        if (e == cudaSuccess && amp.after != FOCSS_AMP_NONE) e = amplify(1, span);
     }
     return e;
 }
@@ -226,17 +318,73 @@ focss_status build_graph(Ctx* ctx, LoopGraph* g, int nf, Field* const* fs, const
                          double dir) {
     g->offset.resize(nf);
     g->batch.resize(nf);
+    g->slot.resize(nf);
     g->body_kernels.assign(nf, 0);
+    // branches: UNIFORM fields of one length together (two-pass runs with plain
+    // loads; the largest step count first), any other field alone
+    std::vector<std::vector<int>> branches;
+    std::vector<char> grouped(nf, 0);
+    auto groupable = [&](int i) {
+        return opts[i].grid == FOCSS_UNIFORM && !ssfm_single_cta(ctx, fs[i]) && plans[i]->staging == FOCSS_STAGING_LOADS;
+    };
     for (int i = 0; i < nf; ++i) {
-        g->offset[i] = g->total;
-        g->batch[i] = fs[i]->batch;
-        g->total += fs[i]->batch;
+        if (grouped[i]) continue;
+        std::vector<int> br{i};
+        int B = fs[i]->batch;
+        for (int j = i + 1; groupable(i) && j < nf; ++j)
+            if (!grouped[j] && groupable(j) && fs[j]->samples == fs[i]->samples && fs[j]->modes == fs[i]->modes &&
+                (long long)(B + fs[j]->batch) * fs[i]->modes <= 65535) {  // realizations are a grid's y
+                br.push_back(j);
+                grouped[j] = 1;
+                B += fs[j]->batch;
+            }
+        std::stable_sort(br.begin(), br.end(), [&](int x, int y) { return opts[x].total_steps > opts[y].total_steps; });
+        branches.push_back(br);
     }
+    int slots = 0;
+    for (const auto& br : branches)
+        for (int i : br) {
+            g->slot[i] = slots++;
+            g->offset[i] = g->total;
+            g->batch[i] = fs[i]->batch;
+            g->total += fs[i]->batch;
+        }
     cudaError_t e = cudaMalloc(&g->d_state, sizeof(SsfmState) * g->total);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_ctr, sizeof(int) * kCtr * nf);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_steps, sizeof(int) * g->total);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_amp, sizeof(unsigned long long) * 2 * nf);
     if (e == cudaSuccess) e = ensure_side(ctx, (size_t)nf + 1, (size_t)nf + 1);
+    if (e == cudaSuccess && branches.size() < (size_t)nf) {
+        std::vector<float2*> data(g->total);
+        std::vector<SsfmParams> prm(g->total);
+        std::vector<AmpField> ampf(nf);
+        for (int i = 0; i < nf; ++i) {
+            const Field* f = fs[i];
+            const PassArgs a = ssfm_args(f, fib, opts[i], dir, nullptr, g->d_ctr + kCtr * g->slot[i]);
+            for (int b = 0; b < f->batch; ++b) {
+                data[g->offset[i] + b] = f->d + (size_t)b * f->modes * f->samples;
+                prm[g->offset[i] + b] = a.prm;
+            }
+            AmpField& af = ampf[g->slot[i]];
+            af.d = f->d;
+            af.n = f->n();
+            af.samples = f->samples;
+            for (int w = 0; w < 2; ++w) {
+                const int op = w ? amp.after : amp.before;
+                double sc = 1, sg = 0;
+                if (op != FOCSS_AMP_NONE) amplifier_coeffs(op, amp.gain, amp.noise_factor, f->f0, f->dt, &sc, &sg);
+                af.scale[w] = split_df(sc);
+                af.sigma[w] = (float)sg;
+            }
+        }
+        e = cudaMalloc(&g->d_data, sizeof(float2*) * g->total);
+        if (e == cudaSuccess) e = cudaMalloc(&g->d_prm, sizeof(SsfmParams) * g->total);
+        if (e == cudaSuccess) e = cudaMalloc(&g->d_ampf, sizeof(AmpField) * nf);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_data, data.data(), sizeof(float2*) * g->total, cudaMemcpyHostToDevice, ctx->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_prm, prm.data(), sizeof(SsfmParams) * g->total, cudaMemcpyHostToDevice, ctx->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_ampf, ampf.data(), sizeof(AmpField) * nf, cudaMemcpyHostToDevice, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    }
     if (e != cudaSuccess) return cuda_check(ctx, e, "span loop set-up");
 
     cudaStream_t s = ctx->stream;
@@ -249,10 +397,14 @@ focss_status build_graph(Ctx* ctx, LoopGraph* g, int nf, Field* const* fs, const
     }
     cudaEvent_t fork = ctx->side_events[nf];
     e = cudaEventRecord(fork, s);
-    for (int i = 0; i < nf && e == cudaSuccess; ++i) {
+    for (size_t r = 0; r < branches.size() && e == cudaSuccess; ++r) {
+        const int i = branches[r][0];
         cudaStream_t b = ctx->side_streams[i];
         e = cudaStreamWaitEvent(b, fork, 0);
-        if (e == cudaSuccess) e = record_branch(ctx, g, i, fs[i], *plans[i], fib, opts[i], amp, spans, dir, b, body_stream);
+        if (e == cudaSuccess)
+            e = branches[r].size() > 1
+                    ? record_group(g, branches[r], fs, *plans[i], opts, amp, spans, b)
+                    : record_branch(ctx, g, i, fs[i], *plans[i], fib, opts[i], amp, spans, dir, b, body_stream);
         // always join, so that the capture can be ended cleanly
         const cudaError_t e1 = cudaEventRecord(ctx->side_events[i], b);
         const cudaError_t e2 = cudaStreamWaitEvent(s, ctx->side_events[i], 0);
@@ -330,8 +482,8 @@ FOCSS_API focss_status focss_span_loop(focss_ctx* c, int n_fields, focss_field* 
     }
     std::vector<unsigned long long> sc(2 * (size_t)n_fields);
     for (int i = 0; i < n_fields; ++i) {
-        sc[2 * i] = amp->seed + (unsigned long long)i;
-        sc[2 * i + 1] = amp->counter0;
+        sc[2 * g->slot[i]] = amp->seed + (unsigned long long)i;
+        sc[2 * g->slot[i] + 1] = amp->counter0;
     }
     cudaStream_t s = c->stream;
     cudaError_t e = cudaMemcpyAsync(g->d_amp, sc.data(), sizeof(unsigned long long) * sc.size(),
@@ -345,19 +497,21 @@ FOCSS_API focss_status focss_span_loop(focss_ctx* c, int n_fields, focss_field* 
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fg::cuda_check(c, e, "span loop run");
     long long kernels = g->static_kernels;
-    for (int i = 0; i < n_fields; ++i) kernels += (long long)ctr[fg::kCtr * i + 4] * g->body_kernels[i];
+    for (int i = 0; i < n_fields; ++i) kernels += (long long)ctr[fg::kCtr * g->slot[i] + 4] * g->body_kernels[i];
     fg::count_launch_graph(kernels);
     for (int i = 0; i < n_fields; ++i) {
-        if (ctr[fg::kCtr * i + 2])
+        const int* ct = &ctr[fg::kCtr * (size_t)g->slot[i]];
+        if (ct[2])
             return fg::set_error(c, FOCSS_ERR_NOT_CONVERGED, "span_loop: step cap reached (field " + std::to_string(i) + ")");
-        if (ctr[fg::kCtr * i + 3]) {
+        if (ct[3]) {
             // a single-CTA run stops a realization at the step cap, unfinished
             if (fg::ssfm_single_cta(c, fs[i]))
                 return fg::set_error(c, FOCSS_ERR_NOT_CONVERGED, "span_loop: step cap reached (field " + std::to_string(i) + ")");
             return fg::set_error(c, FOCSS_ERR_TIMEOUT, "span_loop: a realization did not finish (field " + std::to_string(i) + ")");
         }
     }
-    if (steps_out) std::copy(steps.begin(), steps.end(), steps_out);
+    for (int i = 0; steps_out && i < n_fields; ++i)
+        steps_out = std::copy_n(steps.begin() + g->offset[i], g->batch[i], steps_out);
     return FOCSS_OK;
 }
 

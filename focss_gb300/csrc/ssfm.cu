@@ -389,7 +389,8 @@ focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ss
                 if (e == cudaSuccess) e = cudaEventRecord(pe[2], s);
             } else {
                 e = launch_col(*p, a, f->batch, s);
-                if (e == cudaSuccess) e = launch_row(*p, a, f->batch, s);
+                // (a fixed grid's last column pass leaves nothing for a row pass)
+                if (e == cudaSuccess && !(fixed && i + 1 == n)) e = launch_row(*p, a, f->batch, s);
             }
             if (e != cudaSuccess) {
                 if (ev) cudaEventDestroy(ev);

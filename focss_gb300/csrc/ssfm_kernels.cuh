@@ -389,7 +389,7 @@ __device__ __forceinline__ void col_advance(const PassArgs& a, SsfmState* st, in
             __threadfence();
             const float peak = __uint_as_float(atomicOr(&st->peak_bits, 0u));
             const double sum = op == COL_FWD ? atomicAdd(&st->sum, 0.0) : 0.0;
-            ssfm_advance(*st, a.prm, b, op, peak, sum);
+            ssfm_advance(*st, a.prms ? a.prms[b] : a.prm, b, op, peak, sum);
             st->peak_bits = 0u;
             st->sum = 0.0;
             st->blocks_done = 0u;
@@ -434,8 +434,9 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
     for (int i = threadIdx.x; i < N1; i += blockDim.x) s_fc[i] = a.tw.col[i];
     const int modes = a.modes > 1 ? a.modes : 1;
     float pk = 0.0f, sm = 0.0f;
-    col_work<N1, C>(a, op, st, a.data + ((size_t)b * modes + mo) * a.N, blockIdx.x * C, s_fc, s_B, C, sx, s_x0, mo,
-                    modes, threadIdx.x % (C * P), a.N2, pk, sm);
+    float2* data = a.datas ? a.datas[b] : a.data + (size_t)b * modes * a.N;
+    col_work<N1, C>(a, op, st, data + (size_t)mo * a.N, blockIdx.x * C, s_fc, s_B, C, sx, s_x0, mo, modes,
+                    threadIdx.x % (C * P), a.N2, pk, sm);
     if (st) col_advance(a, st, b, op, pk, sm, red);
 }
 
@@ -612,7 +613,9 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row
     }
     row_tables<N2>(a, st || a.op == ROW_SSFM, g, s_tw, s_T);
     const int rl = threadIdx.x / P, t = threadIdx.x % P;
-    row_work<N2>(a, st ? (int)ROW_SSFM : a.op, a.data + (size_t)b * a.N, blockIdx.x * R + rl, rl, t, s_tw, s_T, sx,
+    float2* data = a.data + (size_t)b * a.N;
+    if (a.datas) data = a.modes > 1 ? a.datas[b >> 1] + (size_t)(b & 1) * a.N : a.datas[b];  // 1 or 2 modes
+    row_work<N2>(a, st ? (int)ROW_SSFM : a.op, data, blockIdx.x * R + rl, rl, t, s_tw, s_T, sx,
                  g, dhi, dlo, N2);
 }
 
