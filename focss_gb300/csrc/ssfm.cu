@@ -93,10 +93,10 @@ std::mutex g_launch_mutex;
 
 // The cached launch of pass kind `kind` (0 column, 1 row, 2 row with
 // bulk-copy staging, 3 row in 64-thread CTAs, 4 column in 64-thread CTAs, 5
-// column with TMA tensor staging) for log2 length lg on the current device,
+// column with TMA tensor staging, 6 row over several blocks) for log2 length lg on the current device,
 // opted in to `smem` bytes of dynamic shared memory.
 cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
-    static Launch cache[kMaxDevices][6][16];
+    static Launch cache[kMaxDevices][7][16];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -114,7 +114,7 @@ cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
     }
     if (!l.fn) return cudaErrorInvalidValue;
     if (!l.attr_set || smem > l.smem) {
-        const void* fn = kind == 5 ? (const void*)l.fn_tma : (const void*)l.fn;
+        const void* fn = kind == 5 ? (const void*)l.fn_tma : kind == 6 ? (const void*)l.fn_loop : (const void*)l.fn;
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         l.attr_set = true;
@@ -133,7 +133,8 @@ cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
 // 2.31 -> 2.13 ms).  Captured into a graph it is a plain kernel node: graph
 // launches already hide that latency, and programmatic edges there measured
 // slower (800 steps of one 2^17 field: 17.8 -> 19.9 us per step).
-cudaError_t launch_pass(const Launch& l, dim3 grid, int threads, size_t smem, cudaStream_t s, const PassArgs& a) {
+template <class... A>
+cudaError_t launch_pass(void (*fn)(A...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... a) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -147,7 +148,7 @@ cudaError_t launch_pass(const Launch& l, dim3 grid, int threads, size_t smem, cu
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, l.fn, a);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, a...);
     count_launch();
     const cudaError_t last = cudaGetLastError();  // consumed, as after a <<<>>> launch
     return e != cudaSuccess ? e : last;
@@ -211,7 +212,7 @@ cudaError_t launch_col(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
     if (p.staging == FOCSS_STAGING_TMA) return launch_col_tma(p, a, batch, modes, smem + 128, s);
     cudaError_t e = cached_launch(narrow ? 4 : 0, p.log2N1, smem, &l);
     if (e != cudaSuccess) return e;
-    return launch_pass(l, dim3(p.N2 / l.per_block, batch), l.threads * modes, smem, s, a);
+    return launch_pass(l.fn, dim3(p.N2 / l.per_block, batch), l.threads * modes, smem, s, a);
 }
 
 cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
@@ -226,8 +227,6 @@ cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
     const int kind = p.staging != FOCSS_STAGING_LOADS ? 2 : narrow ? 3 : 1;
     int R = narrow ? l.per_block_narrow : l.per_block;
     const size_t smem = sizeof(float4) * 512 + sizeof(float2) * ((size_t)p.N2 + (size_t)R * Q * (P + 1));
-    cudaError_t e = cached_launch(kind, p.log2N2, smem, &l);
-    if (e != cudaSuccess) return e;
     a.N = p.N;
     a.N1 = p.N1;
     a.N2 = p.N2;
@@ -235,8 +234,22 @@ cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
     a.tw = tables_at(p.tw, p.N1);
     a.kc = col_kc(p.N1);
     a.batch = batch;
+    if (kind == 1 && l.fn_loop) {
+        // at least four waves: each CTA takes several blocks (with fewer, handing
+        // blocks out as CTAs finish is the better balance: 12 x 2^19, 2.5 waves,
+        // 4 us slower in a chunk each)
+        const int loop = 256 / P, slots = 2 * sm_count();  // CTAs that run at once
+        const long long blocks = (long long)(p.N1 / loop) * rows;
+        if (p.N1 % loop == 0 && blocks > 4ll * slots && rows <= 256) {
+            const size_t sl = sizeof(float4) * 512 + sizeof(float2) * ((size_t)p.N2 + (size_t)loop * Q * (P + 1));
+            const cudaError_t e = cached_launch(6, p.log2N2, sl, &l);
+            return e != cudaSuccess ? e : launch_pass(l.fn_loop, dim3(slots), 256, sl, s, a, rows);
+        }
+    }
+    const cudaError_t e = cached_launch(kind, p.log2N2, smem, &l);
+    if (e != cudaSuccess) return e;
     if (p.N1 % R != 0) return cudaErrorInvalidValue;
-    return launch_pass(l, dim3(p.N1 / R, batch * (a.modes > 1 ? a.modes : 1)), l.threads, smem, s, a);
+    return launch_pass(l.fn, dim3(p.N1 / R, batch * (a.modes > 1 ? a.modes : 1)), l.threads, smem, s, a);
 }
 
 // ---------------------------------------------------------------- SSFM driver

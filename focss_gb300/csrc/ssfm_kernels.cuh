@@ -587,6 +587,9 @@ struct RowShape {
     // (a single field of 2^17 samples at a 128 x 1024 split has 16), four
     // times as many SMs take part.
     static constexpr int RN = 64 / P;
+    // rows per 256-thread CTA of row_kernel_loop (0: not used; at N2 = 512 the
+    // tables are small enough that it gains nothing)
+    static constexpr int LOOP = N2 >= 1024 ? 256 / P : 0;
     // CTAs of r rows per SM the register budget (128 at 512 threads) is sized for
     static constexpr int min_blocks(int r) { return r == RN ? 2 : (512 / (r * P) > 2 ? 512 / (r * P) : 2); }
 };
@@ -617,6 +620,82 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row
     if (a.datas) data = a.modes > 1 ? a.datas[b >> 1] + (size_t)(b & 1) * a.N : a.datas[b];  // 1 or 2 modes
     row_work<N2>(a, st ? (int)ROW_SSFM : a.op, data, blockIdx.x * R + rl, rl, t, s_tw, s_T, sx,
                  g, dhi, dlo, N2);
+}
+
+// The same for a chunk of the launch's (N1 / R) x `rows` row blocks, one after the
+// other, in CTAs that fill the GPU once: the twiddles are loaded once and the
+// rotation table once per realization (16 KB per 64 KB of rows otherwise, in front
+// of each block's work).  126 x 2^19: 303 -> 289 us, 28 x 2^19: 78.5 -> 72.5 us.  512
+// threads: 299 and 74.6 us, 128 threads: 335 and 83 us; requesting the next rows
+// into L2 ahead: 310 and 76.6 us.
+constexpr int kLoopRows = 256;  // rows of a launch, at most (and threads of a CTA)
+template <int N2, int R>
+__global__ void __launch_bounds__(R* PQ<N2>::P, 512 / (R * PQ<N2>::P)) row_kernel_loop(const PassArgs a, int rows) {
+    constexpr int P = PQ<N2>::P, Q = PQ<N2>::Q;
+    extern __shared__ float4 smem4[];
+    float4* s_T = smem4;                                     // g exp(2 pi i j/512)
+    float2* s_tw = reinterpret_cast<float2*>(s_T + 512);     // sub-FFT twiddles
+    float2* sx = s_tw + N2;                                  // R * Q * (P+1)
+    pdl_trigger();
+    const int rl = threadIdx.x / P, t = threadIdx.x % P;
+    const int per = a.N1 / R;
+    pdl_wait();
+    // the rows (realizations' modes) that have a step to do: runs of different
+    // step counts leave the CTAs even shares
+    static_assert(R * P == kLoopRows, "a thread per row");
+    __shared__ unsigned char s_list[kLoopRows];
+    __shared__ int s_count[R * P / 32];
+    if (a.state) {
+        const int i = threadIdx.x;
+        const bool on = i < rows && *(volatile const int*)&a.state[a.modes > 1 ? i >> 1 : i].row_active;
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if ((i & 31) == 0) s_count[i >> 5] = __popc(m);
+        __syncthreads();
+        int n = 0, before = 0;
+        for (int w = 0; w < R * P / 32; ++w) {
+            before += w < (i >> 5) ? s_count[w] : 0;
+            n += s_count[w];
+        }
+        if (on) s_list[before + __popc(m & ((1u << (i & 31)) - 1u))] = (unsigned char)i;
+        __syncthreads();
+        rows = n;
+    }
+    const long long total = (long long)per * rows;
+    const int last = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    int blk = (int)(total * blockIdx.x / gridDim.x);
+    for (int i = threadIdx.x; i < N2; i += R * P) s_tw[i] = a.tw.row[i];
+    int cur = -1;
+    unsigned long long dhi = a.disp_hi, dlo = a.disp_lo;
+    float g = a.scale;
+    float2* data = a.data;
+    for (; blk < last; ++blk) {
+        const int place = blk / per;
+        if (place != cur) {
+            const int b = a.state ? s_list[place] : place;
+            if (a.state) {
+                const SsfmState* st = a.state + (a.modes > 1 ? b >> 1 : b);
+                dhi = st->disp_hi;
+                dlo = st->disp_lo;
+                g = st->lin_gain;
+            }
+            data = a.data + (size_t)b * a.N;
+            if (a.datas) data = a.modes > 1 ? a.datas[b >> 1] + (size_t)(b & 1) * a.N : a.datas[b];
+            __syncthreads();  // the last row's rotations are done
+            if (a.state || a.op == ROW_SSFM)
+                for (int i = threadIdx.x; i < 512; i += R * P) s_T[i] = scale_df(a.tw.turn[i], g);
+            cur = place;
+        }
+        const int k1 = (blk - place * per) * R + rl, op = a.state ? (int)ROW_SSFM : a.op;
+        float2* row = data + (size_t)k1 * N2;
+        float2 v[Q];
+        row_load<N2>(v, row, op == ROW_INV ? row_k2_base<N2>(t) : centred<P>(t));
+        // also without new tables: warps that run apart (each holds whole rows)
+        // compete for the instruction cache (126 x 2^19: 289 -> 296 us)
+        __syncthreads();  // the tables; otherwise a row's warp runs on its own
+        row_core<N2>(a, op, v, k1, rl, t, s_tw, s_T, sx, g, dhi, dlo);
+        row_store<N2>(v, row, op == ROW_FWD ? row_k2_base<N2>(t) : centred<P>(t));
+        __syncwarp();
+    }
 }
 
 // ---------------------------------------------------------------- row pass, bulk-copy staging
@@ -863,10 +942,19 @@ __global__ void __launch_bounds__(kBlockThreads, BlockShape<N1, N2>::SMEM <= 113
 
 typedef void (*PassFn)(PassArgs);
 typedef void (*ColTmaFn)(CUtensorMap, PassArgs);
+typedef void (*RowLoopFn)(PassArgs, int);
+template <int N2>
+RowLoopFn row_loop_fn() {
+    if constexpr (RowShape<N2>::LOOP > 0)
+        return row_kernel_loop<N2, RowShape<N2>::LOOP>;
+    else
+        return nullptr;
+}
 struct Launch {
     PassFn fn = nullptr;
     PassFn fn_bulk = nullptr;  // row pass with bulk-copy staging
     PassFn fn_narrow = nullptr;  // the pass in 64-thread CTAs (few blocks in the whole launch)
+    RowLoopFn fn_loop = nullptr; // row pass with several row blocks per CTA
     ColTmaFn fn_tma = nullptr;   // column pass with TMA tensor staging
     int per_block_narrow = 0;
     int threads = 0, per_block = 0;
@@ -899,6 +987,7 @@ Launch row_launch_for(int log2N2);
         l.fn = row_kernel<L, RowShape<L>::R>;                                  \
         l.fn_bulk = row_kernel_bulk<L, RowShape<L>::R>;                        \
         l.fn_narrow = row_kernel<L, RowShape<L>::RN>;                          \
+        l.fn_loop = row_loop_fn<L>();                                          \
         l.per_block_narrow = RowShape<L>::RN;                                  \
         l.threads = RowShape<L>::R * PQ<L>::P;                                 \
         l.per_block = RowShape<L>::R;                                          \
