@@ -64,7 +64,7 @@ constexpr uint32_t SBO = 128;
 using namespace tcg;
 
 constexpr int STAGES = 4;                  // activation tiles in flight per CTA
-constexpr int FWD_THREADS = 320;           // producer, MMA, two groups of four epilogue warps
+constexpr int FWD_THREADS = 352;           // producer, two MMA warps, two groups of four epilogue warps
 
 template <int CIN, int COUT>
 struct Shape {
@@ -96,7 +96,7 @@ __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-constexpr int FWD_EPI = FWD_THREADS - 64;  // epilogue threads
+constexpr int FWD_EPI = 256;  // epilogue threads (warps 2-9)
 
 // 16-byte asynchronous copy global -> shared; `bytes` = 0 writes zeros.
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, uint32_t bytes) {
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
             tc::mbar_init(&acc_full[i], 1);
             tc::mbar_init(&acc_empty[i], 4);
         }
-        tc::mbar_init(&drain, 1);
+        tc::mbar_init(&drain, 2);
         tc::mbar_init(&wready, tc::FWD_EPI);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = tmem_base;
     const uint32_t a_base = tc::smem_addr(As), bs0 = tc::smem_addr(Bs);
-    if (warp >= 2) {
+    if (warp >= 2 && warp < 10) {
         // the epilogue warps stage the weights while the first tiles load:
         // 16-byte rows W[co][kk][8g .. 8g+7] -> Bs[(kk*KG + g)*COUT + co],
         // made visible to the tensor core's proxy before `wready` completes
@@ -213,11 +213,12 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
                 issued = k + 1;
             }
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 || warp == 10) {
         if (lane == 0 && tc::mbar_wait(&wready, 0, &abort_flag)) {
             const uint64_t bdesc = tc::smem_desc(bs0, S::LBO_B, tc::SBO);
-            for (int i = blockIdx.x, k = 0; i < T; i += gridDim.x, ++k) {
-                const int s = k % ST, ac = k & 1;
+            const int ac = warp == 1 ? 0 : 1;
+            for (int i = blockIdx.x + ac * gridDim.x, k = ac; i < T; i += 2 * gridDim.x, k += 2) {
+                const int s = k % ST;
                 if (!tc::mbar_wait(&full[s], (k / ST) & 1, &abort_flag)) break;
                 if (k >= 2 && !tc::mbar_wait(&acc_empty[ac], ((k >> 1) & 1) ^ 1, &abort_flag)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -259,10 +260,16 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
         // 32q .. 32q+31 = tile rows
         const int q = warp & 3, ac = (warp - 2) >> 2;
         for (int i = blockIdx.x + ac * gridDim.x, k = ac; i < T; i += 2 * gridDim.x, k += 2) {
-            if (!tc::mbar_wait(&acc_full[ac], (k >> 1) & 1, &abort_flag)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int b = i / ntiles, p = (i % ntiles) * tc::M + 32 * q + lane;
             const size_t ob = (size_t)b * L * COUT + (size_t)p * COUT;
+            // the mask does not depend on the accumulator: requested before the wait
+            uint4 mk[COUT / 8] = {};
+            if (mask && p < L) {
+#pragma unroll
+                for (int c = 0; c < COUT / 8; ++c) mk[c] = reinterpret_cast<const uint4*>(mask + ob)[c];
+            }
+            if (!tc::mbar_wait(&acc_full[ac], (k >> 1) & 1, &abort_flag)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             // the whole row of the accumulator in flight at once, one wait
             uint32_t raw[COUT / 16][16];
 #pragma unroll
@@ -270,19 +277,17 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
                 tc::ld_x16_async(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(ac * S::ACC_COLS + 16 * c), raw[c]);
 #pragma unroll
             for (int c = 0; c < COUT / 16; ++c) tc::wait_ld(raw[c]);
+            // it is in registers now: release it before the stores
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&acc_empty[ac]);
 #pragma unroll
             for (int c0 = 0; c0 < COUT; c0 += 16) {
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(raw[c0 / 16][j]);
                 if (p < L) {
-                    uint4 mk[2] = {};
-                    if (mask) {
-                        const uint4* m4 = reinterpret_cast<const uint4*>(mask + ob + c0);
-                        mk[0] = m4[0];
-                        mk[1] = m4[1];
-                    }
-                    const bf16* mb = reinterpret_cast<const bf16*>(mk);
+                    const bf16* mb = reinterpret_cast<const bf16*>(mk + c0 / 8);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         float x = v[j] + s_bias[c0 + j];
@@ -304,10 +309,6 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
                     }
                 }
             }
-            // this warp's reads of the accumulator are complete: release it
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&acc_empty[ac]);
         }
     }
     __syncthreads();
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
         // the CTA leaves (bounded again), then its tiles are marked invalid
         if (warp == 0 && lane == 0)
             for (int k = issued > ST ? issued - ST : 0; k < issued; ++k) tc::mbar_wait(&full[k % ST], (k / ST) & 1, nullptr);
-        if (warp == 1 && lane == 0) {
+        if ((warp == 1 || warp == 10) && lane == 0) {
             tc::mma_commit(&drain);  // completes once every MMA this thread issued has
             tc::mbar_wait(&drain, 0, nullptr);
         }
