@@ -76,7 +76,8 @@ struct Shape {
     static constexpr uint32_t LBO_B = COUT * 16;
     static constexpr size_t SMEM_B = (size_t)KW * (CIN / 8) * COUT * 16;
     static constexpr uint32_t STAGE_BYTES = (CIN / 8) * ROWS * 16;  // one activation tile
-    static constexpr size_t SMEM = SMEM_B + STAGES * (size_t)STAGE_BYTES + 1024;  // + alignment slack
+    // 8 epilogue warps stage 32 rows each (at most 128 + 16 bytes a row)
+    static constexpr size_t SMEM = SMEM_B + STAGES * (size_t)STAGE_BYTES + 8 * 32 * 144 + 1024;  // + alignment slack
     static constexpr uint32_t ACC_COLS = COUT < 32 ? 32 : COUT;   // one FP32 accumulator
     static constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;           // two: a power of two >= 32
 };
@@ -115,6 +116,11 @@ __device__ __forceinline__ void ld_x16(uint32_t taddr, float (&r)[16]) {
 }
 }  // namespace tc
 
+// 0xffff in each half whose bf16 is > 0.
+__device__ __forceinline__ uint32_t positive2(uint32_t m) {
+    return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&m), __float2bfloat162_rn(0.f));
+}
+
 // in: [B][L][CIN] bf16 (read through `amap`, a 3-D tensor map {CIN, L, B}
 // with box {8, ROWS, 1}), W: [COUT][KW][CIN] bf16, bias: [COUT] f32 or null,
 // out [B][L][COUT] (bf16, or f32 when OUT_F32); mask (optional, [B][L][COUT]
@@ -152,7 +158,7 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
     __shared__ __align__(8) unsigned long long full[ST], empty[ST], acc_full[2], acc_empty[2], drain, wready;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
-    __shared__ float s_bias[COUT];
+    __shared__ __align__(16) float s_bias[COUT];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ntiles = (L + tc::M - 1) / tc::M, T = ntiles * B;
     for (int i = threadIdx.x; i < COUT; i += blockDim.x) s_bias[i] = bias ? bias[i] : 0.f;
@@ -258,15 +264,20 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
         // epilogue group ac = (warp - 2) / 4 takes the tiles of accumulator ac
         // (every other tile); warp & 3 selects its tensor-memory lanes
         // 32q .. 32q+31 = tile rows
+        constexpr int E = OUT_F32 ? 4 : 8, RC = COUT / E, PITCH = 16 * RC + 16;  // values per chunk, chunks per row
         const int q = warp & 3, ac = (warp - 2) >> 2;
+        unsigned char* stage = As + tc::STAGES * (size_t)S::STAGE_BYTES + (size_t)(warp - 2) * 32 * PITCH;
         for (int i = blockIdx.x + ac * gridDim.x, k = ac; i < T; i += 2 * gridDim.x, k += 2) {
-            const int b = i / ntiles, p = (i % ntiles) * tc::M + 32 * q + lane;
-            const size_t ob = (size_t)b * L * COUT + (size_t)p * COUT;
+            // the warp's 32 rows of the output are one contiguous block: chunk u of
+            // a lane is 16 bytes at 16 (32 u + lane)
+            const int b = i / ntiles, p0 = (i % ntiles) * tc::M + 32 * q, rows = min(32, L - p0);
+            const size_t ob = ((size_t)b * L + p0) * (COUT / E);
             // the mask does not depend on the accumulator: requested before the wait
-            uint4 mk[COUT / 8] = {};
-            if (mask && p < L) {
+            uint4 mk[RC] = {};
+            if (!OUT_F32 && mask) {
 #pragma unroll
-                for (int c = 0; c < COUT / 8; ++c) mk[c] = reinterpret_cast<const uint4*>(mask + ob)[c];
+                for (int u = 0; u < RC; ++u)
+                    if ((32 * u + lane) / RC < rows) mk[u] = reinterpret_cast<const uint4*>(mask)[ob + 32 * u + lane];
             }
             if (!tc::mbar_wait(&acc_full[ac], (k >> 1) & 1, &abort_flag)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -281,34 +292,46 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&acc_empty[ac]);
+            // lane = row here; a row goes to the stage in 16-byte chunks ...
 #pragma unroll
-            for (int c0 = 0; c0 < COUT; c0 += 16) {
-                float v[16];
+            for (int c = 0; c < RC; ++c) {
+                float v[E];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(raw[c0 / 16][j]);
-                if (p < L) {
-                    const bf16* mb = reinterpret_cast<const bf16*>(mk + c0 / 8);
+                for (int j = 0; j < E; j += 4) {
+                    const float4 bi = *reinterpret_cast<const float4*>(&s_bias[E * c + j]);
+                    const float bj[4] = {bi.x, bi.y, bi.z, bi.w};
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        float x = v[j] + s_bias[c0 + j];
+                    for (int w = 0; w < 4; ++w) {
+                        float x = __uint_as_float(raw[(E * c + j) / 16][(E * c + j) % 16 + w]) + bj[w];
                         if (relu) x = fmaxf(x, 0.f);
-                        if (mask && !(__bfloat162float(mb[j]) > 0.f)) x = 0.f;
-                        v[j] = x;
-                    }
-                    if (OUT_F32) {
-                        float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + ob + c0);
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) o[u] = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
-                    } else {
-                        uint32_t packed[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) packed[j] = pack2(__float2bfloat16(v[2 * j]), __float2bfloat16(v[2 * j + 1]));
-                        uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(out) + ob + c0);
-                        o[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                        o[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                        v[j + w] = x;
                     }
                 }
+                uint4 o;
+                if constexpr (OUT_F32)
+                    o = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+                else
+                    o = make_uint4(pack2(__float2bfloat16(v[0]), __float2bfloat16(v[1])),
+                                   pack2(__float2bfloat16(v[2]), __float2bfloat16(v[3])),
+                                   pack2(__float2bfloat16(v[E - 4]), __float2bfloat16(v[E - 3])),
+                                   pack2(__float2bfloat16(v[E - 2]), __float2bfloat16(v[E - 1])));
+                *reinterpret_cast<uint4*>(stage + lane * PITCH + 16 * c) = o;
             }
+            __syncwarp();
+            // ... and from there to memory in whole 128-byte lines
+#pragma unroll
+            for (int u = 0; u < RC; ++u) {
+                const int e = 32 * u + lane;
+                uint4 o = *reinterpret_cast<const uint4*>(stage + (e / RC) * PITCH + 16 * (e % RC));
+                if (!OUT_F32 && mask) {
+                    o.x &= positive2(mk[u].x);
+                    o.y &= positive2(mk[u].y);
+                    o.z &= positive2(mk[u].z);
+                    o.w &= positive2(mk[u].w);
+                }
+                if (e / RC < rows) reinterpret_cast<uint4*>(out)[ob + e] = o;
+            }
+            __syncwarp();
         }
     }
     __syncthreads();
