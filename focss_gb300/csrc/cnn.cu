@@ -104,16 +104,6 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src, uint32_t byt
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-__device__ __forceinline__ void ld_x16(uint32_t taddr, float (&r)[16]) {
-    uint32_t u[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
-          "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-        : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(u[i]);
-}
 }  // namespace tc
 
 // 0xffff in each half whose bf16 is > 0.
@@ -366,119 +356,129 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
 }
 
 // ------------------------------------------------------------ tcgen05 weight gradient
-// gW[co][kk][ci] += sum_p g[p][co] in[p+kk-4][ci]: per tap a GEMM with
-// M = 64 (the 64-channel side: output channels when COUT = 64, else input
-// channels with the result transposed), N = the other side (64 or 16),
-// K = positions.  Both operands are MN-major (channels contiguous, as
-// stored), no-swizzle canonical layout: 16-byte rows of 8 channels, one row
-// per position, 8-row core matrices LBO = 128 B apart along K (positions),
-// channel groups SBO apart.  The input operand of tap kk is the same buffer
-// starting kk rows further (kk x 16 B), so the tap shift along K is an
-// address offset.  A CTA accumulates three taps in tensor memory over its
-// chunk of positions (a whole number of 128-position tiles).  One thread
-// loads the tiles with TMA tensor copies (one box of 8 channels x 128 or 136
-// rows per channel group, zero-filled outside [0, L)) into a ring of
-// WSTAGES buffers (mbarriers full / empty); one thread issues each tile's
-// MMAs and commits them to the tile's `empty` barrier, and after the last
-// tile to `done`; then all warps add the accumulators to gW.  With M = 64
-// the accumulator row m sits in tensor-memory lane 32 (m / 16) + m % 16.
-// Every wait is bounded (kWaitCap polls); a CTA that gives up drains its
-// copies and MMAs (bounded) and adds NaN, so the failure shows in gW.
+// gW[co][kk][ci] += sum_p g[p][co] in[p+kk-4][ci] and gb[co] += sum_p g[p][co]:
+// GEMMs with M = (tap, input channel), N = output channels, K = positions, 128 a
+// tile.  Both operands are MN-major (channels contiguous, as stored) in the
+// swizzled layout of their TMA boxes: rows of 128 bytes (64 channels) or 32 (16),
+// one per position.  Groups of CIN channels along M lie one row (LBO) apart, so
+// M = 128 covers 128 / CIN consecutive taps of one copy of the tile, and the
+// next MMA's taps start that many rows further: 5 MMAs per 16 positions (64
+// channels; 2 for 16) instead of 9 of M = 64.  The last one has taps to spare: there
+// (64 channels) LBO leads to a block of ones, whose product is the bias gradient
+// (16 channels: a third MMA).
+//
+// A CTA takes an even share of the tiles of all realizations, accumulates them in
+// tensor memory and adds the result to gW once.  Warp 0 loads tiles with TMA
+// (zero-filled outside [0, L)) into a ring of WSTAGES buffers (mbarriers full /
+// empty); warps 1 and 2 issue a share of each tile's MMAs each and commit them to
+// the tile's `empty` barrier (issue from one warp takes ~70 cycles an MMA).  Every
+// wait is bounded (kWaitCap polls); a CTA that gives up drains its copies and MMAs
+// (bounded) and adds NaN, so the failure shows in gW.
+//
+// 12 x 2^15 positions with the bias gradient, 64 -> 64 channels 102 -> 36 us, 64 -> 16
+// 61 -> 26 us, 16 -> 64 72 -> 26 us against three taps per CTA of M = 64 from unswizzled
+// 16-byte boxes and a pass over g for the bias.
 namespace tcw {
 constexpr int P = 128;                // positions per tile
 constexpr int PR = P + 2 * HALF;      // input rows per tile (halo)
-constexpr int TAPS = 3;               // taps per CTA
-constexpr int WSTAGES = 3;            // tiles in flight per CTA
-constexpr uint32_t LBO = 128;
+constexpr int M = 128;
+constexpr int WSTAGES = 4;            // tiles in flight per CTA
+constexpr uint32_t ONES = 2048;       // bytes of ones
 template <int COUT, int CIN>
 struct Shape {
-    static constexpr bool G_IS_A = COUT == 64;           // M side = output-gradient channels
-    static constexpr int NC = G_IS_A ? CIN : COUT;        // N
-    static constexpr uint32_t SMEM_G = (uint32_t)(COUT / 8) * P * 16;
-    static constexpr uint32_t SMEM_I = (uint32_t)(CIN / 8) * PR * 16;
-    static constexpr uint32_t STAGE = SMEM_G + SMEM_I;   // multiples of 128 bytes (TMA destinations)
-    static constexpr size_t SMEM = (size_t)WSTAGES * STAGE + 128;  // + alignment slack
-    static constexpr uint32_t TMEM_COLS = TAPS * NC <= 64 ? 64 : 256;
-    // kind::f16: FP32 D, BF16 A/B, both MN-major (bits 15, 16), N = NC, M = 64.
+    static constexpr int AT = M / CIN;                    // taps per MMA
+    static constexpr int NM = (KW + AT - 1) / AT;         // MMAs (accumulators) per 16 positions
+    static constexpr bool ONES_MMA = AT > 2;              // the ones as an MMA of their own
+    static constexpr int NACC = NM + (ONES_MMA ? 1 : 0);
+    static constexpr uint32_t ROW_G = COUT * 2, ROW_I = CIN * 2;  // bytes per position
+    static constexpr uint32_t SMEM_G = P * ROW_G, SMEM_I = PR * ROW_I;
+    static constexpr uint32_t STAGE = (SMEM_G + SMEM_I + (AT - 1) * ROW_I + 1023) / 1024 * 1024;
+    static constexpr size_t SMEM = (size_t)WSTAGES * STAGE + ONES + 1024;  // + alignment slack
+    static constexpr uint32_t TMEM_COLS = NACC * COUT <= 128 ? 128 : NACC * COUT <= 256 ? 256 : 512;
+    // kind::f16: FP32 D, BF16 A/B, both MN-major (bits 15, 16)
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                                      ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(64 >> 4) << 24);
-    static_assert((COUT == 64 && (CIN == 64 || CIN == 16)) || (COUT == 16 && CIN == 64), "wgrad shapes");
-    static_assert(SMEM_G % 128 == 0 && SMEM_I % 128 == 0, "TMA destinations on 128-byte boundaries");
+                                      ((uint32_t)(COUT >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+    static_assert((COUT == 64 || COUT == 16) && (CIN == 64 || CIN == 16), "swizzles of 128 and 32 bytes");
+    static_assert(SMEM_G % 1024 == 0 && NACC * COUT <= 512 && (NM - 1) * AT <= 2 * HALF, "tile");
 };
+// MN-major operand with rows of ROW bytes (one swizzle span), 8-row groups
+// 8 ROW apart, channel groups along M or N `lbo` bytes apart
+template <uint32_t ROW>
+__device__ __forceinline__ uint64_t desc(uint32_t addr, uint32_t lbo) {
+    constexpr uint64_t mode = ROW == 128 ? 2 : 6;
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(8 * ROW >> 4) << 32) |
+           (1ull << 46) | (mode << 61);
+}
 }  // namespace tcw
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap gmap,
                                                             const __grid_constant__ CUtensorMap imap,
-                                                            float* __restrict__ gW, int L, int chunk) {
+                                                            float* __restrict__ gW, float* __restrict__ gb, int L, int B) {
     using S = tcw::Shape<COUT, CIN>;
-    constexpr int GG = COUT / 8, IG = CIN / 8, ST = tcw::WSTAGES;  // 16-byte channel groups
+    constexpr int ST = tcw::WSTAGES;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long full[ST], empty[ST], done, drain;
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
-    const int tap0 = blockIdx.x * tcw::TAPS;
-    const int b = blockIdx.z;
-    const int c0 = blockIdx.y * chunk;
-    const int c1 = min(L, c0 + chunk);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t raw = tc::smem_addr(smem_raw), base = (raw + 127u) & ~127u;
+    const uint32_t raw = tc::smem_addr(smem_raw), base = (raw + 1023u) & ~1023u, ones = base + ST * S::STAGE;
+    const int ntiles = (L + tcw::P - 1) / tcw::P;
+    const long long T = (long long)ntiles * B;
+    const int first = (int)(T * blockIdx.x / gridDim.x), n = (int)(T * (blockIdx.x + 1) / gridDim.x) - first;
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc::smem_addr(&tmem_base)),
-                     "r"(S::TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
-    }
+    if (warp == 0) tc::tmem_alloc(&tmem_base, S::TMEM_COLS);
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int i = 0; i < ST; ++i) {
             tc::mbar_init(&full[i], 1);
-            tc::mbar_init(&empty[i], 1);
+            tc::mbar_init(&empty[i], 2);
         }
-        tc::mbar_init(&done, 1);
-        tc::mbar_init(&drain, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        tc::mbar_init(&done, 2);
+        tc::mbar_init(&drain, 2);
+        tc::fence_mbar_init();
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    for (int i = threadIdx.x; i < (int)tcw::ONES / 4; i += blockDim.x)
+        reinterpret_cast<uint32_t*>(smem_raw + (ones - raw))[i] = 0x3F803F80u;
+    tc::fence_async_smem();
+    tc::fence_before_sync();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const int n = c1 > c0 ? (c1 - c0 + tcw::P - 1) / tcw::P : 0;
     int issued = 0;
     if (warp == 0 && lane == 0) {
-        // tile t -> stage t % ST: G[cg][r] = g[p0 + r][8cg ..], I[cg][r] = in[p0 - 4 + r][8cg ..]
+        // tile t -> stage t % ST: g rows p0 .., input rows p0 - 4 ..
         for (int t = 0; t < n; ++t) {
-            const int s = t % ST;
+            const int s = t % ST, b = (first + t) / ntiles, p0 = (first + t - b * ntiles) * tcw::P;
             if (t >= ST && !tc::mbar_wait(&empty[s], ((t / ST) & 1) ^ 1, &abort_flag)) break;
-            const int p0 = c0 + t * tcw::P;
-            const uint32_t gb = base + (uint32_t)s * S::STAGE, ib = gb + S::SMEM_G;
-            tc::mbar_expect_tx(&full[s], S::STAGE);
-#pragma unroll
-            for (int cg = 0; cg < GG; ++cg) tc::tma_load_3d(gb + (uint32_t)cg * (tcw::P * 16), &gmap, 8 * cg, p0, b, &full[s]);
-#pragma unroll
-            for (int cg = 0; cg < IG; ++cg)
-                tc::tma_load_3d(ib + (uint32_t)cg * (tcw::PR * 16), &imap, 8 * cg, p0 - HALF, b, &full[s]);
+            const uint32_t gs = base + (uint32_t)s * S::STAGE;
+            tc::mbar_expect_tx(&full[s], S::SMEM_G + S::SMEM_I);
+            tc::tma_load_3d(gs, &gmap, 0, p0, b, &full[s]);
+            tc::tma_load_3d(gs + S::SMEM_G, &imap, 0, p0 - HALF, b, &full[s]);
             issued = t + 1;
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 || warp == 2) {
+        // accumulators j0 .. j1 - 1 of every tile
+        constexpr int HALF_ACC = (S::NACC + (S::ONES_MMA ? 0 : 1)) / 2;
+        const int j0 = warp == 1 ? 0 : HALF_ACC, j1 = warp == 1 ? HALF_ACC : S::NACC;
         for (int t = 0; t < n; ++t) {
             const int s = t % ST;
-            if (!tc::mbar_wait(&full[s], (t / ST) & 1, &abort_flag)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const uint32_t gb = base + (uint32_t)s * S::STAGE, ib = gb + S::SMEM_G;
+            if (!tc::mbar_wait_warp(&full[s], (t / ST) & 1, &abort_flag)) break;
+            tc::fence_after_sync();
+            const uint32_t gs = base + (uint32_t)s * S::STAGE, is = gs + S::SMEM_G;
+            for (int j = j0; j < j1; ++j) {
+                const uint32_t d = tmem + (uint32_t)(COUT * j);
 #pragma unroll
-            for (int j = 0; j < tcw::TAPS; ++j) {
-                const int kk = tap0 + j;
-#pragma unroll
-                for (int ks = 0; ks < tcw::P / 16; ++ks) {  // 16 positions = 2 K core matrices per MMA
-                    const uint64_t gd = tc::smem_desc(gb + ks * 2 * tcw::LBO, tcw::LBO, tcw::P * 16);
-                    const uint64_t id = tc::smem_desc(ib + kk * 16 + ks * 2 * tcw::LBO, tcw::LBO, tcw::PR * 16);
-                    tc::mma_f16(tmem + (uint32_t)(S::NC * j), S::G_IS_A ? gd : id, S::G_IS_A ? id : gd, S::IDESC,
-                                 (t | ks) != 0);
+                for (int ks = 0; ks < tcw::P / 16; ++ks) {
+                    const uint32_t a0 = is + (uint32_t)(j * S::AT + 16 * ks) * S::ROW_I;
+                    uint64_t a = tcw::desc<S::ROW_I>(a0, S::ROW_I);
+                    if (S::ONES_MMA ? j == S::NM : false) a = tcw::desc<S::ROW_I>(ones, S::ROW_I);
+                    if (!S::ONES_MMA && j == S::NM - 1) a = tcw::desc<S::ROW_I>(a0, ones - a0);
+                    tc::mma_f16_warp(d, a, tcw::desc<S::ROW_G>(gs + 16 * ks * S::ROW_G, 16), S::IDESC, (t | ks) != 0);
                 }
             }
-            tc::mma_commit(&empty[s]);  // the stage is free once these MMAs have read it
-            if (t == n - 1) tc::mma_commit(&done);
+            tc::mma_commit_warp(&empty[s]);  // the stage is free once both warps' MMAs have read it
+            if (t == n - 1) tc::mma_commit_warp(&done);
         }
     }
     __syncthreads();
@@ -488,89 +488,41 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(const __grid_constan
         // drain: the queued copies and the issued MMAs complete (bounded) before the CTA leaves
         if (warp == 0 && lane == 0)
             for (int t = issued > ST ? issued - ST : 0; t < issued; ++t) tc::mbar_wait(&full[t % ST], (t / ST) & 1, nullptr);
-        if (warp == 1 && lane == 0) {
-            tc::mma_commit(&drain);
-            tc::mbar_wait(&drain, 0, nullptr);
+        if (warp == 1 || warp == 2) {
+            tc::mma_commit_warp(&drain);
+            tc::mbar_wait_warp(&drain, 0, nullptr);
         }
         __syncthreads();
     }
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    // epilogue: lanes 0-15 of warp w hold M-side channel m = 16 w + lane
+    tc::fence_after_sync();
+    // lane 32 w + lane holds row m of each accumulator: tap m / CIN of its taps,
+    // input channel m % CIN
     if (n > 0) {
-        const int m = 16 * warp + lane;
-        for (int j = 0; j < tcw::TAPS; ++j)
+        const int m = 32 * warp + lane;
+        for (int j = 0; j < S::NACC; ++j) {
+            const int tap = j * S::AT + m / CIN;
+            const bool bias = S::ONES_MMA ? j == S::NM && m == 0 : j == S::NM - 1 && m == CIN;
+            const bool weight = j < S::NM && tap < KW;
 #pragma unroll
-            for (int q = 0; q < S::NC; q += 16) {
-                float v[16];
-                tc::ld_x16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(S::NC * j + q), v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (lane < 16) {
-                    if (!ok)
+            for (int q = 0; q < COUT; q += 16) {
+                uint32_t v[16];
+                tc::ld_x16_async(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(COUT * j + q), v);
+                tc::wait_ld(v);
+                if (weight || bias) {
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) v[e] = __int_as_float(0x7fc00000);
-                    if constexpr (S::G_IS_A) {
-                        // 16 consecutive input channels of output channel m: 4 vector reductions
-                        float* dst = gW + ((size_t)m * KW + tap0 + j) * CIN + q;
-#pragma unroll
-                        for (int e = 0; e < 16; e += 4)
-                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + e), "f"(v[e]),
-                                         "f"(v[e + 1]), "f"(v[e + 2]), "f"(v[e + 3])
-                                         : "memory");
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) atomicAdd(gW + ((size_t)(q + e) * KW + tap0 + j) * CIN + m, v[e]);
-                    }
+                    for (int e = 0; e < 16; ++e)
+                        atomicAdd(weight ? gW + ((size_t)(q + e) * KW + tap) * CIN + m % CIN : gb + q + e,
+                                  __uint_as_float(ok ? v[e] : 0x7fc00000u));
                 }
-            }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(S::TMEM_COLS));
-}
-
-// bias gradient: gb[co] += sum_p g[p][co].  A lane reads 16 bytes (8 channels)
-// of kBiasRows positions before it adds any of them, so that a warp keeps 2 KB
-// in flight; warps and then CTAs combine in shared memory and one atomic per
-// channel per CTA.  12 x 2^15 positions of 64 channels (50 MB): 13.7 us
-// (41 us with one 4-byte load in flight per lane).
-constexpr int kBiasRows = 4;
-template <int C>
-__global__ void __launch_bounds__(256) bias_grad_kernel(const bf16* __restrict__ g, size_t positions,
-                                                        float* __restrict__ gb) {
-    constexpr int L = C / 8, PW = 32 / L;  // lanes per position; positions per warp step
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int cg = lane % L, po = lane / L;
-    float a[8] = {};
-    const size_t step = (size_t)gridDim.x * nw * PW;
-    for (size_t p = ((size_t)blockIdx.x * nw + warp) * PW + po; p < positions; p += kBiasRows * step) {
-        uint4 v[kBiasRows];
-#pragma unroll
-        for (int u = 0; u < kBiasRows; ++u)
-            v[u] = p + u * step < positions ? reinterpret_cast<const uint4*>(g + (p + u * step) * C)[cg] : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int u = 0; u < kBiasRows; ++u) {
-            const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                a[2 * e] += __uint_as_float(w[e] << 16);  // BF16 is the upper half of FP32
-                a[2 * e + 1] += __uint_as_float(w[e] & 0xFFFF0000u);
+                __syncwarp();
             }
         }
     }
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-        for (int o = L; o < 32; o <<= 1) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
-    __shared__ float sh[8][C];
-    if (po == 0)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sh[warp][8 * cg + e] = a[e];
+    tc::fence_before_sync();
     __syncthreads();
-    if (threadIdx.x < C) {
-        float t = 0.f;
-        for (int w = 0; w < nw; ++w) t += sh[w][threadIdx.x];
-        atomicAdd(&gb[threadIdx.x], t);
-    }
+    if (warp == 0) tc::tmem_free(tmem, S::TMEM_COLS);
 }
+
 
 // First-order perturbation triplets fed to the network's idle input channels:
 // feature j of symbol k is T(m_j, n_j) + T(-m_j, -n_j) (T(0, 0) alone) with
@@ -703,36 +655,38 @@ cudaError_t conv_fwd(const bf16* in, const bf16* W, const float* bias, void* out
     return cudaGetLastError();
 }
 
-// [B][L][C] bf16 as a 3-D tensor {C, L, B}; one box = 8 channels (16 bytes)
-// x `rows` positions of one realization, zero-filled outside the tensor.
-cudaError_t channel_group_map(CUtensorMap* map, const bf16* p, int C, int L, int B, int rows) {
+// Tensor map of [B][L][C] bf16 with boxes of all C channels x `rows` positions, in
+// the swizzle that spans a row (128 bytes for 64 channels, 32 for 16).
+cudaError_t position_map(CUtensorMap* map, const bf16* p, int C, int L, int B, int rows) {
     PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     const cudaError_t e = tensor_map_encoder(&encode);
     if (e != cudaSuccess) return e;
     const cuuint64_t dims[3] = {(cuuint64_t)C, (cuuint64_t)L, (cuuint64_t)B};
     const cuuint64_t strides[2] = {(cuuint64_t)C * sizeof(bf16), (cuuint64_t)L * C * sizeof(bf16)};
-    const cuuint32_t box[3] = {8, (cuuint32_t)rows, 1}, estr[3] = {1, 1, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)C, (cuuint32_t)rows, 1}, estr[3] = {1, 1, 1};
     if (encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(p), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+               CU_TENSOR_MAP_INTERLEAVE_NONE, C == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     return cudaSuccess;
 }
 
+// gW and gb += the gradients of weights and bias.
 template <int CIN, int COUT>
-cudaError_t conv_wgrad(const bf16* g, const bf16* in, float* gW, int L, int B, cudaStream_t s) {
+cudaError_t conv_wgrad(const bf16* g, const bf16* in, float* gW, float* gb, int L, int B, cudaStream_t s) {
     using S = tcw::Shape<COUT, CIN>;
-    static_assert(KW % tcw::TAPS == 0, "taps per CTA");
-    const int chunk = 2048;  // a whole number of 128-position tiles: no tile crosses a chunk
     cudaError_t e = cudaFuncSetAttribute(conv_wgrad_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)S::SMEM);
     if (e != cudaSuccess) return e;
     CUtensorMap gmap, imap;
-    e = channel_group_map(&gmap, g, COUT, L, B, tcw::P);
-    if (e == cudaSuccess) e = channel_group_map(&imap, in, CIN, L, B, tcw::PR);
+    e = position_map(&gmap, g, COUT, L, B, tcw::P);
+    if (e == cudaSuccess) e = position_map(&imap, in, CIN, L, B, tcw::PR);
     if (e != cudaSuccess) return e;
-    conv_wgrad_tc_kernel<CIN, COUT><<<dim3(KW / tcw::TAPS, (L + chunk - 1) / chunk, B), 128, S::SMEM, s>>>(
-        gmap, imap, gW, L, chunk);
+    // one CTA per SM, and as many waves as keep a CTA's sums at 32 tiles or less
+    const long long tiles = (long long)((L + tcw::P - 1) / tcw::P) * B;
+    const long long waves = (tiles + 32ll * sm_count() - 1) / (32ll * sm_count());
+    const int grid = (int)std::min<long long>(tiles, waves * sm_count());
+    conv_wgrad_tc_kernel<CIN, COUT><<<grid, 128, S::SMEM, s>>>(gmap, imap, gW, gb, L, B);
     count_launch();
     return cudaGetLastError();
 }
@@ -947,34 +901,19 @@ FOCSS_API focss_status focss_cnn_loss_grad(focss_cnn* m, const focss_field* y, c
     }
     float* G = m->grads;
     // layer 4 (no activation): weights, bias, input gradient masked by out3 > 0
-    if (e == cudaSuccess) e = fg::conv_wgrad<fg::CW, fg::COUT4>(m->g16, m->act[3], G + Y.w[3], L, B, s);
-    if (e == cudaSuccess) {
-        fg::bias_grad_kernel<fg::COUT4><<<fg::sm_count() * 4, 256, 0, s>>>(m->g16, n, G + Y.b[3]);
-        fg::count_launch();
-        e = cudaGetLastError();
-    }
+    if (e == cudaSuccess) e = fg::conv_wgrad<fg::CW, fg::COUT4>(m->g16, m->act[3], G + Y.w[3], G + Y.b[3], L, B, s);
     if (e == cudaSuccess)
         e = fg::conv_fwd<fg::COUT4, fg::CW, false>(m->g16, m->wt[3], nullptr, m->g64a, L, B, 0, m->act[3], s);
     // layers 3, 2 (64 -> 64)
     bf16* g = m->g64a;
     bf16* g2 = m->g64b;
     for (int l = 2; l >= 1 && e == cudaSuccess; --l) {
-        e = fg::conv_wgrad<fg::CW, fg::CW>(g, m->act[l], G + Y.w[l], L, B, s);
-        if (e == cudaSuccess) {
-            fg::bias_grad_kernel<fg::CW><<<fg::sm_count() * 4, 256, 0, s>>>(g, n, G + Y.b[l]);
-            fg::count_launch();
-            e = cudaGetLastError();
-        }
+        e = fg::conv_wgrad<fg::CW, fg::CW>(g, m->act[l], G + Y.w[l], G + Y.b[l], L, B, s);
         if (e == cudaSuccess) e = fg::conv_fwd<fg::CW, fg::CW, false>(g, m->wt[l], nullptr, g2, L, B, 0, m->act[l], s);
         std::swap(g, g2);
     }
     // layer 1: weights and bias only
-    if (e == cudaSuccess) e = fg::conv_wgrad<fg::CIN0, fg::CW>(g, m->act[0], G + Y.w[0], L, B, s);
-    if (e == cudaSuccess) {
-        fg::bias_grad_kernel<fg::CW><<<fg::sm_count() * 4, 256, 0, s>>>(g, n, G + Y.b[0]);
-        fg::count_launch();
-        e = cudaGetLastError();
-    }
+    if (e == cudaSuccess) e = fg::conv_wgrad<fg::CIN0, fg::CW>(g, m->act[0], G + Y.w[0], G + Y.b[0], L, B, s);
     double h = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, m->loss, sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
