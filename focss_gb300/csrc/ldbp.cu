@@ -176,7 +176,6 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
                        &bfull[l & 1]);
     };
 
-    pdl_trigger();
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int i = 0; i < kMaxChain; ++i) {
@@ -430,6 +429,7 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         chain_store(a, a.y, b, n0, true, [&](int) { return make_float2(nan, nan); });
         if (threadIdx.x < a.layers) s_gxi[threadIdx.x] = nan;
     }
+    pdl_trigger();
     if (BWD && a.xi && threadIdx.x < a.layers) atomicAdd(a.gxi + (ptrdiff_t)a.dir * (int)threadIdx.x, s_gxi[threadIdx.x]);
     tcg::fence_before_sync();
     __syncthreads();

@@ -124,15 +124,14 @@ cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
     return cudaSuccess;
 }
 
-// Launches a pass kernel.  Launched directly into a stream, it carries
-// programmatic stream serialization: when the previous operation in the
-// stream is a kernel, this one may be scheduled as soon as that kernel's CTAs
-// have all started, and runs up to its pdl_wait (the column pass computes its
-// six-step factors there) while the other finishes, instead of paying the
-// launch latency after it (one 2^17 field, 100 steps through focss_ssfm_run:
-// 2.31 -> 2.13 ms).  Captured into a graph it is a plain kernel node: graph
-// launches already hide that latency, and programmatic edges there measured
-// slower (800 steps of one 2^17 field: 17.8 -> 19.9 us per step).
+// Launches a pass kernel with programmatic stream serialization: when the previous
+// operation in the stream (or, captured, in the graph's branch) is a kernel, this
+// one may be scheduled once all of that kernel's CTAs have stored their results
+// (pdl_trigger at the end of the pass kernels), and runs up to its pdl_wait while the
+// other finishes.  With the trigger at a pass's start the waiting CTAs held
+// slots and issue cycles of the running one: one 2^17 field 16.6 -> 14.3 us per
+// step, five 23.8 -> 19.1, one 2^19 field 25.8 -> 21.0; captured (plain edges before)
+// 15.3 -> 14.5, 18.7 -> 18.4 and 21.2 -> 20.9.
 template <class... A>
 cudaError_t launch_pass(void (*fn)(A...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... a) {
     cudaLaunchConfig_t cfg{};
@@ -140,14 +139,11 @@ cudaError_t launch_pass(void (*fn)(A...), dim3 grid, int threads, size_t smem, c
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    const cudaError_t ce = cudaStreamIsCapturing(s, &cs);
-    if (ce != cudaSuccess) return ce;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
+    cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, a...);
     count_launch();
     const cudaError_t last = cudaGetLastError();  // consumed, as after a <<<>>> launch
@@ -177,14 +173,11 @@ cudaError_t launch_col_tma(const Plan& p, const PassArgs& a, int batch, int mode
     cfg.blockDim = dim3(l.threads * modes);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    e = cudaStreamIsCapturing(s, &cs);
-    if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
+    cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, l.fn_tma, map, a);
     count_launch();
     const cudaError_t last = cudaGetLastError();

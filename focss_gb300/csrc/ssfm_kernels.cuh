@@ -420,7 +420,6 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
 
     // The six-step factors depend on nothing in memory: computed while the
     // previous pass finishes (programmatic dependent launch).
-    pdl_trigger();
     for (int i = threadIdx.x; i < Q * C; i += blockDim.x)
         s_B[i] = sixstep_column<N1>(i / C, blockIdx.x * C + i % C, a.log2N2);
     pdl_wait();
@@ -437,6 +436,7 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
     float2* data = a.datas ? a.datas[b] : a.data + (size_t)b * modes * a.N;
     col_work<N1, C>(a, op, st, data + (size_t)mo * a.N, blockIdx.x * C, s_fc, s_B, C, sx, s_x0, mo, modes,
                     threadIdx.x % (C * P), a.N2, pk, sm);
+    pdl_trigger();
     if (st) col_advance(a, st, b, op, pk, sm, red);
 }
 
@@ -602,7 +602,6 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row
     float2* s_tw = reinterpret_cast<float2*>(s_T + 512);     // sub-FFT twiddles
     float2* sx = s_tw + N2;                                  // R * Q * (P+1)
 
-    pdl_trigger();
     pdl_wait();
     const int b = blockIdx.y;  // realization * modes + mode
     const SsfmState* st = a.state ? a.state + b / (a.modes > 1 ? a.modes : 1) : nullptr;
@@ -620,6 +619,7 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row
     if (a.datas) data = a.modes > 1 ? a.datas[b >> 1] + (size_t)(b & 1) * a.N : a.datas[b];  // 1 or 2 modes
     row_work<N2>(a, st ? (int)ROW_SSFM : a.op, data, blockIdx.x * R + rl, rl, t, s_tw, s_T, sx,
                  g, dhi, dlo, N2);
+    pdl_trigger();
 }
 
 // The same for a chunk of the launch's (N1 / R) x `rows` row blocks, one after the
@@ -636,7 +636,6 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 512 / (R * PQ<N2>::P)) row_kerne
     float4* s_T = smem4;                                     // g exp(2 pi i j/512)
     float2* s_tw = reinterpret_cast<float2*>(s_T + 512);     // sub-FFT twiddles
     float2* sx = s_tw + N2;                                  // R * Q * (P+1)
-    pdl_trigger();
     const int rl = threadIdx.x / P, t = threadIdx.x % P;
     const int per = a.N1 / R;
     pdl_wait();
@@ -696,6 +695,7 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 512 / (R * PQ<N2>::P)) row_kerne
         row_store<N2>(v, row, op == ROW_FWD ? row_k2_base<N2>(t) : centred<P>(t));
         __syncwarp();
     }
+    pdl_trigger();
 }
 
 // ---------------------------------------------------------------- row pass, bulk-copy staging
@@ -735,7 +735,6 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, 2) row_kernel_bulk(const PassArg
     float2* sx = s_tw + N2;                                  // R * Q * (P+1): landing zone and exchange
     __shared__ __align__(8) unsigned long long bar;
 
-    pdl_trigger();
     pdl_wait();
     const int b = blockIdx.y;  // realization * modes + mode
     const SsfmState* st = a.state ? a.state + b / (a.modes > 1 ? a.modes : 1) : nullptr;
@@ -821,7 +820,6 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB)
     __shared__ float red[64];
     __shared__ __align__(8) unsigned long long bar;
 
-    pdl_trigger();
     for (int i = threadIdx.x; i < Q * C; i += blockDim.x)
         s_B[i] = sixstep_column<N1>(i / C, blockIdx.x * C + i % C, a.log2N2);
     pdl_wait();
@@ -855,6 +853,7 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB)
     float pk = 0.0f, sm = 0.0f;
     col_work<N1, C>(a, op, st, a.data + ((size_t)b * modes + mo) * a.N, blockIdx.x * C, s_fc, s_B, C, sx, s_x0, mo,
                     modes, threadIdx.x % (C * P), a.N2, pk, sm, sx, C);
+    pdl_trigger();
     if (st) col_advance(a, st, b, op, pk, sm, red);
 }
 
