@@ -34,10 +34,15 @@ focss_status get_plan(Ctx* ctx, int N, const Plan** out) {
     return get_plan_split(ctx, N, lg / 2, out);
 }
 
+// Balanced, with the longer side in the rows; but at 2^13 and 2^17 the columns take it:
+// 256- and 64-sample rows keep 16 and 8 samples per thread where 512 and 128 take 32
+// and 16 (one 2^17 field 15.7 -> 14.3 us per step, 64 fields 87.6 -> 82.5; 25 of 2^13
+// 16.6 -> 15.7).  At 2^15 that costs more in the 256-sample columns (64 fields 28.2 ->
+// 31.8), at 2^19 it is even.
 int default_split(int N) {
     int lg = 0;
     while ((1 << lg) < N) ++lg;
-    return lg / 2;
+    return lg == 13 || lg == 17 ? lg / 2 + 1 : lg / 2;
 }
 
 bool split_supported(int N, int log2N1) {
