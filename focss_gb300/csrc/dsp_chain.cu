@@ -17,6 +17,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "fft.cuh"
@@ -190,18 +191,17 @@ __global__ void scale_taps_kernel(double* __restrict__ taps, int len, const doub
 // Decimation gather: out (M samples, two-pass layout M1 x M2) takes bin
 // k_out of the N-point spectrum `in` (two-pass layout N1 x N2; rows from kc on
 // hold the bins k1 - N1 + N1 k2), with the reference's bin map (field.cpp:309-317).
-__global__ void decimate_gather_kernel(const float2* __restrict__ in, float2* __restrict__ out, int N, int N1,
-                                       int N2, int kc_in, int M, int M1, int M2, int kc_out, int rows) {
+__global__ void decimate_gather_kernel(const float2* __restrict__ in, float2* __restrict__ out, int N, int log2N1,
+                                       int N2, int kc_in, int M, int M1, int log2M2, int kc_out) {
     const int cutoff = M / 2, shift = N - M;
-    const size_t total = (size_t)rows * M;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / M;
-        const int p = (int)(i % M);
-        const int k1 = p / M2, k2 = p % M2;
+    in += (size_t)blockIdx.y * N;
+    out += (size_t)blockIdx.y * M;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < M; p += gridDim.x * blockDim.x) {
+        const int k1 = p >> log2M2, k2 = p & ((1 << log2M2) - 1);
         const int kout = ((k1 < kc_out ? k1 : k1 - M1) + M1 * k2) & (M - 1);
         const int kin = kout < cutoff ? kout : kout + shift;
-        const int r1 = kin % N1;
-        out[i] = in[r * N + (size_t)r1 * N2 + ((kin / N1 + (r1 >= kc_in)) & (N2 - 1))];
+        const int r1 = kin & ((1 << log2N1) - 1);
+        out[p] = in[(size_t)r1 * N2 + (((kin >> log2N1) + (r1 >= kc_in)) & (N2 - 1))];
     }
 }
 
@@ -209,19 +209,17 @@ __global__ void decimate_gather_kernel(const float2* __restrict__ in, float2* __
 // repeats the n-point spectrum `in` (layout N1i x N2i) osf times, so pulse
 // shaping needs no transform of the N-point sequence: out (layout N1 x N2)
 // takes bin k mod n times H times g.  Shaping 5 x 2^19 samples from 2^15 symbols
-// each: 72 -> 62 us.
+// each: 72 -> 62 us (this kernel 14.5 us with divisions for the indexes, 8.6 with shifts).
 __global__ void repeat_filter_kernel(const float2* __restrict__ in, const float2* __restrict__ H, float2* __restrict__ out,
-                                     float g, int n, int N1i, int N2i, int kc_in, int N, int N1, int N2, int kc_out,
-                                     int rows) {
-    const size_t total = (size_t)rows * N;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / N;
-        const int p = (int)(i % N);
-        const int k1 = p / N2, k2 = p % N2;
+                                     float g, int n, int log2N1i, int N2i, int kc_in, int N, int N1, int log2N2, int kc_out) {
+    in += (size_t)blockIdx.y * n;
+    out += (size_t)blockIdx.y * N;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) {
+        const int k1 = p >> log2N2, k2 = p & ((1 << log2N2) - 1);
         const int k = ((k1 < kc_out ? k1 : k1 - N1) + N1 * k2) & (n - 1);
-        const int r1 = k % N1i;
-        const float2 v = in[r * n + (size_t)r1 * N2i + ((k / N1i + (r1 >= kc_in)) & (N2i - 1))];
-        out[i] = cscale(cmul(v, H[p]), g);
+        const int r1 = k & ((1 << log2N1i) - 1);
+        const float2 v = in[r1 * N2i + (((k >> log2N1i) + (r1 >= kc_in)) & (N2i - 1))];
+        out[p] = cscale(cmul(v, H[p]), g);
     }
 }
 
@@ -237,20 +235,29 @@ __global__ void freq_shift_kernel(const float2* d, float2* out, int samples, siz
     }
 }
 
-// wdm_mux: out[m,s] = sum_c ch_c[m,s] exp(2 pi i f_c dt s)
+// wdm_mux: out[m,s] = sum_c ch_c[m,s] exp(2 pi i f_c dt s), the channels' turns
+// per sample X passed by value for up to kMuxByValue of them (no copy, and the host
+// does not wait for the call), else in Xd.  Grid y: modes.
+constexpr int kMuxByValue = 128;
+struct MuxTurns {
+    unsigned long long X[kMuxByValue];
+};
 __global__ void wdm_mux_kernel(const float2* __restrict__ ch, int n_ch, int modes, int samples,
-                               const unsigned long long* __restrict__ X, float2* __restrict__ out) {
+                               const __grid_constant__ MuxTurns Xv, const unsigned long long* __restrict__ Xd,
+                               float2* __restrict__ out) {
     const size_t per = (size_t)modes * samples;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < per; i += (size_t)gridDim.x * blockDim.x) {
-        const unsigned long long s = (unsigned long long)(i % (size_t)samples);
+    ch += (size_t)blockIdx.y * samples;
+    out += (size_t)blockIdx.y * samples;
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < samples; s += gridDim.x * blockDim.x) {
         float2 acc = make_float2(0.f, 0.f);
         for (int c = 0; c < n_ch; ++c) {
-            const float x = (float)(long long)(X[c] * s) * 1.0842021724855044e-19f;
+            const unsigned long long X = Xd ? Xd[c] : Xv.X[c];
+            const float x = (float)(long long)(X * (unsigned long long)s) * 1.0842021724855044e-19f;
             float sn, cs;
             sincospif(x, &sn, &cs);
-            acc = cadd(acc, cmul(ch[c * per + i], make_float2(cs, sn)));
+            acc = cadd(acc, cmul(ch[c * per + s], make_float2(cs, sn)));
         }
-        out[i] = acc;
+        out[s] = acc;
     }
 }
 
@@ -284,32 +291,33 @@ __global__ void power_sum_kernel(const float2* __restrict__ d, size_t per, doubl
 // Four calls on 4000 samples (decision, codes, errors, Q): 139 -> 94 us with
 // launches and synchronization.  Above kClusterSamples a cluster's share of
 // the FP64 sums takes longer than a second launch over more CTAs.
-constexpr int kCluster = 8, kClusterThreads = 512;
+constexpr int kCluster = 8, kClusterThreads = 256;
 constexpr size_t kClusterSamples = 16384;
 
-// sum over the realization, valid in thread 0.  CL: by its cluster, whose CTAs
-// end with cluster_done (the partial sums are read remotely), else from psum.
+// Sum over the realization, valid in thread 0 after the next barrier of its warp.  CL:
+// by its cluster, else from psum.  Every CTA writes its partial sum into all CTAs'
+// shared memory before the cluster's barrier, so that afterwards nothing is read
+// remotely and no CTA has to stay for the others.
 template <bool CL>
 __device__ __forceinline__ double realization_power(const float2* __restrict__ d, size_t per, const double* psum) {
     if constexpr (CL) {
         namespace cg = cooperative_groups;
-        __shared__ double sd[32], part;
+        __shared__ double sd[32], part[kCluster];
         const cg::cluster_group cluster = cg::this_cluster();
+        auto started = cluster.barrier_arrive();  // every CTA's shared memory exists once all have
         const double v = block_sum_d(power_partial(d, per, blockIdx.x * (size_t)blockDim.x + threadIdx.x,
                                                    (size_t)gridDim.x * blockDim.x), sd);
-        if (threadIdx.x == 0) part = v;
+        const double mine = __shfl_sync(0xffffffffu, v, 0);
+        cluster.barrier_wait(std::move(started));
+        if (threadIdx.x < kCluster) *cluster.map_shared_rank(&part[blockIdx.x], threadIdx.x) = mine;
         cluster.sync();
         double total = 0.0;
         if (threadIdx.x == 0)
-            for (int r = 0; r < kCluster; ++r) total += *cluster.map_shared_rank(&part, r);
+            for (int r = 0; r < kCluster; ++r) total += part[r];
         return total;
     } else {
         return *psum;
     }
-}
-template <bool CL>
-__device__ __forceinline__ void cluster_done() {
-    if constexpr (CL) cooperative_groups::this_cluster().sync();
 }
 
 // hard_decision_16qam (modulation.cpp:112-120): power = avg/modes,
@@ -330,7 +338,7 @@ __global__ void hard_decision_kernel(const float2* in, float2* out, int modes, i
     const double total = realization_power<CL>(in, per, psum + b);
     if (threadIdx.x == 0) {
         s_sp = sqrt(total / samples / modes);
-        s_inv = (float)(1.0 / s_sp);
+        s_inv = 1.0f / (float)s_sp;  // only for decisions that are not near a boundary
     }
     __syncthreads();
     const double sp = s_sp;
@@ -346,7 +354,6 @@ __global__ void hard_decision_kernel(const float2* in, float2* out, int modes, i
         if (near) c = demod16_div(z.x, z.y, sp);
         out[i] = s_out[c];
     }
-    cluster_done<CL>();
 }
 
 // The FP64 forms of one soft decision (modulation.cpp:122-146) and one
@@ -501,7 +508,6 @@ __global__ void hd_codes_kernel(const float2* __restrict__ in, int32_t* __restri
         if (near) c = demod16_mul(z.x, z.y, sc);
         codes[i] = (int32_t)c;
     }
-    cluster_done<CL>();
 }
 
 // Decision errors over samples [cut, samples - cut) (modulation.cpp:158-223);
@@ -544,7 +550,7 @@ __global__ void error_count_kernel(const float2* __restrict__ tx, const float2* 
     }
     if constexpr (CL) {
         namespace cg = cooperative_groups;
-        __shared__ unsigned long long s_n[2];
+        __shared__ unsigned long long s_n[2], s_all[kCluster][2];
         const cg::cluster_group cluster = cg::this_cluster();
         if (threadIdx.x < 2) s_n[threadIdx.x] = 0ull;
         __syncthreads();
@@ -552,13 +558,14 @@ __global__ void error_count_kernel(const float2* __restrict__ tx, const float2* 
             atomicAdd(&s_n[0], be);
             atomicAdd(&s_n[1], se);
         }
+        __syncthreads();
+        if (threadIdx.x < 2) *cluster.map_shared_rank(&s_all[blockIdx.x][threadIdx.x], 0) = s_n[threadIdx.x];
         cluster.sync();
         if (blockIdx.x == 0 && threadIdx.x < 2) {
             unsigned long long n = 0ull;
-            for (int r = 0; r < kCluster; ++r) n += *cluster.map_shared_rank(&s_n[threadIdx.x], r);
+            for (int r = 0; r < kCluster; ++r) n += s_all[r][threadIdx.x];
             counts[2 * b + threadIdx.x] = n;
         }
-        cluster_done<CL>();
     } else if ((threadIdx.x & 31) == 0) {
         atomicAdd(counts + 2 * b, be);
         atomicAdd(counts + 2 * b + 1, se);
@@ -878,8 +885,8 @@ FOCSS_API focss_status focss_decimate(focss_ctx* c, const focss_field* in, int f
     if (!sp) return fg::set_error(c, FOCSS_ERR_OOM, "decimate scratch");
     st = fg::fft_forward_transposed(c, sp, in->samples, rows, 1.0f / (float)in->samples, in->d);
     if (st != FOCSS_OK) return st;
-    FG_LAUNCH(fg::decimate_gather_kernel<<<fg::grid_for(out->n(), 256), 256, 0, c->stream>>>(
-        sp, out->d, pi->N, pi->N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1, po->N2, fg::col_kc(po->N1), rows));
+    FG_LAUNCH(fg::decimate_gather_kernel<<<fg::grid_per_realization(out->samples, rows), 256, 0, c->stream>>>(
+        sp, out->d, pi->N, pi->log2N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1, po->log2N2, fg::col_kc(po->N1)));
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fg::cuda_check(c, e, "decimate gather");
     return fg::fft_inverse_transposed(c, out->d, out->samples, rows);
@@ -947,9 +954,9 @@ FOCSS_API focss_status focss_rrc_shaping(focss_ctx* c, const focss_field* symbol
         const double N = out->samples;
         st = fg::fft_forward_transposed(c, sp, n, rows, 1.0f, symbols->d);
         if (st != FOCSS_OK) return st;
-        FG_LAUNCH(fg::repeat_filter_kernel<<<fg::grid_for(out->n(), 256), 256, 0, c->stream>>>(
-            sp, H, out->d, (float)(std::sqrt(gain) * osf / (N * N)), pi->N, pi->N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1,
-            po->N2, fg::col_kc(po->N1), rows));
+        FG_LAUNCH(fg::repeat_filter_kernel<<<fg::grid_per_realization(out->samples, rows), 256, 0, c->stream>>>(
+            sp, H, out->d, (float)(std::sqrt(gain) * osf / (N * N)), n, pi->log2N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1,
+            po->log2N2, fg::col_kc(po->N1)));
         st = fg::cuda_check(c, cudaGetLastError(), "rrc_shaping spectrum");
         return st == FOCSS_OK ? fg::fft_inverse_transposed(c, out->d, out->samples, rows) : st;
     }
@@ -1022,12 +1029,19 @@ FOCSS_API focss_status focss_wdm_mux(focss_ctx* c, const focss_field* ch, double
     const int n = ch->batch;
     std::vector<unsigned long long> X(n);
     for (int i = 0; i < n; ++i) X[i] = fg::turns_fix64_host((i - n / 2) * channel_bandwidth * ch->dt);
-    unsigned long long* dX = (unsigned long long*)fg::scratch_buffer(c, 5, sizeof(unsigned long long) * n);
-    if (!dX) return fg::set_error(c, FOCSS_ERR_OOM, "wdm_mux scratch");
-    cudaError_t e = cudaMemcpyAsync(dX, X.data(), sizeof(unsigned long long) * n, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) FG_LAUNCH(fg::wdm_mux_kernel<<<fg::grid_for(out->n(), 256), 256, 0, c->stream>>>(ch->d, n, ch->modes, ch->samples, dX, out->d));
+    fg::MuxTurns v{};
+    unsigned long long* dX = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (n <= fg::kMuxByValue) {
+        std::copy(X.begin(), X.end(), v.X);
+    } else {
+        dX = (unsigned long long*)fg::scratch_buffer(c, 5, sizeof(unsigned long long) * n);
+        if (!dX) return fg::set_error(c, FOCSS_ERR_OOM, "wdm_mux scratch");
+        e = cudaMemcpyAsync(dX, X.data(), sizeof(unsigned long long) * n, cudaMemcpyHostToDevice, c->stream);
+    }
+    if (e == cudaSuccess) FG_LAUNCH(fg::wdm_mux_kernel<<<fg::grid_per_realization(ch->samples, ch->modes), 256, 0, c->stream>>>(ch->d, n, ch->modes, ch->samples, v, dX, out->d));
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess && dX) e = cudaStreamSynchronize(c->stream);  // X
     return fg::cuda_check(c, e, "wdm_mux");
 }
 
