@@ -151,7 +151,6 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
     __shared__ __align__(16) float s_bias[COUT];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ntiles = (L + tc::M - 1) / tc::M, T = ntiles * B;
-    for (int i = threadIdx.x; i < COUT; i += blockDim.x) s_bias[i] = bias ? bias[i] : 0.f;
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int i = 0; i < ST; ++i) {
@@ -171,6 +170,8 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
                      "r"(S::TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
+    pdl_wait();  // nothing in global memory is touched before the launches it depends on are done
+    for (int i = threadIdx.x; i < COUT; i += blockDim.x) s_bias[i] = bias ? bias[i] : 0.f;
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -348,6 +349,7 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
             }
         }
     }
+    pdl_trigger();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -438,6 +440,7 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(const __grid_constan
         tc::mbar_init(&drain, 2);
         tc::fence_mbar_init();
     }
+    pdl_wait();
     for (int i = threadIdx.x; i < (int)tcw::ONES / 4; i += blockDim.x)
         reinterpret_cast<uint32_t*>(smem_raw + (ones - raw))[i] = 0x3F803F80u;
     tc::fence_async_smem();
@@ -518,6 +521,7 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(const __grid_constan
             }
         }
     }
+    pdl_trigger();
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_free(tmem, S::TMEM_COLS);
@@ -621,6 +625,26 @@ inline int gridn(size_t n) {
     return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, (size_t)sm_count() * 16));
 }
 
+// Launches a convolution with programmatic stream serialization: its set-up runs while
+// the kernel before it ends (training step 451 -> 435 us).
+template <class... P, class... A>
+cudaError_t launch_serialized(void (*kern)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    count_launch();
+    const cudaError_t last = cudaGetLastError();
+    return e != cudaSuccess ? e : last;
+}
+
 template <int CIN, int COUT, bool F32>
 cudaError_t conv_fwd(const bf16* in, const bf16* W, const float* bias, void* out, int L, int B, int relu,
                      const bf16* mask, cudaStream_t s) {
@@ -650,9 +674,7 @@ cudaError_t conv_fwd(const bf16* in, const bf16* W, const float* bias, void* out
     per_sm = std::max(1, std::min(per_sm, std::min(2, (int)(512 / S::TMEM_COLS))));
     const long long tiles = (long long)((L + tc::M - 1) / tc::M) * B;
     const int grid = (int)std::max(1ll, std::min(tiles, (long long)sm_count() * per_sm));
-    kern<<<grid, tc::FWD_THREADS, S::SMEM, s>>>(amap, W, bias, out, L, B, relu, mask);
-    count_launch();
-    return cudaGetLastError();
+    return launch_serialized(kern, grid, tc::FWD_THREADS, S::SMEM, s, amap, W, bias, out, L, B, relu, mask);
 }
 
 // Tensor map of [B][L][C] bf16 with boxes of all C channels x `rows` positions, in
@@ -686,9 +708,7 @@ cudaError_t conv_wgrad(const bf16* g, const bf16* in, float* gW, float* gb, int 
     const long long tiles = (long long)((L + tcw::P - 1) / tcw::P) * B;
     const long long waves = (tiles + 32ll * sm_count() - 1) / (32ll * sm_count());
     const int grid = (int)std::min<long long>(tiles, waves * sm_count());
-    conv_wgrad_tc_kernel<CIN, COUT><<<grid, 128, S::SMEM, s>>>(gmap, imap, gW, gb, L, B);
-    count_launch();
-    return cudaGetLastError();
+    return launch_serialized(conv_wgrad_tc_kernel<CIN, COUT>, grid, 128, S::SMEM, s, gmap, imap, gW, gb, L, B);
 }
 
 }  // namespace
