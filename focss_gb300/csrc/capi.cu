@@ -110,7 +110,7 @@ focss_status ensure_state(Ctx* ctx, int batch) {
     if (ctx->d_state) cudaFree(ctx->d_state);
     ctx->d_state = nullptr;
     ctx->state_cap = 0;
-    cudaError_t e = cudaMalloc(&ctx->d_state, sizeof(SsfmState) * (size_t)batch);
+    cudaError_t e = cudaMalloc(&ctx->d_state, sizeof(SsfmState) * 2 * (size_t)batch);  // and the next step's
     if (e != cudaSuccess) return cuda_check(ctx, e, "state alloc");
     ctx->state_cap = batch;
     return FOCSS_OK;

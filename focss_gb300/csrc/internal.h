@@ -99,6 +99,12 @@ struct PassArgs {
     // one's samples (modes x N) and parameters, in place of data and prm
     float2* const* datas;
     SsfmState* state;       // null: plain transform driven by `op`
+    // column passes of a grid known up front (UNIFORM, replayed): where the state
+    // after the pass goes, formed by a CTA of its own while the others work (one 2^17
+    // field 13.8 -> 9.9 us per step: reductions, ticket and FP64 chain of the last CTA
+    // were on the path between the passes); null: the last CTA advances `state` in
+    // place (it may need the pass's peak)
+    SsfmState* next;
     Tables tw;
     int N, N1, N2, log2N2;
     int kc;                 // rows k1 >= kc hold the bins k1 - N1 + N1 k2 (set by the launch helpers)
@@ -205,6 +211,12 @@ void* scratch_buffer(Ctx* ctx, int slot, size_t bytes);
 bool fft_size_supported(int N);
 cudaError_t launch_col(const Plan& p, PassArgs a, int batch, cudaStream_t s);
 cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s);
+// Pass pair k of a grid known up front, `cols` realizations' column passes and `rows`
+// realizations' row passes (rows may be 0).  The state alternates between two
+// buffers, the first zeroed before pass 0; after n passes it is in final_state.
+cudaError_t launch_pair(const Plan& p, PassArgs a, SsfmState* const (&states)[2], long long k, int cols, int rows,
+                        cudaStream_t s);
+inline int final_state(const Plan& p, long long passes) { return p.staging == FOCSS_STAGING_LOADS ? (int)(passes & 1) : 0; }
 // Step-grid record / replay of one ssfm_run: device arrays as in SsfmParams.
 struct StepGrid {
     double* record = nullptr;

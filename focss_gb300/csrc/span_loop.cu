@@ -44,7 +44,7 @@ struct AmpField {
 
 struct LoopGraph {
     cudaGraphExec_t exec = nullptr;
-    SsfmState* d_state = nullptr;         // every field's realizations
+    SsfmState* d_state = nullptr;         // every field's realizations, twice (launch_pair)
     int* d_ctr = nullptr;                 // kCtr counters per field
     int* d_steps = nullptr;               // steps per realization, summed over spans
     unsigned long long* d_amp = nullptr;  // {seed, counter0} per field
@@ -107,8 +107,10 @@ __global__ void amp_group_kernel(const AmpField* __restrict__ fields, const unsi
 
 // span_end_kernel for a group of UNIFORM fields: a realization's counters are
 // found by its n_done.
-__global__ void span_end_group_kernel(const SsfmState* __restrict__ st, const SsfmParams* __restrict__ prm, int n, int* steps) {
+__global__ void span_end_group_kernel(const SsfmState* __restrict__ st0, const SsfmState* __restrict__ st1,
+                                      const SsfmParams* __restrict__ prm, int n, int* steps) {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x) {
+        const SsfmState* st = prm[b].total_steps & 1 ? st1 : st0;  // after total_steps + 2 passes
         if (st[b].action != COL_IDLE) atomicOr(prm[b].n_done + 3, 1);
         steps[b] += st[b].n_steps;
     }
@@ -175,6 +177,8 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
                           cudaStream_t body_stream) {
     const int B = f->batch;
     SsfmState* state = g->d_state + g->offset[i];
+    SsfmState* const states[2] = {state, state + g->total};
+    int done = 0;  // the states buffer at a span's end
     int* ctr = g->d_ctr + kCtr * g->slot[i];
     int* steps = g->d_steps + g->offset[i];
     const size_t n = f->n();
@@ -200,9 +204,9 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
             g->static_kernels += 1;
         } else if (o.grid == FOCSS_UNIFORM) {
             for (int k = 0; k < o.total_steps + 2 && e == cudaSuccess; ++k) {
-                e = launch_col(p, a, B, s);
-                if (e == cudaSuccess && k <= o.total_steps) e = launch_row(p, a, B, s);
+                e = launch_pair(p, a, states, k, B, k <= o.total_steps ? B : 0, s);
             }
+            done = final_state(p, o.total_steps + 2);
             g->static_kernels += 2ll * (o.total_steps + 2) - 1;
         } else {
             // Conditional WHILE node appended to the branch's capture.
@@ -247,7 +251,7 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
             g->body_kernels[i] = 2 * kChunk + 1;
             if (e != cudaSuccess) break;
         }
-        span_end_kernel<<<1, 256, 0, s>>>(state, B, o.grid == FOCSS_ADAPTIVE, ctr, steps);
+        span_end_kernel<<<1, 256, 0, s>>>(states[done], B, o.grid == FOCSS_ADAPTIVE, ctr, steps);
         e = cudaGetLastError();
         g->static_kernels += 1;
         if (e == cudaSuccess && amp.after != FOCSS_AMP_NONE) {
@@ -275,7 +279,7 @@ cudaError_t record_group(LoopGraph* g, const std::vector<int>& group, Field* con
     }
     PassArgs a{};
     a.modes = fs[first]->modes;
-    a.state = g->d_state + off;
+    SsfmState* const states[2] = {g->d_state + off, g->d_state + off + g->total};
     a.datas = g->d_data + off;
     a.prms = g->d_prm + off;
     int* ctr = g->d_ctr + kCtr * slot;
@@ -299,13 +303,12 @@ cudaError_t record_group(LoopGraph* g, const std::vector<int>& group, Field* con
         // K steps take K + 2 column passes with a row pass between any two
         const int passes = opts[first].total_steps + 2;
         for (int k = 0; k < passes && e == cudaSuccess; ++k) {
-            e = launch_col(p, a, active(k - 2), s);
             const int rows = active(k - 1);
-            if (e == cudaSuccess && rows) e = launch_row(p, a, rows, s);
+            e = launch_pair(p, a, states, k, active(k - 2), rows, s);
             g->static_kernels += rows ? 2 : 1;
         }
         if (e != cudaSuccess) break;
-        span_end_group_kernel<<<(B + 255) / 256, 256, 0, s>>>(a.state, a.prms, B, g->d_steps + off);
+        span_end_group_kernel<<<(B + 255) / 256, 256, 0, s>>>(states[0], states[1], a.prms, B, g->d_steps + off);
         e = cudaGetLastError();
         g->static_kernels += 1;
         if (e == cudaSuccess && amp.after != FOCSS_AMP_NONE) e = amplify(1, span);
@@ -349,7 +352,7 @@ focss_status build_graph(Ctx* ctx, LoopGraph* g, int nf, Field* const* fs, const
             g->batch[i] = fs[i]->batch;
             g->total += fs[i]->batch;
         }
-    cudaError_t e = cudaMalloc(&g->d_state, sizeof(SsfmState) * g->total);
+    cudaError_t e = cudaMalloc(&g->d_state, sizeof(SsfmState) * 2 * g->total);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_ctr, sizeof(int) * kCtr * nf);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_steps, sizeof(int) * g->total);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_amp, sizeof(unsigned long long) * 2 * nf);

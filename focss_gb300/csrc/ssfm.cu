@@ -205,7 +205,7 @@ cudaError_t launch_col(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
     if (p.staging == FOCSS_STAGING_TMA) return launch_col_tma(p, a, batch, modes, smem + 128, s);
     cudaError_t e = cached_launch(narrow ? 4 : 0, p.log2N1, smem, &l);
     if (e != cudaSuccess) return e;
-    return launch_pass(l.fn, dim3(p.N2 / l.per_block, batch), l.threads * modes, smem, s, a);
+    return launch_pass(l.fn, dim3(p.N2 / l.per_block + (a.next ? 1 : 0), batch), l.threads * modes, smem, s, a);
 }
 
 cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
@@ -243,6 +243,18 @@ cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     if (p.N1 % R != 0) return cudaErrorInvalidValue;
     return launch_pass(l.fn, dim3(p.N1 / R, batch * (a.modes > 1 ? a.modes : 1)), l.threads, smem, s, a);
+}
+
+cudaError_t launch_pair(const Plan& p, PassArgs a, SsfmState* const (&states)[2], long long k, int cols, int rows,
+                        cudaStream_t s) {
+    const bool early = p.staging == FOCSS_STAGING_LOADS;
+    a.state = states[early ? k & 1 : 0];
+    a.next = early ? states[(k + 1) & 1] : nullptr;
+    cudaError_t e = launch_col(p, a, cols, s);
+    if (early) a.state = a.next;
+    a.next = nullptr;
+    if (e == cudaSuccess && rows) e = launch_row(p, a, rows, s);
+    return e;
 }
 
 // ---------------------------------------------------------------- SSFM driver
@@ -328,7 +340,8 @@ bool ssfm_single_cta(const Ctx* ctx, const Field* f) {
     return it != ctx->ssfm_split.end() && it->second == kSingleCta && f->modes == 1 && block_split(f->samples) != 0;
 }
 
-focss_status ssfm_finish(Ctx* ctx, Field* f, const focss_ssfm_opts& o, int* steps_out, int* recorded_out);
+focss_status ssfm_finish(Ctx* ctx, Field* f, const focss_ssfm_opts& o, const SsfmState* state, int* steps_out,
+                         int* recorded_out);
 
 focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ssfm_opts& o, double dir,
                       int* steps_out, const StepGrid* grid, int* recorded_out) {
@@ -367,11 +380,12 @@ focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ss
     if (ssfm_single_cta(ctx, f)) {
         st = cuda_check(ctx, launch_block(*p, a, f->batch, (int)std::min<long long>(cap, 1 << 30), s), "ssfm block");
         if (st != FOCSS_OK) return st;
-        st = ssfm_finish(ctx, f, o, steps_out, recorded_out);
+        st = ssfm_finish(ctx, f, o, ctx->d_state, steps_out, recorded_out);
         // the kernel stops a realization at the cap, leaving it unfinished
         return st == FOCSS_ERR_TIMEOUT ? set_error(ctx, FOCSS_ERR_NOT_CONVERGED, "ssfm_run: step cap reached") : st;
     }
     const bool fixed = replay || o.grid == FOCSS_UNIFORM;  // pass count known up front
+    SsfmState* const states[2] = {ctx->d_state, ctx->d_state + f->batch};
     const int chunk = 16;
     long long launched = 0;
     bool done = false;
@@ -393,10 +407,12 @@ focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ss
                 if (e == cudaSuccess) e = cudaEventRecord(pe[1], s);
                 if (e == cudaSuccess) e = launch_row(*p, a, f->batch, s);
                 if (e == cudaSuccess) e = cudaEventRecord(pe[2], s);
+            } else if (fixed) {
+                // (its last column pass leaves nothing for a row pass)
+                e = launch_pair(*p, a, states, i, f->batch, i + 1 < n ? f->batch : 0, s);
             } else {
                 e = launch_col(*p, a, f->batch, s);
-                // (a fixed grid's last column pass leaves nothing for a row pass)
-                if (e == cudaSuccess && !(fixed && i + 1 == n)) e = launch_row(*p, a, f->batch, s);
+                if (e == cudaSuccess) e = launch_row(*p, a, f->batch, s);
             }
             if (e != cudaSuccess) {
                 if (ev) cudaEventDestroy(ev);
@@ -425,18 +441,19 @@ focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ss
         }
     }
     if (ev) cudaEventDestroy(ev);
-    return ssfm_finish(ctx, f, o, steps_out, recorded_out);
+    return ssfm_finish(ctx, f, o, states[fixed && !ctx->profiling ? final_state(*p, cap) : 0], steps_out, recorded_out);
 }
 
 // Reads the step states back after a run: every realization must be idle;
 // steps_out gets the step counts, recorded_out the recorded step-size counts.
-focss_status ssfm_finish(Ctx* ctx, Field* f, const focss_ssfm_opts& o, int* steps_out, int* recorded_out) {
+focss_status ssfm_finish(Ctx* ctx, Field* f, const focss_ssfm_opts& o, const SsfmState* state, int* steps_out,
+                         int* recorded_out) {
     cudaStream_t s = ctx->stream;
     focss_status st;
     std::vector<SsfmState> hs(f->batch);
     int fault = 0;
     st = cuda_check(ctx,
-                    cudaMemcpyAsync(hs.data(), ctx->d_state, sizeof(SsfmState) * f->batch,
+                    cudaMemcpyAsync(hs.data(), state, sizeof(SsfmState) * f->batch,
                                     cudaMemcpyDeviceToHost, s),
                     "state readback");
     if (st != FOCSS_OK) return st;

@@ -426,6 +426,17 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
     const int b = blockIdx.y;
     SsfmState* st = a.state ? a.state + b : nullptr;
     int op = a.op;
+    if (a.next && (int)blockIdx.x * C >= a.N2) {  // one CTA more: the step state after this pass
+        if (threadIdx.x == 0) {
+            SsfmState s = *st;
+            if (s.action == COL_IDLE)
+                s.row_active = 0;
+            else
+                ssfm_advance(s, a.prms ? a.prms[b] : a.prm, b, s.action, 0.0f, 0.0);
+            a.next[b] = s;
+        }
+        return;
+    }
     if (st) {
         op = *(volatile int*)&st->action;
         if (op == COL_IDLE) return;
@@ -437,7 +448,7 @@ __global__ void __launch_bounds__(2 * C * ColFFT<N1>::P, ColShape<N1>::MINB) col
     col_work<N1, C>(a, op, st, data + (size_t)mo * a.N, blockIdx.x * C, s_fc, s_B, C, sx, s_x0, mo, modes,
                     threadIdx.x % (C * P), a.N2, pk, sm);
     pdl_trigger();
-    if (st) col_advance(a, st, b, op, pk, sm, red);
+    if (st && !a.next) col_advance(a, st, b, op, pk, sm, red);
 }
 
 // ---------------------------------------------------------------- row pass
