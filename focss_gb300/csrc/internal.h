@@ -113,6 +113,10 @@ struct PassArgs {
     int op;
     float scale;
     int bp_cut;
+    // pass pairs of other grids in small launches: the column pass only collects its
+    // peak in `state`, and every CTA of the row pass advances the state for itself
+    // while its samples load; the first one stores it to `next`
+    int late;
     long long src_off;      // stateless forward column pass: samples from data to its input (0: in place)
     unsigned long long disp_hi, disp_lo;  // stateless ROW_SSFM: dispersion phase as in SsfmState, gain in scale
     const float2* table;    // ROW_TABLE multiplier, transposed layout (k1*N2 + k2), length N
@@ -216,6 +220,11 @@ cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s);
 // buffers, the first zeroed before pass 0; after n passes it is in final_state.
 cudaError_t launch_pair(const Plan& p, PassArgs a, SsfmState* const (&states)[2], long long k, int cols, int rows,
                         cudaStream_t s);
+// Pass pair k of any other grid (states as launch_pair's, with `late` from late_state;
+// otherwise only the first is used).  An even number of pairs ends in states[0].
+cudaError_t launch_pair_adaptive(const Plan& p, PassArgs a, SsfmState* const (&states)[2], long long k, int batch,
+                                 cudaStream_t s);
+bool late_state(const Plan& p, int rows);
 inline int final_state(const Plan& p, long long passes) { return p.staging == FOCSS_STAGING_LOADS ? (int)(passes & 1) : 0; }
 // Step-grid record / replay of one ssfm_run: device arrays as in SsfmParams.
 struct StepGrid {

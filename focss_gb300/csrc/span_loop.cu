@@ -64,7 +64,7 @@ namespace {
 // [2] step cap hit, [3] a realization did not finish, [4] loop iterations
 // over all spans.
 constexpr int kCtr = 8;
-constexpr int kChunk = 8;                // pass pairs per loop-body iteration
+constexpr int kChunk = 8;                // pass pairs per loop-body iteration (even: launch_pair_adaptive)
 constexpr long long kMaxPairs = 1ll << 17;
 constexpr int kMaxIter = (int)(kMaxPairs / kChunk);
 constexpr size_t kMaxCachedGraphs = 64;
@@ -237,10 +237,8 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             e = cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
             if (e != cudaSuccess) break;
-            for (int c = 0; c < kChunk && e == cudaSuccess; ++c) {
-                e = launch_col(p, a, B, body_stream);
-                if (e == cudaSuccess) e = launch_row(p, a, B, body_stream);
-            }
+            for (int c = 0; c < kChunk && e == cudaSuccess; ++c)
+                e = launch_pair_adaptive(p, a, states, c, B, body_stream);
             if (e == cudaSuccess) {
                 loop_check_kernel<<<1, 32, 0, body_stream>>>(ctr, B, h);
                 e = cudaGetLastError();

@@ -93,7 +93,8 @@ std::mutex g_launch_mutex;
 
 // The cached launch of pass kind `kind` (0 column, 1 row, 2 row with
 // bulk-copy staging, 3 row in 64-thread CTAs, 4 column in 64-thread CTAs, 5
-// column with TMA tensor staging, 6 row over several blocks) for log2 length lg on the current device,
+// column with TMA tensor staging, 6 row over several blocks, 8 and 9 row that
+// advances the state, wide and in 64-thread CTAs) for log2 length lg on the current device,
 // opted in to `smem` bytes of dynamic shared memory.
 cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
     static Launch cache[kMaxDevices][7][16];
@@ -106,8 +107,9 @@ cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
     if (!l.fn) {
         l = kind == 0 || kind == 4 || kind == 5 ? col_launch_for(lg) : row_launch_for(lg);
         if (kind == 2) l.fn = l.fn_bulk;
-        if (kind == 3 || kind == 4) {
-            l.fn = l.fn_narrow;
+        if (kind == 8) l.fn = l.fn_late;
+        if (kind == 3 || kind == 4 || kind == 9) {
+            l.fn = kind == 9 ? l.fn_late_narrow : l.fn_narrow;
             l.threads = l.per_block_narrow * (l.threads / l.per_block);
             l.per_block = l.per_block_narrow;
         }
@@ -217,7 +219,7 @@ cudaError_t launch_row(const Plan& p, PassArgs a, int batch, cudaStream_t s) {
     // few row blocks in the whole launch: 64-thread CTAs spread them over more SMs
     const bool narrow = p.staging == FOCSS_STAGING_LOADS && (long long)(p.N1 / l.per_block) * rows < sm_count() &&
                         p.N1 % l.per_block_narrow == 0;
-    const int kind = p.staging != FOCSS_STAGING_LOADS ? 2 : narrow ? 3 : 1;
+    const int kind = p.staging != FOCSS_STAGING_LOADS ? 2 : a.late ? (narrow ? 9 : 8) : narrow ? 3 : 1;
     int R = narrow ? l.per_block_narrow : l.per_block;
     const size_t smem = sizeof(float4) * 512 + sizeof(float2) * ((size_t)p.N2 + (size_t)R * Q * (P + 1));
     a.N = p.N;
@@ -255,6 +257,26 @@ cudaError_t launch_pair(const Plan& p, PassArgs a, SsfmState* const (&states)[2]
     a.next = nullptr;
     if (e == cudaSuccess && rows) e = launch_row(p, a, rows, s);
     return e;
+}
+
+// Threads of a row of 2^lg samples.
+static int row_threads(int lg) {
+    const Launch l = row_launch_for(lg);
+    return l.per_block ? l.threads / l.per_block : 1 << lg;
+}
+
+// Whether every CTA of a row pass over `rows` (realizations' modes) runs at once: up to
+// 512 threads per SM at the passes' register counts.
+bool late_state(const Plan& p, int rows) {
+    return p.staging == FOCSS_STAGING_LOADS && (long long)p.N1 * row_threads(p.log2N2) * rows <= 512ll * sm_count();
+}
+cudaError_t launch_pair_adaptive(const Plan& p, PassArgs a, SsfmState* const (&states)[2], long long k, int batch,
+                                 cudaStream_t s) {
+    a.late = late_state(p, batch * (a.modes > 1 ? a.modes : 1));
+    a.state = states[a.late ? k & 1 : 0];
+    cudaError_t e = launch_col(p, a, batch, s);
+    a.next = a.late ? states[(k + 1) & 1] : nullptr;
+    return e == cudaSuccess ? launch_row(p, a, batch, s) : e;
 }
 
 // ---------------------------------------------------------------- SSFM driver
@@ -411,8 +433,7 @@ focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ss
                 // (its last column pass leaves nothing for a row pass)
                 e = launch_pair(*p, a, states, i, f->batch, i + 1 < n ? f->batch : 0, s);
             } else {
-                e = launch_col(*p, a, f->batch, s);
-                if (e == cudaSuccess) e = launch_row(*p, a, f->batch, s);
+                e = launch_pair_adaptive(*p, a, states, i, f->batch, s);
             }
             if (e != cudaSuccess) {
                 if (ev) cudaEventDestroy(ev);
