@@ -53,6 +53,7 @@ SIGNATURES = {
     "focss_ctx_stream": (P, [P]),
     "focss_ctx_last_error": (C.c_char_p, [P]),
     "focss_field_create": (I, [P, C.POINTER(CDomain), I, C.POINTER(P)]),
+    "focss_field_create_output": (I, [P, C.POINTER(CDomain), I, C.POINTER(P)]),
     "focss_field_destroy": (I, [P]),
     "focss_field_domain": (I, [P, C.POINTER(CDomain), C.POINTER(I)]),
     "focss_field_upload": (I, [P, P, SZ]),

@@ -140,15 +140,25 @@ class Field:
     """Device field: `batch` realizations of one Domain (src/focss/field.h:63-181)."""
 
     def __init__(self, domain: Domain, data=None, batch: int = 1, ctx: Context | None = None):
+        self._create(lib().focss_field_create, domain, batch, ctx)
+        if data is not None:
+            self.upload(data)
+
+    def _create(self, create, domain, batch, ctx):
         self.ctx = ctx or Context.default()
         self.domain = domain
         self.batch = batch
         h = C.c_void_p()
         d = CDomain(domain.modes, domain.samples, domain.time_step, domain.center_frequency)
-        check(lib().focss_field_create(self.ctx.h, C.byref(d), batch, C.byref(h)), self.ctx.h)
+        check(create(self.ctx.h, C.byref(d), batch, C.byref(h)), self.ctx.h)
         self.h = h
-        if data is not None:
-            self.upload(data)
+
+    @classmethod
+    def _output(cls, domain: Domain, batch: int = 1, ctx: Context | None = None):
+        """A field whose samples the next call writes, all of them."""
+        f = cls.__new__(cls)
+        f._create(lib().focss_field_create_output, domain, batch, ctx)
+        return f
 
     @property
     def shape(self):
@@ -176,7 +186,7 @@ class Field:
         return out
 
     def copy(self):
-        f = Field(self.domain, batch=self.batch, ctx=self.ctx)
+        f = Field._output(self.domain, self.batch, self.ctx)
         check(lib().focss_field_copy(f.h, self.h), self.ctx.h)
         return f
 

@@ -77,7 +77,7 @@ class CorrectionCNN:
         return p, g
 
     def forward(self, y: Field) -> Field:
-        z = Field(y.domain, batch=y.batch, ctx=self.ctx)
+        z = Field._output(y.domain, y.batch, self.ctx)
         check(lib().focss_cnn_forward(self.h, y.h, z.h), self.ctx.h)
         return z
 

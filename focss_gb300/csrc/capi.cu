@@ -322,7 +322,7 @@ FOCSS_API void* focss_ctx_stream(focss_ctx* c) { return c ? (void*)c->stream : n
 
 FOCSS_API const char* focss_ctx_last_error(const focss_ctx* c) { return c ? c->last_error.c_str() : ""; }
 
-FOCSS_API focss_status focss_field_create(focss_ctx* c, const focss_domain* d, int batch, focss_field** out) {
+static focss_status field_create(focss_ctx* c, const focss_domain* d, int batch, bool clear, focss_field** out) {
     if (!c || !d || !out) return FOCSS_ERR_INVALID_ARG;
     *out = nullptr;
     // src/focss/field.cpp:25 asserts modes > 0, samples > 0, time_step > 0.
@@ -342,7 +342,7 @@ FOCSS_API focss_status focss_field_create(focss_ctx* c, const focss_domain* d, i
     // stream-ordered: the block is usable by work queued on the context's
     // stream after this call (every library call on the field)
     cudaError_t e = cudaMallocFromPoolAsync((void**)&f->d, sizeof(float2) * f->n(), c->pool, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(f->d, 0, sizeof(float2) * f->n(), c->stream);
+    if (e == cudaSuccess && clear) e = cudaMemsetAsync(f->d, 0, sizeof(float2) * f->n(), c->stream);
     if (e != cudaSuccess) {
         if (f->d) cudaFreeAsync(f->d, c->stream);
         delete f;
@@ -351,6 +351,14 @@ FOCSS_API focss_status focss_field_create(focss_ctx* c, const focss_domain* d, i
     c->fields.insert(f);
     *out = f;
     return FOCSS_OK;
+}
+
+FOCSS_API focss_status focss_field_create(focss_ctx* c, const focss_domain* d, int batch, focss_field** out) {
+    return field_create(c, d, batch, true, out);
+}
+
+FOCSS_API focss_status focss_field_create_output(focss_ctx* c, const focss_domain* d, int batch, focss_field** out) {
+    return field_create(c, d, batch, false, out);
 }
 
 FOCSS_API focss_status focss_field_destroy(focss_field* f) {

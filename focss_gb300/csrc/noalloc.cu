@@ -32,7 +32,7 @@ struct NoallocScratch {
     int counters[16];
 };
 
-// ~52 KB of device memory per device, for the lifetime of the process.
+// ~42 KB of device memory per device, for the lifetime of the process.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoallocScratch)];
 
 std::mutex g_noalloc_mutex;

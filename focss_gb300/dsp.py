@@ -24,12 +24,12 @@ def _like(f: Field, samples=None, dt=None, batch=None):
     d = f.domain
     dom = Domain(d.modes, samples if samples is not None else d.samples,
                  dt if dt is not None else d.time_step, d.center_frequency)
-    return Field(dom, batch=f.batch if batch is None else batch, ctx=f.ctx)
+    return Field._output(dom, f.batch if batch is None else batch, f.ctx)
 
 
 def qam16_map(codes, domain: Domain, batch: int = 1, ctx=None) -> Field:
     """Gray 16QAM symbols (modulation.cpp:9-17) for integer codes shaped (batch, modes, samples)."""
-    out = Field(domain, batch=batch, ctx=ctx)
+    out = Field._output(domain, batch, ctx)
     c = np.ascontiguousarray(np.asarray(codes, dtype=np.int32).reshape(out.shape))
     check(lib().focss_qam16_map(out.ctx.h, _vp(c), c.size, out.h), out.ctx.h)
     return out

@@ -124,8 +124,8 @@ class LearnedDBP:
 
     def forward(self, field: Field) -> Field:
         from .api import Domain
-        out = Field(Domain(1, self.samples // 2, field.domain.time_step * 2, field.domain.center_frequency),
-                    batch=self.batch, ctx=self.ctx)
+        out = Field._output(Domain(1, self.samples // 2, field.domain.time_step * 2, field.domain.center_frequency),
+                            self.batch, self.ctx)
         check(lib().focss_ldbp_forward(self.h, field.h, out.h), self.ctx.h)
         return out
 

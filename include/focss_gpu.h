@@ -108,6 +108,10 @@ FOCSS_API int focss_abi_version(void);
 /* a synchronizing free; no other call may use it once the context is gone. */
 FOCSS_API focss_status focss_field_create(focss_ctx* ctx, const focss_domain* domain, int batch,
                                           focss_field** out);
+/* The same with its samples unset, for the output of a call that writes all of
+ * them (one pass over the memory less). */
+FOCSS_API focss_status focss_field_create_output(focss_ctx* ctx, const focss_domain* domain, int batch,
+                                                 focss_field** out);
 /* ~Field (src/focss/field.cpp:130, 543-547) */
 FOCSS_API focss_status focss_field_destroy(focss_field* field);
 /* Field::domain() (src/focss/field.cpp:232-234) plus the batch count. */
@@ -508,7 +512,7 @@ FOCSS_API focss_status focss_cnn_adam_step(focss_cnn* model, double lr, double b
  * `data` is the caller's device buffer of batch*samples complex64
  * (interleaved float pairs), propagated in place on `stream` (a
  * cudaStream_t; NULL = legacy default stream).  The library allocates
- * nothing: step state and twiddle tables live in one fixed 52 KB
+ * nothing: step state and twiddle tables live in one fixed 42 KB
  * __device__ array per device, held until the process exits.
  * Limits: samples a power of two in [2^8, 2^17], batch <= 256; larger shapes
  * return FOCSS_ERR_UNSUPPORTED before any GPU work.  Single-mode fields only.
