@@ -94,14 +94,15 @@ std::mutex g_launch_mutex;
 // The cached launch of pass kind `kind` (0 column, 1 row, 2 row with
 // bulk-copy staging, 3 row in 64-thread CTAs, 4 column in 64-thread CTAs, 5
 // column with TMA tensor staging, 6 row over several blocks, 8 and 9 row that
-// advances the state, wide and in 64-thread CTAs) for log2 length lg on the current device,
-// opted in to `smem` bytes of dynamic shared memory.
+// advances the state, wide and in 64-thread CTAs) for log2 length lg on the
+// current device, opted in to `smem` bytes of dynamic shared memory.
+constexpr int kLaunchKinds = 10;
 cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
-    static Launch cache[kMaxDevices][7][16];
+    static Launch cache[kMaxDevices][kLaunchKinds][16];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= kMaxDevices || lg < 0 || lg >= 16) return cudaErrorInvalidValue;
+    if (dev < 0 || dev >= kMaxDevices || kind < 0 || kind >= kLaunchKinds || lg < 0 || lg >= 16) return cudaErrorInvalidValue;
     std::lock_guard<std::mutex> lock(g_launch_mutex);
     Launch& l = cache[dev][kind][lg];
     if (!l.fn) {
