@@ -883,6 +883,8 @@ FOCSS_API focss_status focss_decimate(focss_ctx* c, const focss_field* in, int f
     const int rows = in->batch * in->modes;
     float2* sp = (float2*)fg::scratch_buffer(c, 2, sizeof(float2) * in->n());
     if (!sp) return fg::set_error(c, FOCSS_ERR_OOM, "decimate scratch");
+    if (fg::decimated_spectrum(c, sp, in->samples, rows, 1.0f / (float)in->samples, in->d, out->d, out->samples, &st))
+        return st == FOCSS_OK ? fg::fft_inverse_transposed(c, out->d, out->samples, rows) : st;
     st = fg::fft_forward_transposed(c, sp, in->samples, rows, 1.0f / (float)in->samples, in->d);
     if (st != FOCSS_OK) return st;
     FG_LAUNCH(fg::decimate_gather_kernel<<<fg::grid_per_realization(out->samples, rows), 256, 0, c->stream>>>(

@@ -125,6 +125,13 @@ struct PassArgs {
     int* fault;             // set to 1 by a kernel whose bounded wait ran out (may be null)
 };
 
+// Where row_kernel_gather stores a decimated spectrum: bins below M/2 and from N - M/2
+// on, in the two-pass layout M1 x M2 of M samples.
+struct GatherArgs {
+    float2* out;
+    int M, log2M1, M2, kc;
+};
+
 struct Plan {
     int N = 0, N1 = 0, N2 = 0, log2N1 = 0, log2N2 = 0;
     void* tw = nullptr;     // device tables (tables_at)
@@ -281,6 +288,11 @@ focss_status spectral_apply(Ctx* ctx, float2* data, int N, int batch, int row_op
 // src: the input, left as it is (null: data, in place)
 focss_status fft_forward_transposed(Ctx* ctx, float2* data, int N, int batch, float scale, const float2* src = nullptr);
 focss_status fft_inverse_transposed(Ctx* ctx, float2* data, int N, int batch);
+// The spectrum's lowest M bins (see decimate_gather_kernel) into the M-point layout;
+// `data` is left with the column pass's output.  false: not in this form (few rows
+// or staged passes), nothing launched.
+bool decimated_spectrum(Ctx* ctx, float2* data, int N, int batch, float scale, const float2* src, float2* out, int M,
+                        focss_status* st);
 
 // ---- dsp.cu
 cudaError_t launch_scale(float2* d, size_t n, float2 s, cudaStream_t st);

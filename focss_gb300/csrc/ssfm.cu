@@ -93,9 +93,10 @@ std::mutex g_launch_mutex;
 
 // The cached launch of pass kind `kind` (0 column, 1 row, 2 row with
 // bulk-copy staging, 3 row in 64-thread CTAs, 4 column in 64-thread CTAs, 5
-// column with TMA tensor staging, 6 row over several blocks, 8 and 9 row that
-// advances the state, wide and in 64-thread CTAs) for log2 length lg on the
-// current device, opted in to `smem` bytes of dynamic shared memory.
+// column with TMA tensor staging, 6 row over several blocks, 7 row of a
+// decimation, 8 and 9 row that advances the state, wide and in 64-thread CTAs)
+// for log2 length lg on the current device, opted in to `smem` bytes of dynamic
+// shared memory.
 constexpr int kLaunchKinds = 10;
 cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
     static Launch cache[kMaxDevices][kLaunchKinds][16];
@@ -117,7 +118,7 @@ cudaError_t cached_launch(int kind, int lg, size_t smem, Launch* out) {
     }
     if (!l.fn) return cudaErrorInvalidValue;
     if (!l.attr_set || smem > l.smem) {
-        const void* fn = kind == 5 ? (const void*)l.fn_tma : kind == 6 ? (const void*)l.fn_loop : (const void*)l.fn;
+        const void* fn = kind == 5 ? (const void*)l.fn_tma : kind == 6 ? (const void*)l.fn_loop : kind == 7 ? (const void*)l.fn_gather : (const void*)l.fn;
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         l.attr_set = true;
@@ -536,6 +537,38 @@ focss_status fft_forward_transposed(Ctx* ctx, float2* data, int N, int batch, fl
     a.op = ROW_FWD;
     a.scale = scale;
     return cuda_check(ctx, launch_row(*p, a, batch, ctx->stream), "fft row");
+}
+
+bool decimated_spectrum(Ctx* ctx, float2* data, int N, int batch, float scale, const float2* src, float2* out, int M,
+                        focss_status* st) {
+    const Plan *p = nullptr, *po = nullptr;
+    *st = get_plan(ctx, N, &p);
+    if (*st == FOCSS_OK) *st = get_plan(ctx, M, &po);
+    if (*st != FOCSS_OK) return true;
+    Launch l = row_launch_for(p->log2N2);
+    const long long blocks = l.per_block ? (long long)(p->N1 / l.per_block) * batch : 0;
+    if (p->staging != FOCSS_STAGING_LOADS || blocks < sm_count() || p->N1 % l.per_block) return false;
+    PassArgs a{};
+    a.data = data;
+    a.op = COL_FWD;
+    a.src_off = src ? src - data : 0;
+    cudaError_t e = launch_col(*p, a, batch, ctx->stream);
+    a.src_off = 0;
+    a.N = p->N;
+    a.N1 = p->N1;
+    a.N2 = p->N2;
+    a.log2N2 = p->log2N2;
+    a.tw = tables_at(p->tw, p->N1);
+    a.kc = col_kc(p->N1);
+    a.scale = scale;
+    const GatherArgs o{out, M, po->log2N1, po->N2, col_kc(po->N1)};
+    const int P = l.threads / l.per_block, Q = p->N2 / P;
+    const size_t smem = sizeof(float4) * 512 + sizeof(float2) * ((size_t)p->N2 + (size_t)l.per_block * Q * (P + 1));
+    if (e == cudaSuccess) e = cached_launch(7, p->log2N2, smem, &l);
+    if (e == cudaSuccess)
+        e = launch_pass(l.fn_gather, dim3(p->N1 / l.per_block, batch), l.threads, smem, ctx->stream, a, o);
+    *st = cuda_check(ctx, e, "decimated spectrum");
+    return true;
 }
 
 focss_status fft_inverse_transposed(Ctx* ctx, float2* data, int N, int batch) {

@@ -763,6 +763,37 @@ __global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row
     pdl_trigger();
 }
 
+// The forward row pass of a decimation: only the kept bins are stored, straight into
+// the shorter transform's layout (the whole spectrum is not written and no gather reads
+// it; receiver of 12 x 2^19 fields with this step 263 -> 251 us).  Launches with fewer row
+// blocks than SMs keep the 64-thread CTAs of the plain pass and the gather.
+template <int N2, int R>
+__global__ void __launch_bounds__(R* PQ<N2>::P, RowShape<N2>::min_blocks(R)) row_kernel_gather(const PassArgs a, const GatherArgs o) {
+    constexpr int P = PQ<N2>::P, Q = PQ<N2>::Q;
+    extern __shared__ float4 smem4[];
+    float2* s_tw = reinterpret_cast<float2*>(smem4 + 512);   // sub-FFT twiddles
+    float2* sx = s_tw + N2;                                  // R * Q * (P+1)
+    pdl_wait();
+    row_tables<N2>(a, false, 1.0f, s_tw, smem4);
+    const int b = blockIdx.y, rl = threadIdx.x / P, t = threadIdx.x % P, k1 = blockIdx.x * R + rl;
+    const float2* row = a.data + (size_t)b * a.N + (size_t)k1 * N2;
+    float2 v[Q];
+    row_load<N2>(v, row, centred<P>(t));
+    __syncthreads();
+    row_core<N2>(a, ROW_FWD, v, k1, rl, t, s_tw, smem4, sx, a.scale, 0ull, 0ull);
+    const int k1c = k1 < a.kc ? k1 : k1 - a.N1;
+    float2* out = o.out + (size_t)b * o.M;
+#pragma unroll
+    for (int j = 0; j < Q; ++j) {
+        const int k = (k1c + a.N1 * row_k2<N2>(t, j)) & (a.N - 1);
+        if (k < o.M / 2 || k >= a.N - o.M / 2) {
+            const int kout = k & (o.M - 1), r1 = kout & ((1 << o.log2M1) - 1);
+            out[r1 * o.M2 + (((kout >> o.log2M1) + (r1 >= o.kc)) & (o.M2 - 1))] = v[j];
+        }
+    }
+    pdl_trigger();
+}
+
 // ---------------------------------------------------------------- row pass, bulk-copy staging
 // The same row pass with its rows moved by the TMA bulk-copy engine
 // (cp.async.bulk): one thread queues the CTA's R rows (N2 x 8 B each,
@@ -1007,6 +1038,7 @@ __global__ void __launch_bounds__(kBlockThreads, BlockShape<N1, N2>::SMEM <= 113
 typedef void (*PassFn)(PassArgs);
 typedef void (*ColTmaFn)(CUtensorMap, PassArgs);
 typedef void (*RowLoopFn)(PassArgs, int);
+typedef void (*RowGatherFn)(PassArgs, GatherArgs);
 template <int N2>
 RowLoopFn row_loop_fn() {
     if constexpr (RowShape<N2>::LOOP > 0)
@@ -1017,6 +1049,7 @@ RowLoopFn row_loop_fn() {
 struct Launch {
     PassFn fn = nullptr;
     PassFn fn_bulk = nullptr;  // row pass with bulk-copy staging
+    RowGatherFn fn_gather = nullptr;  // forward row pass of a decimation
     PassFn fn_late = nullptr, fn_late_narrow = nullptr;  // row passes that advance the state
     PassFn fn_narrow = nullptr;  // the pass in 64-thread CTAs (few blocks in the whole launch)
     RowLoopFn fn_loop = nullptr; // row pass with several row blocks per CTA
@@ -1054,6 +1087,7 @@ Launch row_launch_for(int log2N2);
         l.fn_narrow = row_kernel<L, RowShape<L>::RN>;                          \
         l.fn_loop = row_loop_fn<L>();                                          \
         l.fn_late = row_kernel_late<L, RowShape<L>::R>;                        \
+        l.fn_gather = row_kernel_gather<L, RowShape<L>::R>;                    \
         l.fn_late_narrow = row_kernel_late<L, RowShape<L>::RN>;                \
         l.per_block_narrow = RowShape<L>::RN;                                  \
         l.threads = RowShape<L>::R * PQ<L>::P;                                 \
