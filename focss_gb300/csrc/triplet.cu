@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
 // KB of B, ~44 cycles whatever its N, hence 16 outputs per row of A; forming
 // Q costs another ~660 cycles of it per group and the epilogue ~130, together
 // ~1900 of the ~2300 cycles a group of R = 75 takes.
-// R = 75 (11 389 terms) on 2^20 symbols: 0.69 ms = 141 TFLOP/s of the sum's 8
-// flops per term, where the FP32 kernel took 2.30 ms (42 TFLOP/s, 53 % of the
+// R = 75 (11 389 terms) on 2^20 symbols: 0.636 ms = 150 TFLOP/s of the sum's 8
+// flops per term (0.69 ms without splitting the tiles of the last wave), where the FP32 kernel took 2.30 ms (42 TFLOP/s, 53 % of the
 // FP32 FMA peak); on the way 0.86 ms with 8 outputs per row of A, 0.82 ms
 // with one thread issuing from divergent code, 0.75 ms with one issuing warp.
 constexpr int TC_ROW = 16;                // outputs per row of A
@@ -747,10 +747,22 @@ focss_status run_triplet_rows(Ctx* c, const float2* in, size_t in_bstride, int m
     dim3 grid((samples + tile - 1) / tile, batch);
     const size_t total = (size_t)batch * modes * samples;
     if (tensor) {
-        // fewer tiles than half the SMs: the groups split over CTAs, whose
-        // partial sums a second kernel joins (at least 4 groups each)
-        const long long tiles = (long long)grid.x * batch;
-        a.splits = (int)std::max(1ll, std::min<long long>({sm_count() / std::max(1ll, tiles), (long long)ng / 4, 32}));
+        // The groups of a tile can be split over CTAs, whose partial sums a second
+        // kernel joins (at least 4 groups each): with fewer tiles than SMs to occupy
+        // them, with more to fill the last wave (2^20 symbols are 3.4 waves of
+        // tiles, 6.7 of half tiles: 0.694 -> 0.636 ms).  Counted in tiles' times:
+        // waves of 1/s tile, each with its set-up (~2 %), and the join.
+        const long long tiles = (long long)grid.x * batch, sms = sm_count();
+        double best = 1e300;
+        for (int s = 1; s <= 32 && (s == 1 || s <= (int)ng / 4); ++s) {
+            if (s > 1 && tiles > 16 * sms) break;  // the last wave is a small part
+            if (s > 8 && tiles > sms) break;       // partial sums' memory
+            const double cost = (double)((tiles * s + sms - 1) / sms) * (1.0 / s + 0.02) + (s > 1 ? 0.02 : 0.0);
+            if (cost < best) {
+                best = cost;
+                a.splits = s;
+            }
+        }
         if (a.splits > 1) {
             a.part = (float2*)scratch_buffer(c, 7, sizeof(float2) * total * a.splits);
             if (!a.part) return set_error(c, FOCSS_ERR_OOM, "triplet scratch");

@@ -113,3 +113,16 @@ def test_silent_field_and_term_cache(ctx):
         c = noise(rng, m.size)
         assert rel_l2(apply(ctx, a, 4, m, n, c), reference(a, 4, m, n, c)) < TOL
     assert not np.any(apply(ctx, np.zeros((1, 1, 1100), complex), 4, m, n, c))
+
+
+@pytest.mark.parametrize("tiles", [100, 153, 400])
+def test_splits_of_long_fields(ctx, tiles):
+    """More tiles than SMs (and not), whose last wave splits fill: groups over
+    several CTAs and their join, ragged end, against the reference."""
+    rng = np.random.default_rng(tiles)
+    a = noise(rng, 1, 1, 2048 * tiles - 1971)
+    m, n, _ = sino.diamond_terms(np.ones((41, 41)), 20)
+    keep = rng.permutation(m.size)[:60] if tiles > 200 else slice(None, None, 9)
+    m, n = np.append(m[keep], np.arange(-20, 21)), np.append(n[keep], np.zeros(41, np.int32))
+    c = noise(rng, m.size)
+    assert rel_l2(apply(ctx, a, 40, m, n, c), reference(a, 40, m, n, c)) < TOL
