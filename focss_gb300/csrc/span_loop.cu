@@ -13,7 +13,7 @@
 //     in one branch (record_group): a pass pair of 25 short fields is two
 //     launches instead of 50, and launches are what such a call is bound by;
 //   * ADAPTIVE / LOGARITHMIC spans are a conditional WHILE node whose body is
-//     kChunk pass pairs plus a one-thread check kernel; the check ends the loop
+//     8 or 16 pass pairs (chunk_pairs) plus a one-thread check kernel; the check ends the loop
 //     once the SSFM state machines of all realizations report the span done
 //     (the counter they increment on completion), or after kMaxPairs passes,
 //     so the loop is bounded whatever the data;
@@ -64,18 +64,23 @@ namespace {
 // [2] step cap hit, [3] a realization did not finish, [4] loop iterations
 // over all spans.
 constexpr int kCtr = 8;
-constexpr int kChunk = 8;                // pass pairs per loop-body iteration (even: launch_pair_adaptive)
+// Pass pairs per loop-body iteration (even: launch_pair_adaptive).  A span takes at
+// least length / maximum step size steps; long ones test the condition (~6 us) half
+// as often (one dual-polarization 2^19 span of ~1090 steps 19.83 -> 19.59 ms; 32
+// pairs 19.56), short ones keep the idle passes after their end few.
+inline int chunk_pairs(const focss_fiber& fib, const focss_ssfm_opts& o) {
+    return fib.length >= 64 * o.maximum_step_size ? 16 : 8;
+}
 constexpr long long kMaxPairs = 1ll << 17;
-constexpr int kMaxIter = (int)(kMaxPairs / kChunk);
 constexpr size_t kMaxCachedGraphs = 64;
 
-__global__ void loop_check_kernel(int* ctr, int batch, cudaGraphConditionalHandle h) {
+__global__ void loop_check_kernel(int* ctr, int batch, int max_iter, cudaGraphConditionalHandle h) {
     if (threadIdx.x != 0) return;
     const int it = ++ctr[1];
     ++ctr[4];
     const bool pending = *(volatile int*)&ctr[0] < batch;
-    if (pending && it >= kMaxIter) ctr[2] = 1;
-    cudaGraphSetConditional(h, (pending && it < kMaxIter) ? 1u : 0u);
+    if (pending && it >= max_iter) ctr[2] = 1;
+    cudaGraphSetConditional(h, (pending && it < max_iter) ? 1u : 0u);
 }
 
 __global__ void span_end_kernel(const SsfmState* __restrict__ st, int batch, int adaptive, int* ctr, int* steps) {
@@ -237,16 +242,17 @@ cudaError_t record_branch(Ctx* ctx, LoopGraph* g, int i, Field* f, const Plan& p
             cudaGraph_t body = cp.conditional.phGraph_out[0];
             e = cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
             if (e != cudaSuccess) break;
-            for (int c = 0; c < kChunk && e == cudaSuccess; ++c)
+            const int chunk = chunk_pairs(fib, o);
+            for (int c = 0; c < chunk && e == cudaSuccess; ++c)
                 e = launch_pair_adaptive(p, a, states, c, B, body_stream);
             if (e == cudaSuccess) {
-                loop_check_kernel<<<1, 32, 0, body_stream>>>(ctr, B, h);
+                loop_check_kernel<<<1, 32, 0, body_stream>>>(ctr, B, (int)(kMaxPairs / chunk), h);
                 e = cudaGetLastError();
             }
             cudaGraph_t done = nullptr;
             const cudaError_t e2 = cudaStreamEndCapture(body_stream, &done);
             if (e == cudaSuccess) e = e2;
-            g->body_kernels[i] = 2 * kChunk + 1;
+            g->body_kernels[i] = 2 * chunk + 1;
             if (e != cudaSuccess) break;
         }
         span_end_kernel<<<1, 256, 0, s>>>(states[done], B, o.grid == FOCSS_ADAPTIVE, ctr, steps);
