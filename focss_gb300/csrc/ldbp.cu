@@ -486,7 +486,7 @@ constexpr uint32_t BUF = 4 * XP + 4 * GP;            // one tile's words; two ti
 constexpr size_t SMEM = 2 * (size_t)BUF + 1024;
 constexpr uint32_t D_COLS = 256;
 static_assert(2 * WIN <= XP && 2 * TILE <= GP && XP % 512 == 0 && GP % 512 == 0, "words");
-static_assert(BUF % 512 == 0 && sizeof(float2) * M * RP <= BUF && sizeof(float2) * (2 * TILE + M) <= BUF, "reuse");
+static_assert(BUF % 512 == 0 && sizeof(float2) * M * RP <= BUF && sizeof(float2) * (TILE + WIN) <= BUF, "reuse");
 // kind::f16, FP32 accumulator, FP16 operands, both MN-major
 __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | (1u << 15) | (1u << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -502,26 +502,32 @@ __device__ __forceinline__ void store(unsigned char* p, uint32_t pitch, int e, f
     *reinterpret_cast<__half*>(p + 2 * pitch) = __float2half_rn((re - rf) * 2048.f);
     *reinterpret_cast<__half*>(p + 3 * pitch) = __float2half_rn((im - jf) * 2048.f);
 }
-// One tile in FP32 on plain buffers: the taps of this CTA's 128 window offsets.
+// One tile in FP32 on plain buffers: the same share of the sums as the CTA's
+// product has.  Tap t = off + d takes the sample pairs whose window offset d + r
+// (r = sample mod 32, here the lane) lies in this CTA's 0 .. 127; what a filter of
+// more than 97 taps has beyond is the share of the CTAs next to it, which may
+// find the same tile within the split's range (their windows differ).
 __device__ __noinline__ void tile_fp32(float2* buf, const float2* x, const float2* gy, const float* xi, float2* gh,
                                        float scale, int n0, int off, int T, int N) {
-    float2 *w = buf, *g = buf + TILE + M;
+    float2 *w = buf, *g = buf + WIN;
     const int c = (T - 1) / 2, lane = threadIdx.x & 31;
     __syncthreads();
-    for (int i = threadIdx.x; i < TILE + M; i += THREADS) {
+    for (int i = threadIdx.x; i < WIN; i += THREADS) {
         const float2 v = x[wrap_index(n0 - c + off + i, N)];
         w[i] = xi ? cmul(v, phase_rotation(*xi * cnorm(v))) : v;
     }
     for (int i = threadIdx.x; i < TILE; i += THREADS) g[i] = n0 + i < N ? gy[n0 + i] : make_float2(0.f, 0.f);
     __syncthreads();
-    for (int t = threadIdx.x >> 5; t < M && off + t < T; t += THREADS / 32) {
+    for (int d = (int)(threadIdx.x >> 5) - (W - 1); d < M && off + d < T; d += THREADS / 32) {
+        if (off + d < 0) continue;
         float2 acc = make_float2(0.f, 0.f);
-        for (int i = lane; i < TILE; i += 32) acc = cadd(acc, cmulc(g[i], w[i + t]));
+        if (d + lane >= 0 && d + lane < M)
+            for (int i = lane; i < TILE; i += W) acc = cadd(acc, cmulc(g[i], w[i + d]));
         acc.x = warp_sum(acc.x) * scale;
         acc.y = warp_sum(acc.y) * scale;
         if (lane == 0) {
-            atomicAdd(&gh[off + t].x, acc.x);
-            atomicAdd(&gh[off + t].y, acc.y);
+            atomicAdd(&gh[off + d].x, acc.x);
+            atomicAdd(&gh[off + d].y, acc.y);
         }
     }
     __syncthreads();
