@@ -788,7 +788,6 @@ struct LdbpModel {
     double* loss = nullptr;
     unsigned char* bmat = nullptr;  // Toeplitz matrices of the layers, of the matched filter; the adjoints'
     float* unscale = nullptr;       // their scales
-    bool stale[2] = {true, true};   // parameters changed since they were built: filters, adjoint filters
     size_t field_n() const { return (size_t)batch * samples; }
     float2* h(int k) const { return (float2*)params + (size_t)k * taps; }
     float* xi(int k) const { return params + (size_t)spans * steps * taps * 2 + k; }
@@ -821,15 +820,16 @@ static unsigned char* matrix(const LdbpModel& M, int k, int adjoint) {
     return M.bmat + adjoint * matrices_bytes(M) + k * layer_bytes(M);
 }
 static float* unscale(const LdbpModel& M, int k, int adjoint) { return M.unscale + adjoint * (M.spans * M.steps + 1) + k; }
-static cudaError_t ldbp_matrices(LdbpModel& M, int adjoint) {
-    if (!M.stale[adjoint]) return cudaSuccess;
+// Queued behind every change of the parameters, so that they are current for
+// whatever follows on the stream, in a replayed graph too.
+static cudaError_t ldbp_matrices(const LdbpModel& M) {
     const int L = M.spans * M.steps;
-    fg::firtc::toeplitz_kernel<<<L + 1, 256, 0, M.ctx->stream>>>(M.h(0), M.taps, L, M.hmf(), M.mf_taps, adjoint,
-                                                                (__half*)matrix(M, 0, adjoint), unscale(M, 0, adjoint));
-    count_launch();
-    const cudaError_t e = cudaGetLastError();
-    M.stale[adjoint] = e != cudaSuccess;
-    return e;
+    for (int adjoint = 0; adjoint < 2; ++adjoint) {
+        fg::firtc::toeplitz_kernel<<<L + 1, 256, 0, M.ctx->stream>>>(M.h(0), M.taps, L, M.hmf(), M.mf_taps, adjoint,
+                                                                    (__half*)matrix(M, 0, adjoint), unscale(M, 0, adjoint));
+        count_launch();
+    }
+    return cudaGetLastError();
 }
 
 // layers per launch: the halo a chain computes twice stays below an eighth
@@ -878,7 +878,7 @@ static cudaError_t launch_chain(const LdbpModel& M, fg::ChainArgs& a) {
 static cudaError_t ldbp_chains(LdbpModel& M, const float2* in, bool keep, float2* symbols) {
     const size_t n = M.field_n();
     const int L = M.spans * M.steps;
-    cudaError_t e = ldbp_matrices(M, 0);
+    cudaError_t e = cudaSuccess;
     float2* bufs[2] = {M.work, M.work + n};
     const int F = chain_length(M);
     const float2* src = in;
@@ -940,9 +940,7 @@ static cudaError_t ldbp_backward(LdbpModel& M, const float2* in) {
     const int L = M.spans * M.steps;
     float2* bufs[2] = {M.work, M.work + n};
     fg::TapGrad t{in, M.acts, M.work, n, M.xi(0), M.ghmf(), 1.0f, L, M.steps, M.mf_taps, M.samples, 0, 0};
-    cudaError_t e = ldbp_matrices(M, 1);
-    if (e != cudaSuccess) return e;
-    e = launch_tap_grad(M, t, 1);
+    cudaError_t e = launch_tap_grad(M, t, 1);
     fg::ChainArgs m{};
     m.layers = 1;
     m.T = M.mf_taps;
@@ -1015,6 +1013,7 @@ FOCSS_API focss_status focss_ldbp_create(focss_ctx* c, int spans, int steps_per_
     if (e == cudaSuccess)
         e = cudaMalloc(&m->bmat, 2 * matrices_bytes(*m));
     if (e == cudaSuccess) e = cudaMalloc(&m->unscale, sizeof(float) * 2 * (nl + 1));
+    if (e == cudaSuccess) e = ldbp_matrices(*m);
     if (e != cudaSuccess) {
         cudaFree(m->params);
         cudaFree(m->acts);
@@ -1048,9 +1047,9 @@ FOCSS_API focss_status focss_ldbp_set_params(focss_ldbp* m, const float* host, i
     if (!m || !host || n != m->n_params) return FOCSS_ERR_INVALID_ARG;
     cudaError_t e = cudaMemcpyAsync(m->params, host, sizeof(float) * n, cudaMemcpyHostToDevice, m->ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->m1, 0, sizeof(float) * 2 * n, m->ctx->stream);
+    if (e == cudaSuccess) e = ldbp_matrices(*m);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->ctx->stream);
     m->adam_t = 0;
-    m->stale[0] = m->stale[1] = true;
     return ldbp_err(m->ctx, e, "ldbp set params");
 }
 
@@ -1102,7 +1101,6 @@ FOCSS_API focss_status focss_ldbp_adam_step(focss_ldbp* m, double lr, double lr_
                                             double eps) {
     if (!m) return FOCSS_ERR_INVALID_ARG;
     m->adam_t += 1;
-    m->stale[0] = m->stale[1] = true;
     const float c1 = (float)(1.0 / (1.0 - std::pow(beta1, m->adam_t)));
     const float c2 = (float)(1.0 / (1.0 - std::pow(beta2, m->adam_t)));
     // complex gradients g = dL/dconj(z) -> real gradient 2 g; xi gradients are already real:
@@ -1112,7 +1110,9 @@ FOCSS_API focss_status focss_ldbp_adam_step(focss_ldbp* m, double lr, double lr_
         m->params, m->grads, m->m1, m->m2, m->n_params, (float)lr, (float)beta1, (float)beta2, (float)eps, c1, c2,
         1.f, xi_lo, xi_lo + m->spans * m->steps, (float)lr_gain);
     count_launch();
-    return ldbp_err(m->ctx, cudaGetLastError(), "ldbp adam");
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = ldbp_matrices(*m);
+    return ldbp_err(m->ctx, e, "ldbp adam");
 }
 
 }  // extern "C"
