@@ -41,9 +41,11 @@ __device__ __forceinline__ int wrap_index(int s, int N) {
 // shared memory (split FP16) and registers (FP32).
 //
 // The input of every layer is scaled by the tile's largest sample (precision:
-// fir_tc.cuh).  Tiles whose input spans more
-// than 2^12 in power (largest sample over the mean of the weakest 32-sample
-// run) or holds non-finite samples run the layers in FP32.  20 x 4 steps of
+// fir_tc.cuh).  Tiles in which a layer's input spans more than 2^12 in power
+// (largest sample over the mean of the weakest run: of 32 samples of the chain's
+// input, of a thread's 8 behind that) or holds samples that are not finite or
+// beyond 1e15 run all layers in FP32, so that an overflow stays within the filters' reach.
+// 20 x 4 steps of
 // 63 taps: relative error of the symbols 1.1e-6 (1.4e-6 with plain FP32 filters).
 //
 // What bounds it: per tile and layer ~1040 cycles of shared-memory bandwidth
@@ -76,6 +78,13 @@ __device__ __forceinline__ float2 phase_grad(float2 g, float2 y, float p, float2
     const float kp = k * p;
     gxi = -2.f * p * q.y;
     return make_float2(fmaf(-k, b.y, fmaf(kp, ge.y, ge.x)), fmaf(k, b.x, fmaf(-kp, ge.x, ge.y)));
+}
+
+// Whether powers of largest value `mx` leave the split's range, `mn` the smallest
+// non-zero sum over a run of `run` samples (both as bits).
+__device__ __forceinline__ bool outside_split(unsigned mx, unsigned mn, int run) {
+    const float pmax = __uint_as_float(mx);
+    return pmax > 0.f && (!(pmax > 1e-36f) || pmax > (float)(4096 / run) * __uint_as_float(mn));
 }
 
 // The CTA's owned samples of a layer's output `v(i)`, i = 0 .. owned-1, to dst.
@@ -159,7 +168,8 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
     __shared__ __align__(8) unsigned long long done, bfull[2];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
-    __shared__ unsigned s_in, s_max[kMaxChain], s_min;  // largest |.|^2: input, filter inputs
+    // largest |.|^2 and weakest run: of the chain's input, of the filters' inputs
+    __shared__ unsigned s_in, s_min_in, s_max[kMaxChain], s_min[kMaxChain];
     __shared__ float s_gxi[kMaxChain];
     __shared__ int s_bad;
     const int ks = ksteps(a.T), cap = qcap(ks), c = (a.T - 1) / 2;
@@ -180,10 +190,11 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         abort_flag = 0;
         for (int i = 0; i < kMaxChain; ++i) {
             s_max[i] = 0u;
+            s_min[i] = 0x7F7FFFFFu;
             s_gxi[i] = 0.f;
         }
         s_in = 0u;
-        s_min = 0x7F7FFFFFu;
+        s_min_in = 0x7F7FFFFFu;
         s_bad = 0;
         tcg::mbar_init(&done, 1);
         tcg::mbar_init(&bfull[0], 1);
@@ -239,7 +250,7 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         if (lane == 0) {
             atomicMax(&s_in, __float_as_uint(mx));
             if (!BWD || !a.xi) atomicMax(&s_max[0], __float_as_uint(mx));
-            atomicMin(&s_min, __float_as_uint(mn));
+            atomicMin(&s_min_in, __float_as_uint(mn));
             if (bad) s_bad = 1;
         }
     }
@@ -247,21 +258,24 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
     __syncthreads();
     tcg::fence_after_sync();
     const uint32_t tmem = tmem_base;
-    const float pmax = __uint_as_float(s_in);
     bool ok = true;
-    if (s_bad || (pmax > 0.f && (!(pmax > 1e-36f) || pmax > 128.f * __uint_as_float(s_min)))) {  // 2^12 over a run's mean
-        ok = tcg::mbar_wait(&bfull[0], 0, &abort_flag);  // the copies land before the buffers are reused
-        if (a.layers > 1) ok = tcg::mbar_wait(&bfull[1], 0, &abort_flag) && ok;
-        chain_tile_fp32<BWD>(a, reinterpret_cast<float2*>(sm), b, n0);
-        __syncthreads();
-        if (warp == 0) tcg::tmem_free(tmem, D_COLS);
-        return;
-    }
+    bool plain = s_bad || outside_split(s_in, s_min_in, 32);  // the layers run in FP32
+    // Largest power and a run of 8 (its sum; whether all of it is valid input) of layer l's filter input.
+    auto note_range = [&](int l, float mx, float sum, bool valid) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+        const unsigned n = __reduce_min_sync(0xffffffffu, valid && sum > 0.f ? __float_as_uint(sum) : 0x7F7FFFFFu);
+        const bool bad = __any_sync(0xffffffffu, valid && !(sum <= 1e30f));
+        if (lane == 0) {
+            atomicMax(&s_max[l], m);
+            atomicMin(&s_min[l], n);
+            if (bad) s_bad = 1;
+        }
+    };
     const int o0 = ROW * (32 * (warp & 3) + lane) + OUT * (warp >> 2);  // first output of the thread
     // Backward, before a layer's filter: the gradient through the phase of the
     // thread's 8 samples at tile elements e0 .. (layer l, its y in the staging
     // buffer), with the gain's gradient over the owned samples.
-    auto grad8 = [&](float2 (&g)[8], int e0, int l, float& mx) {
+    auto grad8 = [&](float2 (&g)[8], int e0, int l, float& mx, float& sum) {
         const float k = a.xi[(ptrdiff_t)a.dir * l];
         const int first = (a.layers - l) * c, left = min(a.owned, a.N - n0);
         float2 y[8];
@@ -283,26 +297,29 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         for (int j = 0; j < 8; ++j) {
             const int i = e0 + j - first;
             if (i >= 0 && i < left) acc += d[j];
-            mx = fmaxf(mx, cnorm(g[j]));
+            const float q = cnorm(g[j]);
+            sum += q;
+            mx = fmaxf(mx, q);
         }
         return acc;
     };
-    if (BWD && a.xi) {
+    if (BWD && a.xi && !plain) {
         stage_in(a.act + row, base);
         __syncthreads();
-        float acc = 0.f, mx = 0.f;
+        float acc = 0.f;
 #pragma unroll
         for (int u = 0; u < LOADS; ++u) {
             const int e0 = 8 * (threadIdx.x + THREADS * u);
-            if (e0 < CAP_MAX) acc += grad8(v[u], e0, 0, mx);
+            float mx = 0.f, sum = 0.f;
+            if (e0 < CAP_MAX) acc += grad8(v[u], e0, 0, mx, sum);
+            note_range(0, mx, sum, e0 + 8 <= len);
         }
-        mx = warp_max(mx);
         acc = warp_sum(acc);
-        if (lane == 0) {
-            atomicMax(&s_max[0], __float_as_uint(mx));
-            atomicAdd(&s_gxi[0], acc);
-        }
+        if (lane == 0) atomicAdd(&s_gxi[0], acc);
         __syncthreads();
+        plain = s_bad || outside_split(s_max[0], s_min[0], 8);
+    }
+    if (BWD && a.xi && !plain) {
 #pragma unroll
         for (int u = 0; u < LOADS; ++u) {
             const int e0 = 8 * (threadIdx.x + THREADS * u);
@@ -313,7 +330,7 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         __syncthreads();
         chain_store(a, a.keep, b, n0, false, [&](int i) { return stage[pad(a.layers * c + i)]; });
     }
-    {
+    if (!plain) {
         const float sc = pow2(-split_exponent(s_max[0]));
 #pragma unroll
         for (int u = 0; u < LOADS; ++u) {
@@ -321,7 +338,8 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
             if (e < cap) split_store8(xs, pitch, e, v[u], sc);
         }
     }
-    for (int l = 0; l < a.layers; ++l) {
+    int next = 0;  // the first layer that has not run
+    for (int l = 0; l < a.layers && !plain; ++l) {
         const bool last = l + 1 == a.layers;
         tcg::fence_async_smem();
         tcg::fence_before_sync();
@@ -349,13 +367,13 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         float2 y[OUT];
         read_outputs(tmem, warp, pow2(split_exponent(s_max[l])) * a.unscale[(ptrdiff_t)a.dir * l] * a.gain[l], y);
         const int first = (a.layers - 1 - l) * c;  // first owned output
-        float mx = 0.f;
+        float mx = 0.f, sum = 0.f;  // powers of the next filter's input
         if (BWD) {
             if (!last) {
 #pragma unroll
                 for (int u = 0; u < TILE / THREADS; ++u) stage[pad(threadIdx.x + THREADS * u)] = ny[u];
                 __syncthreads();
-                const float acc = warp_sum(grad8(y, o0, l + 1, mx));
+                const float acc = warp_sum(grad8(y, o0, l + 1, mx, sum));
                 if (lane == 0) atomicAdd(&s_gxi[l + 1], acc);
                 __syncthreads();
             }
@@ -372,6 +390,7 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
 #pragma unroll
             for (int r = 0; r < OUT; ++r) {
                 pw[r] = cnorm(y[r]);
+                sum += pw[r];
                 mx = fmaxf(mx, pw[r]);
             }
             if (a.xi) {
@@ -385,10 +404,7 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
                 }
             }
         }
-        if (!last) {
-            mx = warp_max(mx);
-            if (lane == 0) atomicMax(&s_max[l + 1], __float_as_uint(mx));
-        }
+        if (!last) note_range(l + 1, mx, sum, o0 + OUT <= a.owned + first * 2);
         if (last || BWD) {
             // staged: the result, or backward the gradient behind the next phase
             if (a.keep && !BWD) __syncthreads();
@@ -411,7 +427,21 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
                     *reinterpret_cast<uint4*>(xs + q * pitch + swz32(16u * e)) = make_uint4(0u, 0u, 0u, 0u);
             }
         __syncthreads();
-        split_store8(xs, pitch, o0, y, pow2(-split_exponent(s_max[l + 1])));
+        next = l + 1;
+        plain = s_bad || outside_split(s_max[next], s_min[next], 8);
+        if (!plain) split_store8(xs, pitch, o0, y, pow2(-split_exponent(s_max[next])));
+    }
+    if (plain) {
+        // the matrices on their way land before their buffers are reused
+        for (int k = next; k < min(next + 2, a.layers); ++k) ok = tcg::mbar_wait(&bfull[k & 1], (k >> 1) & 1, &abort_flag) && ok;
+        tcg::fence_before_sync();
+        ok = !__syncthreads_or(!ok);
+        tcg::fence_after_sync();
+        if (ok) {
+            chain_tile_fp32<BWD>(a, reinterpret_cast<float2*>(sm), b, n0);
+            if (warp == 0) tcg::tmem_free(tmem, D_COLS);
+            return;
+        }
     }
     if (!ok) {
         // a wait ran out: the copies and MMAs in flight land (bounded) before
