@@ -765,7 +765,7 @@ focss_status run_triplet_rows(Ctx* c, const float2* in, size_t in_bstride, int m
         }
         if (a.splits > 1) {
             a.part = (float2*)scratch_buffer(c, 7, sizeof(float2) * total * a.splits);
-            if (!a.part) return set_error(c, FOCSS_ERR_OOM, "triplet scratch");
+            if (!a.part) a.splits = 1;  // no memory for partial sums: unsplit needs none
             grid.z = a.splits;
         }
     }
