@@ -217,6 +217,11 @@ constexpr size_t kResultCap = 256 << 10;  // codes beyond this go through device
 void* result_buffer(Ctx* ctx, size_t bytes);
 unsigned* tickets(Ctx* ctx, size_t n);
 void* scratch_buffer(Ctx* ctx, int slot, size_t bytes);
+// Whether a caller is capturing the stream into a graph.
+inline bool stream_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone;
+}
 
 // ---- ssfm.cu
 bool fft_size_supported(int N);

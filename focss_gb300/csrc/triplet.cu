@@ -667,12 +667,23 @@ focss_status term_plan(Ctx* c, int n_terms, const int32_t* m, const int32_t* n, 
     if (e != cudaSuccess) return cuda_check(c, e, "triplet tables");
     e = cudaMemcpy(p.dev, host.data(), host.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !t.grp.empty()) {
+        // While the context's stream is captured, on a stream of its own: the
+        // entry serves calls made before the graph runs, too.
         char* d = (char*)p.dev;
-        toeplitz_kernel<<<p.ng, 256, 0, c->stream>>>((const float2*)(d + p.coef_offset), (const int*)d + 2 * (size_t)p.ng,
-                                                     (const int4*)(d + p.grp_offset), (const int*)(d + p.len_offset),
-                                                     1.f / p.unscale, (__half*)(d + p.bmat_offset));
-        count_launch();
-        e = cudaGetLastError();
+        const bool aside = stream_capturing(c->stream);
+        cudaStream_t s = c->stream;
+        if (aside) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+        if (e == cudaSuccess) {
+            toeplitz_kernel<<<p.ng, 256, 0, s>>>((const float2*)(d + p.coef_offset), (const int*)d + 2 * (size_t)p.ng,
+                                                 (const int4*)(d + p.grp_offset), (const int*)(d + p.len_offset),
+                                                 1.f / p.unscale, (__half*)(d + p.bmat_offset));
+            count_launch();
+            e = cudaGetLastError();
+            if (aside) {
+                if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+                cudaStreamDestroy(s);
+            }
+        }
     }
     if (e != cudaSuccess) {
         cudaFree(p.dev);
@@ -746,7 +757,7 @@ focss_status run_triplet_rows(Ctx* c, const float2* in, size_t in_bstride, int m
     const int tile = tensor ? TC_K : TK;
     dim3 grid((samples + tile - 1) / tile, batch);
     const size_t total = (size_t)batch * modes * samples;
-    if (tensor) {
+    if (tensor && !stream_capturing(c->stream)) {  // (a graph would hold scratch that a larger call replaces)
         // The groups of a tile can be split over CTAs, whose partial sums a second
         // kernel joins (at least 4 groups each): with fewer tiles than SMs to occupy
         // them, with more to fill the last wave (2^20 symbols are 3.4 waves of
