@@ -951,16 +951,18 @@ FOCSS_API focss_status focss_rrc_shaping(focss_ctx* c, const focss_field* symbol
         if (st == FOCSS_OK) st = fg::rrc_table(c, out->samples, n, osf, roll_off, &H);
         if (st != FOCSS_OK) return st;
         const int rows = symbols->batch * symbols->modes;
-        float2* sp = (float2*)fg::scratch_buffer(c, 2, sizeof(float2) * symbols->n());
-        if (!sp) return fg::set_error(c, FOCSS_ERR_OOM, "rrc_shaping scratch");
-        const double N = out->samples;
-        st = fg::fft_forward_transposed(c, sp, n, rows, 1.0f, symbols->d);
-        if (st != FOCSS_OK) return st;
-        FG_LAUNCH(fg::repeat_filter_kernel<<<fg::grid_per_realization(out->samples, rows), 256, 0, c->stream>>>(
-            sp, H, out->d, (float)(std::sqrt(gain) * osf / (N * N)), n, pi->log2N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1,
-            po->log2N2, fg::col_kc(po->N1)));
-        st = fg::cuda_check(c, cudaGetLastError(), "rrc_shaping spectrum");
-        return st == FOCSS_OK ? fg::fft_inverse_transposed(c, out->d, out->samples, rows) : st;
+        // (a graph would hold scratch that a larger call replaces; the way below needs none)
+        float2* sp = fg::stream_capturing(c->stream) ? nullptr : (float2*)fg::scratch_buffer(c, 2, sizeof(float2) * symbols->n());
+        if (sp) {
+            const double N = out->samples;
+            st = fg::fft_forward_transposed(c, sp, n, rows, 1.0f, symbols->d);
+            if (st != FOCSS_OK) return st;
+            FG_LAUNCH(fg::repeat_filter_kernel<<<fg::grid_per_realization(out->samples, rows), 256, 0, c->stream>>>(
+                sp, H, out->d, (float)(std::sqrt(gain) * osf / (N * N)), n, pi->log2N1, pi->N2, fg::col_kc(pi->N1), po->N, po->N1,
+                po->log2N2, fg::col_kc(po->N1)));
+            st = fg::cuda_check(c, cudaGetLastError(), "rrc_shaping spectrum");
+            return st == FOCSS_OK ? fg::fft_inverse_transposed(c, out->d, out->samples, rows) : st;
+        }
     }
     st = focss_upsample(c, symbols, osf, out);
     if (st != FOCSS_OK) return st;

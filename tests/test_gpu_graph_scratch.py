@@ -2,7 +2,7 @@
 that a later, larger call may replace, and leave no half-made tables behind:
 replays and eager calls around them stay right.
 
-References as in test_gpu_triplet_tiles.py.
+References as in test_gpu_triplet_tiles.py and test_gpu_spectral_paths.py.
 """
 import ctypes as C
 
@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import focss_gb300 as fg
-from focss_gb300 import sino
+from focss_gb300 import dsp, sino
 from focss_gb300._lib import check, lib
 from conftest import rel_l2
 from test_gpu_ldbp_graphs import captured
@@ -45,3 +45,17 @@ def test_triplet_sum(first_seen):
     f.upload(b)
     replay()
     assert rel_l2(out.numpy(), reference(b, 12, m, n, c)) < TOL
+
+
+def test_pulse_shaping():
+    ctx = fg.Context()
+    rng = np.random.default_rng(3)
+    s, t = noise(rng, 2, 1, 512), noise(rng, 2, 1, 512)
+    f = field(ctx, s)
+    want = dsp.rrc_shaping(field(ctx, t), 4, 0.1).numpy()
+    out = dsp.rrc_shaping(f, 4, 0.1)
+    replay = captured(ctx, lambda: check(lib().focss_rrc_shaping(ctx.h, f.h, 4, 0.1, 1.0, out.h), ctx.h))
+    dsp.rrc_shaping(field(ctx, noise(rng, 4, 1, 1 << 16)), 4, 0.1)
+    f.upload(t)
+    replay()
+    assert rel_l2(out.numpy(), want) < 1e-6
