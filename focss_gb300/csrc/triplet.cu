@@ -59,7 +59,7 @@ struct TripletArgs {
     int a_lo, alen;         // the tile reads samples k0 + a_lo + [0, alen)
     int qcap;               // elements of a Q array, a multiple of 8
     int bslot;              // bytes of a Toeplitz buffer
-    float coef_unscale;     // 1 / (power-of-two scale of the matrices)
+    int coef_exp;           // the matrices hold the coefficients times 2^-coef_exp
     float2* part;           // splits > 1: partial sums, splits x batch x modes x N
     int splits;
 };
@@ -187,14 +187,16 @@ __global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
 // the (swizzled) array Q itself is the operand and a step of 16 taps is an
 // address offset.
 //
-// Precision.  Q and C are scaled by powers of two to at most 1 and split into
-// FP16 pairs hi + lo 2^-11 (22 bits, absolute error below 2^-36), and the
+// Precision.  Q and C are scaled by powers of two to just below 2^15 and split
+// into FP16 pairs hi + lo 2^-11 (22 bits down to 2^-28 of the largest, below
+// that an absolute error of 2^-51 of it), and the
 // products hi hi, hi lo, lo hi accumulate in FP32, the last two in columns of
 // their own that join with the factor 2^-11 at the end; lo lo (2^-22 of a
 // product at most) is left out.  The sum over m is compensated (Kahan).  The
 // scale of Q is the tile's largest power; tiles whose power spans more than
 // 2^12 between its largest sample and the mean of its weakest 32-sample run,
-// or with non-finite values, take the FP32 sum.  Relative error against 64
+// or with non-finite values, take the FP32 sum, and so do lists whose
+// coefficients span more than 2^28 (plan_tensor).  Relative error against 64
 // bits at R = 75 on 2^20 symbols: 1.9e-7 .. 2.3e-7 (the FP32 sum 2.7e-7 ..
 // 4.2e-7 on the same inputs).
 //
@@ -217,6 +219,7 @@ constexpr int kEpiWarps = 8, kProdWarps = 6;
 constexpr int kPairs = 2 * 32 * kProdWarps, kBatch = 3;
 constexpr int kMaxKSteps = 14;            // taps per group: 16 * kMaxKSteps - 15
 constexpr int kMaxTcGroups = 512;
+constexpr int kHeadroom = 15;             // both factors' FP16 words reach up to 2^15
 constexpr uint32_t kDCols = 128;          // FP32 columns: (Re Q | Im Q) x (hi hi | mixed) x C re/im x 16 r
 constexpr uint32_t kStepBytes = 2048;     // B bytes per 16 taps: 2 x 64 rows x 16 bytes
 // kind::f16, FP32 accumulator (bits 4-5 = 1), FP16 operands, both K-major
@@ -299,8 +302,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) triplet_tc_kernel(const Triplet
                 triplet_tile_fp32<MODES>(a, reinterpret_cast<float2*>(sm), k, g0, g1);
         return;
     }
-    // |Q| <= pmax < 2^e: scale by 2^-e
-    const int e = pmax > 0.f ? (int)((__float_as_uint(pmax) >> 23) & 255u) - 126 : 0;
+    // |Q| <= pmax < 2^e: scale to below 2^kHeadroom
+    const int e = (pmax > 0.f ? (int)((__float_as_uint(pmax) >> 23) & 255u) - 126 : 0) - kHeadroom;
     const float qscale = __uint_as_float((unsigned)(127 - e) << 23);
     if (warp == 14) tcg::tmem_alloc(&tmem_base, kSt * kDCols);
     tcg::fence_before_sync();
@@ -481,12 +484,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) triplet_tc_kernel(const Triplet
         __syncthreads();
     }
     if (warp < 8) {
-        const float un = ok ? a.coef_unscale : __int_as_float(0x7fc00000);
-        const float uq = __uint_as_float((unsigned)(127 + e) << 23);
+        // both scales back, in two halves: no product leaves the range unless the
+        // sums or the outputs do
+        const int back = e + a.coef_exp, half = back / 2;
+        const float f0 = __uint_as_float((unsigned)(127 + half) << 23);
+        const float f1 = ok ? __uint_as_float((unsigned)(127 + back - half) << 23) : __int_as_float(0x7fc00000);
 #pragma unroll
         for (int p = 0; p < MODES; ++p)
 #pragma unroll
-            for (int r = 0; r < TT; ++r) write_output(a, b, MODES, p, k0 + kl + r, cscale(cscale(cadd(acc[p][r], low[p][r]), uq), un));
+            for (int r = 0; r < TT; ++r) write_output(a, b, MODES, p, k0 + kl + r, cscale(cscale(cadd(acc[p][r], low[p][r]), f0), f1));
     }
     tcg::fence_before_sync();
     __syncthreads();
@@ -502,7 +508,7 @@ struct Terms {
     std::vector<int4> grp;
     size_t bmat_bytes = 0;
     int a_lo = 0, a_hi = 0, ksteps = 0;
-    float unscale = 1.f;
+    int exp = 0;
 };
 
 // Toeplitz matrices of the groups in B's shared-memory layout, FP16: each
@@ -524,20 +530,23 @@ __global__ void toeplitz_kernel(const float2* __restrict__ coef, const int* __re
 }
 
 // Groups of the tensor-core sum.  Left empty when a run has
-// more than 16 kMaxKSteps - 15 taps, there are more than kMaxTcGroups groups
-// or the coefficients' magnitude leaves [2^-100, 2^100].
+// more than 16 kMaxKSteps - 15 taps, there are more than kMaxTcGroups groups,
+// the coefficients' magnitude leaves [2^-100, 2^100] or they span more than
+// 2^28 (zeros aside): the smallest would keep fewer than 22 bits, and where the
+// large ones have no part in a symbol they alone make it up.
 void plan_tensor(Terms& t) {
-    float cmax = 0.f;
+    float cmax = 0.f, cmin = INFINITY;
     for (const float2& c : t.coef) {
         if (!std::isfinite(c.x) || !std::isfinite(c.y)) return;
-        cmax = std::max({cmax, std::fabs(c.x), std::fabs(c.y)});
+        const float mag = std::max(std::fabs(c.x), std::fabs(c.y));
+        cmax = std::max(cmax, mag);
+        if (mag > 0.f) cmin = std::min(cmin, mag);
     }
-    if (!(cmax > 0x1p-100f && cmax < 0x1p100f) || (int)t.gm.size() > kMaxTcGroups) return;
+    if (!(cmax > 0x1p-100f && cmax < 0x1p100f) || cmin < 0x1p-28f * cmax || (int)t.gm.size() > kMaxTcGroups) return;
     for (int l : t.len)
         if (l + 15 > 16 * kMaxKSteps) return;
-    int ex = 0;
-    std::frexp(cmax, &ex);
-    t.unscale = std::ldexp(1.f, ex);
+    std::frexp(cmax, &t.exp);
+    t.exp -= kHeadroom;
     t.a_lo = 0;
     t.a_hi = TC_K;
     for (size_t g = 0; g < t.gm.size(); ++g) {
@@ -596,8 +605,7 @@ struct TermEntry {
     std::vector<int32_t> m, n;
     std::vector<double> coef;
     void* dev = nullptr;
-    int ng = 0, halo_q = 0, halo_a = 0, a_lo = 0, alen = 0, ksteps = 0;
-    float unscale = 1.f;
+    int ng = 0, halo_q = 0, halo_a = 0, a_lo = 0, alen = 0, ksteps = 0, exp = 0;
     size_t coef_offset = 0, grp_offset = 0, len_offset = 0, bmat_offset = 0;
 };
 struct TermCache {
@@ -641,7 +649,7 @@ focss_status term_plan(Ctx* c, int n_terms, const int32_t* m, const int32_t* n, 
     p.a_lo = t.a_lo;
     p.alen = t.a_hi - t.a_lo;
     p.ksteps = t.ksteps;
-    p.unscale = t.unscale;
+    p.exp = t.exp;
     auto up16 = [](size_t v) { return (v + 15) / 16 * 16; };
     p.coef_offset = up16(sizeof(int) * (3 * (size_t)p.ng + 1));
     p.grp_offset = up16(p.coef_offset + sizeof(float2) * t.coef.size());
@@ -676,7 +684,7 @@ focss_status term_plan(Ctx* c, int n_terms, const int32_t* m, const int32_t* n, 
         if (e == cudaSuccess) {
             toeplitz_kernel<<<p.ng, 256, 0, s>>>((const float2*)(d + p.coef_offset), (const int*)d + 2 * (size_t)p.ng,
                                                  (const int4*)(d + p.grp_offset), (const int*)(d + p.len_offset),
-                                                 1.f / p.unscale, (__half*)(d + p.bmat_offset));
+                                                 std::ldexp(1.f, -p.exp), (__half*)(d + p.bmat_offset));
             count_launch();
             e = cudaGetLastError();
             if (aside) {
@@ -748,7 +756,7 @@ focss_status run_triplet_rows(Ctx* c, const float2* in, size_t in_bstride, int m
         a.a_lo = t->a_lo;
         a.alen = t->alen;
         a.qcap = (16 * t->ksteps + TC_K - 16 + 127) / 128 * 128;
-        a.coef_unscale = t->unscale;
+        a.coef_exp = t->exp;
         const size_t need = 1024 + (size_t)kSt * (8 * (size_t)a.qcap + a.bslot) + sizeof(int4) * ng +
                             sizeof(float2) * (size_t)modes * (a.alen + a.alen / 16 + 2);
         tensor = need <= 220 * 1024;
