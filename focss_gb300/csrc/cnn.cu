@@ -369,8 +369,10 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
 // (64 channels) LBO leads to a block of ones, whose product is the bias gradient
 // (16 channels: a third MMA).
 //
-// A CTA takes an even share of the tiles of all realizations, accumulates them in
-// tensor memory and adds the result to gW once.  Warp 0 loads tiles with TMA
+// A CTA (one per SM) takes an even share of the tiles of all realizations,
+// accumulates them in tensor memory and adds the result to gW, in sections of at most
+// SECTION tiles: the accumulator truncates, and on sums of one sign (BF16 factors)
+// loses 3e-7 to 7e-7 over 16 tiles, 1.2e-6 to 2.1e-6 over 32.  Warp 0 loads tiles with TMA
 // (zero-filled outside [0, L)) into a ring of WSTAGES buffers (mbarriers full /
 // empty); warps 1 and 2 issue a share of each tile's MMAs each and commit them to
 // the tile's `empty` barrier (issue from one warp takes ~70 cycles an MMA).  Every
@@ -385,6 +387,7 @@ constexpr int P = 128;                // positions per tile
 constexpr int PR = P + 2 * HALF;      // input rows per tile (halo)
 constexpr int M = 128;
 constexpr int WSTAGES = 4;            // tiles in flight per CTA
+constexpr int SECTION = 16;           // tiles per sum in tensor memory
 constexpr uint32_t ONES = 2048;       // bytes of ones
 template <int COUT, int CIN>
 struct Shape {
@@ -448,78 +451,84 @@ __global__ void __launch_bounds__(128) conv_wgrad_tc_kernel(const __grid_constan
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tmem_base;
+    const int sections = (n + tcw::SECTION - 1) / tcw::SECTION;
     int issued = 0;
-    if (warp == 0 && lane == 0) {
-        // tile t -> stage t % ST: g rows p0 .., input rows p0 - 4 ..
-        for (int t = 0; t < n; ++t) {
-            const int s = t % ST, b = (first + t) / ntiles, p0 = (first + t - b * ntiles) * tcw::P;
-            if (t >= ST && !tc::mbar_wait(&empty[s], ((t / ST) & 1) ^ 1, &abort_flag)) break;
-            const uint32_t gs = base + (uint32_t)s * S::STAGE;
-            tc::mbar_expect_tx(&full[s], S::SMEM_G + S::SMEM_I);
-            tc::tma_load_3d(gs, &gmap, 0, p0, b, &full[s]);
-            tc::tma_load_3d(gs + S::SMEM_G, &imap, 0, p0 - HALF, b, &full[s]);
-            issued = t + 1;
-        }
-    } else if (warp == 1 || warp == 2) {
-        // accumulators j0 .. j1 - 1 of every tile
-        constexpr int HALF_ACC = (S::NACC + (S::ONES_MMA ? 0 : 1)) / 2;
-        const int j0 = warp == 1 ? 0 : HALF_ACC, j1 = warp == 1 ? HALF_ACC : S::NACC;
-        for (int t = 0; t < n; ++t) {
-            const int s = t % ST;
-            if (!tc::mbar_wait_warp(&full[s], (t / ST) & 1, &abort_flag)) break;
-            tc::fence_after_sync();
-            const uint32_t gs = base + (uint32_t)s * S::STAGE, is = gs + S::SMEM_G;
-            for (int j = j0; j < j1; ++j) {
-                const uint32_t d = tmem + (uint32_t)(COUT * j);
-#pragma unroll
-                for (int ks = 0; ks < tcw::P / 16; ++ks) {
-                    const uint32_t a0 = is + (uint32_t)(j * S::AT + 16 * ks) * S::ROW_I;
-                    uint64_t a = tcw::desc<S::ROW_I>(a0, S::ROW_I);
-                    if (S::ONES_MMA ? j == S::NM : false) a = tcw::desc<S::ROW_I>(ones, S::ROW_I);
-                    if (!S::ONES_MMA && j == S::NM - 1) a = tcw::desc<S::ROW_I>(a0, ones - a0);
-                    tc::mma_f16_warp(d, a, tcw::desc<S::ROW_G>(gs + 16 * ks * S::ROW_G, 16), S::IDESC, (t | ks) != 0);
-                }
+    bool ok = true;
+    for (int sec = 0; sec < sections && ok; ++sec) {
+        const int t0 = (int)((long long)n * sec / sections), t1 = (int)((long long)n * (sec + 1) / sections);
+        if (warp == 0 && lane == 0) {
+            // tile t -> stage t % ST: g rows p0 .., input rows p0 - 4 ..; the next
+            // section's first tiles load while this one's sums are added
+            for (int t = issued; t < min(n, t1 + ST); ++t) {
+                const int s = t % ST, b = (first + t) / ntiles, p0 = (first + t - b * ntiles) * tcw::P;
+                if (t >= ST && !tc::mbar_wait(&empty[s], ((t / ST) & 1) ^ 1, &abort_flag)) break;
+                const uint32_t gs = base + (uint32_t)s * S::STAGE;
+                tc::mbar_expect_tx(&full[s], S::SMEM_G + S::SMEM_I);
+                tc::tma_load_3d(gs, &gmap, 0, p0, b, &full[s]);
+                tc::tma_load_3d(gs + S::SMEM_G, &imap, 0, p0 - HALF, b, &full[s]);
+                issued = t + 1;
             }
-            tc::mma_commit_warp(&empty[s]);  // the stage is free once both warps' MMAs have read it
-            if (t == n - 1) tc::mma_commit_warp(&done);
-        }
-    }
-    __syncthreads();
-    bool ok = !abort_flag && (n == 0 || tc::mbar_wait(&done, 0, &abort_flag));
-    ok = !__syncthreads_or(!ok);
-    if (!ok) {
-        // drain: the queued copies and the issued MMAs complete (bounded) before the CTA leaves
-        if (warp == 0 && lane == 0)
-            for (int t = issued > ST ? issued - ST : 0; t < issued; ++t) tc::mbar_wait(&full[t % ST], (t / ST) & 1, nullptr);
-        if (warp == 1 || warp == 2) {
-            tc::mma_commit_warp(&drain);
-            tc::mbar_wait_warp(&drain, 0, nullptr);
+        } else if (warp == 1 || warp == 2) {
+            // accumulators j0 .. j1 - 1 of every tile
+            constexpr int HALF_ACC = (S::NACC + (S::ONES_MMA ? 0 : 1)) / 2;
+            const int j0 = warp == 1 ? 0 : HALF_ACC, j1 = warp == 1 ? HALF_ACC : S::NACC;
+            for (int t = t0; t < t1; ++t) {
+                const int s = t % ST;
+                if (!tc::mbar_wait_warp(&full[s], (t / ST) & 1, &abort_flag)) break;
+                tc::fence_after_sync();
+                const uint32_t gs = base + (uint32_t)s * S::STAGE, is = gs + S::SMEM_G;
+                for (int j = j0; j < j1; ++j) {
+                    const uint32_t d = tmem + (uint32_t)(COUT * j);
+#pragma unroll
+                    for (int ks = 0; ks < tcw::P / 16; ++ks) {
+                        const uint32_t a0 = is + (uint32_t)(j * S::AT + 16 * ks) * S::ROW_I;
+                        uint64_t a = tcw::desc<S::ROW_I>(a0, S::ROW_I);
+                        if (S::ONES_MMA ? j == S::NM : false) a = tcw::desc<S::ROW_I>(ones, S::ROW_I);
+                        if (!S::ONES_MMA && j == S::NM - 1) a = tcw::desc<S::ROW_I>(a0, ones - a0);
+                        tc::mma_f16_warp(d, a, tcw::desc<S::ROW_G>(gs + 16 * ks * S::ROW_G, 16), S::IDESC, t != t0 || ks != 0);
+                    }
+                }
+                tc::mma_commit_warp(&empty[s]);  // the stage is free once both warps' MMAs have read it
+                if (t == t1 - 1) tc::mma_commit_warp(&done);
+            }
         }
         __syncthreads();
-    }
-    tc::fence_after_sync();
-    // lane 32 w + lane holds row m of each accumulator: tap m / CIN of its taps,
-    // input channel m % CIN
-    if (n > 0) {
+        ok = !abort_flag && tc::mbar_wait(&done, sec & 1, &abort_flag);
+        ok = !__syncthreads_or(!ok);
+        if (!ok) {
+            // drain: the queued copies and the issued MMAs complete (bounded) before the CTA leaves
+            if (warp == 0 && lane == 0)
+                for (int t = issued > ST ? issued - ST : 0; t < issued; ++t) tc::mbar_wait(&full[t % ST], (t / ST) & 1, nullptr);
+            if (warp == 1 || warp == 2) {
+                tc::mma_commit_warp(&drain);
+                tc::mbar_wait_warp(&drain, 0, nullptr);
+            }
+            __syncthreads();
+        }
+        tc::fence_after_sync();
+        // lane 32 w + lane holds row m of each accumulator: tap m / CIN of its taps,
+        // input channel m % CIN.  The CTAs, which get here together, start at different
+        // columns.
         const int m = 32 * warp + lane;
-        for (int j = 0; j < S::NACC; ++j) {
+        constexpr int CHUNKS = COUT / 16, ALL = S::NACC * CHUNKS;
+        for (int u = 0; u < ALL; ++u) {
+            const int x = (u + (int)blockIdx.x) % ALL, j = x / CHUNKS, q = 16 * (x % CHUNKS);
             const int tap = j * S::AT + m / CIN;
             const bool bias = S::ONES_MMA ? j == S::NM && m == 0 : j == S::NM - 1 && m == CIN;
-            const bool weight = j < S::NM && tap < KW;
+            uint32_t v[16];
+            tc::ld_x16_async(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(COUT * j + q), v);
+            tc::wait_ld(v);
+            if (bias || (j < S::NM && tap < KW)) {
+                float* dst = bias ? gb + q : gW + ((size_t)q * KW + tap) * CIN + m % CIN;
+                const size_t pitch = bias ? 1 : (size_t)KW * CIN;
 #pragma unroll
-            for (int q = 0; q < COUT; q += 16) {
-                uint32_t v[16];
-                tc::ld_x16_async(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(COUT * j + q), v);
-                tc::wait_ld(v);
-                if (weight || bias) {
-#pragma unroll
-                    for (int e = 0; e < 16; ++e)
-                        atomicAdd(weight ? gW + ((size_t)(q + e) * KW + tap) * CIN + m % CIN : gb + q + e,
-                                  __uint_as_float(ok ? v[e] : 0x7fc00000u));
-                }
-                __syncwarp();
+                for (int e = 0; e < 16; ++e) atomicAdd(dst + e * pitch, __uint_as_float(ok ? v[e] : 0x7fc00000u));
             }
+            __syncwarp();
         }
+        tc::fence_before_sync();
+        __syncthreads();  // the accumulators are read
+        tc::fence_after_sync();
     }
     pdl_trigger();
     tc::fence_before_sync();
@@ -704,10 +713,8 @@ cudaError_t conv_wgrad(const bf16* g, const bf16* in, float* gW, float* gb, int 
     e = position_map(&gmap, g, COUT, L, B, tcw::P);
     if (e == cudaSuccess) e = position_map(&imap, in, CIN, L, B, tcw::PR);
     if (e != cudaSuccess) return e;
-    // one CTA per SM, and as many waves as keep a CTA's sums at 32 tiles or less
     const long long tiles = (long long)((L + tcw::P - 1) / tcw::P) * B;
-    const long long waves = (tiles + 32ll * sm_count() - 1) / (32ll * sm_count());
-    const int grid = (int)std::min<long long>(tiles, waves * sm_count());
+    const int grid = (int)std::min<long long>(tiles, sm_count());
     return launch_serialized(conv_wgrad_tc_kernel<CIN, COUT>, grid, 128, S::SMEM, s, gmap, imap, gW, gb, L, B);
 }
 
