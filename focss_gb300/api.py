@@ -195,6 +195,8 @@ class Field:
         return self
 
     def device_ptr(self):
+        """Address of the samples, ordered on the context's stream: synchronize
+        the context (ctx.sync()) before using it from another stream."""
         return lib().focss_field_device_ptr(self.h)
 
     def copy_realizations(self, dst_first: int, src: "Field", src_first: int, count: int):

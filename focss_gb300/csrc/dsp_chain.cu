@@ -236,8 +236,8 @@ __global__ void freq_shift_kernel(const float2* d, float2* out, int samples, siz
 }
 
 // wdm_mux: out[m,s] = sum_c ch_c[m,s] exp(2 pi i f_c dt s), the channels' turns
-// per sample X passed by value for up to kMuxByValue of them (no copy, and the host
-// does not wait for the call), else in Xd.  Grid y: modes.
+// per sample X passed by value for up to kMuxByValue of them (no copy), else in Xd.
+// Grid y: modes.
 constexpr int kMuxByValue = 128;
 struct MuxTurns {
     unsigned long long X[kMuxByValue];
@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(256) pair_sums_kernel(const float2* __restrict
 }
 
 // Multiplies each realization by its factor, passed by value for small batches
-// (no copy to wait for).
+// (no copy).
 constexpr int kScalesByValue = 64;
 struct Scales {
     float2 s[kScalesByValue];
@@ -1045,7 +1045,7 @@ FOCSS_API focss_status focss_wdm_mux(focss_ctx* c, const focss_field* ch, double
     }
     if (e == cudaSuccess) FG_LAUNCH(fg::wdm_mux_kernel<<<fg::grid_per_realization(ch->samples, ch->modes), 256, 0, c->stream>>>(ch->d, n, ch->modes, ch->samples, v, dX, out->d));
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess && dX) e = cudaStreamSynchronize(c->stream);  // X
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     return fg::cuda_check(c, e, "wdm_mux");
 }
 
@@ -1248,7 +1248,9 @@ static focss_status scale_each(focss_ctx* c, focss_field* f, const std::vector<f
         fg::Scales v{};
         std::copy(s.begin(), s.end(), v.s);
         FG_LAUNCH(fg::scale_some_kernel<<<fg::grid_per_realization(per, f->batch), 256, 0, c->stream>>>(f->d, per, v));
-        return fg::cuda_check(c, cudaGetLastError(), "scale_each");
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        return fg::cuda_check(c, e, "scale_each");
     }
     float2* d = (float2*)fg::scratch_buffer(c, 6, sizeof(float2) * f->batch);
     if (!d) return fg::set_error(c, FOCSS_ERR_OOM, "scale scratch");

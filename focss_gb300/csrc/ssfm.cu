@@ -520,6 +520,7 @@ focss_status linear_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_
     if (e == cudaSuccess) e = launch_row(*p, a, batch, ctx->stream);
     a.op = COL_INV;
     if (e == cudaSuccess) e = launch_col(*p, a, batch, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // complete on return, as every run
     return cuda_check(ctx, e, "linear run");
 }
 

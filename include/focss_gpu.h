@@ -14,7 +14,10 @@
  *    like focss::Field (data[sample + mode*samples], src/focss/field.cpp:140-155).
  *    Host buffers passed to upload/download are interleaved (re, im).
  *  - Calls on one context are ordered on the context's CUDA stream.  Calls
- *    that return host values (reductions, step counts) synchronize the stream.
+ *    that return host values (reductions, step counts), split-step runs,
+ *    focss_cd_compensation, focss_wdm_mux, focss_field_rotate and
+ *    focss_field_scale_each are complete when they return; of the others a
+ *    result is there once the stream is synchronized (focss_ctx_sync).
  *  - One context per host thread; a context is not thread-safe.
  *  - The library owns device memory; the caller owns host memory.
  *  - There is no CPU fallback: without a usable GPU, focss_ctx_create fails.
