@@ -25,7 +25,7 @@ namespace {
 
 constexpr int kNoallocMaxLog2Samples = 17;   // N <= 2^17 samples per realization
 constexpr int kNoallocMaxBatch = 256;        // realizations per call
-// Largest table set: N = 2^17 -> N1 = 256, N2 = 512.
+// Largest table set: N = 2^17 -> 256 and 512 entries, whichever way round.
 struct NoallocScratch {
     alignas(16) unsigned char tw[table_bytes(256, 512)];
     SsfmState state[kNoallocMaxBatch];
@@ -108,8 +108,8 @@ extern "C" FOCSS_API focss_status focss_ssfm_run_noalloc(void* stream, void* dat
 
     Plan p;
     p.N = samples;
-    p.log2N1 = lg / 2;
-    p.log2N2 = lg - lg / 2;
+    p.log2N1 = default_split(samples);
+    p.log2N2 = lg - p.log2N1;
     p.N1 = 1 << p.log2N1;
     p.N2 = 1 << p.log2N2;
     p.tw = sc->tw;

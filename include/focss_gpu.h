@@ -273,9 +273,9 @@ FOCSS_API focss_status focss_span_loop(focss_ctx* ctx, int n_fields, focss_field
 #define FOCSS_SPLIT_SINGLE_CTA (-1)
 FOCSS_API focss_status focss_autotune(focss_ctx* ctx, int samples, int batch, int* log2_n1, double* ms_per_step);
 /* Pin the split used for split-step runs of length `samples` (log2_n1 = 0
- * restores the balanced default; FOCSS_SPLIT_SINGLE_CTA selects the
+ * restores the default; FOCSS_SPLIT_SINGLE_CTA selects the
  * single-CTA kernel for single-mode fields of 2^12..2^14 samples, other
- * fields of that length keep the balanced two-pass split). */
+ * fields of that length keep the default two-pass split). */
 FOCSS_API focss_status focss_set_fft_split(focss_ctx* ctx, int samples, int log2_n1);
 
 /* --------------------------------------------------- TX / resampling DSP */
@@ -509,9 +509,10 @@ FOCSS_API focss_status focss_cnn_adam_step(focss_cnn* model, double lr, double b
  * memory: frameworks that own the device heap through their own pool,
  * latency-critical loops where an allocation and the synchronization it
  * implies are not allowed, or processes with a fixed device-memory budget.
- * It always uses the balanced two-pass FFT split; where focss_set_fft_split
- * or focss_autotune chose another split (or the single-CTA kernel) for
- * focss_ssfm_run, the two fields agree to FP32 rounding, not bit for bit.
+ * It always uses the default two-pass FFT split of the length, which is
+ * focss_ssfm_run's too: the same bits, unless focss_set_fft_split or
+ * focss_autotune chose another split (or the single-CTA kernel) for
+ * focss_ssfm_run; then the two fields agree to FP32 rounding.
  * `data` is the caller's device buffer of batch*samples complex64
  * (interleaved float pairs), propagated in place on `stream` (a
  * cudaStream_t; NULL = legacy default stream).  The library allocates
