@@ -34,11 +34,19 @@ focss_status get_plan(Ctx* ctx, int N, const Plan** out) {
     return get_plan_split(ctx, N, lg / 2, out);
 }
 
-// Balanced, with the longer side in the rows; but at 2^13 and 2^17 the columns take it:
-// 256- and 64-sample rows keep 16 and 8 samples per thread where 512 and 128 take 32
-// and 16 (one 2^17 field 15.7 -> 14.3 us per step, 64 fields 87.6 -> 82.5; 25 of 2^13
-// 16.6 -> 15.7).  At 2^15 that costs more in the 256-sample columns (64 fields 28.2 ->
-// 31.8), at 2^19 it is even.
+// Even exponents have one balanced split.  Odd ones have two, and a column of 2^k
+// costs a pass other than a row of 2^k does: columns run in lane pairs at 32, 128 and
+// 512 samples, rows take 8, 16 and 32 samples a thread at 64, 256 and 1024 but 16 and
+// 32 at 128 and 512 (PQ).  Which is better was measured per exponent; us per step of
+// UNIFORM runs, longer rows | longer columns:
+//   2^9   1 field 6.3 | 6.1, 64 fields 6.8 | 6.5, 512 fields 8.8 | 8.6: little in it
+//   2^11  1 field 6.3 | 6.6, 25 fields 6.9 | 6.9, 256 fields 9.9 | 10.3
+//   2^13  1 field 8.3 | 7.3, 25 fields 8.9 | 7.9, 64 fields 9.8 | 10.6
+//   2^15  1 field 8.3 | 9.2, 25 fields 12.0 | 13.8, 64 fields 22.7 | 26.4
+//   2^17  1 field 11.7 | 10.1, 5 fields 14.9 | 14.3, 64 fields 78.0 | 76.6
+//   2^19  1 field 16.1 | 19.0, 3 fields 25.2 | 24.2
+// The longer side is in the columns where single fields and small batches, which
+// latency bounds, gain clearly: 2^13 and 2^17.
 int default_split(int N) {
     int lg = 0;
     while ((1 << lg) < N) ++lg;
