@@ -499,7 +499,7 @@ focss_status ssfm_finish(Ctx* ctx, Field* f, const focss_ssfm_opts& o, const Ssf
 // One dispersive, lossless, linear step over fib.length (a split step without
 // its nonlinear half-way point: two column passes and one row pass instead of
 // three and two, one rounding of the phase, and no step state to wait for --
-// chromatic-dispersion compensation of 12 x 2^16 samples 82 -> 28 us).  The
+// chromatic-dispersion compensation of 12 x 2^16 samples 77 -> 28 us).  The
 // single-CTA, staged and instrumented runs keep the step machinery.
 focss_status linear_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ssfm_opts& o, double dir) {
     focss_status st = ssfm_validate(ctx, f, fib, o);
