@@ -62,6 +62,7 @@ struct TripletArgs {
     int coef_exp;           // the matrices hold the coefficients times 2^-coef_exp
     float2* part;           // splits > 1: partial sums, splits x batch x modes x N
     int splits;
+    int fp32_units, fp32_pitch;  // teams that sum a tile in FP32 in the tensor-core kernel, and their buffers' pitch
 };
 
 // Output o = sample k of a row: zero outside [radius, N - radius), and the equalizer.
@@ -91,13 +92,17 @@ __global__ void triplet_join_kernel(const TripletArgs a, size_t n) {
 // a register window over Q_m along n, so one shared-memory load feeds TT
 // complex multiply-adds.  Shared arrays use a padded index j + j/8 so the
 // per-thread stride is odd and reads are conflict-free.  Sums groups
-// [g0, g1).  Out of line: the tensor-core kernel calls it for single tiles.
-__device__ __forceinline__ void tile_sync() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
+// [g0, g1).  Out of line: the tensor-core kernel calls it for single tiles, where
+// `unit` numbers the teams of NT threads at work on it, each with buffers of its own.
+// `other`: null, or the buffers of the team two further (two back), which sums the
+// rest of the groups; it leaves its sums there for this one to add.
+__device__ __forceinline__ void team_sync(int id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
 template <int MODES>
-__device__ __noinline__ void triplet_tile_fp32(const TripletArgs& a, float2* sh, int k0, int g0, int g1) {
+__device__ __noinline__ void triplet_tile_fp32(const TripletArgs& a, float2* sh, int k0, int g0, int g1, int unit, float2* other) {
     const int N = a.samples;
-    const int b = blockIdx.y;
-    tile_sync();  // the buffers are free (second tile of a CTA)
+    const int b = blockIdx.y, tid = threadIdx.x % NT;
+    const auto tile_sync = [&] { team_sync(1 + unit, NT); };
+    tile_sync();  // the buffers are free (second tile of a team)
     const int alen = TK + 2 * a.halo_a;
     const int qlen = TK + 2 * a.halo_q;
     float2* As = sh;                           // MODES x padi(alen)
@@ -107,7 +112,7 @@ __device__ __noinline__ void triplet_tile_fp32(const TripletArgs& a, float2* sh,
 
     // A tile: index i <-> sample k0 - halo_a + i (zero outside [0, N))
     for (int p = 0; p < MODES; ++p)
-        for (int i = threadIdx.x; i < alen; i += NT) {
+        for (int i = tid; i < alen; i += NT) {
             const int s = k0 - a.halo_a + i;
             As[p * astride + padi(i)] = (s >= 0 && s < N) ? in[(size_t)p * N + s] : make_float2(0.f, 0.f);
         }
@@ -118,14 +123,14 @@ __device__ __noinline__ void triplet_tile_fp32(const TripletArgs& a, float2* sh,
 #pragma unroll
         for (int r = 0; r < TT; ++r) acc[p][r] = make_float2(0.f, 0.f);
 
-    const int kl = threadIdx.x * TT;  // first local output of this thread
+    const int kl = tid * TT;  // first local output of this thread
     for (int g = g0; g < g1; ++g) {
         const int m = a.g_m[g];
         const int nlo = a.g_nlo[g];
         const int off = a.g_off[g], len = a.g_off[g + 1] - off;
         tile_sync();  // previous Q consumed (and A tile ready on the first)
         // Q tile: index i <-> j = k0 - halo_q + i
-        for (int i = threadIdx.x; i < qlen; i += NT) {
+        for (int i = tid; i < qlen; i += NT) {
             const int ia = i + (a.halo_a - a.halo_q);  // A index of j
             float2 q = make_float2(0.f, 0.f);
 #pragma unroll
@@ -166,16 +171,28 @@ __device__ __noinline__ void triplet_tile_fp32(const TripletArgs& a, float2* sh,
                 acc[p][r] = cadd(acc[p][r], cmul(As[p * astride + padi(kl + r + m + a.halo_a)], s[r]));
     }
 
+    if (unit >= 2) {
+        tile_sync();  // nobody reads the A tile any more
+#pragma unroll
+        for (int p = 0; p < MODES; ++p)
+#pragma unroll
+            for (int r = 0; r < TT; ++r) sh[(p * TT + r) * NT + tid] = acc[p][r];
+    }
+    if (other) team_sync(5 + (unit & 1), 2 * NT);
+    if (unit >= 2) return;
 #pragma unroll
     for (int p = 0; p < MODES; ++p)
 #pragma unroll
-        for (int r = 0; r < TT; ++r) write_output(a, b, MODES, p, k0 + kl + r, acc[p][r]);
+        for (int r = 0; r < TT; ++r) {
+            if (other) acc[p][r] = cadd(acc[p][r], other[(p * TT + r) * NT + tid]);
+            write_output(a, b, MODES, p, k0 + kl + r, acc[p][r]);
+        }
 }
 
 template <int MODES>
 __global__ void __launch_bounds__(NT) triplet_kernel(const TripletArgs a) {
     extern __shared__ float2 sh[];
-    triplet_tile_fp32<MODES>(a, sh, blockIdx.x * TK, 0, a.groups);
+    triplet_tile_fp32<MODES>(a, sh, blockIdx.x * TK, 0, a.groups, 0, nullptr);
 }
 
 // ---------------------------------------------------------------- tensor cores
@@ -297,9 +314,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) triplet_tc_kernel(const Triplet
     __syncthreads();
     const float pmax = __uint_as_float(s_max), pmin = __uint_as_float(s_min);
     if (s_bad || (pmax > 0.f && (!(pmax > 1e-30f) || pmax > 128.f * pmin))) {  // 2^12 over the run's mean
-        if (threadIdx.x < NT)
-            for (int k = k0; k < k0 + TC_K && k < N; k += TK)
-                triplet_tile_fp32<MODES>(a, reinterpret_cast<float2*>(sm), k, g0, g1);
+        // teams of NT threads: one for each TK outputs, or two with half of the groups each
+        // (R = 75 on 2^20 symbols, every tile out of range: 2.6 ms; 4.2 with one team, which
+        // takes both TK in turn, 2.9 in launches of the FP32 kernel alone)
+        const int unit = threadIdx.x / NT, units = a.fp32_units, gm = units == 4 ? (g0 + g1) / 2 : g1;
+        float2* sh = reinterpret_cast<float2*>(sm) + (size_t)unit * a.fp32_pitch;
+        if (unit < units)
+            for (int k = k0 + (units == 1 ? 0 : unit & 1) * TK; k < k0 + TC_K && k < N; k += TK * min(units, 2))
+                triplet_tile_fp32<MODES>(a, sh, k, unit >= 2 ? gm : g0, unit >= 2 ? g1 : gm, unit,
+                                         units < 4 ? nullptr : unit >= 2 ? sh : sh + 2 * (size_t)a.fp32_pitch);
         return;
     }
     // |Q| <= pmax < 2^e: scale to below 2^kHeadroom
@@ -760,7 +783,11 @@ focss_status run_triplet_rows(Ctx* c, const float2* in, size_t in_bstride, int m
         const size_t need = 1024 + (size_t)kSt * (8 * (size_t)a.qcap + a.bslot) + sizeof(int4) * ng +
                             sizeof(float2) * (size_t)modes * (a.alen + a.alen / 16 + 2);
         tensor = need <= 220 * 1024;
-        if (tensor) smem = std::max(smem, need);  // a tile may take the FP32 sum
+        if (tensor) {  // a tile may take the FP32 sum, by as many teams as find room
+            a.fp32_pitch = (int)(smem / sizeof(float2));
+            a.fp32_units = 4 * smem <= 220 * 1024 ? 4 : 2 * smem <= 220 * 1024 ? 2 : 1;
+            smem = std::max(a.fp32_units * smem, need);
+        }
     }
     const int tile = tensor ? TC_K : TK;
     dim3 grid((samples + tile - 1) / tile, batch);
