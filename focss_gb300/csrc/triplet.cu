@@ -558,14 +558,20 @@ __global__ void toeplitz_kernel(const float2* __restrict__ coef, const int* __re
 // 2^28 (zeros aside): the smallest would keep fewer than 22 bits, and where the
 // large ones have no part in a symbol they alone make it up.
 void plan_tensor(Terms& t) {
-    float cmax = 0.f, cmin = INFINITY;
-    for (const float2& c : t.coef) {
-        if (!std::isfinite(c.x) || !std::isfinite(c.y)) return;
-        const float mag = std::max(std::fabs(c.x), std::fabs(c.y));
-        cmax = std::max(cmax, mag);
-        if (mag > 0.f) cmin = std::min(cmin, mag);
+    // magnitudes as bits, which order like non-negative floats (this loop is vectorized)
+    uint32_t top = 0u, low = 0xFFFFFFFFu;  // low: of the smallest non-zero one, less 1
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(t.coef.data());
+    for (size_t i = 0; i < 2 * t.coef.size(); i += 2) {
+        const uint32_t mag = std::max(w[i] & 0x7FFFFFFFu, w[i + 1] & 0x7FFFFFFFu);
+        top = std::max(top, mag);
+        low = std::min(low, mag - 1u);
     }
-    if (!(cmax > 0x1p-100f && cmax < 0x1p100f) || cmin < 0x1p-28f * cmax || (int)t.gm.size() > kMaxTcGroups) return;
+    if (top >= 0x7F800000u || top == 0u || (int)t.gm.size() > kMaxTcGroups) return;  // not finite, or all zero
+    low += 1u;
+    float cmax, cmin;
+    std::memcpy(&cmax, &top, sizeof cmax);
+    std::memcpy(&cmin, &low, sizeof cmin);
+    if (!(cmax > 0x1p-100f && cmax < 0x1p100f) || cmin < 0x1p-28f * cmax) return;
     for (int l : t.len)
         if (l + 15 > 16 * kMaxKSteps) return;
     std::frexp(cmax, &t.exp);
