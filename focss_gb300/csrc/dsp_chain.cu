@@ -589,44 +589,44 @@ constexpr int kPairBlocks = 64;  // CTAs per realization, at most
 // PhaseShiftEqualizer::estimate argmax over i = 0..steps-1 of
 // Re(e^{i 2 pi i / steps} (cr + i ci)) (q2 is monotone in it), the first maximum
 // wins.  Around the peak at -arg(cr + i ci) neighbours fall off by at least
-// ~(2 pi / steps)^2 / 2 of it, far above rounding up to 65536 steps, so the
-// five steps around it decide (an FP32 argument is off by less than 0.01 step);
-// otherwise, or without a usable argument, all steps are tried.  Called by one
-// warp: the FP64 pipe serves ~2 lanes per cycle, so idle warps' copies of the
-// same arithmetic would cost as much again each.
-__device__ int phase_argmax(double cr, double ci, int steps) {
-    const double two_pi = 2 * 3.14159265358979323846264338;
+// ~(2 pi / steps)^2 / 2 of it, far above rounding up to 2^24 steps, so the
+// five steps around it decide (up to 65536 steps an FP32 argument is off by less
+// than 0.01 step), and one warp tries them: the FP64 pipe serves ~2 lanes per cycle, so
+// idle warps' copies of the same arithmetic would cost as much again each.  Otherwise,
+// or without a usable argument, the CTA tries all steps (12 realizations, 100000
+// steps: 2.1 ms; by one warp 4.1).
+__device__ bool phase_peak_known(double cr, double ci, int steps) {
     const double mag = fmax(fabs(cr), fabs(ci));
-    const int lane = threadIdx.x & 31;
-    int first = 0, count = steps;
-    if (steps >= 8 && steps <= 65536 && mag > 1e-290 && mag < 1e290 && !isnan(cr) && !isnan(ci)) {
-        first = __float2int_rn(-atan2f((float)(ci / mag), (float)(cr / mag)) * 0.15915494f * (float)steps) - 2;
-        count = 5;
+    return steps >= 8 && steps <= 1 << 24 && mag > 1e-290 && mag < 1e290 && !isnan(cr) && !isnan(ci);
+}
+struct PhaseBest {
+    double v = -1e308;
+    int i = 0;
+    __device__ void take(double w, int k) {
+        if (w > v || (w == v && k < i)) {
+            v = w;
+            i = k;
+        }
     }
-    double best = -1e308;
-    int bi = 0;
-    for (int k = lane; k < count; k += 32) {
+};
+// Of steps first + k, k = k0, k0 + stride, ... below count, the warp's best (in every lane).
+__device__ PhaseBest phase_argmax(double cr, double ci, int steps, int first, int count, int k0, int stride) {
+    const double two_pi = 2 * 3.14159265358979323846264338;
+    PhaseBest best;
+    for (int k = k0; k < count; k += stride) {
         int i = first + k;
         if (i < 0) i += steps;
         if (i >= steps) i -= steps;
         const double ang = two_pi * (double)i / steps;
         double sn, cs;
         sincos(ang, &sn, &cs);
-        const double v = cr * cs - ci * sn;
-        if (v > best || (v == best && i < bi)) {
-            best = v;
-            bi = i;
-        }
+        best.take(cr * cs - ci * sn, i);
     }
     for (int o = 16; o > 0; o >>= 1) {
-        const double v = __shfl_xor_sync(0xffffffffu, best, o);
-        const int i = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (v > best || (v == best && i < bi)) {
-            best = v;
-            bi = i;
-        }
+        const double v = __shfl_xor_sync(0xffffffffu, best.v, o);
+        best.take(v, __shfl_xor_sync(0xffffffffu, best.i, o));
     }
-    return bi;
+    return best;
 }
 
 template <int WHAT>
@@ -695,9 +695,28 @@ __global__ void __launch_bounds__(256) pair_sums_kernel(const float2* __restrict
     }
     __syncthreads();
     if (WHAT == PAIR_PHASE) {
-        if (warp) return;
-        const int i = phase_argmax(s_sum[0], s_sum[1], steps);
-        if (lane == 0) out[b] = 2 * 3.14159265358979323846264338 * (double)i / steps;
+        const double cr = s_sum[0], ci = s_sum[1];
+        __shared__ double s_v[8];
+        __shared__ int s_i[8];
+        PhaseBest best;
+        if (phase_peak_known(cr, ci, steps)) {
+            if (warp) return;
+            const double mag = fmax(fabs(cr), fabs(ci));
+            const int peak = steps <= 65536
+                                 ? __float2int_rn(-atan2f((float)(ci / mag), (float)(cr / mag)) * 0.15915494f * (float)steps)
+                                 : __double2int_rn(-atan2(ci, cr) * (0.5 / 3.14159265358979323846264338) * steps);
+            best = phase_argmax(cr, ci, steps, peak - 2, 5, lane, 32);
+        } else {
+            best = phase_argmax(cr, ci, steps, 0, steps, threadIdx.x, blockDim.x);
+            if (lane == 0) {
+                s_v[warp] = best.v;
+                s_i[warp] = best.i;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (int w = 1; w < 8; ++w) best.take(s_v[w], s_i[w]);
+        }
+        if (threadIdx.x == 0) out[b] = 2 * 3.14159265358979323846264338 * (double)best.i / steps;
     } else if (threadIdx.x < K) {
         out[(size_t)b * K + threadIdx.x] = s_sum[threadIdx.x];
     }
