@@ -80,11 +80,11 @@ __device__ __forceinline__ float2 phase_grad(float2 g, float2 y, float p, float2
     return make_float2(fmaf(-k, b.y, fmaf(kp, ge.y, ge.x)), fmaf(k, b.x, fmaf(-kp, ge.x, ge.y)));
 }
 
-// Whether powers of largest value `mx` leave the split's range, `mn` the smallest
-// non-zero sum over a run of `run` samples (both as bits).
+// Whether powers of largest value `mx` leave the split's range (infinity and all
+// above 1e30 do), `mn` the smallest non-zero sum over a run of `run` samples (both as bits).
 __device__ __forceinline__ bool outside_split(unsigned mx, unsigned mn, int run) {
     const float pmax = __uint_as_float(mx);
-    return pmax > 0.f && (!(pmax > 1e-36f) || pmax > (float)(4096 / run) * __uint_as_float(mn));
+    return pmax > 0.f && (!(pmax > 1e-36f && pmax <= 1e30f) || pmax > (float)(4096 / run) * __uint_as_float(mn));
 }
 
 // The CTA's owned samples of a layer's output `v(i)`, i = 0 .. owned-1, to dst.
@@ -299,15 +299,15 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
     const uint32_t tmem = tmem_base;
     bool ok = true;
     bool plain = s_bad || outside_split(s_in, s_min_in, 32);  // the layers run in FP32
-    // Largest power and a run of 8 (its sum; whether all of it is valid input) of layer l's filter input.
+    // Largest power and a run of 8 (its sum; whether all of it is valid input) of layer l's filter
+    // input; a run beyond 1e30 or not a number counts as infinite.
     auto note_range = [&](int l, float mx, float sum, bool valid) {
+        if (valid && !(sum <= 1e30f)) mx = __int_as_float(0x7F800000);
         const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
         const unsigned n = __reduce_min_sync(0xffffffffu, valid && sum > 0.f ? __float_as_uint(sum) : 0x7F7FFFFFu);
-        const bool bad = __any_sync(0xffffffffu, valid && !(sum <= 1e30f));
         if (lane == 0) {
             atomicMax(&s_max[l], m);
             atomicMin(&s_min[l], n);
-            if (bad) s_bad = 1;
         }
     };
     const int o0 = ROW * (32 * (warp & 3) + lane) + OUT * (warp >> 2);  // first output of the thread
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
         acc = warp_sum(acc);
         if (lane == 0) atomicAdd(&s_gxi[0], acc);
         __syncthreads();
-        plain = s_bad || outside_split(s_max[0], s_min[0], 8);
+        plain = outside_split(s_max[0], s_min[0], 8);
     }
     if (BWD && a.xi && !plain) {
 #pragma unroll
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(firtc::THREADS, 2) ldbp_chain_kernel(const Cha
             }
         __syncthreads();
         next = l + 1;
-        plain = s_bad || outside_split(s_max[next], s_min[next], 8);
+        plain = outside_split(s_max[next], s_min[next], 8);
         if (!plain) split_store8(xs, pitch, o0, y, pow2(-split_exponent(s_max[next])));
     }
     if (plain) {

@@ -97,3 +97,21 @@ def gain_terms(h, xi, hmf, x, tx, layers):
         out[k] = np.sum(2 * np.abs(g) * p * np.abs(y))
         g = R.fir_adjoint(g * np.conj(e) * (1 - 1j * xi[k] * p) + np.conj(g) * 1j * xi[k] * y ** 2 * e, h[k])
     return out
+
+
+@pytest.mark.parametrize("at", [900, 2044])
+def test_one_overflowing_sample_in_silence(ctx, at):
+    """Nothing else in the field: no run of samples to hold the overflow against."""
+    rng = np.random.default_rng(at)
+    layers, T, N = 3, 31, 4300
+    x = np.zeros((1, N), np.complex64)
+    x[0, at] = 38.0
+    h = np.zeros((layers, T), np.complex64)
+    h[:, T // 2] = [1e18, 1e-18, 1.0]
+    hmf = taps(rng, 1, T, [1.0])[0]
+    m = LearnedDBP(1, layers, T, T, N, 1, 1.0, ctx=ctx)
+    m.set_params(h, np.zeros(layers), hmf)
+    y = m.forward(fg.Field(fg.Domain(1, N, 1.0), data=x[:, None], ctx=ctx)).numpy()[0, 0]
+    reach = np.abs(2 * np.arange(N // 2) - at) <= T // 2 * 3   # of two filters and the matched one
+    assert not np.any(np.isfinite(y[reach]))
+    assert not np.any(y[~reach])
