@@ -427,7 +427,7 @@ def set_row_staging(mode: int, ctx: Context | None = None):
 
 
 def set_fft_split(samples: int, log2_n1: int, ctx: Context | None = None):
-    """Pin the split of length-`samples` split-step runs (0 = balanced
+    """Pin the split of length-`samples` split-step runs (0 = the
     default, SPLIT_SINGLE_CTA = the single-CTA kernel for 2^12..2^14)."""
     ctx = ctx or Context.default()
     check(lib().focss_set_fft_split(ctx.h, samples, log2_n1), ctx.h)

@@ -121,10 +121,10 @@ __device__ __forceinline__ uint32_t positive2(uint32_t m) {
 // Warp 0 (one thread) loads each tile's activations with TMA tensor copies
 // (cp.async.bulk.tensor: one 128-byte-swizzled box of 64 channels x 136 rows,
 // or one box of 8 channels per 8-channel group, zero-filled outside [0, L))
-// into a ring of STAGES buffers (mbarriers full / empty); warp 1 (one thread)
-// waits for the weights, then issues each tile's 9 CIN/16 MMAs into one of
-// two tensor-memory accumulators and commits them to the stage's `empty`
-// barrier and the accumulator's `full` barrier; warps 2-9 stage the weights
+// into a ring of STAGES buffers (mbarriers full / empty); warps 1 and 10 (one
+// thread each) wait for the weights, then issue the 9 CIN/16 MMAs of every other
+// tile, each into a tensor-memory accumulator of its own, and commit them to the
+// stage's `empty` barrier and the accumulator's `full` barrier; warps 2-9 stage the weights
 // once (barrier `wready`) and then run the epilogue in two groups of four
 // (group g takes accumulator g, i.e. every other tile; a warp's lane quarter
 // of tensor memory is warp & 3), so the epilogues of two tiles overlap the
@@ -381,7 +381,8 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
 //
 // 12 x 2^15 positions with the bias gradient, 64 -> 64 channels 102 -> 36 us, 64 -> 16
 // 61 -> 26 us, 16 -> 64 72 -> 26 us against three taps per CTA of M = 64 from unswizzled
-// 16-byte boxes and a pass over g for the bias.
+// 16-byte boxes and a pass over g for the bias (without sections; with them a training
+// step takes 442 us instead of 438).
 namespace tcw {
 constexpr int P = 128;                // positions per tile
 constexpr int PR = P + 2 * HALF;      // input rows per tile (halo)

@@ -13,8 +13,10 @@
 
 namespace fg {
 
-// Per-realization SSFM state machine, device resident.  The last CTA of each
-// column pass advances it (no CTA ever waits on another).
+// Per-realization SSFM state machine, device resident, advanced once a pass pair
+// without any CTA waiting on another: by a CTA beside the column pass's others where
+// the grid is known up front (PassArgs::next), by the row pass's CTAs in small launches
+// of other grids (PassArgs::late), else by the last CTA of the column pass.
 struct SsfmState {
     double distance;               // |z| travelled (ADAPTIVE)
     double h;                      // signed size of the next nonlinear step
@@ -169,7 +171,7 @@ struct Ctx {
     double prof_ms[2] = {0, 0};          // column, row
     long long prof_launches[2] = {0, 0};
     // split-step FFT split (log2 N1) per length picked by the autotuner or
-    // pinned by the caller; lengths absent here use the balanced split
+    // pinned by the caller; lengths absent here use default_split
     std::map<int, int> ssfm_split;
     TermCache* terms = nullptr;      // device tables of recent triplet term lists
     int staging = 0;                 // FOCSS_STAGING_* for new plans (focss_set_pass_staging)
@@ -248,14 +250,14 @@ struct StepGrid {
 };
 focss_status ssfm_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ssfm_opts& o, double dir,
                       int* steps_out, const StepGrid* grid = nullptr, int* recorded_out = nullptr);
-// Argument checks of ssfm_run and the pass arguments of one run (state and
-// finished-realization counter supplied by the caller).
 // Dispersion only (alpha = gamma = 0) over fib.length, o a single UNIFORM step.
 focss_status linear_run(Ctx* ctx, Field* f, const focss_fiber& fib, const focss_ssfm_opts& o, double dir);
+// Argument checks of ssfm_run and the pass arguments of one run (state and
+// finished-realization counter supplied by the caller).
 focss_status ssfm_validate(Ctx* ctx, const Field* f, const focss_fiber& fib, const focss_ssfm_opts& o);
 PassArgs ssfm_args(const Field* f, const focss_fiber& fib, const focss_ssfm_opts& o, double dir, SsfmState* state,
                    int* n_done);
-// The plan ssfm_run uses for length N (autotuned or pinned split, else balanced).
+// The plan ssfm_run uses for length N (autotuned or pinned split, else default_split).
 focss_status ssfm_plan(Ctx* ctx, int N, const Plan** out);
 // Split value selecting the single-CTA kernel (ssfm_block.cu) for a length.
 constexpr int kSingleCta = -1;

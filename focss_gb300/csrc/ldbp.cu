@@ -51,7 +51,7 @@ __device__ __forceinline__ int wrap_index(int s, int N) {
 // What bounds it: per tile and layer ~1040 cycles of shared-memory bandwidth
 // for the products and ~1200 issue cycles for the epilogue (nonlinear phase,
 // splits), with two CTAs per SM (tensor memory) to overlap them.  20 x 4 steps of 63 taps on
-// 16 x 65536 samples: 1368 -> 582 us against one FP32 launch per layer.
+// 16 x 65536 samples: 1368 -> 514 us against one FP32 launch per layer.
 constexpr int kMaxChain = 8;
 struct ChainArgs {
     const float2* x;            // batch x N: samples, or (backward) the gradient

@@ -3,8 +3,9 @@
 //
 // A span loop (forward_propagation / backward_propagation,
 // src/tasks/systems.cpp:26-91) is a long, fixed chain of small launches:
-// per span an optional amplifier, one SSFM run (K+2 column/row pass pairs for
-// a UNIFORM grid, a data-dependent number for ADAPTIVE / LOGARITHMIC) and
+// per span an optional amplifier, one SSFM run (for a UNIFORM grid K+2 column
+// passes with a row pass between any two, for ADAPTIVE / LOGARITHMIC a
+// data-dependent number of pass pairs) and
 // another optional amplifier.  Here the whole chain, for every field of the
 // call, is captured once into one graph:
 //   * fields of different lengths and batches are branches (they run
