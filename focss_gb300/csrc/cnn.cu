@@ -379,10 +379,9 @@ __global__ void __launch_bounds__(tc::FWD_THREADS, 1)
 // wait is bounded (kWaitCap polls); a CTA that gives up drains its copies and MMAs
 // (bounded) and adds NaN, so the failure shows in gW.
 //
-// 12 x 2^15 positions with the bias gradient, 64 -> 64 channels 102 -> 36 us, 64 -> 16
-// 61 -> 26 us, 16 -> 64 72 -> 26 us against three taps per CTA of M = 64 from unswizzled
-// 16-byte boxes and a pass over g for the bias (without sections; with them a training
-// step takes 442 us instead of 438).
+// 12 x 2^15 positions with the bias gradient, 64 -> 64 channels 102 -> 39 us, 64 -> 16
+// 61 -> 27 us, 16 -> 64 72 -> 29 us against three taps per CTA of M = 64 from unswizzled
+// 16-byte boxes and a pass over g for the bias (36, 26 and 26 us without sections).
 namespace tcw {
 constexpr int P = 128;                // positions per tile
 constexpr int PR = P + 2 * HALF;      // input rows per tile (halo)
